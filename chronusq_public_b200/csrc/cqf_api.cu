@@ -802,7 +802,8 @@ void free_basis(cqf_basis* B) {
                     (void*)B->d_sph, (void*)B->d_sphOff, (void*)B->d_ao2shell,
                     (void*)B->d_cart2shell, (void*)B->d_ws, (void*)B->d_counters,
                     (void*)B->d_flags, (void*)B->d_qLL, (void*)B->d_qSS, (void*)B->d_qG, (void*)B->d_qB,
-                    (void*)B->d_relws})
+                    (void*)B->d_relws, (void*)B->d_hg[0], (void*)B->d_hg[1], (void*)B->d_hg[2],
+                    (void*)B->d_hg[3]})
       if (p) cudaFreeAsync(p, st);
     cudaStreamSynchronize(st);
   }
@@ -1178,6 +1179,11 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
     pair_range_kernel<<<grid1(B->npair, 128), 128, 0, B->stream>>>(B->d_pp, B->d_pairs,
                                                                    B->npair, B->d_pairRange);
     CQF_CUDA(cudaGetLastError());
+  }
+  for (int c = 0; c < NCLS; c++) {
+    B->cls_pp_beg[c] = B->cls_cnt[c] ? B->h_pairs[B->cls_beg[c]].pp_off : 0;
+    for (int i = 0; i < B->cls_cnt[c]; i++)
+      B->cls_npp_max[c] = std::max(B->cls_npp_max[c], B->h_pairs[B->cls_beg[c] + i].npp);
   }
   B->h_schwarz.resize((size_t)nshell * nshell);
   CQF_CUDA(cudaMemcpyAsync(B->h_schwarz.data(), B->d_schwarz,

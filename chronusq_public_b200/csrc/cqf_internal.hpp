@@ -71,6 +71,10 @@ struct JKLaunch {
   unsigned long long* counters;  // [0] visited, [1] screened, [2] fp32, [3] fp64
 };
 
+// Coefficient tables of the Hermite-matrix engine (cqf_hgemm.cuh), by the
+// operators on the pair.
+enum HgKind { HG_PLAIN = 0, HG_D6 = 1, HG_D3 = 2, HG_SPIN = 3, HG_NKIND = 4 };
+
 // Whether bra pair p (position in the pair list) belongs to this call's
 // shard of the work (cqf_opts::shard_index / shard_count).
 __host__ __device__ inline bool in_shard(int p, int idx, int cnt) {
@@ -180,6 +184,9 @@ void launch_to_cart(const cqf_basis* B, const double* X, int cplx, double* Xc, c
 // 1/2 (B + B^H) with her = 1, 1/2 B with her = 0 (B = T^T Ac T).
 void launch_from_cart(const cqf_basis* B, const double* Ac, int cplx, int her, double* AX,
                       cudaStream_t st);
+// Builds the engine's coefficient table of one kind for every primitive pair
+// of the basis (once; cqf_hgemm.cu).  Caller holds B->mu, device current.
+cqf_status hg_ensure(cqf_basis* B, int kind);
 // Grows the basis' contraction workspace (B->d_ws) to at least `bytes`.
 cqf_status basis_workspace(cqf_basis* B, size_t bytes);
 
@@ -243,6 +250,11 @@ struct cqf_basis {
   double* d_qG = nullptr;  // Gaunt: qG[d + o * nshell], derivative on shell d
   double* d_qB = nullptr;  // gauge, the same layout
   bool rel_qLL = false, rel_qSS = false, rel_qG = false, rel_qB = false;
+  // coefficient tables of the Hermite-matrix engine (built on first use) and
+  // where each class's begin (doubles; the class's first primitive pair)
+  double* d_hg[cqf::HG_NKIND] = {};
+  size_t hg_beg[cqf::HG_NKIND][cqf::NCLS] = {};
+  int cls_pp_beg[cqf::NCLS] = {0}, cls_npp_max[cqf::NCLS] = {0};
   void* d_relws = nullptr;
   size_t relws_bytes = 0;
   std::mutex mu;

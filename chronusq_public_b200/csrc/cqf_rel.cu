@@ -35,6 +35,7 @@
 
 #include "cqf_deriv.cuh"
 #include "cqf_eri.cuh"
+#include "cqf_hgemm.cuh"
 #include "cqf_internal.hpp"
 
 namespace cqf {
@@ -95,25 +96,6 @@ __device__ __forceinline__ Q4 qmul(const Q4& p, const Q4& q) {
   return r;
 }
 
-// p (m0 + i w . sigma) for real m0 and w: m0 p.s + i p.v.w, and
-// i p.s w + m0 p.v - p.v x w (the general product with the zero parts of the
-// right factor left out)
-__device__ __forceinline__ Q4 qmul_ri(const Q4& p, double m0, double w1, double w2,
-                                      double w3) {
-  const double2 pw = make_double2(p.x.x * w1 + p.y.x * w2 + p.z.x * w3,
-                                  p.x.y * w1 + p.y.y * w2 + p.z.y * w3);
-  Q4 r;
-  r.s = make_double2(m0 * p.s.x - pw.y, m0 * p.s.y + pw.x);
-  // i p.s w_k = (-p.s.y w_k, p.s.x w_k)
-  r.x = make_double2(-p.s.y * w1 + m0 * p.x.x - (p.y.x * w3 - p.z.x * w2),
-                     p.s.x * w1 + m0 * p.x.y - (p.y.y * w3 - p.z.y * w2));
-  r.y = make_double2(-p.s.y * w2 + m0 * p.y.x - (p.z.x * w1 - p.x.x * w3),
-                     p.s.x * w2 + m0 * p.y.y - (p.z.y * w1 - p.x.y * w3));
-  r.z = make_double2(-p.s.y * w3 + m0 * p.z.x - (p.x.x * w2 - p.y.x * w1),
-                     p.s.x * w3 + m0 * p.z.y - (p.x.y * w2 - p.y.y * w1));
-  return r;
-}
-
 // t sigma_k (k = 1, 2, 3): sigma_j sigma_k = delta_jk + i eps_jkl sigma_l, so
 // t sigma_x = (t.x, t.s, i t.z, -i t.y), t sigma_y = (t.y, -i t.z, t.s, i t.x),
 // t sigma_z = (t.z, i t.y, -i t.x, t.s)
@@ -134,15 +116,10 @@ __device__ __forceinline__ void addz(double* A, size_t e, double2 v, double w) {
 
 struct RelLaunch {
   const PairDev* pairs;
-  const PrimPairDev* pp;
-  const ShellDev* shells;
-  const double* prim;
-  const double* boys;
-  const float* boys32;
   const float2* pairRange;  // per pair: FP32 range data (fp32_range_ok)
-  int mixed;      // 1: quartets with bound < cut run in FP32 (second launch)
+  int mixed;                // 1: quartets with bound < cut take FP32 Hermite integrals
   double cut;
-  int braBeg, nBra, ketBeg, nKet, same;
+  int braBeg, nBra, braOff, ketBeg, nKet, same, lsum;
   int screen;
   double thresh;
   const double* norms;  // max shell-block norms of the screening matrices
@@ -156,1728 +133,308 @@ struct RelLaunch {
   double* Jss[4];        // real
   double* K[4];          // complex
   int shardIdx, shardCnt;  // bra pairs p with p % shardCnt == shardIdx only
-  int skipSingle;          // single-primitive quartets: rel_gemm / rel_llss_single_kernel's
-  int contracted;          // some bra or ket pair has more than one primitive pair
-  int nsm;                 // multiprocessors of the device
   unsigned long long* counters;
 };
 
 constexpr int REL_THREADS = 64;
 
-// Digestion of the operator components m of one bra component pair (a, b)
-// against ket component pair (c, d) = (gC, gD) (Cartesian AO indices): the
-// update formulas of the reference with the Pauli algebra of P.  jcol gets
-// the caller's per-column Coulomb sum (J_LL(C,D) for LLSS, J_SS(C,D) for SSSS).
-struct RelCol {
-  int gC, gD;
-  bool dAB, dCD, samePQ;
-  double s34d, w12, wx;
-  double rhoLL;    // LLSS: Re X_CLL(D, C)
-  double rvDC[4];  // SSSS: (Re S, -Im X, -Im Y, -Im Z) of X_CSS(D, C)
-};
-
-template <int TYPE>
-__device__ __forceinline__ void rel_digest(const RelLaunch& a, const PairDev& P, const RelCol& col,
-                                           int ai, int bi, const double* m, double* jcol) {
-  const size_t nc = a.ncart;
-  auto ix = [nc](int r, int c) -> size_t { return (size_t)r + (size_t)c * nc; };
-  const int gC = col.gC, gD = col.gD;
-  const bool dAB = col.dAB, dCD = col.dCD, samePQ = col.samePQ;
-  const double s34d = col.s34d, w12 = col.w12, wx = col.wx, rhoLL = col.rhoLL;
-  const double* rvDC = col.rvDC;
-  const int gA = P.cA + ai, gB = P.cB + bi;
-  if (TYPE == 1) {
-    // Coulomb SS(1,2) from the LL density (:1145-1190)
-    const double wj = w12 * s34d * rhoLL;
-    if (wj != 0.0)
-#pragma unroll
-      for (int op = 0; op < 4; op++) atomicAdd(a.Jss[op] + ix(gA, gB), wj * m[op]);
-    // Coulomb LL(3,4) from the SS density
-    const size_t eBA = ix(gB, gA);
-    jcol[0] += m[0] * __ldg(a.Xss[0] + 2 * eBA) - m[1] * __ldg(a.Xss[1] + 2 * eBA + 1) -
-               m[2] * __ldg(a.Xss[2] + 2 * eBA + 1) - m[3] * __ldg(a.Xss[3] + 2 * eBA + 1);
-    if (!a.exchange) return;
-    // exchange LS: K(t1, t2) -= D(d1, d2) P (:1200-1299)
-    auto ls = [&](int t1, int t2, int d1, int d2, double flip) {
-      const size_t e = ix(d1, d2);
-      Q4 dq{ldz(a.Xk[0], e), ldz(a.Xk[1], e), ldz(a.Xk[2], e), ldz(a.Xk[3], e)};
-      // dq (m0 + i flip m.sigma)
-      const Q4 r = qmul_ri(dq, m[0], flip * m[1], flip * m[2], flip * m[3]);
-      const size_t t = ix(t1, t2);
-      addz(a.K[0], t, r.s, -1.0);
-      addz(a.K[1], t, r.x, -1.0);
-      addz(a.K[2], t, r.y, -1.0);
-      addz(a.K[3], t, r.z, -1.0);
-    };
-    ls(gC, gB, gD, gA, 1.0);
-    if (!dAB) ls(gC, gA, gD, gB, -1.0);
-    if (!dCD) {
-      ls(gD, gB, gC, gA, 1.0);
-      if (!dAB) ls(gD, gA, gC, gB, -1.0);
-    }
-  } else {
-    // m[a * 4 + b]; Coulomb SS(1,2) from D(4,3), and SS(3,4) from
-    // D(2,1) when the bra and ket pairs differ (:2342-2380)
-#pragma unroll
-    for (int op = 0; op < 4; op++) {
-      const double v = m[op * 4 + 0] * rvDC[0] + m[op * 4 + 1] * rvDC[1] +
-                       m[op * 4 + 2] * rvDC[2] + m[op * 4 + 3] * rvDC[3];
-      if (v != 0.0) atomicAdd(a.Jss[op] + ix(gA, gB), w12 * s34d * v);
-    }
-    if (!samePQ) {
-      const size_t eBA = ix(gB, gA);
-      const double rvBA[4] = {__ldg(a.Xss[0] + 2 * eBA), -__ldg(a.Xss[1] + 2 * eBA + 1),
-                              -__ldg(a.Xss[2] + 2 * eBA + 1),
-                              -__ldg(a.Xss[3] + 2 * eBA + 1)};
-#pragma unroll
-      for (int b = 0; b < 4; b++)
-        jcol[b] += m[0 * 4 + b] * rvBA[0] + m[1 * 4 + b] * rvBA[1] +
-                   m[2 * 4 + b] * rvBA[2] + m[3 * 4 + b] * rvBA[3];
-    }
-    if (!a.exchange) return;
-    // exchange SS: K(t1, t2) -= P_12 D(d1, d2) P_34 with the bra / ket
-    // orientation signs f1, f2 (:2381-2445); the Hermitian-conjugate
-    // images come from the completion in the back transform
-    auto ex = [&](int t1, int t2, int d1, int d2, double f1, double f2) {
-      const size_t e = ix(d1, d2);
-      const Q4 dq{ldz(a.Xk[0], e), ldz(a.Xk[1], e), ldz(a.Xk[2], e), ldz(a.Xk[3], e)};
-      Q4 r{make_double2(0, 0), make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-#pragma unroll 1
-      for (int b = 0; b < 4; b++) {
-        // left operator sum_a c_ab sigma_a, c_ab = m_ab (i f1)^[a>0] (i f2)^[b>0]
-        double2 cs = make_double2(m[0 * 4 + b], 0.0);
-        double2 cx = make_double2(0.0, f1 * m[1 * 4 + b]);
-        double2 cy = make_double2(0.0, f1 * m[2 * 4 + b]);
-        double2 cz = make_double2(0.0, f1 * m[3 * 4 + b]);
-        if (b > 0) {
-          cs = make_double2(-f2 * cs.y, f2 * cs.x);
-          cx = make_double2(-f2 * cx.y, f2 * cx.x);
-          cy = make_double2(-f2 * cy.y, f2 * cy.x);
-          cz = make_double2(-f2 * cz.y, f2 * cz.x);
-        }
-        const Q4 Lq{cs, cx, cy, cz};
-        const Q4 ld = qmul(Lq, dq);
-        const Q4 t = b == 0 ? ld : qsig(ld, b);  // (Lq dq) sigma_b
-        r.s = cadd(r.s, t.s);
-        r.x = cadd(r.x, t.x);
-        r.y = cadd(r.y, t.y);
-        r.z = cadd(r.z, t.z);
-      }
-      const size_t t = ix(t1, t2);
-      addz(a.K[0], t, r.s, -wx);
-      addz(a.K[1], t, r.x, -wx);
-      addz(a.K[2], t, r.y, -wx);
-      addz(a.K[3], t, r.z, -wx);
-    };
-    ex(gA, gD, gB, gC, 1.0, 1.0);
-    if (!dCD) ex(gA, gC, gB, gD, 1.0, -1.0);
-    if (!dAB) {
-      ex(gB, gD, gA, gC, -1.0, 1.0);
-      if (!dCD) ex(gB, gC, gA, gD, -1.0, -1.0);
-    }
-  }
-}
-
+// Planning pass of one class pair: per (bra pair, word of 32 kets) the
+// quartets that survive the screen, as FP64 and FP32 lane masks, and the
+// lists of non-empty words (the layout of jk_plan_kernel).
 // TYPE 1: LLSS (bra = SS pair, differentiated; ket = LL pair), all
 // (bra, ket) combinations (direct4C_libcint.hpp:907-929).
 // TYPE 2: SSSS, unique quartets of pairs (:2018-2047).
-// The ket's Cartesian component pairs (c, d) of a quartet are split over
-// nsplit threads (grid y = ket tiles x nsplit): the heavy classes with few
-// quartets (f shells) still fill the GPU.
-// T: primitive arithmetic (double; float for the small-bound quartets of a
-// mixed launch); operator components, digestion and accumulation in FP64.
-template <int LM, int TYPE, typename T>
-__global__ void __launch_bounds__(REL_THREADS)
-    rel_kernel(const RelLaunch a, int la, int lb, int lc, int ld, int nsplit) {
-  constexpr bool IS32 = sizeof(T) == 4;
-  const int ib = blockIdx.x;
-  if (!in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;  // another shard's bra
-  const int split = blockIdx.y % nsplit;
-  const int jk = (blockIdx.y / nsplit) * REL_THREADS + threadIdx.x;
-  const int ns = a.nShell;
-  bool visited = jk < a.nKet && !(TYPE == 2 && a.same && jk > ib);
-  const PairDev P = a.pairs[a.braBeg + ib];
-  PairDev Q = P;
-  bool work = false, mine = false;
-  if (visited) {
-    Q = a.pairs[a.ketBeg + jk];
-    if (a.skipSingle && P.npp == 1 && Q.npp == 1) visited = false;  // rel_gemm_kernel's
-  }
-  if (visited) {
-    int s1, s2, s3, s4;
-    double q12, q34;
-    if (TYPE == 1) {
-      s1 = P.s1; s2 = P.s2; s3 = Q.s1; s4 = Q.s2;
-      q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-      q34 = __ldg(a.qLL + s3 + (size_t)s4 * ns);
-    } else {
-      const bool pRef = P.lex >= Q.lex;
-      const PairDev& R12 = pRef ? P : Q;
-      const PairDev& R34 = pRef ? Q : P;
-      s1 = R12.s1; s2 = R12.s2; s3 = R34.s1; s4 = R34.s2;
-      q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-      q34 = __ldg(a.qSS + s3 + (size_t)s4 * ns);
+constexpr int REL_RUN = 32;
+template <int TYPE>
+__global__ void __launch_bounds__(256)
+    rel_plan_kernel(const RelLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
+                    int* __restrict__ list32, unsigned* __restrict__ lcount) {
+  const int lane = threadIdx.x & 31, ns = a.nShell;
+  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  const int nTiles = (a.nKet + WTILE - 1) / WTILE, nWords = a.nBra * nTiles;
+  unsigned long long cVis = 0, cScr = 0, c32 = 0, c64 = 0;
+  for (int run = gw; run * REL_RUN < nWords; run += nw) {
+    int my64 = -1, my32 = -1, n64 = 0, n32 = 0;
+    const int wEnd = min((run + 1) * REL_RUN, nWords);
+    for (int word = run * REL_RUN; word < wEnd; word++) {
+      const int ib = word / nTiles, jk = (word - ib * nTiles) * WTILE + lane;
+      const bool visited = jk < a.nKet && !(TYPE == 2 && a.same && jk > ib + a.braOff) &&
+                           in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt);
+      bool work = false, lo = false;
+      if (visited) {
+        const PairDev P = a.pairs[a.braBeg + ib], Q = a.pairs[a.ketBeg + jk];
+        const bool pRef = TYPE == 1 || P.lex >= Q.lex;
+        const int s1 = pRef ? P.s1 : Q.s1, s2 = pRef ? P.s2 : Q.s2;
+        const int s3 = pRef ? Q.s1 : P.s1, s4 = pRef ? Q.s2 : P.s2;
+        // shMax * Q12 * Q34 < thresh (:947-948, :2059-2061)
+        const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) *
+                             __ldg(a.qSS + P.s1 + (size_t)P.s2 * ns) *
+                             __ldg((TYPE == 1 ? a.qLL : a.qSS) + Q.s1 + (size_t)Q.s2 * ns);
+        work = !a.screen || bound >= a.thresh;
+        lo = work && a.mixed && bound < a.cut &&
+             fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
+                           __ldg(a.pairRange + a.ketBeg + jk), a.lsum + (TYPE == 2 ? 4 : 2), 1,
+                           TYPE == 2);
+      }
+      const unsigned bv = __ballot_sync(0xffffffffu, visited);
+      const unsigned bw = __ballot_sync(0xffffffffu, work);
+      const unsigned b32 = __ballot_sync(0xffffffffu, lo), b64 = bw & ~b32;
+      cVis += __popc(bv);
+      cScr += __popc(bv & ~bw);
+      c32 += __popc(b32);
+      c64 += __popc(b64);
+      if (lane == 0) masks[word] = make_uint2(b64, b32);
+      if (b64) {
+        if (lane == n64) my64 = word;
+        n64++;
+      }
+      if (b32) {
+        if (lane == n32) my32 = word;
+        n32++;
+      }
     }
-    // shMax * Q12 * Q34 < thresh (:947-948, :2059-2061)
-    const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) * q12 * q34;
-    work = !a.screen || bound >= a.thresh;
-    const bool lo = a.mixed && bound < a.cut &&
-                    fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                                  __ldg(a.pairRange + a.ketBeg + jk),
-                                  la + lb + lc + ld + 2 + 2 * (TYPE == 2), 1, TYPE == 2);
-    mine = work && (IS32 ? lo : !lo);
-  }
-  if (split == 0) {
-    const unsigned mask = __activemask();
-    const unsigned bv = __ballot_sync(mask, visited), bw = __ballot_sync(mask, work);
-    const unsigned bm = __ballot_sync(mask, mine);
-    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) {
-      if (!IS32 && bv) atomicAdd(a.counters + 0, (unsigned long long)__popc(bv));
-      if (!IS32 && (bv & ~bw)) atomicAdd(a.counters + 1, (unsigned long long)__popc(bv & ~bw));
-      if (bm) atomicAdd(a.counters + (IS32 ? 2 : 3), (unsigned long long)__popc(bm));
+    unsigned base64 = 0, base32 = 0;
+    if (lane == 0) {
+      if (n64) base64 = atomicAdd(lcount + 0, (unsigned)n64);
+      if (n32) base32 = atomicAdd(lcount + 1, (unsigned)n32);
     }
+    base64 = __shfl_sync(0xffffffffu, base64, 0);
+    base32 = __shfl_sync(0xffffffffu, base32, 0);
+    if (lane < n64) list64[base64 + lane] = my64;
+    if (lane < n32) list32[base32 + lane] = my32;
   }
+  if (lane == 0) {
+    if (cVis) atomicAdd(a.counters + 0, cVis);
+    if (cScr) atomicAdd(a.counters + 1, cScr);
+    if (c32) atomicAdd(a.counters + 2, c32);
+    if (c64) atomicAdd(a.counters + 3, c64);
+  }
+}
 
-  constexpr int NB = (TYPE == 2) ? 4 : 1;  // ket operator components
-  constexpr int NC = 4 * NB;               // operator components per integral
-  constexpr int NCL = ncart(LM);
-  constexpr int E1 = (LM + 2) * (LM + 2) * (2 * LM + 3);
-  constexpr int HB = nherm(2 * LM + 2);
-  constexpr int HL = nherm(4 * LM + 2 + 2 * (TYPE == 2));
-  constexpr int FL = 2 * LM + 3;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb;
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  if (!mine) return;
-  const T* boysT = reinterpret_cast<const T*>(IS32 ? (const void*)a.boys32 : (const void*)a.boys);
+// left product (i f)^[a > 0] sigma_a d of a Pauli quaternion: a permutation
+// of its components with signs
+__device__ __forceinline__ Q4 left_sigma(const Q4& d, int a, double f) {
+  if (a == 0) return d;
+  // sigma_k (s + v.sigma) = v_k + s sigma_k + i (k x v).sigma; times i f
+  auto fi = [f](double2 z) { return make_double2(-f * z.y, f * z.x); };  // i f z
+  auto fr = [f](double2 z, double g) { return make_double2(f * g * z.x, f * g * z.y); };
+  if (a == 1) return Q4{fi(d.x), fi(d.s), fr(d.z, 1.0), fr(d.y, -1.0)};
+  if (a == 2) return Q4{fi(d.y), fr(d.z, -1.0), fi(d.s), fr(d.x, 1.0)};
+  return Q4{fi(d.z), fr(d.y, 1.0), fr(d.x, -1.0), fi(d.s)};
+}
+// sum_b (i f)^[b > 0] t_b sigma_b of four quaternions of 8 reals each
+__device__ __forceinline__ Q4 right_sigmas(const double (&t)[4][8], double f) {
+  auto q = [&](int b) {
+    return Q4{make_double2(t[b][0], t[b][1]), make_double2(t[b][2], t[b][3]),
+              make_double2(t[b][4], t[b][5]), make_double2(t[b][6], t[b][7])};
+  };
+  Q4 r = q(0);
+#pragma unroll
+  for (int b = 1; b < 4; b++) {
+    const Q4 u = qsig(q(b), b);
+    r.s = cadd(r.s, make_double2(-f * u.s.y, f * u.s.x));
+    r.x = cadd(r.x, make_double2(-f * u.x.y, f * u.x.x));
+    r.y = cadd(r.y, make_double2(-f * u.y.y, f * u.y.x));
+    r.z = cadd(r.z, make_double2(-f * u.z.y, f * u.z.x));
+  }
+  return r;
+}
 
-  const int dK = (TYPE == 2) ? 1 : 0;
-  const int Lb = la + lb + 2, Lk = lc + ld + 2 * dK, L = Lb + Lk;
-  const ShellDev SC = a.shells[Q.shA], SD = a.shells[Q.shB];
+// Digestion of one quartet's operator components (TYPE 1: M[(ab, op)][cd],
+// TYPE 2: M[(ab, op)][(cd, op')]): the reference's updates with the sums
+// over the other two component indices taken before the one atomic of each
+// output element (J: over cd or ab; K: over the two contracted indices).
+// Work units of the exchange are (target, its bra and ket component, a share
+// of the contracted bra components); a unit sums m times the density over
+// its elements per operator and applies the Pauli matrices once at its end.
+// The element-wise digestion this replaces sent up to 36 atomics per element
+// (11.7e9 for one Ag atom's LLSS; the L2 takes 185e9 scattered ones per
+// second).
+template <int TYPE>
+__device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& z) {
+  constexpr int NB = TYPE == 2 ? 4 : 1;
+  const PairDev &P = *z.P, &Q = *z.Q;
+  const int tid = threadIdx.x, nt = blockDim.x, ms = z.ms[0];
+  const double* M = z.M[0];
+  const size_t nc = a.ncart;
+  auto ix = [nc](int r, int c) -> size_t { return (size_t)r + (size_t)c * nc; };
+  const int na = ncart(z.la), nb = ncart(z.lb), ncc = ncart(z.lc), nd = ncart(z.ld);
+  const int nAB = z.ab1 - z.ab0, nCD = z.cd1 - z.cd0;
   const bool dAB = P.shA == P.shB, dCD = Q.shA == Q.shB, samePQ = P.lex == Q.lex;
   const double s12d = dAB ? 1.0 : 2.0, s34d = dCD ? 1.0 : 2.0;
   // the back transform adds the transpose (Hermitian completion): a
   // contribution on a pair's own diagonal block is counted twice there
   const double w12 = dAB ? 0.5 : 1.0, w34 = dCD ? 0.5 : 1.0;
-  const bool single = P.npp == 1 && Q.npp == 1;  // digest without accumulating
-  const size_t nc = a.ncart;
-  auto ix = [nc](int r, int c) -> size_t { return (size_t)r + (size_t)c * nc; };
-
-  T Ea[3][E1], Ec[3][E1];
-  T G[NB][HB];
-  T Rv[HL];
-  T F[4 * LM + 5];
-  double acc[NCL * NCL * NC];
-  T fa[3][4][FL], fc[3][4][FL];
-  int nfa[3][4], nfc[3][4];
-
-#pragma unroll 1
-  for (int cd = split; cd < ncc * nd; cd += nsplit) {
-    {
-      const int c = cd / nd, d = cd % nd;
-      const int ci[3] = {cart_lx(lc, c), cart_ly(lc, c), cart_lz(lc, c)};
-      const int di[3] = {cart_lx(ld, d), cart_ly(ld, d), cart_lz(ld, d)};
-      const int gC = Q.cA + c, gD = Q.cB + d;
-      // per-column Coulomb accumulators (LLSS: J_LL(C,D); SSSS: J_SS(C,D))
-      double jcol[4] = {0.0, 0.0, 0.0, 0.0};
-      double rhoLL = 0.0;
-      double rvDC[4] = {0.0, 0.0, 0.0, 0.0};
-      if (TYPE == 1) {
-        rhoLL = __ldg(a.Xll + 2 * ix(gD, gC));
-      } else {
-        const size_t eDC = ix(gD, gC);
-        rvDC[0] = __ldg(a.Xss[0] + 2 * eDC);
-        rvDC[1] = -__ldg(a.Xss[1] + 2 * eDC + 1);
-        rvDC[2] = -__ldg(a.Xss[2] + 2 * eDC + 1);
-        rvDC[3] = -__ldg(a.Xss[3] + 2 * eDC + 1);
+  // Coulomb SS(1,2) from D(4,3) (:1145-1190, :2342-2380): unit (ab, op)
+  for (int u = tid; u < nAB * 4; u += nt) {
+    const double* m = M + (size_t)u * ms;
+    double s = 0.0;
+    for (int k = 0; k < nCD; k++) {
+      const int cd = z.cd0 + k, c = cd / nd, d = cd - c * nd;
+      const size_t e = ix(Q.cB + d, Q.cA + c);
+      if (TYPE == 1)
+        s += m[k] * __ldg(a.Xll + 2 * e);
+      else
+        s += m[4 * k] * __ldg(a.Xss[0] + 2 * e) - m[4 * k + 1] * __ldg(a.Xss[1] + 2 * e + 1) -
+             m[4 * k + 2] * __ldg(a.Xss[2] + 2 * e + 1) -
+             m[4 * k + 3] * __ldg(a.Xss[3] + 2 * e + 1);
+    }
+    const int ab = z.ab0 + (u >> 2), ai = ab / nb, bi = ab - ai * nb;
+    if (s != 0.0) atomicAdd(a.Jss[u & 3] + ix(P.cA + ai, P.cB + bi), w12 * s34d * s);
+  }
+  // Coulomb LL(3,4) / SS(3,4) from D(2,1) (SSSS: when the pairs differ):
+  // unit (cd, op')
+  if (TYPE == 1 || !samePQ)
+    for (int u = tid; u < nCD * NB; u += nt) {
+      double s = 0.0;
+      for (int k = 0; k < nAB; k++) {
+        const int ab = z.ab0 + k, ai = ab / nb, bi = ab - ai * nb;
+        const size_t e = ix(P.cB + bi, P.cA + ai);
+        const double* m = M + (size_t)(4 * k) * ms + u;
+        s += m[0] * __ldg(a.Xss[0] + 2 * e) - m[ms] * __ldg(a.Xss[1] + 2 * e + 1) -
+             m[2 * (size_t)ms] * __ldg(a.Xss[2] + 2 * e + 1) -
+             m[3 * (size_t)ms] * __ldg(a.Xss[3] + 2 * e + 1);
       }
-
-      const RelCol col{gC, gD, dAB, dCD, samePQ, s34d, w12, samePQ ? 0.5 : 1.0, rhoLL,
-                       {rvDC[0], rvDC[1], rvDC[2], rvDC[3]}};
-
-      if (!single)
-#pragma unroll 1
-        for (int k = 0; k < nab * NC; k++) acc[k] = 0.0;
-#pragma unroll 1
-      for (int ip = 0; ip < P.npp; ip++) {
-        const PrimPairDev& A = a.pp[P.pp_off + ip];
-        double ea, eb;
-        pair_exps(SA, SB, a.prim, A, ea, eb);
-#pragma unroll 1
-        for (int x = 0; x < 3; x++)
-          hermite_E_rt<T, LM + 1>(la + 1, lb + 1, T(A.o2p), T(A.PA[x]), T(A.PB[x]), Ea[x]);
-        const T p = T(A.p);
-#pragma unroll 1
-        for (int b = 0; b < NB; b++)
-#pragma unroll 1
-          for (int h = 0; h < nherm(Lb); h++) G[b][h] = T(0);
-#pragma unroll 1
-        for (int iq = 0; iq < Q.npp; iq++) {
-          const PrimPairDev& B = a.pp[Q.pp_off + iq];
-          double ec, ed;
-          pair_exps(SC, SD, a.prim, B, ec, ed);
-          const T q = T(B.p);
-#pragma unroll 1
-          for (int x = 0; x < 3; x++)
-            hermite_E_rt<T, LM + 1>(lc + dK, ld + dK, T(B.o2p), T(B.PA[x]), T(B.PB[x]), Ec[x]);
-          const T X = T(A.P[0] - B.P[0]), Y = T(A.P[1] - B.P[1]), Z = T(A.P[2] - B.P[2]);
-          const T pq = p + q, alpha = p * q / pq;
-          const T Targ = alpha * (X * X + Y * Y + Z * Z);
-          const T pref = T(PI52X2) / sqrt(pq) * T(A.Kp) * T(B.Kp);
-          boys_rt<T>(L, Targ, F, boysT);
-          hermite_R_rt<T>(L, alpha, X, Y, Z, F, Rv);
-          const int ntk = (TYPE == 2) ? 4 : 1;
-#pragma unroll 1
-          for (int x = 0; x < 3; x++)
-#pragma unroll 1
-            for (int ty = 0; ty < ntk; ty++) {
-              nfc[x][ty] = axis_factor<T>(Ec[x], ld + dK, lc + ld + 2 * dK + 1, ci[x], di[x], ty,
-                                          T(2.0 * ec), T(2.0 * ed), fc[x][ty]);
-#pragma unroll 1
-              for (int t = 1; t < nfc[x][ty]; t += 2) fc[x][ty][t] = -fc[x][ty][t];
-            }
-          if (TYPE == 1) {
-            ket_add<T>(G[0], pref, fc[0][0], nfc[0][0], fc[1][0], nfc[1][0], fc[2][0], nfc[2][0],
-                       Lb, Rv);
-          } else {
-#pragma unroll 1
-            for (int kk = 0; kk < 3; kk++)
-#pragma unroll 1
-              for (int ll = 0; ll < 3; ll++) {
-                int op;
-                double sg;
-                op_of(kk, ll, op, sg);
-                const int tx = (kk == 0) | ((ll == 0) << 1), ty = (kk == 1) | ((ll == 1) << 1),
-                          tz = (kk == 2) | ((ll == 2) << 1);
-                ket_add<T>(G[op < NB ? op : 0], T(sg) * pref, fc[0][tx], nfc[0][tx], fc[1][ty],
-                           nfc[1][ty], fc[2][tz], nfc[2][tz], Lb, Rv);
-              }
-          }
-        }
-        // bra: the 9 derivative pairs of every component pair (a, b)
-#pragma unroll 1
-        for (int ai = 0; ai < na; ai++)
-#pragma unroll 1
-          for (int bi = 0; bi < nb; bi++) {
-            const int ab = ai * nb + bi;
-            const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-            const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-#pragma unroll 1
-            for (int x = 0; x < 3; x++)
-#pragma unroll 1
-              for (int ty = 0; ty < 4; ty++)
-                nfa[x][ty] = axis_factor<T>(Ea[x], lb + 1, la + lb + 3, ax[x], bx[x], ty,
-                                            T(2.0 * ea), T(2.0 * eb), fa[x][ty]);
-            double mloc[NC];
-            double* m = single ? mloc : acc + ab * NC;
-            if (single)
+      const int cd = z.cd0 + u / NB, c = cd / nd, d = cd - c * nd;
+      if (s != 0.0)
+        atomicAdd((TYPE == 1 ? a.Jll : a.Jss[u % NB]) + ix(Q.cA + c, Q.cB + d), w34 * s12d * s);
+    }
+  if (!a.exchange) return;
+  // exchange targets (bra index of the output A or B, ket index C or D):
+  // LLSS (:1200-1299) K(c,b) -= D(d,a) P, K(c,a) -= D(d,b) P^(-), ...;
+  // SSSS (:2381-2445) K(a,d) -= P D(b,c) P, K(a,c), K(b,d), K(b,c)
+  const int total = 4 * (na > nb ? na : nb) * (ncc > nd ? ncc : nd);
+  for (int tgt = 0; tgt < 4; tgt++) {
+    const bool outA = TYPE == 1 ? (tgt & 1) : tgt < 2;   // output bra index: A (else B)
+    const bool outC = TYPE == 1 ? tgt < 2 : (tgt & 1);   // output ket index: C (else D)
+    if (TYPE == 1 ? ((outA && dAB) || (!outC && dCD)) : ((!outA && dAB) || (outC && dCD))) continue;
+    const double f1 = TYPE == 1 ? (outA ? -1.0 : 1.0) : (outA ? 1.0 : -1.0);
+    const double f2 = TYPE == 1 ? f1 : (outC ? -1.0 : 1.0);
+    const int no = outA ? na : nb, ni = outA ? nb : na;    // bra: output, contracted
+    const int ko = outC ? ncc : nd, ki = outC ? nd : ncc;  // ket
+    const int parts = total < nt ? ni : 1;
+    for (int u = tid; u < no * ko * parts; u += nt) {
+      const int part = u / (no * ko), r = u - part * (no * ko), kO = r / no, bO = r - kO * no;
+      double t[4][8];
 #pragma unroll
-              for (int k = 0; k < NC; k++) mloc[k] = 0.0;
-#pragma unroll 1
-            for (int mu = 0; mu < 3; mu++)
-#pragma unroll 1
-              for (int nu = 0; nu < 3; nu++) {
-                int op;
-                double sg;
-                op_of(mu, nu, op, sg);
-                const int tx = (mu == 0) | ((nu == 0) << 1), ty = (mu == 1) | ((nu == 1) << 1),
-                          tz = (mu == 2) | ((nu == 2) << 1);
-#pragma unroll 1
-                for (int b = 0; b < NB; b++)
-                  m[op * NB + b] += sg * double(bra_dot<T>(fa[0][tx], nfa[0][tx], fa[1][ty],
-                                                           nfa[1][ty], fa[2][tz], nfa[2][tz], G[b]));
-              }
-            if (single) rel_digest<TYPE>(a, P, col, ai, bi, mloc, jcol);
-          }
-      }
-      if (!single)
-#pragma unroll 1
-        for (int ab = 0; ab < nab; ab++) rel_digest<TYPE>(a, P, col, ab / nb, ab % nb, acc + ab * NC, jcol);
-
-      // per-column Coulomb flush
-      if (TYPE == 1) {
-        if (jcol[0] != 0.0) atomicAdd(a.Jll + ix(gC, gD), w34 * s12d * jcol[0]);
-      } else if (!samePQ) {
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-          if (jcol[b] != 0.0) atomicAdd(a.Jss[b] + ix(gC, gD), w34 * s12d * jcol[b]);
-      }
-    }
-  }
-}
-
-// Hermite index (t, u, v) of compact index e (inverse of hidx).
-__device__ __forceinline__ void hinv(int e, int& t, int& u, int& v) {
-  int sdeg = 0;
-  while (nherm(sdeg) <= e) sdeg++;
-  int r = e - nherm(sdeg - 1), k = 0;
-  while ((k + 1) * (k + 2) / 2 <= r) k++;
-  v = r - k * (k + 1) / 2;
-  u = k - v;
-  t = sdeg - k;
-}
-
-constexpr int RB_THREADS = 128;
-
-// The block kernels' table of Hermite indices: tab[h] = t | u << 8 | v << 16
-// for h < n (hinv once per block instead of per use).
-__device__ __forceinline__ void htab_fill(int* tab, int n) {
-  for (int h = threadIdx.x; h < n; h += blockDim.x) {
-    int t, u, v;
-    hinv(h, t, u, v);
-    tab[h] = t | (u << 8) | (v << 16);
-  }
-}
-__device__ __forceinline__ void htab_get(const int* tab, int h, int& t, int& u, int& v) {
-  const int w = tab[h];
-  t = w & 255;
-  u = (w >> 8) & 255;
-  v = w >> 16;
-}
-
-// Division by a runtime divisor d >= 1 as a multiply-high: with
-// m = ceil(2^32 / d), floor(x m / 2^32) = floor(x / d) for 0 <= x < 2^32 / d
-// (the error of m is below d).  The kernels' element indices are < 2^20.
-struct FastDiv {
-  unsigned m;
-  int d;
-  __device__ __forceinline__ explicit FastDiv(int dv)
-      : m(dv == 1 ? 0u : 0xFFFFFFFFu / (unsigned)dv + 1u), d(dv) {}
-  __device__ __forceinline__ int div(int x) const {
-    return d == 1 ? x : (int)__umulhi((unsigned)x, m);
-  }
-  __device__ __forceinline__ void divmod(int x, int& q, int& r) const {
-    q = div(x);
-    r = x - q * d;
-  }
-};
-
-// Shared-memory layout of rel_block_kernel (doubles), per launch.
-struct RelBlockLayout {
-  int oR0, oR1, oEb, oEk, oFa, oFc, oG, oM, oF, oJ, oT, total;
-};
-__host__ __device__ inline RelBlockLayout rel_block_layout(int la, int lb, int lc, int ld,
-                                                           int type) {
-  const int dK = type == 2 ? 1 : 0;
-  const int Lb = la + lb + 2, L = Lb + lc + ld + 2 * dK;
-  const int NB = type == 2 ? 4 : 1;
-  const int nab = ncart(la) * ncart(lb);
-  const int FL = 2 * (la > lb ? la : lb) + 3;
-  const int FLk = 2 * (lc > ld ? lc : ld) + 3;
-  RelBlockLayout Lo;
-  int o = 0;
-  auto take = [&](int n) { int r = o; o += (n + 1) / 2 * 2; return r; };
-  Lo.oR0 = take(nherm(L));
-  Lo.oR1 = take(nherm(L));
-  Lo.oEb = take(3 * (la + 2) * (lb + 2) * (la + lb + 3));
-  Lo.oEk = take(3 * (lc + 1 + dK) * (ld + 1 + dK) * (lc + ld + 1 + 2 * dK));
-  Lo.oFa = take(3 * (la + 1) * (lb + 1) * 4 * FL);  // per (axis, exponent pair, type)
-  Lo.oFc = take(12 * FLk);
-  Lo.oG = take(NB * nherm(Lb));
-  Lo.oM = take(nab * 4 * NB);
-  Lo.oF = take(L + 1);
-  Lo.oJ = take(4);
-  Lo.oT = take((nherm(L) + 1) / 2);  // packed (t, u, v) of each Hermite index, int
-  Lo.total = o;
-  return Lo;
-}
-
-// Block-cooperative form of rel_kernel for the heavy classes (d and f
-// shells): one block per unique quartet, everything in shared memory.  Per
-// primitive quartet: E tables, R (level by level, ping-pong buffers, all
-// threads), the bra factors of every component pair; per ket component pair
-// (c, d): its ket factors, G[b][tuv] (one entry per thread), the operator
-// components of every bra component pair (one (ab, b) unit per thread) and
-// their digestion (one ab per thread), the per-column Coulomb sum reduced in
-// shared memory.  Same quartet set, screens and updates as rel_kernel.
-template <int TYPE, typename T>
-__global__ void __launch_bounds__(RB_THREADS)
-    rel_block_kernel(const RelLaunch a, int la, int lb, int lc, int ld) {
-  constexpr bool IS32 = sizeof(T) == 4;
-  extern __shared__ double sm[];
-  const long long q = blockIdx.x + (long long)blockIdx.y * gridDim.x;
-  int ib, jk;
-  if (TYPE == 2 && a.same) {  // SSSS, one class: unordered pairs jk <= ib
-    long long r = (long long)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
-    while (r * (r + 1) / 2 > q) r--;
-    while ((r + 1) * (r + 2) / 2 <= q) r++;
-    ib = (int)r;
-    jk = (int)(q - r * (r + 1) / 2);
-  } else {
-    ib = (int)(q / a.nKet);
-    jk = (int)(q % a.nKet);
-  }
-  if (ib >= a.nBra || !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;
-  const int ns = a.nShell;
-  const PairDev P = a.pairs[a.braBeg + ib];
-  const PairDev Q = a.pairs[a.ketBeg + jk];
-  if (a.skipSingle && P.npp == 1 && Q.npp == 1) return;  // rel_gemm_kernel's
-  bool work, mine;
-  {
-    int s1, s2, s3, s4;
-    double q12, q34;
-    if (TYPE == 1) {
-      s1 = P.s1; s2 = P.s2; s3 = Q.s1; s4 = Q.s2;
-      q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-      q34 = __ldg(a.qLL + s3 + (size_t)s4 * ns);
-    } else {
-      const bool pRef = P.lex >= Q.lex;
-      const PairDev& R12 = pRef ? P : Q;
-      const PairDev& R34 = pRef ? Q : P;
-      s1 = R12.s1; s2 = R12.s2; s3 = R34.s1; s4 = R34.s2;
-      q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-      q34 = __ldg(a.qSS + s3 + (size_t)s4 * ns);
-    }
-    const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) * q12 * q34;
-    work = !a.screen || bound >= a.thresh;
-    const bool lo = a.mixed && bound < a.cut &&
-                    fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                                  __ldg(a.pairRange + a.ketBeg + jk),
-                                  la + lb + lc + ld + 2 + 2 * (TYPE == 2), 1, TYPE == 2);
-    mine = work && (IS32 ? lo : !lo);
-  }
-  if (threadIdx.x == 0) {
-    if (!IS32) atomicAdd(a.counters + 0, 1ull);
-    if (!IS32 && !work) atomicAdd(a.counters + 1, 1ull);
-    if (mine) atomicAdd(a.counters + (IS32 ? 2 : 3), 1ull);
-  }
-  if (!mine) return;  // block-uniform
-  const T* boysT = reinterpret_cast<const T*>(IS32 ? (const void*)a.boys32 : (const void*)a.boys);
-
-  constexpr int NB = (TYPE == 2) ? 4 : 1;
-  constexpr int NC = 4 * NB;
-  const int tid = threadIdx.x;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb;
-  const int dK = (TYPE == 2) ? 1 : 0;
-  const int Lb = la + lb + 2, L = Lb + lc + ld + 2 * dK;
-  const int FL = 2 * max(la, lb) + 3, FLk = 2 * max(lc, ld) + 3;
-  const RelBlockLayout Lo = rel_block_layout(la, lb, lc, ld, TYPE);
-  int* htab = reinterpret_cast<int*>(sm + Lo.oT);
-  htab_fill(htab, nherm(L));  // read after prep's first barrier
-  const FastDiv fhbB(nherm(Lb)), fnbB(nb);
-  T* Rb[2] = {reinterpret_cast<T*>(sm + Lo.oR0), reinterpret_cast<T*>(sm + Lo.oR1)};
-  T* Eb = reinterpret_cast<T*>(sm + Lo.oEb);
-  T* Ek = reinterpret_cast<T*>(sm + Lo.oEk);
-  T* fa = reinterpret_cast<T*>(sm + Lo.oFa);
-  T* fc = reinterpret_cast<T*>(sm + Lo.oFc);
-  T* G = reinterpret_cast<T*>(sm + Lo.oG);
-  double* Mc = sm + Lo.oM;
-  T* Fs = reinterpret_cast<T*>(sm + Lo.oF);
-  double* Js = sm + Lo.oJ;
-  const int E1b = (la + 2) * (lb + 2) * (la + lb + 3);
-  const int E1k = (lc + 1 + dK) * (ld + 1 + dK) * (lc + ld + 1 + 2 * dK);
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  const ShellDev SC = a.shells[Q.shA], SD = a.shells[Q.shB];
-  const bool dAB = P.shA == P.shB, dCD = Q.shA == Q.shB, samePQ = P.lex == Q.lex;
-  const double s12d = dAB ? 1.0 : 2.0, s34d = dCD ? 1.0 : 2.0;
-  const double w12 = dAB ? 0.5 : 1.0, w34 = dCD ? 0.5 : 1.0;
-  const size_t nc = a.ncart;
-  const T* R = Rb[0];  // R^(0) after the recursion
-  double ec = 0.0, ed = 0.0;
-  T pref = T(0);
-
-  // E tables, R and the bra factors of primitive quartet (ip, iq)
-  auto prep = [&](int ip, int iq) {
-    const PrimPairDev& A = a.pp[P.pp_off + ip];
-    const PrimPairDev& B = a.pp[Q.pp_off + iq];
-    double ea, eb;
-    pair_exps(SA, SB, a.prim, A, ea, eb);
-    pair_exps(SC, SD, a.prim, B, ec, ed);
-    if (tid < 3)
-      hermite_E_rt<T, LMAX + 1>(la + 1, lb + 1, T(A.o2p), T(A.PA[tid]), T(A.PB[tid]),
-                                Eb + tid * E1b);
-    else if (tid < 6)
-      hermite_E_rt<T, LMAX + 1>(lc + dK, ld + dK, T(B.o2p), T(B.PA[tid - 3]), T(B.PB[tid - 3]),
-                                Ek + (tid - 3) * E1k);
-    const T X = T(A.P[0] - B.P[0]), Y = T(A.P[1] - B.P[1]), Z = T(A.P[2] - B.P[2]);
-    const T pq = T(A.p) + T(B.p), alpha = T(A.p) * T(B.p) / pq;
-    pref = T(PI52X2) / sqrt(pq) * T(A.Kp) * T(B.Kp);
-    if (tid >= 32 && tid < 64)
-      boys_lanes<T>(L, alpha * (X * X + Y * Y + Z * Z), Fs, boysT, tid - 32);
-    __syncthreads();
-    // R^(n)_tuv, n = L .. 0, from R^(n+1); level n in Rb[n & 1]
-    const T m2a = T(-2) * alpha;
-    for (int n = L; n >= 0; n--) {
-      T* cur = Rb[n & 1];
-      const T* prv = Rb[(n + 1) & 1];
-      const int cnt = nherm(L - n);
-      for (int e = tid; e < cnt; e += RB_THREADS) {
-        int t, u, v;
-        htab_get(htab, e, t, u, v);
-        T val;
-        if (e == 0) {
-          T f = T(1);
-          for (int k = 0; k < n; k++) f *= m2a;
-          val = f * Fs[n];
-        } else if (t > 0) {
-          val = X * prv[hidx(t - 1, u, v)];
-          if (t > 1) val += T(t - 1) * prv[hidx(t - 2, u, v)];
-        } else if (u > 0) {
-          val = Y * prv[hidx(0, u - 1, v)];
-          if (u > 1) val += T(u - 1) * prv[hidx(0, u - 2, v)];
-        } else {
-          val = Z * prv[hidx(0, 0, v - 1)];
-          if (v > 1) val += T(v - 1) * prv[hidx(0, 0, v - 2)];
-        }
-        cur[e] = val;
-      }
-      __syncthreads();
-    }
-    // bra factors of every axis, exponent pair and derivative type
-    for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += RB_THREADS) {
-      const int ty = it % 4, jb = (it / 4) % (lb + 1), ia = (it / 4 / (lb + 1)) % (la + 1),
-                x = it / 4 / (lb + 1) / (la + 1);
-      axis_factor<T>(Eb + x * E1b, lb + 1, la + lb + 3, ia, jb, ty, T(2.0 * ea), T(2.0 * eb),
-                     fa + (size_t)it * FL);
-    }
-    __syncthreads();
-  };
-  auto faOf = [&](int x, int i, int j, int ty) {
-    return fa + (size_t)(((x * (la + 1) + i) * (lb + 1) + j) * 4 + ty) * FL;
-  };
-
-  const bool single = P.npp == 1 && Q.npp == 1;
-  if (single) prep(0, 0);
-  if (tid < 4) Js[tid] = 0.0;
-#pragma unroll 1
-  for (int cd = 0; cd < ncc * nd; cd++) {
-    const int c = cd / nd, d = cd % nd;
-    const int gC = Q.cA + c, gD = Q.cB + d;
-    for (int e = tid; e < nab * NC; e += RB_THREADS) Mc[e] = 0.0;
-#pragma unroll 1
-    for (int ip = 0; ip < P.npp; ip++)
-#pragma unroll 1
-      for (int iq = 0; iq < Q.npp; iq++) {
-        if (!single) prep(ip, iq);  // ends with a barrier
-        // ket factors of this component pair (sign (-1)^t folded in)
-        const int ntk = (TYPE == 2) ? 4 : 1;
-        if (tid < 3 * ntk) {
-          const int x = tid / ntk, ty = tid % ntk;
-          const int ci = x == 0 ? cart_lx(lc, c) : (x == 1 ? cart_ly(lc, c) : cart_lz(lc, c));
-          const int di = x == 0 ? cart_lx(ld, d) : (x == 1 ? cart_ly(ld, d) : cart_lz(ld, d));
-          T* f = fc + (x * 4 + ty) * FLk;
-          const int n = axis_factor<T>(Ek + x * E1k, ld + dK, lc + ld + 2 * dK + 1, ci, di, ty,
-                                       T(2.0 * ec), T(2.0 * ed), f);
-          for (int t = 1; t < n; t += 2) f[t] = -f[t];
-        }
-        __syncthreads();
-        // G[b][tuv]
-        const int hb = nherm(Lb);
-        for (int e = tid; e < NB * hb; e += RB_THREADS) {
-          int b, h;
-          fhbB.divmod(e, b, h);
-          int t, u, v;
-          htab_get(htab, h, t, u, v);
-          const int ci[3] = {cart_lx(lc, c), cart_ly(lc, c), cart_lz(lc, c)};
-          const int di[3] = {cart_lx(ld, d), cart_ly(ld, d), cart_lz(ld, d)};
-          T gsum = T(0);
-          for (int kk = 0; kk < (TYPE == 2 ? 3 : 1); kk++)
-            for (int ll = 0; ll < (TYPE == 2 ? 3 : 1); ll++) {
-              int op = 0;
-              double sg = 1.0;
-              int tyx = 0, tyy = 0, tyz = 0;
-              if (TYPE == 2) {
-                op_of(kk, ll, op, sg);
-                if (op != b) continue;
-                tyx = (kk == 0) | ((ll == 0) << 1);
-                tyy = (kk == 1) | ((ll == 1) << 1);
-                tyz = (kk == 2) | ((ll == 2) << 1);
-              }
-              const T* fx = fc + (0 * 4 + tyx) * FLk;
-              const T* fy = fc + (1 * 4 + tyy) * FLk;
-              const T* fz = fc + (2 * 4 + tyz) * FLk;
-              const int nx = ci[0] + di[0] + (tyx & 1) + (tyx >> 1) + 1;
-              const int ny = ci[1] + di[1] + (tyy & 1) + (tyy >> 1) + 1;
-              const int nz = ci[2] + di[2] + (tyz & 1) + (tyz >> 1) + 1;
-              T acc = T(0);
-              for (int i = 0; i < nx; i++) {
-                if (fx[i] == T(0)) continue;
-                for (int j = 0; j < ny; j++) {
-                  const T fxy = fx[i] * fy[j];
-                  if (fxy == T(0)) continue;
-                  acc += fxy * hdot_v(fz, nz, R, t + i, u + j, v);
-                }
-              }
-              gsum += T(sg) * acc;
-            }
-          G[e] = pref * gsum;
-        }
-        __syncthreads();
-        // operator components of every bra component pair: unit (ab, b)
-        for (int e = tid; e < nab * NB; e += RB_THREADS) {
-          const int ab = e / NB, b = e % NB;
-          int ai, bi;
-          fnbB.divmod(ab, ai, bi);
-          const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-          const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-          double m4[4] = {0.0, 0.0, 0.0, 0.0};
-          for (int mu = 0; mu < 3; mu++)
-            for (int nu = 0; nu < 3; nu++) {
-              int op;
-              double sg;
-              op_of(mu, nu, op, sg);
-              const int tx = (mu == 0) | ((nu == 0) << 1), ty = (mu == 1) | ((nu == 1) << 1),
-                        tz = (mu == 2) | ((nu == 2) << 1);
-              const T* gx = faOf(0, ax[0], bx[0], tx);
-              const T* gy = faOf(1, ax[1], bx[1], ty);
-              const T* gz = faOf(2, ax[2], bx[2], tz);
-              m4[op] += sg * (double)bra_dot<T>(gx, ax[0] + bx[0] + (tx & 1) + (tx >> 1) + 1, gy,
-                                     ax[1] + bx[1] + (ty & 1) + (ty >> 1) + 1, gz,
-                                     ax[2] + bx[2] + (tz & 1) + (tz >> 1) + 1, G + b * hb);
-            }
-          for (int op = 0; op < 4; op++) Mc[ab * NC + op * NB + b] += m4[op];
-        }
-        __syncthreads();
-      }
-    // digestion, one bra component pair per thread
-    RelCol col{gC, gD, dAB, dCD, samePQ, s34d, w12, samePQ ? 0.5 : 1.0, 0.0, {0, 0, 0, 0}};
-    if (TYPE == 1) {
-      col.rhoLL = __ldg(a.Xll + 2 * ((size_t)gD + (size_t)gC * nc));
-    } else {
-      const size_t eDC = (size_t)gD + (size_t)gC * nc;
-      col.rvDC[0] = __ldg(a.Xss[0] + 2 * eDC);
-      col.rvDC[1] = -__ldg(a.Xss[1] + 2 * eDC + 1);
-      col.rvDC[2] = -__ldg(a.Xss[2] + 2 * eDC + 1);
-      col.rvDC[3] = -__ldg(a.Xss[3] + 2 * eDC + 1);
-    }
-    for (int ab = tid; ab < nab; ab += RB_THREADS) {
-      double jl[4] = {0.0, 0.0, 0.0, 0.0};
-      rel_digest<TYPE>(a, P, col, ab / nb, ab % nb, Mc + ab * NC, jl);
       for (int b = 0; b < 4; b++)
-        if (jl[b] != 0.0) atomicAdd(Js + b, jl[b]);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const size_t eCD = (size_t)gC + (size_t)gD * nc;
-      if (TYPE == 1) {
-        if (Js[0] != 0.0) atomicAdd(a.Jll + eCD, w34 * s12d * Js[0]);
-      } else if (!samePQ) {
-        for (int b = 0; b < 4; b++)
-          if (Js[b] != 0.0) atomicAdd(a.Jss[b] + eCD, w34 * s12d * Js[b]);
-      }
-      for (int b = 0; b < 4; b++) Js[b] = 0.0;
-    }
-    __syncthreads();
-  }
-}
-
-// Shared-memory layout of rel_llss_block_kernel (doubles).  The axis
-// factors depend on a component pair only through its two exponents on the
-// axis, so they are kept per (axis, i, j[, derivative type]); single-primitive
-// launches digest each element as it is made and keep no accumulator Mc.
-struct LlssBlockLayout {
-  int oR0, oR1, oEb, oEk, oFa, oFc, oG, oM, oF, oJ, oT, total;
-};
-__host__ __device__ inline LlssBlockLayout llss_block_layout(int la, int lb, int lc, int ld,
-                                                             bool single) {
-  const int Lb = la + lb + 2, L = Lb + lc + ld;
-  const int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld);
-  const int FL = 2 * (la > lb ? la : lb) + 3, FLk = lc + ld + 1;
-  LlssBlockLayout Lo;
-  int o = 0;
-  auto take = [&](int n) { int r = o; o += (n + 1) / 2 * 2; return r; };
-  Lo.oR0 = take(nherm(L));
-  Lo.oR1 = take(nherm(L));
-  Lo.oEb = take(3 * (la + 2) * (lb + 2) * (la + lb + 3));
-  Lo.oEk = take(3 * (lc + 1) * (ld + 1) * (lc + ld + 1));
-  Lo.oFa = take(3 * (la + 1) * (lb + 1) * 4 * FL);
-  Lo.oFc = take(3 * (lc + 1) * (ld + 1) * FLk);
-  Lo.oG = take(ncd * nherm(Lb));
-  Lo.oM = take(single ? 0 : nab * ncd * 4);
-  Lo.oF = take(L + 1);
-  Lo.oJ = take(ncd);
-  Lo.oT = take((nherm(L) + 1) / 2);  // packed (t, u, v) of each Hermite index, int
-  Lo.total = o;
-  return Lo;
-}
-
-// LLSS form of the block kernel: the ket pair is undifferentiated, so the
-// ket-contracted Hermite sums G[cd][tuv] of every ket component pair are
-// built at once, and the operator components of every (bra, ket) component
-// element are one work unit per thread (nab x ncd units); digestion per
-// element, the per-column Coulomb sums J_LL(C,D) reduced in shared memory.
-// With skipSingle set the quartets of two single-primitive pairs are
-// rel_llss_single_kernel's.
-template <typename T>
-__global__ void __launch_bounds__(RB_THREADS)
-    rel_llss_block_kernel(const RelLaunch a, int la, int lb, int lc, int ld) {
-  constexpr bool IS32 = sizeof(T) == 4;
-  extern __shared__ double sm[];
-  const long long q = blockIdx.x + (long long)blockIdx.y * gridDim.x;
-  const int ib = (int)(q / a.nKet), jk = (int)(q % a.nKet);
-  if (ib >= a.nBra || !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;
-  const int ns = a.nShell;
-  const PairDev P = a.pairs[a.braBeg + ib];
-  const PairDev Q = a.pairs[a.ketBeg + jk];
-  if (a.skipSingle && P.npp == 1 && Q.npp == 1) return;  // rel_llss_single_kernel's
-  const double bound = sh_max(a.norms, P.s1, P.s2, Q.s1, Q.s2, ns) *
-                       __ldg(a.qSS + P.s1 + (size_t)P.s2 * ns) *
-                       __ldg(a.qLL + Q.s1 + (size_t)Q.s2 * ns);
-  const bool work = !a.screen || bound >= a.thresh;
-  const bool lo = a.mixed && bound < a.cut &&
-                  fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                                __ldg(a.pairRange + a.ketBeg + jk), la + lb + lc + ld + 2, 1, 0);
-  const bool mine = work && (IS32 ? lo : !lo);
-  if (threadIdx.x == 0) {
-    if (!IS32) atomicAdd(a.counters + 0, 1ull);
-    if (!IS32 && !work) atomicAdd(a.counters + 1, 1ull);
-    if (mine) atomicAdd(a.counters + (IS32 ? 2 : 3), 1ull);
-  }
-  if (!mine) return;  // block-uniform
-  const T* boysT = reinterpret_cast<const T*>(IS32 ? (const void*)a.boys32 : (const void*)a.boys);
-
-  const int tid = threadIdx.x;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb, ncd = ncc * nd;
-  const int Lb = la + lb + 2, L = Lb + lc + ld;
-  const int hb = nherm(Lb);
-  const int FL = 2 * max(la, lb) + 3, FLk = lc + ld + 1;
-  const LlssBlockLayout Lo = llss_block_layout(la, lb, lc, ld, false);
-  int* htab = reinterpret_cast<int*>(sm + Lo.oT);
-  htab_fill(htab, nherm(L));  // read after the first barrier of the primitive loop
-  T* Rb[2] = {reinterpret_cast<T*>(sm + Lo.oR0), reinterpret_cast<T*>(sm + Lo.oR1)};
-  T* Eb = reinterpret_cast<T*>(sm + Lo.oEb);
-  T* Ek = reinterpret_cast<T*>(sm + Lo.oEk);
-  T* fa = reinterpret_cast<T*>(sm + Lo.oFa);
-  T* fc = reinterpret_cast<T*>(sm + Lo.oFc);
-  T* G = reinterpret_cast<T*>(sm + Lo.oG);
-  double* Mc = sm + Lo.oM;
-  T* Fs = reinterpret_cast<T*>(sm + Lo.oF);
-  double* Js = sm + Lo.oJ;
-  const int E1b = (la + 2) * (lb + 2) * (la + lb + 3);
-  const int E1k = (lc + 1) * (ld + 1) * (lc + ld + 1);
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  const ShellDev SC = a.shells[Q.shA], SD = a.shells[Q.shB];
-  const bool dAB = P.shA == P.shB, dCD = Q.shA == Q.shB;
-  const double s12d = dAB ? 1.0 : 2.0, s34d = dCD ? 1.0 : 2.0;
-  const double w12 = dAB ? 0.5 : 1.0, w34 = dCD ? 0.5 : 1.0;
-  const size_t nc = a.ncart;
-  const T* R = Rb[0];
-
-  for (int e = tid; e < nab * ncd * 4; e += RB_THREADS) Mc[e] = 0.0;
-  for (int e = tid; e < ncd; e += RB_THREADS) Js[e] = 0.0;
-  // the axis factor vectors of (axis x, bra exponents i, j, type ty) and
-  // (axis x, ket exponents i, j)
-  auto faOf = [&](int x, int i, int j, int ty) {
-    return fa + (size_t)(((x * (la + 1) + i) * (lb + 1) + j) * 4 + ty) * FL;
-  };
-  auto fcOf = [&](int x, int i, int j) {
-    return fc + (size_t)((x * (lc + 1) + i) * (ld + 1) + j) * FLk;
-  };
+#pragma unroll
+        for (int k = 0; k < 8; k++) t[b][k] = 0.0;
+      bool any = false;
 #pragma unroll 1
-  for (int ip = 0; ip < P.npp; ip++)
+      for (int bI = part; bI < ni; bI += parts) {
+        const int ab = (outA ? bO * nb + bI : bI * nb + bO) - z.ab0;
+        if (ab < 0 || ab >= nAB) continue;
 #pragma unroll 1
-    for (int iq = 0; iq < Q.npp; iq++) {
-      const PrimPairDev& A = a.pp[P.pp_off + ip];
-      const PrimPairDev& B = a.pp[Q.pp_off + iq];
-      double ea, eb, ec, ed;
-      pair_exps(SA, SB, a.prim, A, ea, eb);
-      pair_exps(SC, SD, a.prim, B, ec, ed);
-      __syncthreads();  // the previous primitive quartet's readers are done
-      if (tid < 3)
-        hermite_E_rt<T, LMAX + 1>(la + 1, lb + 1, T(A.o2p), T(A.PA[tid]), T(A.PB[tid]),
-                                  Eb + tid * E1b);
-      else if (tid < 6)
-        hermite_E_rt<T, LMAX + 1>(lc, ld, T(B.o2p), T(B.PA[tid - 3]), T(B.PB[tid - 3]),
-                                  Ek + (tid - 3) * E1k);
-      const T X = T(A.P[0] - B.P[0]), Y = T(A.P[1] - B.P[1]), Z = T(A.P[2] - B.P[2]);
-      const T pq = T(A.p) + T(B.p), alpha = T(A.p) * T(B.p) / pq;
-      const T pref = T(PI52X2) / sqrt(pq) * T(A.Kp) * T(B.Kp);
-      if (tid >= 32 && tid < 64)
-        boys_lanes<T>(L, alpha * (X * X + Y * Y + Z * Z), Fs, boysT, tid - 32);
-      __syncthreads();
-      const T m2a = T(-2) * alpha;
-      for (int n = L; n >= 0; n--) {
-        T* cur = Rb[n & 1];
-        const T* prv = Rb[(n + 1) & 1];
-        const int cnt = nherm(L - n);
-        for (int e = tid; e < cnt; e += RB_THREADS) {
-          int t, u, v;
-          htab_get(htab, e, t, u, v);
-          T val;
-          if (e == 0) {
-            T f = T(1);
-            for (int k = 0; k < n; k++) f *= m2a;
-            val = f * Fs[n];
-          } else if (t > 0) {
-            val = X * prv[hidx(t - 1, u, v)];
-            if (t > 1) val += T(t - 1) * prv[hidx(t - 2, u, v)];
-          } else if (u > 0) {
-            val = Y * prv[hidx(0, u - 1, v)];
-            if (u > 1) val += T(u - 1) * prv[hidx(0, u - 2, v)];
-          } else {
-            val = Z * prv[hidx(0, 0, v - 1)];
-            if (v > 1) val += T(v - 1) * prv[hidx(0, 0, v - 2)];
-          }
-          cur[e] = val;
-        }
-        __syncthreads();
-      }
-      // bra factors (every axis, exponent pair, derivative type); ket factors
-      // (undifferentiated, sign (-1)^t folded in)
-      for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += RB_THREADS) {
-        const int ty = it % 4, jb = (it / 4) % (lb + 1), ia = (it / 4 / (lb + 1)) % (la + 1),
-                  x = it / 4 / (lb + 1) / (la + 1);
-        axis_factor<T>(Eb + x * E1b, lb + 1, la + lb + 3, ia, jb, ty, T(2.0 * ea), T(2.0 * eb),
-                       fa + (size_t)it * FL);
-      }
-      for (int it = tid; it < 3 * (lc + 1) * (ld + 1); it += RB_THREADS) {
-        const int di = it % (ld + 1), ci = (it / (ld + 1)) % (lc + 1),
-                  x = it / (ld + 1) / (lc + 1);
-        T* f = fc + (size_t)it * FLk;
-        const int n = axis_factor<T>(Ek + x * E1k, ld, lc + ld + 1, ci, di, 0, T(0), T(0), f);
-        for (int t = 1; t < n; t += 2) f[t] = -f[t];
-      }
-      __syncthreads();
-      // G[cd][tuv] of every ket component pair
-      for (int e = tid; e < ncd * hb; e += RB_THREADS) {
-        const int cd = e / hb, h = e % hb, c = cd / nd, d = cd % nd;
-        int t, u, v;
-        htab_get(htab, h, t, u, v);
-        const T* fx = fcOf(0, cart_lx(lc, c), cart_lx(ld, d));
-        const T* fy = fcOf(1, cart_ly(lc, c), cart_ly(ld, d));
-        const T* fz = fcOf(2, cart_lz(lc, c), cart_lz(ld, d));
-        const int nx = cart_lx(lc, c) + cart_lx(ld, d) + 1;
-        const int ny = cart_ly(lc, c) + cart_ly(ld, d) + 1;
-        const int nz = cart_lz(lc, c) + cart_lz(ld, d) + 1;
-        T acc = T(0);
-        for (int i = 0; i < nx; i++) {
-          if (fx[i] == T(0)) continue;
-          for (int j = 0; j < ny; j++) {
-            const T fxy = fx[i] * fy[j];
-            if (fxy == T(0)) continue;
-            acc += fxy * hdot_v(fz, nz, R, t + i, u + j, v);
-          }
-        }
-        G[e] = pref * acc;
-      }
-      __syncthreads();
-      // operator components of every (bra, ket) component element
-      for (int e = tid; e < nab * ncd; e += RB_THREADS) {
-        const int ab = e / ncd, cd = e % ncd;
-        const int ai = ab / nb, bi = ab % nb;
-        const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-        const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-        double m4[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int mu = 0; mu < 3; mu++)
-          for (int nu = 0; nu < 3; nu++) {
-            int op;
-            double sg;
-            op_of(mu, nu, op, sg);
-            const int tx = (mu == 0) | ((nu == 0) << 1), ty = (mu == 1) | ((nu == 1) << 1),
-                      tz = (mu == 2) | ((nu == 2) << 1);
-            m4[op] += sg * (double)bra_dot<T>(faOf(0, ax[0], bx[0], tx),
-                                   ax[0] + bx[0] + (tx & 1) + (tx >> 1) + 1,
-                                   faOf(1, ax[1], bx[1], ty),
-                                   ax[1] + bx[1] + (ty & 1) + (ty >> 1) + 1,
-                                   faOf(2, ax[2], bx[2], tz),
-                                   ax[2] + bx[2] + (tz & 1) + (tz >> 1) + 1, G + (size_t)cd * hb);
-          }
-        for (int op = 0; op < 4; op++) Mc[(size_t)e * 4 + op] += m4[op];
-      }
-    }
-  __syncthreads();
-  // digestion, one (bra, ket) component element per thread
-  for (int e = tid; e < nab * ncd; e += RB_THREADS) {
-    const int ab = e / ncd, cd = e % ncd;
-    const int gC = Q.cA + cd / nd, gD = Q.cB + cd % nd;
-    RelCol col{gC, gD, dAB, dCD, false, s34d, w12, 1.0,
-               __ldg(a.Xll + 2 * ((size_t)gD + (size_t)gC * nc)), {0, 0, 0, 0}};
-    double jl[4] = {0.0, 0.0, 0.0, 0.0};
-    rel_digest<1>(a, P, col, ab / nb, ab % nb, Mc + (size_t)e * 4, jl);
-    if (jl[0] != 0.0) atomicAdd(Js + cd, jl[0]);
-  }
-  __syncthreads();
-  for (int cd = tid; cd < ncd; cd += RB_THREADS)
-    if (Js[cd] != 0.0)
-      atomicAdd(a.Jll + (size_t)(Q.cA + cd / nd) + (size_t)(Q.cB + cd % nd) * nc,
-                w34 * s12d * Js[cd]);
-}
-
-// LLSS quartets of two single-primitive pairs (every quartet of an
-// uncontracted basis): one block per bra pair and tile of kt ket pairs (kt
-// up to LS_KT; 1 for launches too small to fill the GPU otherwise).
-// The bra pair's E tables and axis factors are made once; per ket its E
-// tables, Boys values and R (level by level over the block), the ket factors,
-// G[cd][tuv] of every ket component pair, then the operator components of
-// every (bra, ket) component element, digested as they are made (one
-// primitive quartet: nothing to accumulate).  Same quartet set, screens and
-// updates as rel_llss_block_kernel.
-constexpr int LS_KT = 8;
-
-template <typename T>
-__global__ void __launch_bounds__(RB_THREADS, 8)
-    rel_llss_single_kernel(const RelLaunch a, int la, int lb, int lc, int ld, int kt) {
-  constexpr bool IS32 = sizeof(T) == 4;
-  extern __shared__ double sm[];
-  const int nTiles = (a.nKet + kt - 1) / kt;
-  const long long q = blockIdx.x + (long long)blockIdx.y * gridDim.x;
-  const int ib = (int)(q / nTiles), tile = (int)(q % nTiles);
-  if (ib >= a.nBra || !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;
-  const PairDev P = a.pairs[a.braBeg + ib];
-  if (P.npp != 1) return;  // contracted bra: rel_llss_block_kernel
-  const int jkEnd = min(tile * kt + kt, a.nKet);
-  const int ns = a.nShell;
-  const T* boysT = reinterpret_cast<const T*>(IS32 ? (const void*)a.boys32 : (const void*)a.boys);
-
-  const int tid = threadIdx.x;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb, ncd = ncc * nd;
-  const int Lb = la + lb + 2, L = Lb + lc + ld;
-  const int hb = nherm(Lb);
-  const int FL = 2 * max(la, lb) + 3, FLk = lc + ld + 1;
-  const LlssBlockLayout Lo = llss_block_layout(la, lb, lc, ld, true);
-  int* htab = reinterpret_cast<int*>(sm + Lo.oT);
-  htab_fill(htab, nherm(L));  // read after the bra phase's barrier
-  T* Rb[2] = {reinterpret_cast<T*>(sm + Lo.oR0), reinterpret_cast<T*>(sm + Lo.oR1)};
-  T* Eb = reinterpret_cast<T*>(sm + Lo.oEb);
-  T* Ek = reinterpret_cast<T*>(sm + Lo.oEk);
-  T* fa = reinterpret_cast<T*>(sm + Lo.oFa);
-  T* fc = reinterpret_cast<T*>(sm + Lo.oFc);
-  T* G = reinterpret_cast<T*>(sm + Lo.oG);
-  T* Fs = reinterpret_cast<T*>(sm + Lo.oF);
-  double* Js = sm + Lo.oJ;
-  const int E1b = (la + 2) * (lb + 2) * (la + lb + 3);
-  const int E1k = (lc + 1) * (ld + 1) * (lc + ld + 1);
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  const bool dAB = P.shA == P.shB;
-  const double s12d = dAB ? 1.0 : 2.0, w12 = dAB ? 0.5 : 1.0;
-  const size_t nc = a.ncart;
-  const T* R = Rb[0];
-  auto faOf = [&](int x, int i, int j, int ty) {
-    return fa + (size_t)(((x * (la + 1) + i) * (lb + 1) + j) * 4 + ty) * FL;
-  };
-  auto fcOf = [&](int x, int i, int j) {
-    return fc + (size_t)((x * (lc + 1) + i) * (ld + 1) + j) * FLk;
-  };
-  const FastDiv fncd(ncd), fnb(nb), fnd(nd), fhb(hb);
-
-  // ---- bra phase: E tables and axis factors of every axis, exponent pair
-  // and derivative type
-  const PrimPairDev& A = a.pp[P.pp_off];
-  double ea, eb;
-  pair_exps(SA, SB, a.prim, A, ea, eb);
-  if (tid < 3)
-    hermite_E_rt<T, LMAX + 1>(la + 1, lb + 1, T(A.o2p), T(A.PA[tid]), T(A.PB[tid]),
-                              Eb + tid * E1b);
-  __syncthreads();
-  for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += RB_THREADS) {
-    const int ty = it % 4, jb = (it / 4) % (lb + 1), ia = (it / 4 / (lb + 1)) % (la + 1),
-              x = it / 4 / (lb + 1) / (la + 1);
-    axis_factor<T>(Eb + x * E1b, lb + 1, la + lb + 3, ia, jb, ty, T(2.0 * ea), T(2.0 * eb),
-                   fa + (size_t)it * FL);
-  }
-  // (read after the barriers of the first ket)
-
-  // ---- the tile's kets
-#pragma unroll 1
-  for (int jk = tile * kt; jk < jkEnd; jk++) {
-    const PairDev Q = a.pairs[a.ketBeg + jk];
-    if (Q.npp != 1) continue;  // contracted ket: rel_llss_block_kernel (block-uniform)
-    const double bound = sh_max(a.norms, P.s1, P.s2, Q.s1, Q.s2, ns) *
-                         __ldg(a.qSS + P.s1 + (size_t)P.s2 * ns) *
-                         __ldg(a.qLL + Q.s1 + (size_t)Q.s2 * ns);
-    const bool work = !a.screen || bound >= a.thresh;
-    const bool lo = a.mixed && bound < a.cut &&
-                    fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                                  __ldg(a.pairRange + a.ketBeg + jk), la + lb + lc + ld + 2, 1,
-                                  0);
-    const bool mine = work && (IS32 ? lo : !lo);
-    if (tid == 0) {
-      if (!IS32) atomicAdd(a.counters + 0, 1ull);
-      if (!IS32 && !work) atomicAdd(a.counters + 1, 1ull);
-      if (mine) atomicAdd(a.counters + (IS32 ? 2 : 3), 1ull);
-    }
-    if (!mine) continue;  // block-uniform
-    const bool dCD = Q.shA == Q.shB;
-    const double s34d = dCD ? 1.0 : 2.0, w34 = dCD ? 0.5 : 1.0;
-    const PrimPairDev& B = a.pp[Q.pp_off];
-    const T X = T(A.P[0] - B.P[0]), Y = T(A.P[1] - B.P[1]), Z = T(A.P[2] - B.P[2]);
-    const T pq = T(A.p) + T(B.p), alpha = T(A.p) * T(B.p) / pq;
-    const T pref = T(PI52X2) / sqrt(pq) * T(A.Kp) * T(B.Kp);
-    // the previous ket's readers are past the barrier that ended its loop
-    if (tid < 3)
-      hermite_E_rt<T, LMAX + 1>(lc, ld, T(B.o2p), T(B.PA[tid]), T(B.PB[tid]), Ek + tid * E1k);
-    else if (tid >= 32 && tid < 64)
-      boys_lanes<T>(L, alpha * (X * X + Y * Y + Z * Z), Fs, boysT, tid - 32);
-    for (int e = tid; e < ncd; e += RB_THREADS) Js[e] = 0.0;
-    __syncthreads();
-    const T m2a = T(-2) * alpha;
-    for (int n = L; n >= 0; n--) {
-      T* cur = Rb[n & 1];
-      const T* prv = Rb[(n + 1) & 1];
-      const int cnt = nherm(L - n);
-      for (int e = tid; e < cnt; e += RB_THREADS) {
-        int t, u, v;
-        htab_get(htab, e, t, u, v);
-        T val;
-        if (e == 0) {
-          T f = T(1);
-          for (int k = 0; k < n; k++) f *= m2a;
-          val = f * Fs[n];
-        } else if (t > 0) {
-          val = X * prv[hidx(t - 1, u, v)];
-          if (t > 1) val += T(t - 1) * prv[hidx(t - 2, u, v)];
-        } else if (u > 0) {
-          val = Y * prv[hidx(0, u - 1, v)];
-          if (u > 1) val += T(u - 1) * prv[hidx(0, u - 2, v)];
-        } else {
-          val = Z * prv[hidx(0, 0, v - 1)];
-          if (v > 1) val += T(v - 1) * prv[hidx(0, 0, v - 2)];
-        }
-        cur[e] = val;
-      }
-      if (n == L) {  // the ket factors beside the first level (Ek is complete)
-        for (int it = tid; it < 3 * (lc + 1) * (ld + 1); it += RB_THREADS) {
-          const int di = it % (ld + 1), ci = (it / (ld + 1)) % (lc + 1),
-                    x = it / (ld + 1) / (lc + 1);
-          T* f = fc + (size_t)it * FLk;
-          const int nf = axis_factor<T>(Ek + x * E1k, ld, lc + ld + 1, ci, di, 0, T(0), T(0), f);
-          for (int t = 1; t < nf; t += 2) f[t] = -f[t];
-        }
-      }
-      __syncthreads();
-    }
-    // G[cd][tuv] of every ket component pair
-    for (int e = tid; e < ncd * hb; e += RB_THREADS) {
-      int cd, h, c, d;
-      fhb.divmod(e, cd, h);
-      fnd.divmod(cd, c, d);
-      int t, u, v;
-      htab_get(htab, h, t, u, v);
-      const T* fx = fcOf(0, cart_lx(lc, c), cart_lx(ld, d));
-      const T* fy = fcOf(1, cart_ly(lc, c), cart_ly(ld, d));
-      const T* fz = fcOf(2, cart_lz(lc, c), cart_lz(ld, d));
-      const int nx = cart_lx(lc, c) + cart_lx(ld, d) + 1;
-      const int ny = cart_ly(lc, c) + cart_ly(ld, d) + 1;
-      const int nz = cart_lz(lc, c) + cart_lz(ld, d) + 1;
-      T acc = T(0);
-      for (int i = 0; i < nx; i++) {
-        if (fx[i] == T(0)) continue;
-        for (int j = 0; j < ny; j++) {
-          const T fxy = fx[i] * fy[j];
-          if (fxy == T(0)) continue;
-          acc += fxy * hdot_v(fz, nz, R, t + i, u + j, v);
-        }
-      }
-      G[e] = pref * acc;
-    }
-    __syncthreads();
-    // operator components of every (bra, ket) component element, digested
-    for (int e = tid; e < nab * ncd; e += RB_THREADS) {
-      int ab, cd, ai, bi, c, d;
-      fncd.divmod(e, ab, cd);
-      fnb.divmod(ab, ai, bi);
-      fnd.divmod(cd, c, d);
-      const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-      const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-      double m4[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int mu = 0; mu < 3; mu++)
-        for (int nu = 0; nu < 3; nu++) {
-          int op;
-          double sg;
-          op_of(mu, nu, op, sg);
-          const int tx = (mu == 0) | ((nu == 0) << 1), ty = (mu == 1) | ((nu == 1) << 1),
-                    tz = (mu == 2) | ((nu == 2) << 1);
-          m4[op] += sg * (double)bra_dot<T>(faOf(0, ax[0], bx[0], tx),
-                                 ax[0] + bx[0] + (tx & 1) + (tx >> 1) + 1,
-                                 faOf(1, ax[1], bx[1], ty),
-                                 ax[1] + bx[1] + (ty & 1) + (ty >> 1) + 1,
-                                 faOf(2, ax[2], bx[2], tz),
-                                 ax[2] + bx[2] + (tz & 1) + (tz >> 1) + 1, G + (size_t)cd * hb);
-        }
-      const int gC = Q.cA + c, gD = Q.cB + d;
-      RelCol col{gC, gD, dAB, dCD, false, s34d, w12, 1.0,
-                 __ldg(a.Xll + 2 * ((size_t)gD + (size_t)gC * nc)), {0, 0, 0, 0}};
-      double jl[4] = {0.0, 0.0, 0.0, 0.0};
-      rel_digest<1>(a, P, col, ai, bi, m4, jl);
-      if (jl[0] != 0.0) atomicAdd(Js + cd, jl[0]);
-    }
-    __syncthreads();
-    for (int cd = tid; cd < ncd; cd += RB_THREADS)
-      if (Js[cd] != 0.0)
-        atomicAdd(a.Jll + (size_t)(Q.cA + cd / nd) + (size_t)(Q.cB + cd % nd) * nc,
-                  w34 * s12d * Js[cd]);
-    __syncthreads();  // the ket's shared memory is free for the next one
-  }
-}
-
-// ---------------------------------------- GEMM form of the block kernels
-// For a single-primitive quartet (every quartet of an uncontracted basis)
-// the block kernels' work is two dense products per ket chunk:
-//   G[h][(cd, b)] = sum_h' K[h'][(cd, b)] Rm[h'][h],
-//   M[(ab, op)][(cd, b)] = sum_h H[h][(ab, op)] G[h][(cd, b)],
-// with H / K the bra / ket Hermite coefficients of every component pair
-// already combined over the derivative pairs of each operator component
-// (H[(ab, op)][tuv] = sum_{mu nu -> op} sg f_x f_y f_z), and
-// Rm[h'][h] = pref R_{t+tau, u+nu, v+phi} (ket sign folded into K).  Both
-// run as register-tiled loops over shared memory, every lane busy: a thread
-// owns a 4 x 4 tile, for the second product (one bra pair's 4 operator
-// components) x (one ket pair's 4 components; LLSS: 4 ket pairs), which is
-// then digested from registers at the reference's update sites.  A block
-// takes one bra pair and a tile of up to KT ket pairs: the bra's E tables,
-// axis factors and H are built once and stay in shared memory while the
-// block walks its kets; per ket the R recursion runs over the block from a
-// table of Hermite indices.  Same quartet set, screens
-// and digestion as the block kernels, which keep the contracted quartets
-// (and the classes whose layout does not fit).
-constexpr int RG_THREADS = 256;
-constexpr size_t RG_SMEM_MAX = 224 * 1024;
-constexpr size_t RG_SMEM_HALF = 112 * 1024;  // two blocks per SM (228 KB, 1 KB reserved each)
-
-struct RelGemmLayout {
-  int HB, HBp, HK, HR, CH, CR, CRp, NT;
-  int oH, oRm, oFk, oJs, oTuv, oScr;
-  int oEb, oFa;                 // bra phase, in the scratch area
-  int oEk, oR0, oR1, oF;        // per-ket phase, in the scratch area
-  int oK, oG;                   // per ket chunk, in the scratch area
-  int total;
-};
-__host__ __device__ inline int rg_round(int n, int m) { return (n + m - 1) / m * m; }
-// offsets and total in elements of esz bytes (8: FP64, 4: FP32 arithmetic)
-__host__ __device__ inline RelGemmLayout rel_gemm_layout(int la, int lb, int lc, int ld, int type,
-                                                         int CH, int esz) {
-  const int dK = type == 2 ? 1 : 0, NB = type == 2 ? 4 : 1;
-  const int Lb = la + lb + 2, Lk = lc + ld + 2 * dK, L = Lb + Lk;
-  const int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld);
-  const int FL = 2 * (la > lb ? la : lb) + 3, FLk = 2 * (lc > ld ? lc : ld) + 3;
-  RelGemmLayout Lo;
-  Lo.HB = nherm(Lb);
-  Lo.HBp = rg_round(Lo.HB, 4);
-  Lo.HK = nherm(Lk);
-  Lo.HR = nab * 4;
-  Lo.CH = CH;
-  Lo.CR = CH * NB;
-  Lo.CRp = rg_round(Lo.CR, 4);
-  Lo.NT = nherm(L);
-  int o = 0;
-  auto take = [&](int n) { int r = o; o += rg_round(n, 4); return r; };
-  Lo.oH = take(Lo.HB * Lo.HR);
-  Lo.oRm = take(Lo.HK * Lo.HBp);
-  Lo.oFk = take(ncd * 12 * FLk);
-  Lo.oJs = take(CH * 4 * 8 / esz);           // per-column Coulomb sums, double
-  Lo.oTuv = take((Lo.NT * 4 + esz - 1) / esz);  // packed (t, u, v) of each Hermite index, int
-  Lo.oScr = o;
-  int p = o;
-  auto takeB = [&](int n) { int r = p; p += rg_round(n, 4); return r; };
-  Lo.oEb = takeB(3 * (la + 2) * (lb + 2) * (la + lb + 3));
-  Lo.oFa = takeB(3 * (la + 1) * (lb + 1) * 4 * FL);  // per (axis, exponent pair, type)
-  int k = o;
-  auto takeK = [&](int n) { int r = k; k += rg_round(n, 4); return r; };
-  Lo.oEk = takeK(3 * (lc + 1 + dK) * (ld + 1 + dK) * (lc + ld + 1 + 2 * dK));
-  Lo.oR0 = takeK(nherm(L));
-  Lo.oR1 = takeK(nherm(L));
-  Lo.oF = takeK(L + 1);
-  int q = o;
-  auto takeC = [&](int n) { int r = q; q += rg_round(n, 4); return r; };
-  Lo.oK = takeC(Lo.HK * Lo.CRp);
-  Lo.oG = takeC(Lo.HBp * Lo.CRp);
-  Lo.total = p > k ? p : k;
-  if (q > Lo.total) Lo.total = q;
-  return Lo;
-}
-// the ket chunk: the largest whose layout leaves two blocks per SM, if that
-// is at least 4 ket pairs (or all of them); else the largest that fits at
-// all (one block per SM); 0: the class does not fit
-inline int rel_gemm_chunk(int la, int lb, int lc, int ld, int type, int esz) {
-  const int ncd = ncart(lc) * ncart(ld);
-  for (int ch = ncd; ch >= 1; ch--)
-    if ((size_t)rel_gemm_layout(la, lb, lc, ld, type, ch, esz).total * esz <= RG_SMEM_HALF) {
-      if (ch >= 4 || ch == ncd) return ch;
-      break;
-    }
-  for (int ch = ncd; ch >= 1; ch--)
-    if ((size_t)rel_gemm_layout(la, lb, lc, ld, type, ch, esz).total * esz <= RG_SMEM_MAX)
-      return ch;
-  return 0;
-}
-// four consecutive elements (16-byte aligned)
-__device__ __forceinline__ void rg_ld4(const double* p, double (&v)[4]) {
-  const double2 a = *reinterpret_cast<const double2*>(p);
-  const double2 b = *reinterpret_cast<const double2*>(p + 2);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void rg_ld4(const float* p, float (&v)[4]) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void rg_st4(double* p, double a, double b, double c, double d) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
-  reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
-}
-__device__ __forceinline__ void rg_st4(float* p, float a, float b, float c, float d) {
-  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-// ket pairs per block
-constexpr int RG_KT = 8;
-
-// T: primitive arithmetic (double; float for the small-bound quartets of a
-// mixed launch); the operator components are digested in FP64.
-template <int TYPE, typename T>
-__global__ void __launch_bounds__(RG_THREADS, 2)
-    rel_gemm_kernel(const RelLaunch a, int la, int lb, int lc, int ld, int CH) {
-  constexpr bool IS32 = sizeof(T) == 4;
-  extern __shared__ double sm[];
-  T* smT = reinterpret_cast<T*>(sm);
-  const int nTiles = (a.nKet + RG_KT - 1) / RG_KT;
-  const long long q = blockIdx.x + (long long)blockIdx.y * gridDim.x;
-  const int ib = (int)(q / nTiles), tile = (int)(q % nTiles);
-  if (ib >= a.nBra || !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;
-  const bool tri = (TYPE == 2 && a.same);  // SSSS, one class: kets jk <= ib
-  if (tri && tile * RG_KT > ib) return;
-  const PairDev P = a.pairs[a.braBeg + ib];
-  if (P.npp != 1) return;  // contracted: the block kernels
-  const int jkEnd = min(tile * RG_KT + RG_KT, tri ? ib + 1 : a.nKet);
-  const int ns = a.nShell;
-
-  constexpr int NB = (TYPE == 2) ? 4 : 1;
-  const int tid = threadIdx.x;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb, ncd = ncc * nd;
-  const int dK = (TYPE == 2) ? 1 : 0;
-  const int Lb = la + lb + 2, Lk = lc + ld + 2 * dK, L = Lb + Lk;
-  const int FL = 2 * max(la, lb) + 3, FLk = 2 * max(lc, ld) + 3;
-  const RelGemmLayout Lo = rel_gemm_layout(la, lb, lc, ld, TYPE, CH, (int)sizeof(T));
-  const int HB = Lo.HB, HBp = Lo.HBp, HK = Lo.HK, HR = Lo.HR, CRp = Lo.CRp;
-  const FastDiv fHBp(HBp), fCRp(CRp), ftr(CRp / 4), fnab(nab), fnb(nb), fnd(nd);
-  T* Hs = smT + Lo.oH;
-  T* Rm = smT + Lo.oRm;
-  T* fk = smT + Lo.oFk;
-  double* Js = reinterpret_cast<double*>(smT + Lo.oJs);
-  int* tuv = reinterpret_cast<int*>(smT + Lo.oTuv);
-  T* Eb = smT + Lo.oEb;
-  T* fa = smT + Lo.oFa;
-  T* Ek = smT + Lo.oEk;
-  T* Rb[2] = {smT + Lo.oR0, smT + Lo.oR1};
-  T* Fs = smT + Lo.oF;
-  T* Ks = smT + Lo.oK;
-  T* Gs = smT + Lo.oG;
-  const T* boysT = reinterpret_cast<const T*>(IS32 ? (const void*)a.boys32 : (const void*)a.boys);
-  const int E1b = (la + 2) * (lb + 2) * (la + lb + 3);
-  const int E1k = (lc + 1 + dK) * (ld + 1 + dK) * (lc + ld + 1 + 2 * dK);
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  const bool dAB = P.shA == P.shB;
-  const double s12d = dAB ? 1.0 : 2.0;
-  const double w12 = dAB ? 0.5 : 1.0;
-  const size_t nc = a.ncart;
-  auto unpack = [&](int h, int& t, int& u, int& v) {
-    const int w = tuv[h];
-    t = w & 255;
-    u = (w >> 8) & 255;
-    v = w >> 16;
-  };
-
-  // ---- bra phase, once per block: E tables, axis factors, H
-  const PrimPairDev& A = a.pp[P.pp_off];
-  double ea, eb;
-  pair_exps(SA, SB, a.prim, A, ea, eb);
-  if (tid < 3)
-    hermite_E_rt<T, LMAX + 1>(la + 1, lb + 1, T(A.o2p), T(A.PA[tid]), T(A.PB[tid]),
-                              Eb + tid * E1b);
-  for (int h = tid; h < Lo.NT; h += RG_THREADS) {
-    int t, u, v;
-    hinv(h, t, u, v);
-    tuv[h] = t | (u << 8) | (v << 16);
-  }
-  for (int e = tid; e < 4 * CH; e += RG_THREADS) Js[e] = 0.0;
-  __syncthreads();
-  for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += RG_THREADS) {
-    const int ty = it % 4, jb = (it / 4) % (lb + 1), ia = (it / 4 / (lb + 1)) % (la + 1),
-              x = it / 4 / (lb + 1) / (la + 1);
-    axis_factor<T>(Eb + x * E1b, lb + 1, la + lb + 3, ia, jb, ty, T(2.0 * ea), T(2.0 * eb),
-                   fa + (size_t)it * FL);
-  }
-  __syncthreads();
-  auto faOf = [&](int x, int i, int j, int ty) {
-    return fa + (size_t)(((x * (la + 1) + i) * (lb + 1) + j) * 4 + ty) * FL;
-  };
-  for (int e = tid; e < HB * HR; e += RG_THREADS) {
-    const int h = e / HR, row = e % HR, ab = row / 4, op = row % 4;
-    const int ai = ab / nb, bi = ab % nb;
-    int t, u, v;
-    unpack(h, t, u, v);
-    const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-    const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-    T val = T(0);
-    for (int mu = 0; mu < 3; mu++)
-      for (int nu = 0; nu < 3; nu++) {
-        int o2;
-        double sg;
-        op_of(mu, nu, o2, sg);
-        if (o2 != op) continue;
-        const int tx = (mu == 0) | ((nu == 0) << 1), ty = (mu == 1) | ((nu == 1) << 1),
-                  tz = (mu == 2) | ((nu == 2) << 1);
-        if (t >= ax[0] + bx[0] + (tx & 1) + (tx >> 1) + 1 ||
-            u >= ax[1] + bx[1] + (ty & 1) + (ty >> 1) + 1 ||
-            v >= ax[2] + bx[2] + (tz & 1) + (tz >> 1) + 1)
-          continue;
-        val += T(sg) * faOf(0, ax[0], bx[0], tx)[t] * faOf(1, ax[1], bx[1], ty)[u] *
-               faOf(2, ax[2], bx[2], tz)[v];
-      }
-    Hs[e] = val;
-  }
-  __syncthreads();  // H is complete; the bra scratch (Eb, fa) is free
-
-  // ---- the block's kets, one at a time
-#pragma unroll 1
-  for (int jk = tile * RG_KT; jk < jkEnd; jk++) {
-    const PairDev Q = a.pairs[a.ketBeg + jk];
-    if (Q.npp != 1) continue;  // contracted: the block kernels (block-uniform)
-    bool work, mine;
-    {
-      int s1, s2, s3, s4;
-      double q12, q34;
-      if (TYPE == 1) {
-        s1 = P.s1; s2 = P.s2; s3 = Q.s1; s4 = Q.s2;
-        q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-        q34 = __ldg(a.qLL + s3 + (size_t)s4 * ns);
-      } else {
-        const bool pRef = P.lex >= Q.lex;
-        const PairDev& R12 = pRef ? P : Q;
-        const PairDev& R34 = pRef ? Q : P;
-        s1 = R12.s1; s2 = R12.s2; s3 = R34.s1; s4 = R34.s2;
-        q12 = __ldg(a.qSS + s1 + (size_t)s2 * ns);
-        q34 = __ldg(a.qSS + s3 + (size_t)s4 * ns);
-      }
-      const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) * q12 * q34;
-      work = !a.screen || bound >= a.thresh;
-      const bool lo = a.mixed && bound < a.cut &&
-                      fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                                    __ldg(a.pairRange + a.ketBeg + jk),
-                                    la + lb + lc + ld + 2 + 2 * (TYPE == 2), 1, TYPE == 2);
-      mine = work && (IS32 ? lo : !lo);
-    }
-    if (tid == 0) {
-      if (!IS32) atomicAdd(a.counters + 0, 1ull);
-      if (!IS32 && !work) atomicAdd(a.counters + 1, 1ull);
-      if (mine) atomicAdd(a.counters + (IS32 ? 2 : 3), 1ull);
-    }
-    if (!mine) continue;  // block-uniform
-    const ShellDev SC = a.shells[Q.shA], SD = a.shells[Q.shB];
-    const bool dCD = Q.shA == Q.shB, samePQ = P.lex == Q.lex;
-    const double w34 = dCD ? 0.5 : 1.0;
-    const PrimPairDev& B = a.pp[Q.pp_off];
-    double ec, ed;
-    pair_exps(SC, SD, a.prim, B, ec, ed);
-    const T X = T(A.P[0] - B.P[0]), Y = T(A.P[1] - B.P[1]), Z = T(A.P[2] - B.P[2]);
-    const T pq = T(A.p) + T(B.p), alpha = T(A.p) * T(B.p) / pq;
-    const T pref = T(PI52X2) / sqrt(pq) * T(A.Kp) * T(B.Kp);
-    // Boys (one thread) and the ket E tables, then R level by level over the
-    // block, indices from the table
-    if (tid < 32) boys_lanes<T>(L, alpha * (X * X + Y * Y + Z * Z), Fs, boysT, tid);
-    else if (tid >= 32 && tid < 35)
-      hermite_E_rt<T, LMAX + 1>(lc + dK, ld + dK, T(B.o2p), T(B.PA[tid - 32]),
-                                T(B.PB[tid - 32]), Ek + (tid - 32) * E1k);
-    __syncthreads();
-    {
-      const T m2a = T(-2) * alpha;
-      for (int n = L; n >= 0; n--) {
-        T* cur = Rb[n & 1];
-        const T* prv = Rb[(n + 1) & 1];
-        const int cnt = nherm(L - n);
-        for (int e = tid; e < cnt; e += RG_THREADS) {
-          int t, u, v;
-          unpack(e, t, u, v);
-          T val;
-          if (e == 0) {
-            T f = T(1);
-            for (int k = 0; k < n; k++) f *= m2a;
-            val = f * Fs[n];
-          } else if (t > 0) {
-            val = X * prv[hidx(t - 1, u, v)];
-            if (t > 1) val += T(t - 1) * prv[hidx(t - 2, u, v)];
-          } else if (u > 0) {
-            val = Y * prv[hidx(0, u - 1, v)];
-            if (u > 1) val += T(u - 1) * prv[hidx(0, u - 2, v)];
-          } else {
-            val = Z * prv[hidx(0, 0, v - 1)];
-            if (v > 1) val += T(v - 1) * prv[hidx(0, 0, v - 2)];
-          }
-          cur[e] = val;
-        }
-        __syncthreads();
-      }
-    }
-    const T* R = Rb[0];
-    for (int it = tid; it < ncd * 12; it += RG_THREADS) {
-      const int cd = it / 12, x = (it % 12) / 4, ty = it % 4;
-      if (TYPE == 1 && ty) continue;
-      const int c = cd / nd, d = cd % nd;
-      const int ci = x == 0 ? cart_lx(lc, c) : (x == 1 ? cart_ly(lc, c) : cart_lz(lc, c));
-      const int di = x == 0 ? cart_lx(ld, d) : (x == 1 ? cart_ly(ld, d) : cart_lz(ld, d));
-      T* f = fk + (size_t)it * FLk;
-      const int n = axis_factor<T>(Ek + x * E1k, ld + dK, lc + ld + 2 * dK + 1, ci, di, ty,
-                                   T(2.0 * ec), T(2.0 * ed), f);
-      for (int t = 1; t < n; t += 2) f[t] = -f[t];
-    }
-    for (int e = tid; e < HK * HBp; e += RG_THREADS) {
-      int hp, h;
-      fHBp.divmod(e, hp, h);
-      T val = T(0);
-      if (h < HB) {
-        int t, u, v, t2, u2, v2;
-        unpack(h, t, u, v);
-        unpack(hp, t2, u2, v2);
-        val = pref * R[hidx(t + t2, u + u2, v + v2)];
-      }
-      Rm[e] = val;
-    }
-    __syncthreads();  // fk and Rm are complete; the per-ket scratch is free
-
-    // ---- ket chunks
-#pragma unroll 1
-    for (int cd0 = 0; cd0 < ncd; cd0 += CH) {
-      const int nch = min(CH, ncd - cd0);
-      // K[h'][(cdl, b)]
-      for (int e = tid; e < HK * CRp; e += RG_THREADS) {
-        int hp, r;
-        fCRp.divmod(e, hp, r);
-        const int cdl = r / NB, b = r % NB;
-        T val = T(0);
-        if (cdl < nch) {
-          const int cd = cd0 + cdl;
-          int c, d;
-          fnd.divmod(cd, c, d);
-          const int ci[3] = {cart_lx(lc, c), cart_ly(lc, c), cart_lz(lc, c)};
-          const int di[3] = {cart_lx(ld, d), cart_ly(ld, d), cart_lz(ld, d)};
-          int t, u, v;
-          unpack(hp, t, u, v);
-          const T* f0 = fk + (size_t)cd * 12 * FLk;
+        for (int kI = 0; kI < ki; kI++) {
+          const int cd = (outC ? kO * nd + kI : kI * nd + kO) - z.cd0;
+          if (cd < 0 || cd >= nCD) continue;
+          any = true;
+          const int gB = (outA ? P.cB : P.cA) + bI, gK = (outC ? Q.cB : Q.cA) + kI;
+          const size_t e = TYPE == 1 ? ix(gK, gB) : ix(gB, gK);
+          const Q4 d{ldz(a.Xk[0], e), ldz(a.Xk[1], e), ldz(a.Xk[2], e), ldz(a.Xk[3], e)};
+          const double* m = M + (size_t)(4 * ab) * ms + NB * cd;
           if (TYPE == 1) {
-            if (t <= ci[0] + di[0] && u <= ci[1] + di[1] && v <= ci[2] + di[2])
-              val = f0[(0 * 4) * FLk + t] * f0[(1 * 4) * FLk + u] * f0[(2 * 4) * FLk + v];
+            // (D (m0 + i f m.sigma)): per operator m_op D
+#pragma unroll
+            for (int op = 0; op < 4; op++) {
+              const double v = m[(size_t)op * ms];
+              t[op][0] += v * d.s.x; t[op][1] += v * d.s.y;
+              t[op][2] += v * d.x.x; t[op][3] += v * d.x.y;
+              t[op][4] += v * d.y.x; t[op][5] += v * d.y.y;
+              t[op][6] += v * d.z.x; t[op][7] += v * d.z.y;
+            }
           } else {
-            for (int kk = 0; kk < 3; kk++)
-              for (int ll = 0; ll < 3; ll++) {
-                int o2;
-                double sg;
-                op_of(kk, ll, o2, sg);
-                if (o2 != b) continue;
-                const int tx = (kk == 0) | ((ll == 0) << 1), ty = (kk == 1) | ((ll == 1) << 1),
-                          tz = (kk == 2) | ((ll == 2) << 1);
-                if (t >= ci[0] + di[0] + (tx & 1) + (tx >> 1) + 1 ||
-                    u >= ci[1] + di[1] + (ty & 1) + (ty >> 1) + 1 ||
-                    v >= ci[2] + di[2] + (tz & 1) + (tz >> 1) + 1)
-                  continue;
-                val += T(sg) * f0[(0 * 4 + tx) * FLk + t] * f0[(1 * 4 + ty) * FLk + u] *
-                       f0[(2 * 4 + tz) * FLk + v];
+#pragma unroll
+            for (int op = 0; op < 4; op++) {
+              const Q4 l = left_sigma(d, op, f1);
+              const double2 m01 = *reinterpret_cast<const double2*>(m + (size_t)op * ms);
+              const double2 m23 = *reinterpret_cast<const double2*>(m + (size_t)op * ms + 2);
+              const double v[4] = {m01.x, m01.y, m23.x, m23.y};
+#pragma unroll
+              for (int b = 0; b < 4; b++) {
+                t[b][0] += v[b] * l.s.x; t[b][1] += v[b] * l.s.y;
+                t[b][2] += v[b] * l.x.x; t[b][3] += v[b] * l.x.y;
+                t[b][4] += v[b] * l.y.x; t[b][5] += v[b] * l.y.y;
+                t[b][6] += v[b] * l.z.x; t[b][7] += v[b] * l.z.y;
               }
-          }
-        }
-        Ks[e] = val;
-      }
-      __syncthreads();
-      // G = K^T Rm, 4 x 4 tiles (rows of K, columns h)
-      {
-        const int tr = CRp / 4, th = HBp / 4;
-        for (int unit = tid; unit < tr * th; unit += RG_THREADS) {
-          int hq, rq;
-          ftr.divmod(unit, hq, rq);
-          const int r0 = rq * 4, h0 = hq * 4;
-          T acc[4][4];
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = T(0);
-#pragma unroll 2
-          for (int hp = 0; hp < HK; hp++) {
-            T kv[4], mv[4];
-            rg_ld4(Ks + (size_t)hp * CRp + r0, kv);
-            rg_ld4(Rm + (size_t)hp * HBp + h0, mv);
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-              for (int j = 0; j < 4; j++) acc[i][j] = fma(kv[i], mv[j], acc[i][j]);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            rg_st4(Gs + (size_t)(h0 + j) * CRp + r0, acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-          }
-        }
-      }
-      __syncthreads();
-      // M = H^T G, one 4 x 4 tile per unit, digested from registers
-      {
-        const int ngrp = (TYPE == 2) ? nch : (nch + 3) / 4;
-        for (int unit = tid; unit < nab * ngrp; unit += RG_THREADS) {
-          int grp, ab;
-          fnab.divmod(unit, grp, ab);
-          const int col0 = (TYPE == 2) ? grp * 4 : grp * 4;  // first column of the tile
-          T acc[4][4];
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = T(0);
-#pragma unroll 2
-          for (int h = 0; h < HB; h++) {
-            T hv[4], gv[4];
-            rg_ld4(Hs + (size_t)h * HR + ab * 4, hv);
-            rg_ld4(Gs + (size_t)h * CRp + col0, gv);
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-              for (int j = 0; j < 4; j++) acc[i][j] = fma(hv[i], gv[j], acc[i][j]);
-          }
-          int ai, bi;
-          fnb.divmod(ab, ai, bi);
-          auto column = [&](int cdl) {
-            int c, d;
-            fnd.divmod(cd0 + cdl, c, d);
-            const int gC = Q.cA + c, gD = Q.cB + d;
-            RelCol col{gC, gD, dAB, dCD, samePQ, dCD ? 1.0 : 2.0, w12, samePQ ? 0.5 : 1.0, 0.0,
-                       {0, 0, 0, 0}};
-            if (TYPE == 1) {
-              col.rhoLL = __ldg(a.Xll + 2 * ((size_t)gD + (size_t)gC * nc));
-            } else {
-              const size_t eDC = (size_t)gD + (size_t)gC * nc;
-              col.rvDC[0] = __ldg(a.Xss[0] + 2 * eDC);
-              col.rvDC[1] = -__ldg(a.Xss[1] + 2 * eDC + 1);
-              col.rvDC[2] = -__ldg(a.Xss[2] + 2 * eDC + 1);
-              col.rvDC[3] = -__ldg(a.Xss[3] + 2 * eDC + 1);
-            }
-            return col;
-          };
-          if (TYPE == 2) {
-            double m[16];
-#pragma unroll
-            for (int op = 0; op < 4; op++)
-#pragma unroll
-              for (int b = 0; b < 4; b++) m[op * 4 + b] = (double)acc[op][b];
-            double jl[4] = {0.0, 0.0, 0.0, 0.0};
-            rel_digest<TYPE>(a, P, column(grp), ai, bi, m, jl);
-#pragma unroll
-            for (int b = 0; b < 4; b++)
-              if (jl[b] != 0.0) atomicAdd(Js + grp * 4 + b, jl[b]);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              const int cdl = grp * 4 + k;
-              if (cdl >= nch) break;
-              double m[4] = {(double)acc[0][k], (double)acc[1][k], (double)acc[2][k],
-                             (double)acc[3][k]};
-              double jl[4] = {0.0, 0.0, 0.0, 0.0};
-              rel_digest<TYPE>(a, P, column(cdl), ai, bi, m, jl);
-              if (jl[0] != 0.0) atomicAdd(Js + cdl * 4, jl[0]);
             }
           }
         }
       }
-      __syncthreads();
-      // per-column Coulomb flush (as the block kernels)
-      for (int cdl = tid; cdl < nch; cdl += RG_THREADS) {
-        const int cd = cd0 + cdl, c = cd / nd, d = cd % nd;
-        const size_t eCD = (size_t)(Q.cA + c) + (size_t)(Q.cB + d) * nc;
-        if (TYPE == 1) {
-          if (Js[cdl * 4] != 0.0) atomicAdd(a.Jll + eCD, w34 * s12d * Js[cdl * 4]);
-        } else if (!samePQ) {
-          for (int b = 0; b < 4; b++)
-            if (Js[cdl * 4 + b] != 0.0) atomicAdd(a.Jss[b] + eCD, w34 * s12d * Js[cdl * 4 + b]);
-        }
-        for (int b = 0; b < 4; b++) Js[cdl * 4 + b] = 0.0;
-      }
-      __syncthreads();
+      if (!any) continue;
+      const Q4 k4 = right_sigmas(t, f2);
+      const int gO = (outA ? P.cA : P.cB) + bO, gP = (outC ? Q.cA : Q.cB) + kO;
+      const size_t e = TYPE == 1 ? ix(gP, gO) : ix(gO, gP);
+      const double w = TYPE == 2 && samePQ ? -0.5 : -1.0;
+      addz(a.K[0], e, k4.s, w);
+      addz(a.K[1], e, k4.x, w);
+      addz(a.K[2], e, k4.y, w);
+      addz(a.K[3], e, k4.z, w);
     }
-  }  // kets
-}
-
-// Dynamic shared-memory limit of the block kernels (SSSS (ff|ff) takes 51 KB;
-// the one LLSS layout above the limit, (ff|ff) at 165 KB, runs per thread).
-constexpr size_t REL_SMEM_MAX = 160 * 1024;
-
-// One class in one arithmetic precision: the instance in T computes the
-// quartets that precision owns (every surviving one for double without the
-// mixed mode; with it, double takes bound >= cut and float the rest).
-template <int TYPE, typename T>
-void launch_rel_prec(const RelLaunch& aIn, int la, int lb, int lc, int ld, cudaStream_t st) {
-  RelLaunch a = aIn;
-  a.skipSingle = 0;
-  const int lmax = std::max(std::max(la, lb), std::max(lc, ld));
-  if constexpr (TYPE == 2) if (lmax >= 2) {
-    // single-primitive SSSS quartets of the d and f classes: the GEMM form,
-    // when its layout fits; the other kernels skip them.  (LLSS quartets are
-    // lighter -- one ket operator -- and the LLSS kernels, with every ket
-    // component pair's Hermite sums built at once, measured faster: one Ag
-    // atom 0.31 s in the GEMM form against 0.27 s for the first of them.)
-    const int esz = (int)sizeof(T);
-    const int CH = rel_gemm_chunk(la, lb, lc, ld, TYPE, esz);
-    if (CH > 0) {
-      const size_t smem = (size_t)rel_gemm_layout(la, lb, lc, ld, TYPE, CH, esz).total * esz;
-      cudaFuncSetAttribute(rel_gemm_kernel<TYPE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)RG_SMEM_MAX);
-      const long long nb = (long long)a.nBra * ((a.nKet + RG_KT - 1) / RG_KT);
-      const unsigned gx = (unsigned)std::min<long long>(nb, 65535);
-      const unsigned gy = (unsigned)((nb + gx - 1) / gx);
-      rel_gemm_kernel<TYPE, T><<<dim3(gx, gy), RG_THREADS, smem, st>>>(a, la, lb, lc, ld, CH);
-      a.skipSingle = 1;
-    }
-  }
-  const int tiles = (a.nKet + REL_THREADS - 1) / REL_THREADS;
-  // split each quartet's ket components over enough threads to fill the GPU
-  // (~256k threads per launch), at most one component pair per thread
-  const long long quartets = (long long)a.nBra * a.nKet;
-  const int ncd = ncart(lc) * ncart(ld);
-  int nsplit = (int)std::min<long long>(ncd, std::max<long long>(1, (1 << 18) / quartets));
-  nsplit = std::max(1, std::min(nsplit, 65535 / tiles));
-  dim3 grid(a.nBra, tiles * nsplit);
-  const int lm = std::max(std::max(la, lb), std::max(lc, ld));
-  if (lm <= 1) {
-    rel_kernel<1, TYPE, T><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-    return;
-  }
-  if constexpr (TYPE == 1) {
-    // LLSS d/f classes: one block per quartet with every ket component at
-    // once, when it fits in shared memory (single-primitive quartets in
-    // their own instance); else per thread
-    const long long nq = (long long)a.nBra * a.nKet;
-    const unsigned gx = (unsigned)std::min<long long>(nq, 65535);
-    const unsigned gy = (unsigned)((nq + gx - 1) / gx);
-    const size_t smem1 = (size_t)llss_block_layout(la, lb, lc, ld, true).total * sizeof(double);
-    if (smem1 <= REL_SMEM_MAX) {
-      // always the same limit (on the current device), never one below a
-      // launch still queued
-      cudaFuncSetAttribute(rel_llss_single_kernel<T>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REL_SMEM_MAX);
-      // ket tiles only where the launch keeps ~64 blocks per SM without them
-      const int kt = (int)std::max<long long>(
-          1, std::min<long long>(LS_KT, nq / (64LL * std::max(1, a.nsm))));
-      const long long nb1 = (long long)a.nBra * ((a.nKet + kt - 1) / kt);
-      const unsigned gx1 = (unsigned)std::min<long long>(nb1, 65535);
-      const unsigned gy1 = (unsigned)((nb1 + gx1 - 1) / gx1);
-      rel_llss_single_kernel<T><<<dim3(gx1, gy1), RB_THREADS, smem1, st>>>(a, la, lb, lc, ld,
-                                                                           kt);
-      a.skipSingle = 1;
-      if (!a.contracted) return;
-    }
-    const size_t smem = (size_t)llss_block_layout(la, lb, lc, ld, false).total * sizeof(double);
-    if (smem <= REL_SMEM_MAX) {
-      cudaFuncSetAttribute(rel_llss_block_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)REL_SMEM_MAX);
-      rel_llss_block_kernel<T><<<dim3(gx, gy), RB_THREADS, smem, st>>>(a, la, lb, lc, ld);
-    } else if (lm == 2) {
-      rel_kernel<2, TYPE, T><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-    } else {
-      rel_kernel<3, TYPE, T><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-    }
-  } else {
-    // SSSS d and f classes: one block per quartet, intermediates in shared memory
-    const RelBlockLayout Lo = rel_block_layout(la, lb, lc, ld, TYPE);
-    const size_t smem = (size_t)Lo.total * sizeof(double);
-    cudaFuncSetAttribute(rel_block_kernel<TYPE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)REL_SMEM_MAX);
-    const long long nq = a.same ? (long long)a.nBra * (a.nBra + 1) / 2
-                                : (long long)a.nBra * a.nKet;
-    const unsigned gx = (unsigned)std::min<long long>(nq, 65535);
-    const unsigned gy = (unsigned)((nq + gx - 1) / gx);
-    rel_block_kernel<TYPE, T><<<dim3(gx, gy), RB_THREADS, smem, st>>>(a, la, lb, lc, ld);
   }
 }
 
 template <int TYPE>
-void launch_rel(const RelLaunch& a, int la, int lb, int lc, int ld, cudaStream_t st) {
-  if (a.nBra == 0 || a.nKet == 0) return;
-  launch_rel_prec<TYPE, double>(a, la, lb, lc, ld, st);
-  if (a.mixed) launch_rel_prec<TYPE, float>(a, la, lb, lc, ld, st);
+struct RelDig {
+  using Args = RelLaunch;
+  static constexpr int NP = 1;
+  static constexpr int ABU = 4, CDU = TYPE == 2 ? 4 : 16;  // components per 16-row tile
+  __host__ __device__ static constexpr int tb(int) { return HG_SPIN; }
+  __host__ __device__ static constexpr int tk(int) { return TYPE == 2 ? HG_SPIN : HG_PLAIN; }
+  __host__ __device__ static constexpr int rtu(int) { return 1; }
+  __host__ __device__ static constexpr int ctu(int) { return 1; }
+  static __device__ __forceinline__ void digest(const RelLaunch& a, const HgQuartet& z) {
+    rel_digest<TYPE>(a, z);
+  }
+};
+
+// One class pair: planning pass and engine, in slabs of bra pairs whose mask
+// words fit the stream's region (maskWords words of 16 B; work: its four
+// counters).
+template <int TYPE>
+cqf_status launch_rel(cqf_basis* B, const RelLaunch& aIn, int cb, int ck, uint2* masks,
+                      long long maskWords, unsigned* work, cudaStream_t st) {
+  int la, lb, lc, ld;
+  class_ls(cb, la, lb);
+  class_ls(ck, lc, ld);
+  const int kk = TYPE == 2 ? HG_SPIN : HG_PLAIN;
+  const int nTiles = (aIn.nKet + WTILE - 1) / WTILE;
+  const int slab = (int)std::max<long long>(1, maskWords / nTiles);
+  for (int ib0 = 0; ib0 < aIn.nBra; ib0 += slab) {
+    RelLaunch a = aIn;
+    a.braBeg += ib0;
+    a.braOff = ib0;
+    a.nBra = std::min(slab, aIn.nBra - ib0);
+    a.lsum = la + lb + lc + ld;
+    const long long nWords = (long long)a.nBra * nTiles;
+    int* list64 = reinterpret_cast<int*>(masks + nWords);
+    int* list32 = list64 + nWords;
+    CQF_RCUDA(cudaMemsetAsync(work, 0, 4 * sizeof(unsigned), st));
+    const unsigned gp = (unsigned)std::min<long long>(
+        ((nWords + REL_RUN - 1) / REL_RUN + 7) / 8, (long long)B->nsm * 8);
+    rel_plan_kernel<TYPE><<<gp, 256, 0, st>>>(a, masks, list64, list32, work + 2);
+    HgLaunch h{};
+    h.pairs = B->d_pairs;
+    h.pp = B->d_pp;
+    h.boys = B->d_boys64;
+    h.boys32 = B->d_boys32;
+    h.la = la; h.lb = lb; h.lc = lc; h.ld = ld;
+    h.braBeg = a.braBeg;
+    h.ketBeg = a.ketBeg;
+    h.nTiles = nTiles;
+    h.masks = masks;
+    h.list64 = list64;
+    h.list32 = list32;
+    h.lcount = work + 2;
+    h.counter = work;
+    h.bra[0] = {B->d_hg[HG_SPIN] + B->hg_beg[HG_SPIN][cb], B->cls_pp_beg[cb]};
+    h.ket[0] = {B->d_hg[kk] + B->hg_beg[kk][ck], B->cls_pp_beg[ck]};
+    CQF_RTRY(hg_launch<RelDig<TYPE>>(h, a, nWords, (long long)a.nBra * a.nKet,
+                                     B->cls_npp_max[cb] * B->cls_npp_max[ck], B->nsm, st));
+  }
+  return CQF_OK;
 }
 
 // ------------------------------------------------------------------ Gaunt
@@ -2864,12 +1421,29 @@ size_t align32(size_t n) { return (n + 31) / 32 * 32; }
 // precision / fp32_cutoff (CQF_MIXED: quartets whose screening bound is below
 // the cutoff run in FP32 arithmetic, the rest in FP64).  cnt: total,
 // screened, FP32, FP64 quartet counts, added to.
-size_t rel_ws_doubles(const cqf_basis* B) {
+size_t rel_core_doubles(const cqf_basis* B) {
   const size_t nc2 = (size_t)B->ncart * B->ncart, ns2 = (size_t)B->nshell * B->nshell;
   const size_t dc = align32(9 * 2 * nc2) + align32(13 * nc2) + align32(10 * ns2);
   // Gaunt: 20 Cartesian complex densities | 16 complex accumulators | norms
   const size_t ga = align32(20 * 2 * nc2) + align32(16 * 2 * nc2) + align32(18 * ns2);
   return std::max(dc, ga) + 64;
+}
+// Mask words of one launch stream's region: the largest class pair (either
+// orientation) up to MASK_CAP_WORDS, at least one bra row of the widest class.
+long long rel_mask_words(const cqf_basis* B) {
+  size_t need = 1, row = 1;
+  for (int cb = 0; cb < NCLS; cb++)
+    for (int ck = 0; ck < NCLS; ck++) {
+      const size_t w = ((size_t)B->cls_cnt[ck] + WTILE - 1) / WTILE;
+      row = std::max(row, w);
+      need = std::max(need, (size_t)B->cls_cnt[cb] * w);
+    }
+  return (long long)std::max(row, std::min(need, MASK_CAP_WORDS));
+}
+// The contraction's arrays, then per launch stream the masks and word lists
+// (16 B a word), then four counters each.
+size_t rel_ws_doubles(const cqf_basis* B) {
+  return rel_core_doubles(B) + (size_t)(2 * rel_mask_words(B) + 2) * (NAUX + 1);
 }
 
 // The entries a contraction type writes (the others are neither zeroed nor
@@ -3014,11 +1588,6 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
 
   RelLaunch a{};
   a.pairs = B->d_pairs;
-  a.pp = B->d_pp;
-  a.shells = B->d_shells;
-  a.prim = B->d_prim;
-  a.boys = B->d_boys64;
-  a.boys32 = B->d_boys32;
   a.pairRange = B->d_pairRange;
   a.mixed = mixed ? 1 : 0;
   a.cut = opts.fp32_cutoff;
@@ -3041,27 +1610,41 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
   a.shardIdx = opts.shard_index;
   a.shardCnt = std::max(1, opts.shard_count);
   a.counters = dcnt;
-  a.nsm = B->nsm;
-  for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck < NCLS; ck++) {
+  CQF_RTRY(hg_ensure(B, HG_SPIN));
+  if (llss) CQF_RTRY(hg_ensure(B, HG_PLAIN));
+  // class pairs round-robin over the call's stream and the auxiliary ones
+  // (they only add into the accumulators), the largest angular sums first,
+  // so that one launch's tail overlaps the next one's start
+  const long long maskWords = rel_mask_words(B);
+  uint2* masks = reinterpret_cast<uint2*>(ws + rel_core_doubles(B));
+  unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
+  CQF_RCUDA(cudaEventRecord(B->evFork, st));
+  cudaStream_t lanes[NAUX + 1] = {st};
+  for (int i = 0; i < NAUX; i++) {
+    lanes[1 + i] = B->aux[i];
+    CQF_RCUDA(cudaStreamWaitEvent(B->aux[i], B->evFork, 0));
+  }
+  int nlaunch = 0;
+  cqf_status rc = CQF_OK;
+  for (int cb = NCLS - 1; cb >= 0 && rc == CQF_OK; cb--)
+    for (int ck = NCLS - 1; ck >= 0 && rc == CQF_OK; ck--) {
       if (!llss && ck > cb) continue;
       if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
-      int la, lb, lc, ld;
-      class_ls(cb, la, lb);
-      class_ls(ck, lc, ld);
       a.braBeg = B->cls_beg[cb];
       a.nBra = B->cls_cnt[cb];
       a.ketBeg = B->cls_beg[ck];
       a.nKet = B->cls_cnt[ck];
       a.same = (cb == ck);
-      a.contracted = 0;
-      for (int i = 0; i < a.nBra && !a.contracted; i++)
-        a.contracted = B->h_pairs[a.braBeg + i].npp > 1;
-      for (int i = 0; i < a.nKet && !a.contracted; i++)
-        a.contracted = B->h_pairs[a.ketBeg + i].npp > 1;
-      if (llss) launch_rel<1>(a, la, lb, lc, ld, st);
-      else launch_rel<2>(a, la, lb, lc, ld, st);
+      const int li = nlaunch++ % (NAUX + 1);
+      uint2* mk = masks + 2 * maskWords * li;
+      rc = llss ? launch_rel<1>(B, a, cb, ck, mk, maskWords, work + 4 * li, lanes[li])
+                : launch_rel<2>(B, a, cb, ck, mk, maskWords, work + 4 * li, lanes[li]);
     }
+  for (int i = 0; i < NAUX; i++) {
+    CQF_RCUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
+    CQF_RCUDA(cudaStreamWaitEvent(st, B->evJoin[i], 0));
+  }
+  CQF_RTRY(rc);
   CQF_RCUDA(cudaGetLastError());
   auto back = [&](const double* src, int mode, double* dst) {
     rel_from_cart_kernel<<<rgrid(NN, 256), 256, 0, st>>>(src, mode, N, nc, B->d_shells,

@@ -1,0 +1,51 @@
+"""The Hermite-matrix engine (csrc/cqf_hgemm.cuh) at the sizes where its work
+split changes, against the oracle: contracted f pairs (several chunks of rows
+and columns, the integrals made again for each), long contractions (a
+quartet's primitives in batches of 32 and over several blocks), one single
+shell (tiles almost empty), and FP32 Hermite integrals.  FP64 results agree
+to 1e-11 of the largest element (sums of some 1e4 terms in another order);
+mixed ones to 1e-6 at the cutoff used."""
+import numpy as np
+import pytest
+
+import oracle as O
+from chronusq_public_b200.basis import BasisSet, Molecule, parse_gbs
+from chronusq_public_b200.contraction import (LLSS, SSSS, DirectTPI, GTODirectRelERIContraction,
+                                              TwoBodyContraction)
+from test_gpu_rel import OUTS, max_rel, rel_inputs
+
+pytestmark = pytest.mark.gpu
+
+BASES = {
+    # contracted f on two centres, and a pure s partner
+    "f2": ("He 0\nF 2 1.00\n  1.7 0.4\n  0.6 0.7\nS 1 1.00\n  0.8 1.0\n",
+           "H 0\nF 2 1.00\n  1.1 0.5\n  0.4 0.6\n"),
+    # 11 x 11 primitive pairs of s, with a contracted p
+    "long": ("He 0\nS 11 1.00\n" + "".join("  %g %g\n" % (0.12 * 2.2 ** k, 0.2 + 0.05 * k)
+                                           for k in range(11)) + "P 3 1.00\n  2.9 0.3\n"
+             "  0.9 0.6\n  0.3 0.4\n", "H 0\nS 2 1.00\n  1.9 0.3\n  0.4 0.8\n"),
+    "one": ("He 0\nS 1 1.00\n  0.9 1.0\n", "H 0\nS 1 1.00\n  0.5 1.0\n"),
+}
+
+
+def basis(name):
+    he, h = BASES[name]
+    mol = Molecule.from_angstrom([("He", 0.0, 0.0, 0.0), ("H", 0.3, -0.2, 0.9)])
+    return BasisSet.build(mol, parse_gbs("****\n%s****\n%s****\n" % (he, h)))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ctype", [LLSS, SSSS])
+@pytest.mark.parametrize("name", sorted(BASES))
+def test_engine_rel(name, ctype, precision):
+    bs = basis(name)
+    N = bs.nbasis
+    _D, X = rel_inputs(N, 61)
+    ref = O.OracleBasis(bs).rel_contract(X, ctype, True)
+    lst = [TwoBodyContraction(X[m], np.zeros((N, N), complex)) for m in range(17)]
+    c = GTODirectRelERIContraction(DirectTPI(bs))
+    c.twoBodyContract(lst, ctype, precision=precision, fp32_cutoff=1e-2)
+    s = c.last_stats
+    assert s["fp32"] + s["fp64"] + s["screened"] == s["total"]
+    for m in OUTS[ctype]:
+        assert max_rel(lst[m].AX, ref[m]) < (1e-11 if precision == "fp64" else 1e-6), m
