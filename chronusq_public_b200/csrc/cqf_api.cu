@@ -1201,6 +1201,9 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
   CQF_CUDA(cudaMallocAsync(&B->d_flags, MAXMAT * sizeof(int), B->stream));
   B->h_flags.assign(MAXMAT, 0);
   CQF_CUDA(cudaStreamSynchronize(B->stream));
+  // the engine's tables, here so that contractions (captured or no-alloc
+  // ones among them) allocate nothing
+  if (B->maxL > 2) CQF_TRY(hg_ensure(B, HG_PLAIN));
   return CQF_OK;
 }
 
@@ -1385,7 +1388,7 @@ void launch_to_cart(const cqf_basis* B, const double* X, int cplx, double* Xc, c
 
 cqf_status basis_workspace(cqf_basis* B, size_t bytes) { return ensure_ws(B, bytes); }
 
-WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts) {
+WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan) {
   const int cw = opts.is_complex ? 2 : 1;
   const size_t matN = (size_t)B->nbasis * B->nbasis * cw;
   const size_t matC = (size_t)B->ncart * B->ncart * cw;
@@ -1411,15 +1414,17 @@ WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts) {
   // FP32 copy of the Cartesian densities (mixed real builds)
   const bool mixed = opts.precision == CQF_MIXED && opts.fp32_cutoff > 0.0 && !opts.is_complex;
   L.oXc32 = take(mixed ? (matC * nMat + 1) / 2 : 0);
-  // quartet masks of the fast class kernels: one region per launch stream,
-  // as many mask words as the largest class pair needs (either orientation)
+  // quartet masks of the fast class kernels and the engine: one region per
+  // launch stream, as many mask words as the largest class pair needs (either orientation)
   // up to MASK_CAP_WORDS, and at least one bra row of the widest class;
   // larger class pairs run in slabs of bra pairs
   size_t need = 0, row = 1;
   for (int cb = 0; cb < NCLS; cb++) {
     row = std::max<size_t>(row, ((size_t)B->cls_cnt[cb] + WTILE - 1) / WTILE);
     for (int ck = 0; ck <= cb; ck++) {
-      if (opts.is_complex || !B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
+      // complex matrices: only the class pairs with f shells are planned
+      if (opts.is_complex && (!plan || cb < class_id(LMAX, 0))) continue;
+      if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
       const size_t nb = B->cls_cnt[cb], nk = B->cls_cnt[ck];
       need = std::max(need, std::max(nb * ((nk + WTILE - 1) / WTILE),
                                      nk * ((nb + WTILE - 1) / WTILE)));
@@ -1446,7 +1451,7 @@ cqf_status check_contract_args(const cqf_basis* B, const cqf_contraction* list, 
 cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
                          const cqf_opts& opts, cqf_stats* stats, double* ws, bool capture,
                          const int* d_flags_pre, const double* const* normSrc,
-                         double* pinned);
+                         double* pinned, bool plan);
 
 struct PinnedBuf {
   double* p;
@@ -1629,7 +1634,7 @@ cqf_status contract_complex_split_on(cqf_basis* B, const cqf_contraction* list, 
 cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
                          const cqf_opts& opts, cqf_stats* stats, double* ws, bool capture,
                          const int* d_flags_pre, const double* const* normSrc,
-                         double* pinned) {
+                         double* pinned, bool plan) {
   if (opts.shard_count < 1 || opts.shard_index < 0 || opts.shard_index >= opts.shard_count)
     return fail(CQF_EINVAL, "shard_index must lie in [0, shard_count)");
   cudaStream_t st = opts.stream ? (cudaStream_t)opts.stream : B->stream;
@@ -1637,7 +1642,7 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
   const int cw = opts.is_complex ? 2 : 1;
   const size_t matN = (size_t)N * N * cw, matC = (size_t)nc * nc * cw;
   const size_t ns2 = (size_t)ns * ns;
-  const WsLayout Lw = ws_layout(B, nMat, opts);
+  const WsLayout Lw = ws_layout(B, nMat, opts, plan);
   const bool host = !opts.device_pointers;
   const size_t oX = Lw.oX, oAX = Lw.oAX, oXc = Lw.oXc, oAc = Lw.oAc, oNm = Lw.oNm,
                oNmM = Lw.oNmM, oG = Lw.oG;
@@ -1766,8 +1771,9 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
   cudaStream_t lanes[NAUX + 1] = {st};
   for (int i = 0; i < NAUX; i++) lanes[1 + i] = B->aux[i];
   int nlaunch = 0;
+  cqf_status hgRc = CQF_OK;
   for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck <= cb; ck++) {
+    for (int ck = 0; ck <= cb && hgRc == CQF_OK; ck++) {
       if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
       int la, lb, lc, ld;
       class_ls(cb, la, lb);
@@ -1787,9 +1793,11 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
       if (tune) CQF_CUDA(cudaEventRecord(B->tune_ev[2 * (cb * NCLS + ck)], st));
       uint2* masks = reinterpret_cast<uint2*>(ws + Lw.oMask) + 2 * Lw.maskWords * li;
       a.braOff = 0;
-      if (!(fastOK && lm <= 2 &&
-            launch_jk_fast(a, la, lb, lc, ld, masks, (long long)Lw.maskWords, work + 4 * li,
-                           B->nsm, ls, B->blocks_per_sm[cb][ck])))
+      if (lm > 2 && Lw.maskWords > 0)
+        hgRc = launch_jk_hg(B, a, cb, ck, masks, (long long)Lw.maskWords, work + 4 * li, ls);
+      else if (!(fastOK && lm <= 2 &&
+                 launch_jk_fast(a, la, lb, lc, ld, masks, (long long)Lw.maskWords, work + 4 * li,
+                                B->nsm, ls, B->blocks_per_sm[cb][ck])))
         launch_jk_generic(a, la, lb, lc, ld, ls);
       if (tune) CQF_CUDA(cudaEventRecord(B->tune_ev[2 * (cb * NCLS + ck) + 1], st));
     }
@@ -1797,6 +1805,7 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
     CQF_CUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
     CQF_CUDA(cudaStreamWaitEvent(st, B->evJoin[i], 0));
   }
+  CQF_TRY(hgRc);
   CQF_CUDA(cudaGetLastError());
   for (int m = 0; m < nMat; m++)
     from_cart_kernel<<<grid1((size_t)N * N, 256), 256, 0, st>>>(

@@ -99,7 +99,13 @@ struct WsLayout {
   size_t oX, oAX, oXc, oAc, oNm, oNmM, oG, oNmT, oPN, oWork, oXc32, oMask, total;
   size_t maskWords;  // mask words of each launch stream's region
 };
-WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts);
+// plan = false leaves the masks of a complex contraction out (its class pairs
+// with f shells then run on the generic kernel): what the fixed scratch of
+// the no-alloc entry point falls back to.
+WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan = true);
+// J and K of a class pair with an f shell (cqf_hg_eri.cu).
+cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* masks,
+                        long long maskWords, unsigned* work, cudaStream_t st);
 cqf_status check_contract_args(const cqf_basis* B, const cqf_contraction* list, int nMat);
 // The contraction on a caller-provided device workspace of ws_layout().total
 // doubles; the caller holds B->mu and has made B's device current.
@@ -157,7 +163,7 @@ cqf_status contract_complex_split_on(cqf_basis* B, const cqf_contraction* list, 
 cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
                          const cqf_opts& opts, cqf_stats* stats, double* ws, bool capture,
                          const int* d_flags_pre, const double* const* normSrc = nullptr,
-                         double* pinned = nullptr);
+                         double* pinned = nullptr, bool plan = true);
 // Page-locked host staging buffers of host-pointer contractions, shared by
 // every basis of the process: acquire returns a buffer of at least `bytes`
 // that no other call holds (allocating one only when none fits), release

@@ -12,6 +12,7 @@
 #pragma once
 
 #include "cqf_jk_kernels.cuh"
+#include "cqf_jk_plan.cuh"
 #include "gen/cqf_gen_jk.cuh"
 
 #include <algorithm>
@@ -72,115 +73,6 @@ __device__ __forceinline__ const float* boys_rows<float>(const JKLaunch& a, int 
   return a.boys32 + (size_t)L * BOYS_NPTS * BOYS_ROW32;
 }
 
-
-// Shell-block norm maximum of a quartet in the reference's roles
-// (direct.hpp:1693-1736), with the warp-uniform bra pair P: the pair norms
-// come from the per-pair array, and the four cross terms are read from the
-// column of a bra shell (normsT holds the transpose), so a warp's lanes read
-// one column instead of 32 scattered ones.
-__device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P,
-                                             const PairDev& Q, double nP, double nQ,
-                                             bool pRef) {
-  const int ns = a.nShell;
-  double m;
-  if (pRef) {  // rows from P (uniform): B(r, c) = normsT[c + r ns]
-    const double* c1 = a.normsT + (size_t)P.s1 * ns;
-    const double* c2 = a.normsT + (size_t)P.s2 * ns;
-    m = fmax(fmax(__ldg(c1 + Q.s1), __ldg(c2 + Q.s1)), fmax(__ldg(c1 + Q.s2), __ldg(c2 + Q.s2)));
-  } else {     // rows from Q, columns from P (uniform): B(r, c) = norms[r + c ns]
-    const double* c1 = a.norms + (size_t)P.s1 * ns;
-    const double* c2 = a.norms + (size_t)P.s2 * ns;
-    m = fmax(fmax(__ldg(c1 + Q.s1), __ldg(c1 + Q.s2)), fmax(__ldg(c2 + Q.s1), __ldg(c2 + Q.s2)));
-  }
-  return fmax(m, fmax(nP, nQ));
-}
-
-// Planning pass of one class pair: for every (bra pair, tile of 32 kets) the
-// quartets that survive the Schwarz x density screen, split by precision --
-// mask.x: lanes computed in FP64, mask.y: lanes computed in FP32 (mixed
-// builds: screening bound below the cut and inside the FP32 range guard).
-// Quartet set, screens and counts are those of the reference's loop
-// (direct.hpp:1642-1805); in the same class a ket sits at or before its bra
-// (each unordered pair of pairs once).  The masks form one row-major
-// sequence of words (bra pair, ket tile); a warp takes runs of 32
-// consecutive words and appends the indices of its non-empty words to one
-// list per precision (lengths in lcount[0 / 1]), so the class kernels visit
-// only words that name quartets of their precision.
-constexpr int PLAN_RUN = 32;
-template <bool MIXED>
-__global__ void __launch_bounds__(256)
-    jk_plan_kernel(const JKLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
-                   int* __restrict__ list32, unsigned int* __restrict__ lcount) {
-  const int lane = threadIdx.x & 31;
-  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-  const int nTiles = (a.nKet + WTILE - 1) / WTILE;
-  const int nWords = a.nBra * nTiles;
-  const int nRuns = (nWords + PLAN_RUN - 1) / PLAN_RUN;
-  const double cut = MIXED ? a.fp32_cut : 0.0;
-  unsigned long long cVis = 0, cScr = 0, c32 = 0, c64 = 0;
-  for (int run = gw; run < nRuns; run += nw) {
-    int my64 = -1, my32 = -1, n64 = 0, n32 = 0;
-    const int wEnd = min((run + 1) * PLAN_RUN, nWords);
-    for (int word = run * PLAN_RUN; word < wEnd; word++) {
-      const int ib = word / nTiles, tile = word - ib * nTiles;
-      unsigned b64 = 0u, b32 = 0u;
-      const int ibc = ib + a.braOff;  // the bra's position in its class
-      // else: no quartet in this word (above the diagonal, or another shard's bra)
-      if (!(a.same && tile * WTILE > ibc) && in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) {
-        const int jk = tile * WTILE + lane;
-        const PairDev P = a.pairs[a.braBeg + ib];
-        const bool visited = jk < a.nKet && !(a.same && jk > ibc);
-        const double tileMax = __ldg(a.maxNorm) * P.Q * __ldg(a.qWin + a.ketBeg + tile * WTILE);
-        bool screened = false, w32 = false;
-        if (a.screen && tileMax < a.thresh) {
-          screened = true;
-        } else if (visited && a.screen) {
-          const PairDev Q = a.pairs[a.ketBeg + jk];
-          const bool pRef = P.lex >= Q.lex;
-          const double bound = sh_max_bra(a, P, Q, __ldg(a.pairNorm + a.braBeg + ib),
-                                          __ldg(a.pairNorm + a.ketBeg + jk), pRef) * P.Q * Q.Q;
-          screened = bound < a.thresh;
-          w32 = MIXED && !screened && bound < cut &&
-                fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                              __ldg(a.pairRange + a.ketBeg + jk), a.lsum, 0, 0);
-        }  // without the screen every quartet runs in FP64
-        const unsigned bv = __ballot_sync(0xffffffffu, visited);
-        const unsigned bs = __ballot_sync(0xffffffffu, visited && screened);
-        b32 = __ballot_sync(0xffffffffu, visited && !screened && w32);
-        b64 = bv & ~bs & ~b32;
-        cVis += __popc(bv);
-        cScr += __popc(bs);
-        c32 += __popc(b32);
-        c64 += __popc(b64);
-      }
-      if (lane == 0) masks[word] = make_uint2(b64, b32);
-      if (b64) {
-        if (lane == n64) my64 = word;
-        n64++;
-      }
-      if (b32) {
-        if (lane == n32) my32 = word;
-        n32++;
-      }
-    }
-    unsigned int base64 = 0, base32 = 0;
-    if (lane == 0) {
-      if (n64) base64 = atomicAdd(lcount + 0, (unsigned)n64);
-      if (n32) base32 = atomicAdd(lcount + 1, (unsigned)n32);
-    }
-    base64 = __shfl_sync(0xffffffffu, base64, 0);
-    base32 = __shfl_sync(0xffffffffu, base32, 0);
-    if (lane < n64) list64[base64 + lane] = my64;
-    if (lane < n32) list32[base32 + lane] = my32;
-  }
-  if (lane == 0) {
-    if (cVis) atomicAdd(a.counters + 0, cVis);
-    if (cScr) atomicAdd(a.counters + 1, cScr);
-    if (c32) atomicAdd(a.counters + 2, c32);
-    if (c64) atomicAdd(a.counters + 3, c64);
-  }
-}
 
 // Position of the n-th (0-based) set bit of m (n < popc(m)).
 __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
@@ -377,15 +269,10 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
       c.braOff = b.braOff + ib0;
       cudaMemsetAsync(work, 0, 4 * sizeof(unsigned int), st);
       const long long nWords = (long long)c.nBra * nTiles;
-      const long long nRuns = (nWords + PLAN_RUN - 1) / PLAN_RUN;
-      const unsigned gp = (unsigned)std::min<long long>((nRuns + 7) / 8, (long long)nsm * 8);
       // word lists: FP64 then FP32, nWords entries each; counts in work[2..3]
       int* list64 = reinterpret_cast<int*>(masks + nWords);
       int* list32 = list64 + nWords;
-      if (mixed)
-        jk_plan_kernel<true><<<gp, 256, 0, st>>>(c, masks, list64, list32, work + 2);
-      else
-        jk_plan_kernel<false><<<gp, 256, 0, st>>>(c, masks, list64, list32, work + 2);
+      launch_jk_plan(c, mixed, masks, list64, list32, work + 2, nsm, st);
       constexpr int WPB = JK_THREADS / 32;
       auto grid = [&](long long items) {
         return (unsigned)std::max<long long>(

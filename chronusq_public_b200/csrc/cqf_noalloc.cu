@@ -87,8 +87,11 @@ extern "C" cqf_status cqf_two_body_contract_noalloc(cqf_basis* B, const cqf_cont
   bool allHer = true;
   std::vector<cqf_contraction> list = cqf::normalized_list(listIn, nMat, &allHer);
   const bool split = allHer && cqf::split_eligible(B, list.data(), nMat, opts);
+  // without the masks of complex contractions with f shells where they do
+  // not fit (those class pairs then take the generic kernel)
+  const bool plan = split || cqf::ws_layout(B, nMat, opts).total <= kScratchDoubles;
   const size_t need = split ? cqf::complex_split_ws_doubles(B, list.data(), nMat, opts)
-                            : cqf::ws_layout(B, nMat, opts).total;
+                            : cqf::ws_layout(B, nMat, opts, plan).total;
   if (need > kScratchDoubles) {
     char msg[256];
     std::snprintf(msg, sizeof msg,
@@ -105,5 +108,6 @@ extern "C" cqf_status cqf_two_body_contract_noalloc(cqf_basis* B, const cqf_cont
   s = scratch_address(B->device, &ws);
   if (s != CQF_OK) return s;
   if (split) return cqf::contract_complex_split_on(B, list.data(), nMat, opts, stats, ws);
-  return cqf::contract_core(B, list.data(), nMat, opts, stats, ws, false, nullptr);
+  return cqf::contract_core(B, list.data(), nMat, opts, stats, ws, false, nullptr, nullptr,
+                            nullptr, plan);
 }

@@ -23,6 +23,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "cqf_hgemm.cuh"
 #include "cqf_internal.hpp"
 
 namespace {
@@ -243,7 +244,15 @@ unsigned long long cqf_fock_footprint(const cqf_shell* shells, int nshell) {
   const unsigned long long ws =
       8 * (2 * nmat * N * N + 2 * nmat * nc * nc + (nmat + 1) * ns * ns) + 4 * nmat * nc * nc +
       masks;
-  return pairs + ws;
+  // bases with f shells hold the Hermite-matrix engine's tables
+  unsigned long long maxl = 0, tabs = 0;
+  for (int s = 0; s < nshell; s++) maxl = std::max<unsigned long long>(maxl, shells[s].l);
+  if (maxl > 2)
+    for (int s = 0; s < nshell; s++)
+      for (int t = 0; t <= s; t++)
+        tabs += 8ull * cqf::hg_size(cqf::HG_PLAIN, shells[s].l, shells[t].l) *
+                std::max(0, shells[s].nprim) * std::max(0, shells[t].nprim);
+  return pairs + ws + tabs;
 }
 
 cqf_status cqf_server_create(const cqf_server_opts* opts, cqf_server** out) {

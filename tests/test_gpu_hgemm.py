@@ -10,8 +10,9 @@ import pytest
 
 import oracle as O
 from chronusq_public_b200.basis import BasisSet, Molecule, parse_gbs
-from chronusq_public_b200.contraction import (LLSS, SSSS, DirectTPI, GTODirectRelERIContraction,
-                                              TwoBodyContraction)
+from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, LLSS, SSSS, DirectTPI,
+                                              GTODirectRelERIContraction,
+                                              GTODirectTPIContraction, TwoBodyContraction)
 from test_gpu_rel import OUTS, max_rel, rel_inputs
 
 pytestmark = pytest.mark.gpu
@@ -24,6 +25,11 @@ BASES = {
     "long": ("He 0\nS 11 1.00\n" + "".join("  %g %g\n" % (0.12 * 2.2 ** k, 0.2 + 0.05 * k)
                                            for k in range(11)) + "P 3 1.00\n  2.9 0.3\n"
              "  0.9 0.6\n  0.3 0.4\n", "H 0\nS 2 1.00\n  1.9 0.3\n  0.4 0.8\n"),
+    # f beside an s of 8 primitives (64 x 64 primitive quartets), p, d, f
+    "mix": ("He 0\nS 8 1.00\n" + "".join("  %g %g\n" % (0.15 * 2.6 ** k, 0.2 + 0.1 * k)
+                                          for k in range(8)) + "F 1 1.00\n  1.3 1.0\n",
+            "H 0\nS 2 1.00\n  1.9 0.3\n  0.4 0.8\nP 1 1.00\n  0.7 1.0\nD 1 1.00\n  0.9 1.0\n"
+            "F 1 1.00\n  0.8 1.0\n"),
     "one": ("He 0\nS 1 1.00\n  0.9 1.0\n", "H 0\nS 1 1.00\n  0.5 1.0\n"),
 }
 
@@ -49,3 +55,28 @@ def test_engine_rel(name, ctype, precision):
     assert s["fp32"] + s["fp64"] + s["screened"] == s["total"]
     for m in OUTS[ctype]:
         assert max_rel(lst[m].AX, ref[m]) < (1e-11 if precision == "fp64" else 1e-6), m
+
+
+@pytest.mark.parametrize("kind", ["real", "real_nonher", "complex", "complex_nonher", "mixed"])
+@pytest.mark.parametrize("name", ["f2", "mix"])
+def test_engine_jk(name, kind):
+    """J and K of bases with f shells: every Hermitian / complex flavour and
+    mixed precision (three matrices a call)."""
+    bs = basis(name)
+    N = bs.nbasis
+    rng = np.random.default_rng(62)
+    cplx, her = kind.startswith("complex"), not kind.endswith("nonher")
+    mats = []
+    for _ in range(3):
+        A = 0.1 * rng.standard_normal((N, N))
+        if cplx:
+            A = A + 0.1j * rng.standard_normal((N, N))
+        mats.append(np.asfortranarray(A + A.conj().T if her else A))
+    types = [COULOMB, EXCHANGE, EXCHANGE]
+    ref = O.OracleBasis(bs).contract(mats, [int(her)] * 3, types)
+    out = [np.zeros((N, N), mats[0].dtype, order="F") for _ in mats]
+    c = GTODirectTPIContraction(DirectTPI(bs))
+    c.twoBodyContract([TwoBodyContraction(m, o, her, t) for m, o, t in zip(mats, out, types)],
+                      precision="mixed" if kind == "mixed" else "fp64", fp32_cutoff=1e-3)
+    for o, r in zip(out, ref):
+        assert max_rel(o, np.asarray(r)) < (1e-6 if kind == "mixed" else 1e-11)
