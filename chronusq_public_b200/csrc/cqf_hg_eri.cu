@@ -157,42 +157,19 @@ cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* m
   class_ls(ck, lc, ld);
   a.lsum = la + lb + lc + ld;
   const bool mixed = a.precision == 1 && a.fp32_cut > 0.0;
-  const int nTiles = (a.nKet + WTILE - 1) / WTILE;
-  const int slab = (int)std::max<long long>(1, maskWords / nTiles);
-  for (int ib0 = 0; ib0 < a.nBra; ib0 += slab) {
+  auto plan = [&](int ib0, int n, uint2* mk, int* list64, int* list32, unsigned* lcount,
+                  unsigned) {
     JKLaunch c = a;
     c.braBeg = a.braBeg + ib0;
-    c.nBra = std::min(slab, a.nBra - ib0);
+    c.nBra = n;
     c.braOff = ib0;
-    const long long nWords = (long long)c.nBra * nTiles;
-    int* list64 = reinterpret_cast<int*>(masks + nWords);
-    int* list32 = list64 + nWords;
-    cudaMemsetAsync(work, 0, 4 * sizeof(unsigned), st);
-    launch_jk_plan(c, mixed, masks, list64, list32, work + 2, B->nsm, st);
-    HgLaunch h{};
-    h.pairs = a.pairs;
-    h.pp = a.pp;
-    h.boys = a.boys64;
-    h.boys32 = a.boys32;
-    h.la = la; h.lb = lb; h.lc = lc; h.ld = ld;
-    h.braBeg = c.braBeg;
-    h.ketBeg = c.ketBeg;
-    h.nTiles = nTiles;
-    h.masks = masks;
-    h.list64 = list64;
-    h.list32 = list32;
-    h.lcount = work + 2;
-    h.counter = work;
-    h.bra[0] = {B->d_hg[HG_PLAIN] + B->hg_beg[HG_PLAIN][cb], B->cls_pp_beg[cb]};
-    h.ket[0] = {B->d_hg[HG_PLAIN] + B->hg_beg[HG_PLAIN][ck], B->cls_pp_beg[ck]};
-    const long long nq = (long long)c.nBra * c.nKet;
-    const int np = B->cls_npp_max[cb] * B->cls_npp_max[ck];
-    const cqf_status s =
-        a.cplx ? hg_launch<EriDig<true>>(h, c, nWords, nq, np, B->nsm, st)
-               : hg_launch<EriDig<false>>(h, c, nWords, nq, np, B->nsm, st);
-    if (s != CQF_OK) return s;
-  }
-  return CQF_OK;
+    launch_jk_plan(c, mixed, mk, list64, list32, lcount, B->nsm, st);
+  };
+  const HgRegion r{masks, maskWords, work};
+  return a.cplx ? hg_contract<EriDig<true>>(B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a,
+                                            st, plan)
+                : hg_contract<EriDig<false>>(B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a,
+                                             st, plan);
 }
 
 }  // namespace cqf

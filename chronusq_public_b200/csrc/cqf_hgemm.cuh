@@ -457,7 +457,75 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
+// Planning pass over the words (bra pair, 32 kets) of nBra x nKet quartets:
+// f(ib, jk, work, lo) returns whether quartet (ib, jk) exists and sets
+// whether it is computed, and with FP32 Hermite integrals.  Masks, lists of
+// non-empty words (lengths in lcount[0 / 1], zero on entry) and the counters
+// visited / screened / FP32 / FP64; the layout of jk_plan_kernel.
+template <class F>
+__device__ __forceinline__ void hg_plan(int nBra, int nKet, uint2* __restrict__ masks,
+                                        int* __restrict__ list64, int* __restrict__ list32,
+                                        unsigned* __restrict__ lcount,
+                                        unsigned long long* counters, F f) {
+  const int lane = threadIdx.x & 31;
+  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  const int nTiles = (nKet + WTILE - 1) / WTILE, nWords = nBra * nTiles;
+  unsigned long long cVis = 0, cScr = 0, c32 = 0, c64 = 0;
+  for (int run = gw; run * 32 < nWords; run += nw) {
+    int my64 = -1, my32 = -1, n64 = 0, n32 = 0;
+    const int wEnd = min((run + 1) * 32, nWords);
+    for (int word = run * 32; word < wEnd; word++) {
+      const int ib = word / nTiles, jk = (word - ib * nTiles) * WTILE + lane;
+      bool work = false, lo = false;
+      const bool visited = jk < nKet && f(ib, jk, work, lo);
+      work = work && visited;
+      const unsigned bv = __ballot_sync(0xffffffffu, visited);
+      const unsigned bw = __ballot_sync(0xffffffffu, work);
+      const unsigned b32 = __ballot_sync(0xffffffffu, work && lo), b64 = bw & ~b32;
+      cVis += __popc(bv);
+      cScr += __popc(bv & ~bw);
+      c32 += __popc(b32);
+      c64 += __popc(b64);
+      if (lane == 0) masks[word] = make_uint2(b64, b32);
+      if (b64) {
+        if (lane == n64) my64 = word;
+        n64++;
+      }
+      if (b32) {
+        if (lane == n32) my32 = word;
+        n32++;
+      }
+    }
+    unsigned base64 = 0, base32 = 0;
+    if (lane == 0) {
+      if (n64) base64 = atomicAdd(lcount + 0, (unsigned)n64);
+      if (n32) base32 = atomicAdd(lcount + 1, (unsigned)n32);
+    }
+    base64 = __shfl_sync(0xffffffffu, base64, 0);
+    base32 = __shfl_sync(0xffffffffu, base32, 0);
+    if (lane < n64) list64[base64 + lane] = my64;
+    if (lane < n32) list32[base32 + lane] = my32;
+  }
+  if (lane == 0) {
+    if (cVis) atomicAdd(counters + 0, cVis);
+    if (cScr) atomicAdd(counters + 1, cScr);
+    if (c32) atomicAdd(counters + 2, c32);
+    if (c64) atomicAdd(counters + 3, c64);
+  }
+}
+
 // ---------------------------------------------------------- host side
+// The engine on nBra x nKet quartets of class pair (cb | ck) in slabs of bra
+// pairs whose mask words fit the stream's region (maskWords words of 16 B;
+// work: its four counters).  plan(ib0, n, masks, list64, list32, lcount,
+// grid) launches the planning pass on bra pairs [ib0, ib0 + n) of the class;
+// digest arguments may depend on the slab: args(ib0, n).
+struct HgRegion {
+  uint2* masks;
+  long long maskWords;
+  unsigned* work;
+};
 // Chunk of rows and columns: as few chunks as fit in the shared memory of
 // two blocks per SM, else of one (the R cube and the recursion buffers of
 // the f classes take up to 60 KB by themselves); 0 rows when nothing fits.
@@ -530,6 +598,48 @@ inline cqf_status hg_launch(HgLaunch a, const typename D::Args& args, long long 
   const unsigned grid =
       (unsigned)std::max<long long>(1, std::min(slots, nWords * a.nsub * a.parts));
   hg_kernel<D><<<grid, 32 * W, smem, st>>>(a, args);
+  return CQF_OK;
+}
+
+template <class D, class Plan>
+inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, int nBra, int ketBeg,
+                              int nKet, const HgRegion& r, const typename D::Args& args,
+                              cudaStream_t st, Plan plan) {
+  HgLaunch h{};
+  h.pairs = B->d_pairs;
+  h.pp = B->d_pp;
+  h.boys = B->d_boys64;
+  h.boys32 = B->d_boys32;
+  class_ls(cb, h.la, h.lb);
+  class_ls(ck, h.lc, h.ld);
+  h.ketBeg = ketBeg;
+  h.nTiles = (nKet + WTILE - 1) / WTILE;
+  h.masks = r.masks;
+  h.lcount = r.work + 2;
+  h.counter = r.work;
+  for (int q = 0; q < D::NP; q++) {
+    const int tb = D::tb(q), tk = D::tk(q);
+    h.bra[q] = {B->d_hg[tb] + B->hg_beg[tb][cb], B->cls_pp_beg[cb]};
+    h.ket[q] = {B->d_hg[tk] + B->hg_beg[tk][ck], B->cls_pp_beg[ck]};
+  }
+  const int slab = (int)std::max<long long>(1, r.maskWords / h.nTiles);
+  for (int ib0 = 0; ib0 < nBra; ib0 += slab) {
+    const int n = std::min(slab, nBra - ib0);
+    const long long nWords = (long long)n * h.nTiles;
+    int* list64 = reinterpret_cast<int*>(r.masks + nWords);
+    int* list32 = list64 + nWords;
+    h.list64 = list64;
+    h.list32 = list32;
+    h.braBeg = braBeg + ib0;
+    if (cudaMemsetAsync(r.work, 0, 4 * sizeof(unsigned), st) != cudaSuccess)
+      return fail(CQF_ECUDA, "hg_contract: counters");
+    const unsigned gp =
+        (unsigned)std::min<long long>(((nWords + 31) / 32 + 7) / 8, (long long)B->nsm * 8);
+    plan(ib0, n, r.masks, list64, list32, r.work + 2, gp);
+    const cqf_status s = hg_launch<D>(h, args, nWords, (long long)n * nKet,
+                                      B->cls_npp_max[cb] * B->cls_npp_max[ck], B->nsm, st);
+    if (s != CQF_OK) return s;
+  }
   return CQF_OK;
 }
 

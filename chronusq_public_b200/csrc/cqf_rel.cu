@@ -144,72 +144,31 @@ constexpr int REL_THREADS = 64;
 // TYPE 1: LLSS (bra = SS pair, differentiated; ket = LL pair), all
 // (bra, ket) combinations (direct4C_libcint.hpp:907-929).
 // TYPE 2: SSSS, unique quartets of pairs (:2018-2047).
-constexpr int REL_RUN = 32;
 template <int TYPE>
 __global__ void __launch_bounds__(256)
     rel_plan_kernel(const RelLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
                     int* __restrict__ list32, unsigned* __restrict__ lcount) {
-  const int lane = threadIdx.x & 31, ns = a.nShell;
-  const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-  const int nTiles = (a.nKet + WTILE - 1) / WTILE, nWords = a.nBra * nTiles;
-  unsigned long long cVis = 0, cScr = 0, c32 = 0, c64 = 0;
-  for (int run = gw; run * REL_RUN < nWords; run += nw) {
-    int my64 = -1, my32 = -1, n64 = 0, n32 = 0;
-    const int wEnd = min((run + 1) * REL_RUN, nWords);
-    for (int word = run * REL_RUN; word < wEnd; word++) {
-      const int ib = word / nTiles, jk = (word - ib * nTiles) * WTILE + lane;
-      const bool visited = jk < a.nKet && !(TYPE == 2 && a.same && jk > ib + a.braOff) &&
-                           in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt);
-      bool work = false, lo = false;
-      if (visited) {
-        const PairDev P = a.pairs[a.braBeg + ib], Q = a.pairs[a.ketBeg + jk];
-        const bool pRef = TYPE == 1 || P.lex >= Q.lex;
-        const int s1 = pRef ? P.s1 : Q.s1, s2 = pRef ? P.s2 : Q.s2;
-        const int s3 = pRef ? Q.s1 : P.s1, s4 = pRef ? Q.s2 : P.s2;
-        // shMax * Q12 * Q34 < thresh (:947-948, :2059-2061)
-        const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) *
-                             __ldg(a.qSS + P.s1 + (size_t)P.s2 * ns) *
-                             __ldg((TYPE == 1 ? a.qLL : a.qSS) + Q.s1 + (size_t)Q.s2 * ns);
-        work = !a.screen || bound >= a.thresh;
-        lo = work && a.mixed && bound < a.cut &&
-             fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
-                           __ldg(a.pairRange + a.ketBeg + jk), a.lsum + (TYPE == 2 ? 4 : 2), 1,
-                           TYPE == 2);
-      }
-      const unsigned bv = __ballot_sync(0xffffffffu, visited);
-      const unsigned bw = __ballot_sync(0xffffffffu, work);
-      const unsigned b32 = __ballot_sync(0xffffffffu, lo), b64 = bw & ~b32;
-      cVis += __popc(bv);
-      cScr += __popc(bv & ~bw);
-      c32 += __popc(b32);
-      c64 += __popc(b64);
-      if (lane == 0) masks[word] = make_uint2(b64, b32);
-      if (b64) {
-        if (lane == n64) my64 = word;
-        n64++;
-      }
-      if (b32) {
-        if (lane == n32) my32 = word;
-        n32++;
-      }
-    }
-    unsigned base64 = 0, base32 = 0;
-    if (lane == 0) {
-      if (n64) base64 = atomicAdd(lcount + 0, (unsigned)n64);
-      if (n32) base32 = atomicAdd(lcount + 1, (unsigned)n32);
-    }
-    base64 = __shfl_sync(0xffffffffu, base64, 0);
-    base32 = __shfl_sync(0xffffffffu, base32, 0);
-    if (lane < n64) list64[base64 + lane] = my64;
-    if (lane < n32) list32[base32 + lane] = my32;
-  }
-  if (lane == 0) {
-    if (cVis) atomicAdd(a.counters + 0, cVis);
-    if (cScr) atomicAdd(a.counters + 1, cScr);
-    if (c32) atomicAdd(a.counters + 2, c32);
-    if (c64) atomicAdd(a.counters + 3, c64);
-  }
+  const int ns = a.nShell;
+  hg_plan(a.nBra, a.nKet, masks, list64, list32, lcount, a.counters,
+          [&](int ib, int jk, bool& work, bool& lo) {
+            if ((TYPE == 2 && a.same && jk > ib + a.braOff) ||
+                !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt))
+              return false;
+            const PairDev P = a.pairs[a.braBeg + ib], Q = a.pairs[a.ketBeg + jk];
+            const bool pRef = TYPE == 1 || P.lex >= Q.lex;
+            const int s1 = pRef ? P.s1 : Q.s1, s2 = pRef ? P.s2 : Q.s2;
+            const int s3 = pRef ? Q.s1 : P.s1, s4 = pRef ? Q.s2 : P.s2;
+            // shMax * Q12 * Q34 < thresh (:947-948, :2059-2061)
+            const double bound = sh_max(a.norms, s1, s2, s3, s4, ns) *
+                                 __ldg(a.qSS + P.s1 + (size_t)P.s2 * ns) *
+                                 __ldg((TYPE == 1 ? a.qLL : a.qSS) + Q.s1 + (size_t)Q.s2 * ns);
+            work = !a.screen || bound >= a.thresh;
+            lo = work && a.mixed && bound < a.cut &&
+                 fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
+                               __ldg(a.pairRange + a.ketBeg + jk),
+                               a.lsum + (TYPE == 2 ? 4 : 2), 1, TYPE == 2);
+            return true;
+          });
 }
 
 // left product (i f)^[a > 0] sigma_a d of a Pauli quaternion: a permutation
@@ -390,60 +349,27 @@ struct RelDig {
   }
 };
 
-// One class pair: planning pass and engine, in slabs of bra pairs whose mask
-// words fit the stream's region (maskWords words of 16 B; work: its four
-// counters).
+// One class pair: planning pass and engine.
 template <int TYPE>
-cqf_status launch_rel(cqf_basis* B, const RelLaunch& aIn, int cb, int ck, uint2* masks,
-                      long long maskWords, unsigned* work, cudaStream_t st) {
-  int la, lb, lc, ld;
-  class_ls(cb, la, lb);
-  class_ls(ck, lc, ld);
-  const int kk = TYPE == 2 ? HG_SPIN : HG_PLAIN;
-  const int nTiles = (aIn.nKet + WTILE - 1) / WTILE;
-  const int slab = (int)std::max<long long>(1, maskWords / nTiles);
-  for (int ib0 = 0; ib0 < aIn.nBra; ib0 += slab) {
-    RelLaunch a = aIn;
-    a.braBeg += ib0;
-    a.braOff = ib0;
-    a.nBra = std::min(slab, aIn.nBra - ib0);
-    a.lsum = la + lb + lc + ld;
-    const long long nWords = (long long)a.nBra * nTiles;
-    int* list64 = reinterpret_cast<int*>(masks + nWords);
-    int* list32 = list64 + nWords;
-    CQF_RCUDA(cudaMemsetAsync(work, 0, 4 * sizeof(unsigned), st));
-    const unsigned gp = (unsigned)std::min<long long>(
-        ((nWords + REL_RUN - 1) / REL_RUN + 7) / 8, (long long)B->nsm * 8);
-    rel_plan_kernel<TYPE><<<gp, 256, 0, st>>>(a, masks, list64, list32, work + 2);
-    HgLaunch h{};
-    h.pairs = B->d_pairs;
-    h.pp = B->d_pp;
-    h.boys = B->d_boys64;
-    h.boys32 = B->d_boys32;
-    h.la = la; h.lb = lb; h.lc = lc; h.ld = ld;
-    h.braBeg = a.braBeg;
-    h.ketBeg = a.ketBeg;
-    h.nTiles = nTiles;
-    h.masks = masks;
-    h.list64 = list64;
-    h.list32 = list32;
-    h.lcount = work + 2;
-    h.counter = work;
-    h.bra[0] = {B->d_hg[HG_SPIN] + B->hg_beg[HG_SPIN][cb], B->cls_pp_beg[cb]};
-    h.ket[0] = {B->d_hg[kk] + B->hg_beg[kk][ck], B->cls_pp_beg[ck]};
-    CQF_RTRY(hg_launch<RelDig<TYPE>>(h, a, nWords, (long long)a.nBra * a.nKet,
-                                     B->cls_npp_max[cb] * B->cls_npp_max[ck], B->nsm, st));
-  }
-  return CQF_OK;
+cqf_status launch_rel(cqf_basis* B, const RelLaunch& a, int cb, int ck, const HgRegion& r,
+                      cudaStream_t st) {
+  return hg_contract<RelDig<TYPE>>(
+      B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, st,
+      [&](int ib0, int n, uint2* masks, int* list64, int* list32, unsigned* lcount, unsigned gp) {
+        RelLaunch c = a;
+        c.braBeg += ib0;
+        c.braOff = ib0;
+        c.nBra = n;
+        rel_plan_kernel<TYPE><<<gp, 256, 0, st>>>(c, masks, list64, list32, lcount);
+      });
 }
 
 // ------------------------------------------------------------------ Gaunt
 // The Gaunt term -alpha_1.alpha_2 / r12 (direct4C_libcint.hpp:2833-3907).
 // The reference runs over unordered pairs of (differentiated, other) shell
 // pairs X = (s2, s1), Y = (s3, s4) with the integrals (m d_j n | d_l k l).
-// Here a thread takes an unordered quartet of unordered significant pairs
-// {P, Q} (P = (A, B), Q = (C, D)) and computes, per Cartesian element, the
-// 36 blocks (A B with d_j on A or B | C D with d_l on C or D) at once: the
+// Here an unordered quartet of unordered significant pairs {P, Q}
+// (P = (A, B), Q = (C, D)) gives, per Cartesian element, the 36 blocks (A B with d_j on A or B | C D with d_l on C or D) at once: the
 // four (or, for P = Q, three) reference quartets {X, Y} the placements
 // make, each screened on its own by shMax Q^G(X) Q^G(Y).  Per element and
 // surviving quartet, in the reference's orientation (X >= Y as (deriv,
@@ -464,7 +390,7 @@ struct GauntLaunch {
   const ShellDev* shells;
   const double* prim;
   const double* boys;
-  int braBeg, nBra, ketBeg, nKet, same;
+  int braBeg, nBra, braOff, ketBeg, nKet, same;
   int screen;
   double thresh;
   const double* norms;  // max shell-block norms of the 16 exchange densities
@@ -482,10 +408,6 @@ struct GauntLaunch {
   int shardIdx, shardCnt;  // bra pairs p with p % shardCnt == shardIdx only
   unsigned long long* counters;
 };
-
-// bra component pairs per unit of work (the accumulator holds 36 blocks
-// of each): a whole (pp) or (dd) pair, a fifth of an (ff) one
-__host__ __device__ constexpr int gaunt_abch(int lm) { return lm <= 1 ? 9 : (lm == 2 ? 36 : 20); }
 
 struct GInv {
   double T[3][3], t, tau[3], S[3][3];
@@ -753,39 +675,99 @@ __device__ void gauge_sites(const GauntLaunch& a, const GVd& V, const GVd& Vt, i
 // accumulator holds 7 x 36 blocks of each)
 __host__ __device__ constexpr int gauge_abch(int lm) { return lm <= 2 ? 9 : 4; }
 
+// The reference quartets of {P, Q} that survive their own screen: bit
+// 2 pb + pk, derivative on B (pb) / D (pk) instead of A / C.
+__device__ __forceinline__ unsigned gaunt_alive(const GauntLaunch& a, const PairDev& P,
+                                                const PairDev& Q) {
+  const int ns = a.nShell;
+  const double shMax = sh_max(a.norms, P.s1, P.s2, Q.s1, Q.s2, ns);
+  const bool samePQ = P.lex == Q.lex;
+  unsigned alive = 0;
+#pragma unroll
+  for (int pb = 0; pb < 2; pb++)
+#pragma unroll
+    for (int pk = 0; pk < 2; pk++) {
+      if ((pb && P.shA == P.shB) || (pk && Q.shA == Q.shB) || (samePQ && pb > pk)) continue;
+      const int xd = pb ? P.shB : P.shA, xo = pb ? P.shA : P.shB;
+      const int yd = pk ? Q.shB : Q.shA, yo = pk ? Q.shA : Q.shB;
+      const double bound = shMax * __ldg(a.qG + xd + (size_t)xo * ns) *
+                           __ldg(a.qG + yd + (size_t)yo * ns);
+      if (!a.screen || bound >= a.thresh) alive |= 1u << (2 * pb + pk);
+    }
+  return alive;
+}
+
+__global__ void __launch_bounds__(256)
+    gaunt_plan_kernel(const GauntLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
+                      int* __restrict__ list32, unsigned* __restrict__ lcount) {
+  hg_plan(a.nBra, a.nKet, masks, list64, list32, lcount, a.counters,
+          [&](int ib, int jk, bool& work, bool&) {
+            if ((a.same && jk > ib + a.braOff) ||
+                !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt))
+              return false;
+            work = gaunt_alive(a, a.pairs[a.braBeg + ib], a.pairs[a.ketBeg + jk]) != 0;
+            return true;
+          });
+}
+
+// Gaunt on the engine: M[(ab, pb, j)][(cd, pk, l)], every surviving reference
+// quartet of every element one unit of work.
+struct GauntDig {
+  using Args = GauntLaunch;
+  static constexpr int NP = 1, ABU = 8, CDU = 8;  // 8 component pairs: three row tiles
+  __host__ __device__ static constexpr int tb(int) { return HG_D6; }
+  __host__ __device__ static constexpr int tk(int) { return HG_D6; }
+  __host__ __device__ static constexpr int rtu(int) { return 3; }
+  __host__ __device__ static constexpr int ctu(int) { return 3; }
+  static __device__ __forceinline__ void digest(const GauntLaunch& a, const HgQuartet& z) {
+    const PairDev &P = *z.P, &Q = *z.Q;
+    const unsigned alive = gaunt_alive(a, P, Q);
+    const int nb = ncart(z.lb), nd = ncart(z.ld), nCD = z.cd1 - z.cd0;
+    for (int u = threadIdx.x; u < (z.ab1 - z.ab0) * nCD * 4; u += blockDim.x) {
+      const int blk = u & 3, e = u >> 2, r = e / nCD, c = e - r * nCD;
+      if (!(alive & (1u << blk))) continue;
+      const int pb = blk >> 1, pk = blk & 1;
+      const int ab = z.ab0 + r, cd = z.cd0 + c;
+      const int gA = P.cA + ab / nb, gB = P.cB + ab % nb;
+      const int gC = Q.cA + cd / nd, gD = Q.cB + cd % nd;
+      const int xd = pb ? P.shB : P.shA, xo = pb ? P.shA : P.shB;
+      const int yd = pk ? Q.shB : Q.shA, yo = pk ? Q.shA : Q.shB;
+      const int xdA = pb ? gB : gA, xoA = pb ? gA : gB;
+      const int ydA = pk ? gD : gC, yoA = pk ? gC : gD;
+      // the reference's orientation: bra X (j on X) or Y (j on Y)
+      const bool xb = xd > yd || (xd == yd && xo >= yo);
+      const double* m = z.M[0] + (size_t)(r * 6 + pb * 3) * z.ms[0] + c * 6 + pk * 3;
+      double v[9];
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int l = 0; l < 3; l++)
+          v[3 * j + l] = xb ? m[(size_t)j * z.ms[0] + l] : m[(size_t)l * z.ms[0] + j];
+      if (xb) gaunt_sites(a, v, xo, xd, yd, yo, xoA, xdA, ydA, yoA);
+      else gaunt_sites(a, v, yo, yd, xd, xo, yoA, ydA, xdA, xoA);
+    }
+  }
+};
+
 // One thread per (quartet {P, Q}, unit); units = ket component pairs (c, d)
-// x slices of bra component pairs, split over nsplit threads.  GAUNT: one
-// operator, 1 / r12.  GAUGE: seven -- 1 / r12 and d_i d_i' r12 for the six
-// pairs i <= i' -- each a pass over the primitive pairs (the r12 passes on
-// the auxiliary functions of r12_aux, the Hermite index shifted by
-// e_i + e_i').
-template <int LM, bool GAUGE>
+// x slices of bra component pairs, split over nsplit threads.  Seven
+// operators -- 1 / r12 and d_i d_i' r12 for the six pairs i <= i' -- each a
+// pass over the primitive pairs (the r12 passes on the auxiliary functions
+// of r12_aux, the Hermite index shifted by e_i + e_i').
+template <int LM>
 __global__ void __launch_bounds__(REL_THREADS)
-    gaunt_kernel(const GauntLaunch a, int la, int lb, int lc, int ld, int nsplit, int nslice) {
+    gauge_kernel(const GauntLaunch a, int la, int lb, int lc, int ld, int nsplit, int nslice) {
   const int ib = blockIdx.x;
   if (!in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;  // another shard's bra
   const int split = blockIdx.y % nsplit;
   const int jk = (blockIdx.y / nsplit) * REL_THREADS + threadIdx.x;
-  const int ns = a.nShell;
   const bool visited = jk < a.nKet && !(a.same && jk > ib);
   const PairDev P = a.pairs[a.braBeg + ib];
   PairDev Q = P;
-  unsigned alive = 0;  // bit 2 pb + pk: derivative on B (pb) / D (pk)
+  unsigned alive = 0;
   if (visited) {
     Q = a.pairs[a.ketBeg + jk];
-    const double shMax = sh_max(a.norms, P.s1, P.s2, Q.s1, Q.s2, ns);
-    const bool samePQ = P.lex == Q.lex;
-#pragma unroll
-    for (int pb = 0; pb < 2; pb++)
-#pragma unroll
-      for (int pk = 0; pk < 2; pk++) {
-        if ((pb && P.shA == P.shB) || (pk && Q.shA == Q.shB) || (samePQ && pb > pk)) continue;
-        const int xd = pb ? P.shB : P.shA, xo = pb ? P.shA : P.shB;
-        const int yd = pk ? Q.shB : Q.shA, yo = pk ? Q.shA : Q.shB;
-        const double bound = shMax * __ldg(a.qG + xd + (size_t)xo * ns) *
-                             __ldg(a.qG + yd + (size_t)yo * ns);
-        if (!a.screen || bound >= a.thresh) alive |= 1u << (2 * pb + pk);
-      }
+    alive = gaunt_alive(a, P, Q);
   }
   if (split == 0) {
     const unsigned mask = __activemask();
@@ -798,12 +780,12 @@ __global__ void __launch_bounds__(REL_THREADS)
   }
   if (!alive) return;
 
-  constexpr int NOP = GAUGE ? 7 : 1;
+  constexpr int NOP = 7;
   constexpr int E1 = (LM + 2) * (LM + 2) * (2 * LM + 3);
   constexpr int HB = nherm(2 * LM + 1);
-  constexpr int HL = nherm(4 * LM + 2 + (GAUGE ? 2 : 0));
+  constexpr int HL = nherm(4 * LM + 4);
   constexpr int FL = 2 * LM + 3;
-  constexpr int ABCH = GAUGE ? gauge_abch(LM) : gaunt_abch(LM);
+  constexpr int ABCH = gauge_abch(LM);
   const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
   const int nab = na * nb, ncd = ncc * nd;
   const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
@@ -945,15 +927,7 @@ __global__ void __launch_bounds__(REL_THREADS)
             return xb ? m[o * 36 + ((pb * 3 + j) * 2 + pk) * 3 + l]
                       : m[o * 36 + ((pb * 3 + l) * 2 + pk) * 3 + j];
           };
-          if (!GAUGE) {
-            double v[9];
-#pragma unroll
-            for (int j = 0; j < 3; j++)
-#pragma unroll
-              for (int l = 0; l < 3; l++) v[3 * j + l] = comp(0, j, l);
-            if (xb) gaunt_sites(a, v, xo, xd, yd, yo, xoA, xdA, ydA, yoA);
-            else gaunt_sites(a, v, yo, yd, xd, xo, yoA, ydA, xdA, xoA);
-          } else {
+          {
             GVd V, Vt;
 #pragma unroll 1
             for (int k = 0; k < 6; k++) {
@@ -980,25 +954,22 @@ __global__ void __launch_bounds__(REL_THREADS)
   }
 }
 
-template <bool GAUGE>
-void launch_gaunt(const GauntLaunch& a, int la, int lb, int lc, int ld, cudaStream_t st) {
+void launch_gauge(const GauntLaunch& a, int la, int lb, int lc, int ld, cudaStream_t st) {
   if (a.nBra == 0 || a.nKet == 0) return;
   const int tiles = (a.nKet + REL_THREADS - 1) / REL_THREADS;
   const int lm = std::max(std::max(la, lb), std::max(lc, ld));
   const int nab = ncart(la) * ncart(lb);
-  const int abch = GAUGE ? gauge_abch(std::max(lm, 1)) : gaunt_abch(std::max(lm, 1));
+  const int abch = gauge_abch(std::max(lm, 1));
   const int nslice = (nab + abch - 1) / abch;
   const long long quartets = (long long)a.nBra * a.nKet;
   const int units = ncart(lc) * ncart(ld) * nslice;
   int nsplit = (int)std::min<long long>(units, std::max<long long>(1, (1 << 18) / quartets));
   nsplit = std::max(1, std::min(nsplit, 65535 / tiles));
   dim3 grid(a.nBra, tiles * nsplit);
-  if (lm <= 1)
-    gaunt_kernel<1, GAUGE><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
+  if (lm <= 1) gauge_kernel<1><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
   else if (lm == 2)
-    gaunt_kernel<2, GAUGE><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
-  else
-    gaunt_kernel<3, GAUGE><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
+    gauge_kernel<2><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
+  else gauge_kernel<3><<<grid, REL_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit, nslice);
 }
 
 // ------------------------------------------------------------ 4C Schwarz
@@ -1479,6 +1450,37 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
                               bool gauge, const cqf_opts& opts, cudaStream_t st, double* ws,
                               unsigned long long* cnt);
 
+// go(cb, ck, region, stream) for every class pair with quartets (every
+// ordered one, or ck <= cb), round-robin over the call's stream and the
+// auxiliary ones with a mask region each: the launches only add into the
+// accumulators, so one's tail overlaps the next one's start; the largest
+// angular momenta first.
+template <class Go>
+cqf_status for_class_pairs(cqf_basis* B, bool ordered, double* ws, cudaStream_t st, Go go) {
+  const long long maskWords = rel_mask_words(B);
+  uint2* masks = reinterpret_cast<uint2*>(ws + rel_core_doubles(B));
+  unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
+  CQF_RCUDA(cudaEventRecord(B->evFork, st));
+  cudaStream_t lanes[NAUX + 1] = {st};
+  for (int i = 0; i < NAUX; i++) {
+    lanes[1 + i] = B->aux[i];
+    CQF_RCUDA(cudaStreamWaitEvent(B->aux[i], B->evFork, 0));
+  }
+  int nlaunch = 0;
+  cqf_status rc = CQF_OK;
+  for (int cb = NCLS - 1; cb >= 0 && rc == CQF_OK; cb--)
+    for (int ck = ordered ? NCLS - 1 : cb; ck >= 0 && rc == CQF_OK; ck--) {
+      if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
+      const int li = nlaunch++ % (NAUX + 1);
+      rc = go(cb, ck, HgRegion{masks + 2 * maskWords * li, maskWords, work + 4 * li}, lanes[li]);
+    }
+  for (int i = 0; i < NAUX; i++) {
+    CQF_RCUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
+    CQF_RCUDA(cudaStreamWaitEvent(st, B->evJoin[i], 0));
+  }
+  return rc;
+}
+
 cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const* AX, int type,
                             int exch, const cqf_opts& opts, cudaStream_t st, double* ws,
                             unsigned long long* cnt) {
@@ -1612,39 +1614,19 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
   a.counters = dcnt;
   CQF_RTRY(hg_ensure(B, HG_SPIN));
   if (llss) CQF_RTRY(hg_ensure(B, HG_PLAIN));
-  // class pairs round-robin over the call's stream and the auxiliary ones
-  // (they only add into the accumulators), the largest angular sums first,
-  // so that one launch's tail overlaps the next one's start
-  const long long maskWords = rel_mask_words(B);
-  uint2* masks = reinterpret_cast<uint2*>(ws + rel_core_doubles(B));
-  unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
-  CQF_RCUDA(cudaEventRecord(B->evFork, st));
-  cudaStream_t lanes[NAUX + 1] = {st};
-  for (int i = 0; i < NAUX; i++) {
-    lanes[1 + i] = B->aux[i];
-    CQF_RCUDA(cudaStreamWaitEvent(B->aux[i], B->evFork, 0));
-  }
-  int nlaunch = 0;
-  cqf_status rc = CQF_OK;
-  for (int cb = NCLS - 1; cb >= 0 && rc == CQF_OK; cb--)
-    for (int ck = NCLS - 1; ck >= 0 && rc == CQF_OK; ck--) {
-      if (!llss && ck > cb) continue;
-      if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
-      a.braBeg = B->cls_beg[cb];
-      a.nBra = B->cls_cnt[cb];
-      a.ketBeg = B->cls_beg[ck];
-      a.nKet = B->cls_cnt[ck];
-      a.same = (cb == ck);
-      const int li = nlaunch++ % (NAUX + 1);
-      uint2* mk = masks + 2 * maskWords * li;
-      rc = llss ? launch_rel<1>(B, a, cb, ck, mk, maskWords, work + 4 * li, lanes[li])
-                : launch_rel<2>(B, a, cb, ck, mk, maskWords, work + 4 * li, lanes[li]);
-    }
-  for (int i = 0; i < NAUX; i++) {
-    CQF_RCUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
-    CQF_RCUDA(cudaStreamWaitEvent(st, B->evJoin[i], 0));
-  }
-  CQF_RTRY(rc);
+  CQF_RTRY(for_class_pairs(
+      B, llss, ws, st, [&](int cb, int ck, const HgRegion& r, cudaStream_t ls) {
+        int la, lb, lc, ld;
+        class_ls(cb, la, lb);
+        class_ls(ck, lc, ld);
+        a.braBeg = B->cls_beg[cb];
+        a.nBra = B->cls_cnt[cb];
+        a.ketBeg = B->cls_beg[ck];
+        a.nKet = B->cls_cnt[ck];
+        a.same = (cb == ck);
+        a.lsum = la + lb + lc + ld;
+        return llss ? launch_rel<1>(B, a, cb, ck, r, ls) : launch_rel<2>(B, a, cb, ck, r, ls);
+      }));
   CQF_RCUDA(cudaGetLastError());
   auto back = [&](const double* src, int mode, double* dst) {
     rel_from_cart_kernel<<<rgrid(NN, 256), 256, 0, st>>>(src, mode, N, nc, B->d_shells,
@@ -1755,20 +1737,32 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
   a.shardIdx = opts.shard_index;
   a.shardCnt = std::max(1, opts.shard_count);
   a.counters = dcnt;
-  for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck <= cb; ck++) {
-      if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
-      int la, lb, lc, ld;
-      class_ls(cb, la, lb);
-      class_ls(ck, lc, ld);
-      a.braBeg = B->cls_beg[cb];
-      a.nBra = B->cls_cnt[cb];
-      a.ketBeg = B->cls_beg[ck];
-      a.nKet = B->cls_cnt[ck];
-      a.same = (cb == ck);
-      if (gauge) launch_gaunt<true>(a, la, lb, lc, ld, st);
-      else launch_gaunt<false>(a, la, lb, lc, ld, st);
-    }
+  if (!gauge) CQF_RTRY(hg_ensure(B, HG_D6));
+  CQF_RTRY(for_class_pairs(
+      B, false, ws, st, [&](int cb, int ck, const HgRegion& r, cudaStream_t ls) {
+        int la, lb, lc, ld;
+        class_ls(cb, la, lb);
+        class_ls(ck, lc, ld);
+        a.braBeg = B->cls_beg[cb];
+        a.nBra = B->cls_cnt[cb];
+        a.ketBeg = B->cls_beg[ck];
+        a.nKet = B->cls_cnt[ck];
+        a.same = (cb == ck);
+        if (gauge) {
+          launch_gauge(a, la, lb, lc, ld, ls);
+          return CQF_OK;
+        }
+        return hg_contract<GauntDig>(
+            B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, ls,
+            [&](int ib0, int n, uint2* masks, int* list64, int* list32, unsigned* lcount,
+                unsigned gp) {
+              GauntLaunch c = a;
+              c.braBeg += ib0;
+              c.braOff = ib0;
+              c.nBra = n;
+              gaunt_plan_kernel<<<gp, 256, 0, ls>>>(c, masks, list64, list32, lcount);
+            });
+      }));
   CQF_RCUDA(cudaGetLastError());
   auto back = [&](const double* srcAcc, int mode, double* dst) {
     rel_from_cart_kernel<<<rgrid(NN, 256), 256, 0, st>>>(srcAcc, mode, N, nc, B->d_shells,

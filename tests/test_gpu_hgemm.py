@@ -10,9 +10,10 @@ import pytest
 
 import oracle as O
 from chronusq_public_b200.basis import BasisSet, Molecule, parse_gbs
-from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, LLSS, SSSS, DirectTPI,
+from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, GAUNT, LLSS, SSSS, DirectTPI,
                                               GTODirectRelERIContraction,
                                               GTODirectTPIContraction, TwoBodyContraction)
+from test_gpu_gaunt import OUTS_C, OUTS_X, gaunt_inputs
 from test_gpu_rel import OUTS, max_rel, rel_inputs
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +81,15 @@ def test_engine_jk(name, kind):
                       precision="mixed" if kind == "mixed" else "fp64", fp32_cutoff=1e-3)
     for o, r in zip(out, ref):
         assert max_rel(o, np.asarray(r)) < (1e-6 if kind == "mixed" else 1e-11)
+
+
+@pytest.mark.parametrize("name", sorted(BASES))
+def test_engine_gaunt(name):
+    bs = basis(name)
+    N = bs.nbasis
+    _D, X = gaunt_inputs(N, 63)
+    ref = O.OracleBasis(bs).rel_contract(X, GAUNT, True)
+    lst = [TwoBodyContraction(X[m], np.zeros((N, N), complex)) for m in range(29)]
+    GTODirectRelERIContraction(DirectTPI(bs)).twoBodyContract(lst, GAUNT)
+    for m in OUTS_X + OUTS_C:
+        assert max_rel(lst[m].AX, ref[m]) < 1e-11, m
