@@ -13,20 +13,21 @@
 // its shells is minus the d/dr of that shell's functions; each of the 12
 // (4 centres x 3 axes) goes to the component of the shell's atom.
 //
-// One thread per unique shell quartet and ket Cartesian component pair:
-// per bra primitive pair the Hermite tables raised by one on both centres,
-// the ket-contracted Hermite sums of the plain ket and of its six
-// derivatives (on C or D, x / y / z), and for every bra component pair the
-// 12 derivative integrals -- six from differentiated bra factors against the
-// plain ket sums, six from plain bra factors against the differentiated
-// ones.  Accumulators are Cartesian, FP64 atomics, one per (component,
-// matrix); the back transform symmetrises.  FP64.
+// Quartets run on the Hermite-matrix engine (cqf_hgemm.cuh): the first
+// derivatives on A and B against the plain ket, and the plain bra against
+// those on C, are two matrix products per primitive quartet; those on D are
+// minus the sum (translational invariance).  The derivatives of one atom are
+// summed before the digestion, and a quartet on a single atom, whose
+// derivatives cancel, is dropped by the planning pass.  Accumulators are
+// Cartesian, one per (component, matrix); the back transform symmetrises.
+// FP64.  The kernel this replaces (one thread per quartet and ket component,
+// 12 x 6 atomics per element) took 268 ms for (H2O)4 / cc-pVDZ.
 #include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
 
-#include "cqf_deriv.cuh"
+#include "cqf_hg_digest.cuh"
 #include "cqf_internal.hpp"
 
 namespace cqf {
@@ -40,16 +41,11 @@ namespace {
                   std::string(#call) + ": " + cudaGetErrorString(e_));                     \
   } while (0)
 
-constexpr int GRAD_THREADS = 64;
 constexpr int GRAD_MAXMAT = 8;  // matrices per call
 
 struct GradLaunch {
   const PairDev* pairs;
-  const PrimPairDev* pp;
-  const ShellDev* shells;
-  const double* prim;
-  const double* boys;
-  int braBeg, nBra, ketBeg, nKet, same;
+  int braBeg, nBra, braOff, ketBeg, nKet, same;
   int ncart, nMat;
   int type[GRAD_MAXMAT];  // COULOMB / EXCHANGE
   const int* shellAtom;   // per shell (device)
@@ -59,187 +55,69 @@ struct GradLaunch {
   unsigned long long* counters;
 };
 
-template <int LM>
-__global__ void __launch_bounds__(GRAD_THREADS)
-    grad_kernel(const GradLaunch a, int la, int lb, int lc, int ld, int nsplit) {
-  const int ib = blockIdx.x;
-  if (!in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) return;  // another shard's bra
-  const int split = blockIdx.y % nsplit;
-  const int jk = (blockIdx.y / nsplit) * GRAD_THREADS + threadIdx.x;
-  const bool visited = jk < a.nKet && !(a.same && jk > ib);
-  if (split == 0) {
-    const unsigned mask = __activemask();
-    const unsigned bv = __ballot_sync(mask, visited);
-    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1 && bv) {
-      atomicAdd(a.counters + 0, (unsigned long long)__popc(bv));
-      atomicAdd(a.counters + 3, (unsigned long long)__popc(bv));
-    }
-  }
-  if (!visited) return;
-  const PairDev P = a.pairs[a.braBeg + ib];
-  const PairDev Q = a.pairs[a.ketBeg + jk];
+__global__ void __launch_bounds__(256)
+    grad_plan_kernel(const GradLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
+                     int* __restrict__ list32, unsigned* __restrict__ lcount) {
+  hg_plan(a.nBra, a.nKet, masks, list64, list32, lcount, a.counters,
+          [&](int ib, int jk, bool& work, bool&) {
+            if ((a.same && jk > ib + a.braOff) ||
+                !in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt))
+              return false;
+            const PairDev P = a.pairs[a.braBeg + ib], Q = a.pairs[a.ketBeg + jk];
+            const int t = __ldg(a.shellAtom + P.shA);
+            work = __ldg(a.shellAtom + P.shB) != t || __ldg(a.shellAtom + Q.shA) != t ||
+                   __ldg(a.shellAtom + Q.shB) != t;
+            return true;
+          });
+}
 
-  constexpr int NCL = ncart(LM);
-  constexpr int E1 = (LM + 2) * (LM + 2) * (2 * LM + 3);
-  constexpr int HB = nherm(2 * LM + 1);
-  constexpr int HL = nherm(4 * LM + 1);
-  constexpr int FL = 2 * LM + 3;
-  const int na = ncart(la), nb = ncart(lb), ncc = ncart(lc), nd = ncart(ld);
-  const int nab = na * nb;
-  const ShellDev SA = a.shells[P.shA], SB = a.shells[P.shB];
-  const ShellDev SC = a.shells[Q.shA], SD = a.shells[Q.shB];
-  const int Lb = la + lb + 1, Lk = lc + ld + 1, L = la + lb + lc + ld + 1;
-  // the reference's orientation: (s1 s2 | s3 s4) with (s1, s2) the pair
-  // later in its loop order; its degeneracy (direct.hpp:2365-2398), and
-  // d/dA = -d/dr
-  const bool pRef = P.lex >= Q.lex;
-  const PairDev& R12 = pRef ? P : Q;
-  const PairDev& R34 = pRef ? Q : P;
-  const double deg = (R12.s1 == R12.s2 ? 1.0 : 2.0) * (R34.s1 == R34.s2 ? 1.0 : 2.0) *
-                     ((R12.s1 == R34.s1) ? (R12.s2 == R34.s2 ? 1.0 : 2.0) : 2.0);
-  const double f = -0.5 * deg;
-  // atom of each differentiated centre: A, B, C, D
-  const int atom[4] = {__ldg(a.shellAtom + P.shA), __ldg(a.shellAtom + P.shB),
+struct GradDig {
+  using Args = GradLaunch;
+  static constexpr int NP = 2, ABU = 16, CDU = 16;
+  __host__ __device__ static constexpr int tb(int q) { return q == 0 ? HG_D6 : HG_PLAIN; }
+  __host__ __device__ static constexpr int tk(int q) { return q == 0 ? HG_PLAIN : HG_D3; }
+  __host__ __device__ static constexpr int rtu(int q) { return q == 0 ? 6 : 1; }
+  __host__ __device__ static constexpr int ctu(int q) { return q == 0 ? 1 : 3; }
+  static __device__ __forceinline__ void digest(const GradLaunch& a, const HgQuartet& z) {
+    const PairDev &P = *z.P, &Q = *z.Q;
+    const int at[4] = {__ldg(a.shellAtom + P.shA), __ldg(a.shellAtom + P.shB),
                        __ldg(a.shellAtom + Q.shA), __ldg(a.shellAtom + Q.shB)};
-  const size_t nc = a.ncart, nc2 = nc * nc;
-
-  double Ea[3][E1], Ec[3][E1];
-  double G[7][HB];  // plain ket, then d/dC x y z, d/dD x y z
-  double Rv[HL];
-  double F[4 * LM + 3];
-  double acc[NCL * NCL * 12];  // [ab][centre * 3 + xyz]
-  double fa[3][3][FL], fc[3][3][FL];
-  int nfa[3][3], nfc[3][3];
-
-#pragma unroll 1
-  for (int cd = split; cd < ncc * nd; cd += nsplit) {
-    const int c = cd / nd, d = cd % nd;
-    const int ci[3] = {cart_lx(lc, c), cart_ly(lc, c), cart_lz(lc, c)};
-    const int di[3] = {cart_lx(ld, d), cart_ly(ld, d), cart_lz(ld, d)};
-#pragma unroll 1
-    for (int k = 0; k < nab * 12; k++) acc[k] = 0.0;
-#pragma unroll 1
-    for (int ip = 0; ip < P.npp; ip++) {
-      const PrimPairDev& A = a.pp[P.pp_off + ip];
-      double ea, eb;
-      pair_exps(SA, SB, a.prim, A, ea, eb);
-#pragma unroll 1
-      for (int x = 0; x < 3; x++)
-        hermite_E_rt<double, LM + 1>(la + 1, lb + 1, A.o2p, A.PA[x], A.PB[x], Ea[x]);
-#pragma unroll 1
-      for (int k = 0; k < 7; k++)
-#pragma unroll 1
-        for (int h = 0; h < nherm(Lb); h++) G[k][h] = 0.0;
-#pragma unroll 1
-      for (int iq = 0; iq < Q.npp; iq++) {
-        const PrimPairDev& Bq = a.pp[Q.pp_off + iq];
-        double ec, ed;
-        pair_exps(SC, SD, a.prim, Bq, ec, ed);
-#pragma unroll 1
-        for (int x = 0; x < 3; x++)
-          hermite_E_rt<double, LM + 1>(lc + 1, ld + 1, Bq.o2p, Bq.PA[x], Bq.PB[x], Ec[x]);
-        const double X = A.P[0] - Bq.P[0], Y = A.P[1] - Bq.P[1], Z = A.P[2] - Bq.P[2];
-        const double pq = A.p + Bq.p, alpha = A.p * Bq.p / pq;
-        const double pref = PI52X2 / sqrt(pq) * A.Kp * Bq.Kp;
-        boys_rt<double>(L, alpha * (X * X + Y * Y + Z * Z), F, a.boys);
-        hermite_R_rt<double>(L, alpha, X, Y, Z, F, Rv);
-#pragma unroll 1
-        for (int x = 0; x < 3; x++)
-#pragma unroll 1
-          for (int ty = 0; ty < 3; ty++) {
-            nfc[x][ty] = axis_factor<double>(Ec[x], ld + 1, lc + ld + 3, ci[x], di[x], ty,
-                                             2.0 * ec, 2.0 * ed, fc[x][ty]);
-#pragma unroll 1
-            for (int t = 1; t < nfc[x][ty]; t += 2) fc[x][ty][t] = -fc[x][ty][t];
-          }
-        // plain ket (the bra derivatives need only Lb - 1 < Lb Hermite orders)
-        ket_add<double>(G[0], pref, fc[0][0], nfc[0][0], fc[1][0], nfc[1][0], fc[2][0],
-                        nfc[2][0], Lb, Rv);
-#pragma unroll 1
-        for (int k = 0; k < 6; k++) {
-          const int side = k / 3, dir = k % 3;  // 0: C, 1: D
-          const int tx = dir == 0 ? 1 + side : 0, ty = dir == 1 ? 1 + side : 0,
-                    tz = dir == 2 ? 1 + side : 0;
-          ket_add<double>(G[1 + k], pref, fc[0][tx], nfc[0][tx], fc[1][ty], nfc[1][ty],
-                          fc[2][tz], nfc[2][tz], Lb - 1, Rv);
-        }
-      }
-#pragma unroll 1
-      for (int ab = 0; ab < nab; ab++) {
-        const int ai = ab / nb, bi = ab % nb;
-        const int ax[3] = {cart_lx(la, ai), cart_ly(la, ai), cart_lz(la, ai)};
-        const int bx[3] = {cart_lx(lb, bi), cart_ly(lb, bi), cart_lz(lb, bi)};
-#pragma unroll 1
-        for (int x = 0; x < 3; x++)
-#pragma unroll 1
-          for (int ty = 0; ty < 3; ty++)
-            nfa[x][ty] = axis_factor<double>(Ea[x], lb + 1, la + lb + 3, ax[x], bx[x], ty,
-                                             2.0 * ea, 2.0 * eb, fa[x][ty]);
-        double* m = acc + ab * 12;
-#pragma unroll 1
-        for (int k = 0; k < 6; k++) {  // d/dr on A or B against the plain ket
-          const int side = k / 3, dir = k % 3;
-          const int tx = dir == 0 ? 1 + side : 0, ty = dir == 1 ? 1 + side : 0,
-                    tz = dir == 2 ? 1 + side : 0;
-          m[k] += bra_dot<double>(fa[0][tx], nfa[0][tx], fa[1][ty], nfa[1][ty], fa[2][tz],
-                                  nfa[2][tz], G[0]);
-        }
-#pragma unroll 1
-        for (int k = 0; k < 6; k++)  // plain bra against d/dr on C or D
-          m[6 + k] += bra_dot<double>(fa[0][0], nfa[0][0], fa[1][0], nfa[1][0], fa[2][0],
-                                      nfa[2][0], G[1 + k]);
+    // the quartet's atoms, and the weight of the derivatives on A, B, C in
+    // each atom's (the one on D is minus their sum; d/dR = -d/dr)
+    int atom[4] = {at[0], 0, 0, 0}, n = 1;
+#pragma unroll
+    for (int k = 1; k < 4; k++) {
+      bool seen = false;
+#pragma unroll
+      for (int s = 0; s < 4; s++) seen = seen || (s < n && atom[s] == at[k]);
+      if (!seen) {
+#pragma unroll
+        for (int s = 1; s < 4; s++)
+          if (s == n) atom[s] = at[k];
+        n++;
       }
     }
-    // digestion at the reference's update sites (direct.hpp:2470-2520)
-    const int gC = Q.cA + c, gD = Q.cB + d;
-#pragma unroll 1
-    for (int ab = 0; ab < nab; ab++) {
-      const int gA = P.cA + ab / nb, gB = P.cB + ab % nb;
-      // Cartesian AO index of the function of shells s1..s4 (a pair with
-      // s1 == s2 maps shA to s1)
-      const int pa1 = (P.s1 == P.shA) ? gA : gB, pa2 = (P.s1 == P.shA) ? gB : gA;
-      const int qa1 = (Q.s1 == Q.shA) ? gC : gD, qa2 = (Q.s1 == Q.shA) ? gD : gC;
-      const int b1 = pRef ? pa1 : qa1, b2 = pRef ? pa2 : qa2;
-      const int b3 = pRef ? qa1 : pa1, b4 = pRef ? qa2 : pa2;
-      const double* m = acc + ab * 12;
-#pragma unroll 1
-      for (int k = 0; k < 12; k++) {
-        const double v = f * m[k];
-        if (v == 0.0) continue;
-        const int g = atom[k / 3] * 3 + k % 3;
-#pragma unroll 1
-        for (int mt = 0; mt < a.nMat; mt++) {
-          const double* X = a.Xc + (size_t)mt * nc2;
-          double* A = a.Ac + ((size_t)g * a.nMat + mt) * nc2;
-          auto x = [&](int r, int cc) { return __ldg(X + r + (size_t)cc * nc); };
-          if (a.type[mt] == CQF_COULOMB) {
-            atomicAdd(A + b1 + (size_t)b2 * nc, x(b4, b3) * v);
-            atomicAdd(A + b4 + (size_t)b3 * nc, x(b1, b2) * v);
-          } else {
-            atomicAdd(A + b1 + (size_t)b3 * nc, 0.5 * x(b4, b2) * v);
-            atomicAdd(A + b4 + (size_t)b2 * nc, 0.5 * x(b3, b1) * v);
-            atomicAdd(A + b4 + (size_t)b1 * nc, 0.5 * x(b3, b2) * v);
-            atomicAdd(A + b2 + (size_t)b3 * nc, 0.5 * x(b4, b1) * v);
-          }
-        }
-      }
-    }
+    auto atomOf = [&](int s) {
+      return s == 0 ? atom[0] : (s == 1 ? atom[1] : (s == 2 ? atom[2] : atom[3]));
+    };
+    const double *M0 = z.M[0], *M1 = z.M[1];
+    const int m0 = z.ms[0], m1 = z.ms[1];
+    const size_t nc2 = (size_t)a.ncart * a.ncart;
+    auto val = [&](int k, int ab, int cd) {
+      const int s = k / 3, x = k - 3 * s, t = atomOf(s);
+      const double w = t == at[3] ? -1.0 : 0.0;
+      const double* r = M0 + (size_t)(6 * ab + x) * m0 + cd;
+      return (w + (t == at[0])) * r[0] + (w + (t == at[1])) * r[(size_t)3 * m0] +
+             (w + (t == at[2])) * M1[(size_t)ab * m1 + 3 * cd + x];
+    };
+    for (int mt = 0; mt < a.nMat; mt++)
+      hg_digest_her(z, a.ncart, a.type[mt] != CQF_COULOMB, -1.0, true, a.Xc + mt * nc2, 3 * n,
+                    val, [&](int k) {
+                      const int s = k / 3, x = k - 3 * s;
+                      return a.Ac + ((size_t)(atomOf(s) * 3 + x) * a.nMat + mt) * nc2;
+                    });
   }
-}
-
-void launch_grad(const GradLaunch& a, int la, int lb, int lc, int ld, cudaStream_t st) {
-  if (a.nBra == 0 || a.nKet == 0) return;
-  const int tiles = (a.nKet + GRAD_THREADS - 1) / GRAD_THREADS;
-  const long long quartets = (long long)a.nBra * a.nKet;
-  const int ncd = ncart(lc) * ncart(ld);
-  int nsplit = (int)std::min<long long>(ncd, std::max<long long>(1, (1 << 18) / quartets));
-  nsplit = std::max(1, std::min(nsplit, 65535 / tiles));
-  dim3 grid(a.nBra, tiles * nsplit);
-  const int lm = std::max(std::max(la, lb), std::max(lc, ld));
-  if (lm <= 1) grad_kernel<1><<<grid, GRAD_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-  else if (lm == 2) grad_kernel<2><<<grid, GRAD_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-  else grad_kernel<3><<<grid, GRAD_THREADS, 0, st>>>(a, la, lb, lc, ld, nsplit);
-}
+};
 
 }  // namespace
 }  // namespace cqf
@@ -284,7 +162,23 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   // scratch (stream-ordered): shell atoms | Cartesian X | Cartesian
   // accumulators | host staging of X and AX
   const size_t host = o.device_pointers ? 0 : (size_t)nMat * NN + (size_t)nGrad * nMat * NN;
-  const size_t doubles = (size_t)nMat * nc2 + (size_t)nGrad * nMat * nc2 + host;
+  // then, per launch stream, the planning pass's masks and lists and four
+  // counters
+  size_t need = 1, row = 1;
+  for (int cb = 0; cb < NCLS; cb++)
+    for (int ck = 0; ck <= cb; ck++) {
+      const size_t w = ((size_t)B->cls_cnt[ck] + WTILE - 1) / WTILE;
+      row = std::max(row, w);
+      need = std::max(need, (size_t)B->cls_cnt[cb] * w);
+    }
+  const size_t maskWords = std::max(row, std::min(need, MASK_CAP_WORDS));
+  const size_t lists = (2 * maskWords + 2) * (NAUX + 1);
+  const size_t fixed = ((size_t)nMat * nc2 + (size_t)nGrad * nMat * nc2 + host + 1) / 2 * 2;
+  const size_t doubles = fixed + lists;
+  for (int k : {(int)HG_PLAIN, (int)HG_D6, (int)HG_D3}) {
+    const cqf_status s = hg_ensure(B, k);
+    if (s != CQF_OK) return s;
+  }
   double* ws = nullptr;
   int* dAtom = nullptr;
   CQF_GCUDA(cudaMallocAsync(&ws, doubles * sizeof(double), st));
@@ -310,10 +204,6 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
 
   GradLaunch a{};
   a.pairs = B->d_pairs;
-  a.pp = B->d_pp;
-  a.shells = B->d_shells;
-  a.prim = B->d_prim;
-  a.boys = B->d_boys64;
   a.ncart = nc;
   a.nMat = nMat;
   for (int m = 0; m < nMat; m++) a.type[m] = list[m].type;
@@ -323,19 +213,49 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   a.shardIdx = o.shard_index;
   a.shardCnt = o.shard_count;
   a.counters = B->d_counters;
-  for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck <= cb; ck++) {
+  // class pairs round-robin over the call's stream and the auxiliary ones
+  // (they only add into the accumulators), the largest first
+  uint2* masks = reinterpret_cast<uint2*>(ws + fixed);
+  unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
+  CQF_GCUDA(cudaEventRecord(B->evFork, st));
+  cudaStream_t lanes[NAUX + 1] = {st};
+  for (int i = 0; i < NAUX; i++) {
+    lanes[1 + i] = B->aux[i];
+    CQF_GCUDA(cudaStreamWaitEvent(B->aux[i], B->evFork, 0));
+  }
+  int nlaunch = 0;
+  cqf_status rc = CQF_OK;
+  for (int cb = NCLS - 1; cb >= 0; cb--)
+    for (int ck = cb; ck >= 0 && rc == CQF_OK; ck--) {
       if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
-      int la, lb, lc, ld;
-      class_ls(cb, la, lb);
-      class_ls(ck, lc, ld);
       a.braBeg = B->cls_beg[cb];
       a.nBra = B->cls_cnt[cb];
       a.ketBeg = B->cls_beg[ck];
       a.nKet = B->cls_cnt[ck];
       a.same = (cb == ck);
-      launch_grad(a, la, lb, lc, ld, st);
+      const int li = nlaunch++ % (NAUX + 1);
+      const cudaStream_t ls = lanes[li];
+      const HgRegion r{masks + 2 * maskWords * li, (long long)maskWords, work + 4 * li};
+      rc = hg_contract<GradDig>(
+          B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, ls,
+          [&](int ib0, int n, uint2* mk, int* list64, int* list32, unsigned* lcount,
+              unsigned gp) {
+            GradLaunch c = a;
+            c.braBeg += ib0;
+            c.braOff = ib0;
+            c.nBra = n;
+            grad_plan_kernel<<<gp, 256, 0, ls>>>(c, mk, list64, list32, lcount);
+          });
     }
+  for (int i = 0; i < NAUX; i++) {
+    CQF_GCUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
+    CQF_GCUDA(cudaStreamWaitEvent(st, B->evJoin[i], 0));
+  }
+  if (rc != CQF_OK) {
+    cudaFreeAsync(ws, st);
+    cudaFreeAsync(dAtom, st);
+    return rc;
+  }
   CQF_GCUDA(cudaGetLastError());
   // AX += 1/2 (A + A^T) per component and matrix (:2550-2560)
   for (int k = 0; k < nGrad * nMat; k++) {
@@ -359,7 +279,7 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   CQF_GCUDA(cudaStreamSynchronize(st));
   if (stats) {
     stats->quartets_total = (long long)h[0];
-    stats->quartets_screened = 0;
+    stats->quartets_screened = (long long)h[1];  // on one atom: the derivatives cancel
     stats->quartets_fp32 = 0;
     stats->quartets_fp64 = (long long)h[3];
     float ms = 0.f;

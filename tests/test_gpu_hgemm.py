@@ -10,7 +10,8 @@ import pytest
 
 import oracle as O
 from chronusq_public_b200.basis import BasisSet, Molecule, parse_gbs
-from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, GAUNT, LLSS, SSSS, DirectTPI,
+from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, GAUNT, LLSS, SSSS,
+                                              DirectGradContraction, DirectTPI,
                                               GTODirectRelERIContraction,
                                               GTODirectTPIContraction, TwoBodyContraction)
 from test_gpu_gaunt import OUTS_C, OUTS_X, gaunt_inputs
@@ -93,3 +94,22 @@ def test_engine_gaunt(name):
     GTODirectRelERIContraction(DirectTPI(bs)).twoBodyContract(lst, GAUNT)
     for m in OUTS_X + OUTS_C:
         assert max_rel(lst[m].AX, ref[m]) < 1e-11, m
+
+
+@pytest.mark.parametrize("name", sorted(BASES))
+def test_engine_gradient(name):
+    """J and K gradient contractions: two atoms share a quartet in every
+    arrangement, the quartets of one atom drop out."""
+    bs = basis(name)
+    N = bs.nbasis
+    rng = np.random.default_rng(64)
+    A = rng.standard_normal((N, N))
+    D = 0.1 * (A + A.T)
+    atoms = np.array([s.atom for s in bs.shells], dtype=np.int32)
+    ref = O.OracleBasis(bs).grad_contract([D, D], [O.COULOMB, O.EXCHANGE], atoms, 2)
+    cl = [[TwoBodyContraction(D, np.zeros((N, N), order="F"), True, t)
+           for t in (COULOMB, EXCHANGE)] for _ in range(6)]
+    DirectGradContraction(DirectTPI(bs)).gradTwoBodyContract(cl, atoms)
+    for g in range(6):
+        for m in range(2):
+            assert max_rel(cl[g][m].AX, np.asarray(ref[g][m])) < 1e-11, (g, m)
