@@ -803,7 +803,7 @@ void free_basis(cqf_basis* B) {
                     (void*)B->d_cart2shell, (void*)B->d_ws, (void*)B->d_counters,
                     (void*)B->d_flags, (void*)B->d_qLL, (void*)B->d_qSS, (void*)B->d_qG, (void*)B->d_qB,
                     (void*)B->d_relws, (void*)B->d_hg[0], (void*)B->d_hg[1], (void*)B->d_hg[2],
-                    (void*)B->d_hg[3]})
+                    (void*)B->d_hg[3], (void*)B->d_pairsHg})
       if (p) cudaFreeAsync(p, st);
     cudaStreamSynchronize(st);
   }
@@ -1182,8 +1182,11 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
   }
   for (int c = 0; c < NCLS; c++) {
     B->cls_pp_beg[c] = B->cls_cnt[c] ? B->h_pairs[B->cls_beg[c]].pp_off : 0;
-    for (int i = 0; i < B->cls_cnt[c]; i++)
-      B->cls_npp_max[c] = std::max(B->cls_npp_max[c], B->h_pairs[B->cls_beg[c] + i].npp);
+    for (int i = 0; i < B->cls_cnt[c]; i++) {
+      const int npp = B->h_pairs[B->cls_beg[c] + i].npp;
+      B->cls_npp_max[c] = std::max(B->cls_npp_max[c], npp);
+      B->cls_npp_sum[c] += npp;
+    }
   }
   B->h_schwarz.resize((size_t)nshell * nshell);
   CQF_CUDA(cudaMemcpyAsync(B->h_schwarz.data(), B->d_schwarz,
@@ -1431,6 +1434,8 @@ WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan
     }
   }
   L.maskWords = need == 0 ? 0 : std::max(row, std::min(need, MASK_CAP_WORDS));
+  // the engine cuts the words of contracted f classes into several items
+  if (plan && B->maxL > 2 && need > 0) L.maskWords = std::max(L.maskWords, HG_MIN_WORDS);
   // per word: the uint2 mask and one entry in each of the two word lists
   L.oMask = take(std::max<size_t>(2 * L.maskWords * (NAUX + 1), 1));
   L.total = off;

@@ -78,44 +78,44 @@ struct GradDig {
   __host__ __device__ static constexpr int tk(int q) { return q == 0 ? HG_PLAIN : HG_D3; }
   __host__ __device__ static constexpr int rtu(int q) { return q == 0 ? 6 : 1; }
   __host__ __device__ static constexpr int ctu(int q) { return q == 0 ? 1 : 3; }
+  __host__ __device__ static int stage(int la, int lb, int lc, int ld, int nk) {
+    return hg_her_stage(la, lb, lc, ld, nk);
+  }
   static __device__ __forceinline__ void digest(const GradLaunch& a, const HgQuartet& z) {
-    const PairDev &P = *z.P, &Q = *z.Q;
-    const int at[4] = {__ldg(a.shellAtom + P.shA), __ldg(a.shellAtom + P.shB),
-                       __ldg(a.shellAtom + Q.shA), __ldg(a.shellAtom + Q.shB)};
-    // the quartet's atoms, and the weight of the derivatives on A, B, C in
-    // each atom's (the one on D is minus their sum; d/dR = -d/dr)
-    int atom[4] = {at[0], 0, 0, 0}, n = 1;
-#pragma unroll
-    for (int k = 1; k < 4; k++) {
-      bool seen = false;
-#pragma unroll
-      for (int s = 0; s < 4; s++) seen = seen || (s < n && atom[s] == at[k]);
-      if (!seen) {
-#pragma unroll
-        for (int s = 1; s < 4; s++)
-          if (s == n) atom[s] = at[k];
-        n++;
-      }
-    }
-    auto atomOf = [&](int s) {
-      return s == 0 ? atom[0] : (s == 1 ? atom[1] : (s == 2 ? atom[2] : atom[3]));
-    };
+    const PairDev& P = *z.P;
+    const int aA = __ldg(a.shellAtom + P.shA), aB = __ldg(a.shellAtom + P.shB);
     const double *M0 = z.M[0], *M1 = z.M[1];
     const int m0 = z.ms[0], m1 = z.ms[1];
     const size_t nc2 = (size_t)a.ncart * a.ncart;
-    auto val = [&](int k, int ab, int cd) {
-      const int s = k / 3, x = k - 3 * s, t = atomOf(s);
-      const double w = t == at[3] ? -1.0 : 0.0;
-      const double* r = M0 + (size_t)(6 * ab + x) * m0 + cd;
-      return (w + (t == at[0])) * r[0] + (w + (t == at[1])) * r[(size_t)3 * m0] +
-             (w + (t == at[2])) * M1[(size_t)ab * m1 + 3 * cd + x];
+    // the nine derivatives on A, B and C; the one on D is minus their sum.
+    // Each atom gets the sum of its functions' (d/dR = -d/dr is the factor -1
+    // below)
+    auto val = [&](int q, int ab, int cd, double (&v)[9]) {
+#pragma unroll
+      for (int k = 0; k < 6; k++) v[k] = M0[hg_row(6 * ab + k, m0) + q * z.cw[0] + cd];
+#pragma unroll
+      for (int x = 0; x < 3; x++) v[6 + x] = M1[hg_row(ab, m1) + q * z.cw[1] + 3 * cd + x];
     };
-    for (int mt = 0; mt < a.nMat; mt++)
-      hg_digest_her(z, a.ncart, a.type[mt] != CQF_COULOMB, -1.0, true, a.Xc + mt * nc2, 3 * n,
-                    val, [&](int k) {
-                      const int s = k / 3, x = k - 3 * s;
-                      return a.Ac + ((size_t)(atomOf(s) * 3 + x) * a.nMat + mt) * nc2;
-                    });
+    for (int mt = 0; mt < a.nMat; mt++) {
+      if (mt > 0) __syncthreads();  // the last matrix's densities are done with
+      hg_digest_her<9>(
+          z, a.ncart, a.type[mt] != CQF_COULOMB, -1.0, true, a.Xc + mt * nc2, val,
+          [&](int q, size_t e, const double (&s)[9]) {
+            const int aC = __ldg(a.shellAtom + z.Q[q].shA), aD = __ldg(a.shellAtom + z.Q[q].shB);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const int t = k == 0 ? aA : (k == 1 ? aB : (k == 2 ? aC : aD));
+              if ((k > 0 && t == aA) || (k > 1 && t == aB) || (k > 2 && t == aC)) continue;
+              const double w = t == aD ? -1.0 : 0.0;
+              const double wa = w + (t == aA), wb = w + (t == aB), wc = w + (t == aC);
+#pragma unroll
+              for (int x = 0; x < 3; x++) {
+                const double v = wa * s[x] + wb * s[3 + x] + wc * s[6 + x];
+                if (v != 0.0) atomicAdd(a.Ac + ((size_t)(t * 3 + x) * a.nMat + mt) * nc2 + e, v);
+              }
+            }
+          });
+    }
   }
 };
 
@@ -164,14 +164,10 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   const size_t host = o.device_pointers ? 0 : (size_t)nMat * NN + (size_t)nGrad * nMat * NN;
   // then, per launch stream, the planning pass's masks and lists and four
   // counters
-  size_t need = 1, row = 1;
-  for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck <= cb; ck++) {
-      const size_t w = ((size_t)B->cls_cnt[ck] + WTILE - 1) / WTILE;
-      row = std::max(row, w);
-      need = std::max(need, (size_t)B->cls_cnt[cb] * w);
-    }
-  const size_t maskWords = std::max(row, std::min(need, MASK_CAP_WORDS));
+  size_t row = 1;
+  for (int c = 0; c < NCLS; c++)
+    row = std::max(row, ((size_t)B->cls_cnt[c] + WTILE - 1) / WTILE);
+  const size_t maskWords = std::max(row, MASK_CAP_WORDS);
   const size_t lists = (2 * maskWords + 2) * (NAUX + 1);
   const size_t fixed = ((size_t)nMat * nc2 + (size_t)nGrad * nMat * nc2 + host + 1) / 2 * 2;
   const size_t doubles = fixed + lists;

@@ -8,92 +8,148 @@ namespace cqf {
 
 // The reference's Hermitian updates of a real matrix (direct.hpp:1858-1918,
 // :2470-2520) with the sums over the other two components taken before the
-// atomic of each output element:
+// atomics of each output element:
 //   J(1,2) += X(4,3) I, J(4,3) += X(1,2) I;
 //   K(1,3), (4,2), (4,1), (2,3) += h X(4,2), X(1,3), X(2,3), X(4,1) I,
-// in the reference's roles of the four functions.  nCombo integrals per
-// element (derivative components), val(k, ab, cd) (components counted from
-// the chunk's first) into the accumulator acc(k); work units are (combo,
-// output element, a share of the contracted bra components when the outputs
-// alone do not fill the block).  xT: exchange densities are read with rows
-// and columns exchanged in the updates whose row is function 1 or 2 (the
-// gradient's orientation).
-template <class V, class Acc>
-__device__ __forceinline__ void hg_digest_her(const HgQuartet& z, size_t nc, bool exch, double f,
-                                              bool xT, const double* __restrict__ X, int nCombo,
-                                              V val, Acc acc) {
-  const PairDev &P = *z.P, &Q = *z.Q;
+// in the reference's roles of the four functions.  An element has NV
+// integrals (derivative components), val(q, ab, cd, v) of ket q (components
+// counted from the chunk's first); out(q, element, s) adds their sums, scaled.
+// The density blocks are read once into shared memory, in the orientation
+// their update wants.  Work units are (ket, output element), shared by a few
+// lanes where there are few.
+// xT: exchange densities are read with rows and columns exchanged in the
+// updates whose row is function 1 or 2 (the gradient's orientation).
+struct HgRoles {
+  bool pRef, swP, swQ;
+  double deg;
+};
+__device__ __forceinline__ HgRoles hg_roles(const PairDev& P, const PairDev& Q) {
+  HgRoles r;
+  r.pRef = P.lex >= Q.lex;
+  r.swP = P.shA != P.s1;
+  r.swQ = Q.shA != Q.s1;
+  const PairDev &R12 = r.pRef ? P : Q, &R34 = r.pRef ? Q : P;
+  r.deg = (R12.s1 == R12.s2 ? 1.0 : 2.0) * (R34.s1 == R34.s2 ? 1.0 : 2.0) *
+          (R12.s1 == R34.s1 && R12.s2 == R34.s2 ? 1.0 : 2.0);
+  return r;
+}
+__host__ __device__ inline int hg_her_stage(int la, int lb, int lc, int ld, int nk) {
+  const int nx = (ncart(la) + ncart(lb)) * (ncart(lc) + ncart(ld));
+  const int nj = ncart(la) * ncart(lb) + ncart(lc) * ncart(ld);
+  return nk * (nx > nj ? nx : nj);
+}
+template <int NV, class V, class Out>
+__device__ __forceinline__ void hg_digest_her(const HgQuartet& z, int nc, bool exch, double f,
+                                              bool xT, const double* __restrict__ X, V val,
+                                              Out out) {
+  const PairDev& P = *z.P;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int na = ncart(z.la), nb = ncart(z.lb), ncc = ncart(z.lc), nd = ncart(z.ld);
   const int nAB = z.ab1 - z.ab0, nCD = z.cd1 - z.cd0;
-  const bool pRef = P.lex >= Q.lex;
-  const bool swP = P.shA != P.s1, swQ = Q.shA != Q.s1;
-  const PairDev &R12 = pRef ? P : Q, &R34 = pRef ? Q : P;
-  const double deg = (R12.s1 == R12.s2 ? 1.0 : 2.0) * (R34.s1 == R34.s2 ? 1.0 : 2.0) *
-                     (R12.s1 == R34.s1 && R12.s2 == R34.s2 ? 1.0 : 2.0);
+  double* xs = z.st;
   if (!exch) {
-    const double v = 0.5 * f * deg;
     // rows of an output and of its density are the pair's first function
-    // (1, 3) or its second
-    for (int uu = tid; uu < nCombo * (nAB + nCD); uu += nt) {
-      const int k0 = uu / (nAB + nCD), u = uu - k0 * (nAB + nCD);
-      const bool toBra = u < nAB;
-      const bool to12 = toBra == pRef;  // the output pair is (1, 2)
-      const bool swO = toBra ? swP : swQ, swI = toBra ? swQ : swP;
-      const PairDev& O = toBra ? P : Q;
-      const PairDev& I = toBra ? Q : P;
-      const int nO2 = toBra ? nb : nd, nI2 = toBra ? nd : nb;
-      const int base = toBra ? z.cd0 : z.ab0, n = toBra ? nCD : nAB;
-      // X's row is the first function of (1, 2) but the second of (4, 3)
-      const bool rowFirstI = to12 ? swI : !swI;
-      double s = 0.0;
-      for (int k = 0; k < n; k++) {
-        const int p = base + k, i = p / nI2, j = p - i * nI2;
-        const int gi = I.cA + i, gj = I.cB + j;
-        s += (toBra ? val(k0, u, k) : val(k0, k, u - nAB)) *
-             __ldg(X + (rowFirstI ? gi + (size_t)gj * nc : gj + (size_t)gi * nc));
+    // (1, 3) or its second; X's row is the first function of (1, 2) but the
+    // second of (4, 3).  Per ket: X over ab (orders J(cd)), X over cd
+    const int per = nAB + nCD;
+    for (int uu = tid; uu < z.nk * per; uu += nt) {
+      const int q = uu / per, u = uu - q * per;
+      const PairDev& Q = z.Q[q];
+      const HgRoles ro = hg_roles(P, Q);
+      const bool bra = u < nAB;
+      const bool is12 = bra == ro.pRef, sw = bra ? ro.swP : ro.swQ;
+      const int p = bra ? z.ab0 + u : z.cd0 + u - nAB, n2 = bra ? nb : nd;
+      const int i = p / n2, j = p - i * n2;
+      const int gi = (bra ? P.cA : Q.cA) + i, gj = (bra ? P.cB : Q.cB) + j;
+      const bool rowFirst = is12 ? !sw : sw;
+      xs[uu] = __ldg(X + (rowFirst ? gi + (size_t)gj * nc : gj + (size_t)gi * nc));
+    }
+    __syncthreads();
+    for (int uu = tid; uu < z.nk * per; uu += nt) {
+      const int q = uu / per, u = uu - q * per;
+      if (!z.have(q)) continue;
+      const PairDev& Q = z.Q[q];
+      const HgRoles ro = hg_roles(P, Q);
+      const bool bra = u < nAB;
+      const double* x = xs + q * per + (bra ? nAB : 0);
+      double s[NV];
+#pragma unroll
+      for (int k = 0; k < NV; k++) s[k] = 0.0;
+      for (int k = 0; k < (bra ? nCD : nAB); k++) {
+        double v[NV];
+        val(q, bra ? u : k, bra ? k : u - nAB, v);
+#pragma unroll
+        for (int t = 0; t < NV; t++) s[t] += v[t] * x[k];
       }
-      const int p = toBra ? z.ab0 + u : z.cd0 + (u - nAB), i = p / nO2, j = p - i * nO2;
-      const int gi = O.cA + i, gj = O.cB + j;
-      const bool rowFirstO = to12 ? !swO : swO;
-      if (s != 0.0)
-        atomicAdd(acc(k0) + (rowFirstO ? gi + (size_t)gj * nc : gj + (size_t)gi * nc), v * s);
+      const bool is12 = bra == ro.pRef, sw = bra ? ro.swP : ro.swQ;
+      const int p = bra ? z.ab0 + u : z.cd0 + u - nAB, n2 = bra ? nb : nd;
+      const int i = p / n2, j = p - i * n2;
+      const int gi = (bra ? P.cA : Q.cA) + i, gj = (bra ? P.cB : Q.cB) + j;
+      const bool rowFirst = is12 ? !sw : sw;
+#pragma unroll
+      for (int k = 0; k < NV; k++) s[k] *= 0.5 * f * ro.deg;
+      out(q, rowFirst ? gi + (size_t)gj * nc : gj + (size_t)gi * nc, s);
     }
     return;
   }
-  const double h = 0.25 * f * deg;
-  const int total = 4 * nCombo * (na > nb ? na : nb) * (ncc > nd ? ncc : nd);
-  for (int up = 0; up < 4; up++) {
-    const bool f12 = up == 0 || up == 2, f34 = up == 0 || up == 3;  // first function of the pair
-    const bool row12 = up == 0 || up == 3, rowI12 = !xT && (up == 1 || up == 2);
-    const bool outA = (pRef ? f12 : f34) != swP, outC = (pRef ? f34 : f12) != swQ;
-    const bool rowBra = row12 == pRef, rowBraI = rowI12 == pRef;
-    const int no = outA ? na : nb, ni = outA ? nb : na;
-    const int ko = outC ? ncc : nd, ki = outC ? nd : ncc;
-    const int gO0 = outA ? P.cA : P.cB, gI0 = outA ? P.cB : P.cA;
-    const int hO0 = outC ? Q.cA : Q.cB, hI0 = outC ? Q.cB : Q.cA;
-    const int parts = total < nt ? ni : 1;
-    for (int uu = tid; uu < nCombo * no * ko * parts; uu += nt) {
-      const int k0 = uu / (no * ko * parts), u = uu - k0 * (no * ko * parts);
-      const int part = u / (no * ko), r = u - part * (no * ko), kO = r / no, bO = r - kO * no;
-      double s = 0.0;
+  // (output A or B) x (output C or D): from the roles, whether the output's
+  // row and the density's row are the bra's function.  (1,3), (2,3) have row
+  // (1,2) and read X with row (3,4); (4,2), (4,1) the reverse
+  const int nx = (na + nb) * (ncc + nd);
+  for (int uu = tid; uu < z.nk * nx; uu += nt) {
+    const int q = uu / nx, r = uu - q * nx, i = r / (ncc + nd), j = r - i * (ncc + nd);
+    const PairDev& Q = z.Q[q];
+    const HgRoles ro = hg_roles(P, Q);
+    const bool inA = i < na, inC = j < ncc;
+    // the output holds the first function of (3, 4): it has the other bra
+    // and the other ket function
+    const bool f34 = ro.pRef ? (!inC != ro.swQ) : (!inA != ro.swP);
+    const bool rowBra = (!xT && !f34) == ro.pRef;
+    const int gb = inA ? P.cA + i : P.cB + i - na, gk = inC ? Q.cA + j : Q.cB + j - ncc;
+    xs[uu] = __ldg(X + (rowBra ? gb + (size_t)gk * nc : gk + (size_t)gb * nc));
+  }
+  __syncthreads();
+  const int sh = hg_share(z.nk * nx, na < nb ? na : nb);
+  for (int uu = tid; uu < ((z.nk * nx) << sh); uu += nt) {
+    const int part = uu & ((1 << sh) - 1), w = uu >> sh, q = w / nx, r = w - q * nx;
+    if (!z.have(q)) continue;
+    const int kO2 = r / (na + nb), bO2 = r - kO2 * (na + nb);
+    const bool outA = bO2 < na, outC = kO2 < ncc;
+    const int bO = outA ? bO2 : bO2 - na, kO = outC ? kO2 : kO2 - ncc;
+    const int ni = outA ? nb : na, ki = outC ? nd : ncc;
+    const int abI = outA ? 1 : nb, cdI = outC ? 1 : nd;
+    const int ab0 = (outA ? bO * nb : bO) - z.ab0, cd0 = (outC ? kO * nd : kO) - z.cd0;
+    const PairDev& Q = z.Q[q];
+    const HgRoles ro = hg_roles(P, Q);
+    const double* xq = xs + q * nx + (outA ? na : 0) * (ncc + nd) + (outC ? ncc : 0);
+    double s[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) s[k] = 0.0;
 #pragma unroll 1
-      for (int bI = part; bI < ni; bI += parts) {
-        const int ab = (outA ? bO * nb + bI : bI * nb + bO) - z.ab0;
-        if (ab < 0 || ab >= nAB) continue;
-        const int gb = gI0 + bI;
-        for (int kI = 0; kI < ki; kI++) {
-          const int cd = (outC ? kO * nd + kI : kI * nd + kO) - z.cd0;
-          if (cd < 0 || cd >= nCD) continue;
-          const int gk = hI0 + kI;
-          s += val(k0, ab, cd) *
-               __ldg(X + (rowBraI ? gb + (size_t)gk * nc : gk + (size_t)gb * nc));
-        }
+    for (int bI = part; bI < ni; bI += 1 << sh) {
+      const int ab = ab0 + bI * abI;
+      if (ab < 0 || ab >= nAB) continue;
+      const double* x = xq + bI * (ncc + nd);
+      int cd = cd0;
+      for (int kI = 0; kI < ki; kI++, cd += cdI) {
+        if (cd < 0 || cd >= nCD) continue;
+        double v[NV];
+        val(q, ab, cd, v);
+#pragma unroll
+        for (int t = 0; t < NV; t++) s[t] += v[t] * x[kI];
       }
-      const int go = gO0 + bO, gp = hO0 + kO;
-      if (s != 0.0)
-        atomicAdd(acc(k0) + (rowBra ? go + (size_t)gp * nc : gp + (size_t)go * nc), h * s);
     }
+    if (sh > 0) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) s[k] = hg_group_sum(s[k], sh);
+      if (part) continue;
+    }
+    const bool f34 = ro.pRef ? (outC != ro.swQ) : (outA != ro.swP);
+    const bool rowBra = f34 == ro.pRef;
+    const int go = (outA ? P.cA : P.cB) + bO, gp = (outC ? Q.cA : Q.cB) + kO;
+#pragma unroll
+    for (int k = 0; k < NV; k++) s[k] *= 0.25 * f * ro.deg;
+    out(q, rowBra ? go + (size_t)gp * nc : gp + (size_t)go * nc, s);
   }
 }
 

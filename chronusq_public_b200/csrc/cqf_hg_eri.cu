@@ -15,20 +15,25 @@ namespace {
 template <bool CPLX>
 __device__ __forceinline__ void eri_digest_any(const JKLaunch& a, const HgQuartet& z, int fl,
                                                const double* __restrict__ X, double* A) {
-  const PairDev &P = *z.P, &Q = *z.Q;
+  const PairDev& P = *z.P;
   const int nb = ncart(z.lb), nd = ncart(z.ld), nCD = z.cd1 - z.cd0;
-  const bool pRef = P.lex >= Q.lex;
-  const bool swP = P.shA != P.s1, swQ = Q.shA != Q.s1;
-  const PairDev &R12 = pRef ? P : Q, &R34 = pRef ? Q : P;
-  const double deg = (R12.s1 == R12.s2 ? 1.0 : 2.0) * (R34.s1 == R34.s2 ? 1.0 : 2.0) *
-                     (R12.s1 == R34.s1 && R12.s2 == R34.s2 ? 1.0 : 2.0);
-  for (int e = threadIdx.x; e < (z.ab1 - z.ab0) * nCD; e += blockDim.x) {
+  const int per = (z.ab1 - z.ab0) * nCD;
+  for (int uu = threadIdx.x; uu < z.nk * per; uu += blockDim.x) {
+    const int q = uu / per, e = uu - q * per;
+    if (!z.have(q)) continue;
+    const PairDev& Q = z.Q[q];
+    const bool pRef = P.lex >= Q.lex;
+    const bool swP = P.shA != P.s1, swQ = Q.shA != Q.s1;
+    const PairDev &R12 = pRef ? P : Q, &R34 = pRef ? Q : P;
+    const double deg = (R12.s1 == R12.s2 ? 1.0 : 2.0) * (R34.s1 == R34.s2 ? 1.0 : 2.0) *
+                       (R12.s1 == R34.s1 && R12.s2 == R34.s2 ? 1.0 : 2.0);
     const int r = e / nCD, c = e - r * nCD, ab = z.ab0 + r, cd = z.cd0 + c;
     const int ga = P.cA + ab / nb, gb = P.cB + ab % nb, gc = Q.cA + cd / nd, gd = Q.cB + cd % nd;
     const int pa = swP ? gb : ga, pb = swP ? ga : gb;
     const int qc = swQ ? gd : gc, qd = swQ ? gc : gd;
     digest_one<CPLX>(fl, X, A, a.ncart, pRef ? pa : qc, pRef ? pb : qd, pRef ? qc : pa,
-                     pRef ? qd : pb, 0.5 * deg * z.M[0][(size_t)r * z.ms[0] + c]);
+                     pRef ? qd : pb,
+                     0.5 * deg * z.M[0][hg_row(r, z.ms[0]) + q * z.cw[0] + c]);
   }
 }
 
@@ -40,17 +45,28 @@ struct EriDig {
   __host__ __device__ static constexpr int tk(int) { return HG_PLAIN; }
   __host__ __device__ static constexpr int rtu(int) { return 1; }
   __host__ __device__ static constexpr int ctu(int) { return 1; }
+  __host__ __device__ static int stage(int la, int lb, int lc, int ld, int nk) {
+    return CPLX ? 0 : hg_her_stage(la, lb, lc, ld, nk);
+  }
   static __device__ __forceinline__ void digest(const JKLaunch& a, const HgQuartet& z) {
     const size_t stride = (size_t)a.ncart * a.ncart * (CPLX ? 2 : 1);
     for (int m = 0; m < a.nMat; m++) {
       const int fl = __ldg(a.flags + m);
       const double* X = a.Xc + m * stride;
       double* A = a.Ac + m * stride;
-      if (!CPLX && (fl & 1))
-        hg_digest_her(z, a.ncart, fl & 2, 1.0, false, X, 1,
-                      [&](int, int ab, int cd) { return z.M[0][(size_t)ab * z.ms[0] + cd]; },
-                      [&](int) { return A; });
-      else eri_digest_any<CPLX>(a, z, fl, X, A);
+      if (!CPLX && (fl & 1)) {
+        if (m > 0) __syncthreads();  // the last matrix's densities are done with
+        hg_digest_her<1>(
+            z, a.ncart, fl & 2, 1.0, false, X,
+            [&](int q, int ab, int cd, double (&v)[1]) {
+              v[0] = z.M[0][hg_row(ab, z.ms[0]) + q * z.cw[0] + cd];
+            },
+            [&](int, size_t e, const double (&s)[1]) {
+              if (s[0] != 0.0) atomicAdd(A + e, s[0]);
+            });
+      } else {
+        eri_digest_any<CPLX>(a, z, fl, X, A);
+      }
     }
   }
 };

@@ -86,10 +86,35 @@ __global__ void __launch_bounds__(HT_THREADS)
   }
 }
 
+// The pairs with npp cut to the primitive pairs that can contribute: they are
+// sorted by their Schwarz bound, and one below 1e-34 (a tight primitive on
+// another centre, exp(-mu R^2) = 0) stays below rounding against any partner
+// and through four derivatives.
+__global__ void hg_pairs_kernel(const PairDev* __restrict__ in, const double* __restrict__ ppQ,
+                                int n, PairDev* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  PairDev P = in[i];
+  while (P.npp > 1 && ppQ[P.pp_off + P.npp - 1] < 1e-34) P.npp--;
+  out[i] = P;
+}
+
 }  // namespace
 
 cqf_status hg_ensure(cqf_basis* B, int kind) {
   if (B->d_hg[kind]) return CQF_OK;
+  if (!B->d_pairsHg) {
+    const int n = std::max(1, B->npair);
+    cudaError_t e = cudaMallocAsync((void**)&B->d_pairsHg, n * sizeof(PairDev), B->stream);
+    if (e == cudaSuccess) {
+      hg_pairs_kernel<<<(n + 127) / 128, 128, 0, B->stream>>>(B->d_pairs, B->d_ppQ, B->npair,
+                                                              B->d_pairsHg);
+      e = cudaGetLastError();
+    }
+    if (e != cudaSuccess)
+      return fail(e == cudaErrorMemoryAllocation ? CQF_ENOMEM : CQF_ECUDA,
+                  std::string("hg_ensure: ") + cudaGetErrorString(e));
+  }
   size_t total = 0;
   for (int c = 0; c < NCLS; c++) {
     B->hg_beg[kind][c] = total;

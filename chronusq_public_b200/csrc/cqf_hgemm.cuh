@@ -13,14 +13,17 @@
 // they are stored in the order in which a warp's A fragment reads them
 // (16 rows x 4 orders = 512 consecutive bytes).
 //
-// A block takes quartets one after the other from the planning pass's masks:
-// Boys values (one lane per primitive quartet, or one lane per order for a
-// single one), R level by level from a table of parents into a cube
-// [t][u][v] (so the index of h + h' is the sum of two table entries), G and
-// M in shared memory, then the digestion D::digest of the operator
-// components.  G sums over the ket primitives, M over the bra primitives, so
-// a contracted quartet is digested once.  Quartets whose components do not
-// fit in shared memory go in chunks of rows and columns.
+// A block takes one bra pair and a batch of its kets from the planning pass's
+// masks: the Boys values of a batch of primitive quartets (a lane each; for a
+// single one a lane per order), R level by level for the whole batch from a
+// table of parents into cubes [t][u][v] (so the index of h + h' is the sum of
+// two table entries), G and M in shared memory with the kets' columns side by
+// side, then the digestion D::digest of the operator components.  G sums over
+// the ket primitives, M over the bra primitives, so a contracted quartet is
+// digested once.  The s and p classes batch up to 32 kets and primitives (one
+// primitive quartet at a time the barriers and a nearly empty matrix tile
+// were most of their time); quartets whose components do not fit in shared
+// memory go one ket at a time in chunks of rows and columns.
 //
 // What bounds it: the per-thread kernels this replaces spent their time on
 // integer index work over local arrays at a few percent of the FP64 rate;
@@ -31,6 +34,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 
 #include "cqf_eri.cuh"
 #include "cqf_internal.hpp"
@@ -83,55 +87,75 @@ struct HgLaunch {
   const int* list32;
   const unsigned* lcount;          // lengths of the two lists
   unsigned* counter;               // next item
-  int nsub, parts;                 // items per word, and parts of a quartet's primitives
+  int nsub;                        // items per word (when items is null)
+  const uint2* items;              // or the list hg_expand_kernel made,
+  const unsigned* nItems;          // and its length
   int nru, ncu;                    // row / column units per chunk
+  int nk, nr;                      // kets and primitive quartets (a power of two) per batch
   HgSide bra[HG_MAXPASS], ket[HG_MAXPASS];
 };
 
-// One quartet's work as the digestion sees it: the components of rows
-// [ab0, ab1) and columns [cd0, cd1) are in M.
+// A batch as the digestion sees it: kets Q[0 .. nk), those with pre[q + 1] >
+// pre[q] computed; the components of rows [ab0, ab1) and columns [cd0, cd1)
+// of ket q are in M[pass] at column q * cw[pass].
 struct HgQuartet {
   const PairDev* P;
   const PairDev* Q;
-  int la, lb, lc, ld;
+  const int* pre;
+  int nk, la, lb, lc, ld;
   int ab0, ab1, cd0, cd1;
   const double* M[HG_MAXPASS];
-  int ms[HG_MAXPASS];              // row strides of M
+  int ms[HG_MAXPASS], cw[HG_MAXPASS];  // row strides of M (hg_row), columns per ket
+  double* st;                          // D::stage() doubles of shared memory
+  __device__ __forceinline__ bool have(int q) const { return pre[q + 1] > pre[q]; }
 };
+
+// Row r of M: stride ms (8 modulo 16: the fragments' stores hit every bank
+// once) and two more per four rows (the digestion reads M by rows, four per
+// component pair, from many threads at once).
+__host__ __device__ __forceinline__ int hg_row(int r, int ms) { return r * ms + 2 * (r >> 2); }
 
 // Shared-memory layout (doubles).
 struct HgLayout {
-  int L, S, FS;
-  int oF, oR0, oR1, oCube, oG[HG_MAXPASS], oM[HG_MAXPASS], oRec, oOff, oItem, total;
-  int ms[HG_MAXPASS], gs[HG_MAXPASS];
+  int L, S, FS, NH, RS, CS;        // strides of F, of a recursion buffer and of a cube (odd)
+  int oF, oR0, oR1, oCube, oG[HG_MAXPASS], oM[HG_MAXPASS], oSt, oRec, oOff, oKet, oPre, total;
+  int ms[HG_MAXPASS], gs[HG_MAXPASS], cw[HG_MAXPASS];
 };
 template <class D>
-__host__ __device__ inline HgLayout hg_layout(int la, int lb, int lc, int ld, int nru, int ncu) {
+__host__ __device__ inline HgLayout hg_layout(int la, int lb, int lc, int ld, int nru, int ncu,
+                                              int nk, int nr) {
   HgLayout o;
   const int lab = la + lb, lcd = lc + ld;
   o.L = lab + lcd + hg_rise(D::tb(0)) + hg_rise(D::tk(0));
   o.S = o.L + 1;
-  o.FS = (o.L + 5) | 1;  // F_0 .. F_L, X, Y, Z, alpha
+  o.FS = (o.L + 5) | 1;  // F_0 .. F_L, X, Y, Z
+  o.NH = nherm(o.L);
+  o.RS = nherm(o.L - 1) | 1;
+  o.CS = o.L * o.S * o.S + 1;  // t = L is the last index; L (L + 1)^2 is even
   int p = 0;
   auto take = [&](int n) { int r = p; p += (n + 1) / 2 * 2; return r; };
-  o.oF = take(32 * o.FS);
-  o.oR0 = take(nherm(o.L));
-  o.oR1 = take(nherm(o.L));
-  o.oCube = take(o.S * o.S * o.S);
+  o.oKet = take(32 * (int)(sizeof(PairDev) / sizeof(double)));
+  o.oPre = take(34);  // 33 prefix sums, the item, 32 first primitives
+  o.oF = take(nr * o.FS);
+  o.oR0 = take(nr * o.RS);
+  o.oR1 = take(nr * o.RS);
+  o.oCube = take(nr * o.CS);
   for (int q = 0; q < D::NP; q++) {
     const int rt = hg_tiles(D::tb(q), la, lb), ct = hg_tiles(D::tk(q), lc, ld);
     const int r = nru * D::rtu(q) < rt ? nru * D::rtu(q) : rt;
-    const int c = ncu * D::ctu(q) < ct ? ncu * D::ctu(q) : ct;
+    o.cw[q] = ncu * D::ctu(q) < ct ? ncu * D::ctu(q) * 16
+                                   : ncart(lc) * ncart(ld) * hg_ops(D::tk(q));
+    const int c = (nk * o.cw[q] + 15) / 16;
     // strides free of bank conflicts for the fragments' reads and writes
     o.gs[q] = c * 16 + 4;
     o.ms[q] = c * 16 + 8;
     const int hb = (nherm(lab + hg_rise(D::tb(q))) + 7) / 8 * 8;
     o.oG[q] = take(hb * o.gs[q]);
-    o.oM[q] = take(r * 16 * o.ms[q]);
+    o.oM[q] = take(r * 16 * o.ms[q] + r * 8);
   }
-  o.oRec = take((nherm(o.L) + 1) / 2);
-  o.oOff = take((nherm(o.L) + 1) / 2);
-  o.oItem = take(2);
+  o.oSt = take(D::stage(la, lb, lc, ld, nk));
+  o.oRec = take((o.NH + 1) / 2);
+  o.oOff = take((o.NH + 1) / 2);
   o.total = p;
   return o;
 }
@@ -207,50 +231,53 @@ __device__ __forceinline__ void hg_boys_lanes(const PrimPairDev& A, const PrimPa
   }
 }
 
-// R~ into the cube, level by level over the block; ends with a barrier.
+// R~ of nb <= nr primitive quartets (nr = 2^ln) into their cubes, level by
+// level over the block, the quartets in the fastest index; ends with a
+// barrier.
 template <typename T>
-__device__ __forceinline__ void hg_R(int L, const double* f, T* r0, T* r1, double* cube,
-                                     const unsigned* rec, const int* off) {
-  const T X = T(f[L + 1]), Y = T(f[L + 2]), Z = T(f[L + 3]);
+__device__ __forceinline__ void hg_R(const HgLayout& o, int ln, int nb, const double* F, T* r0,
+                                     T* r1, double* cube, const unsigned* rec, const int* off) {
+  const int L = o.L;
   for (int n = L; n >= 0; n--) {
     T* cur = (n & 1) ? r1 : r0;
     const T* prv = (n & 1) ? r0 : r1;
-    const int cnt = nherm(L - n);
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+    const int cnt = nherm(L - n) << ln;
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+      const int e = i >> ln, j = i & ((1 << ln) - 1);
+      if (j >= nb) continue;
+      const double* f = F + j * o.FS;
       T v;
       if (e == 0) {
         v = T(f[n]);
       } else {
         const unsigned w = rec[e];
-        const int ax = (w >> 20) & 3;
-        v = (ax == 0 ? X : (ax == 1 ? Y : Z)) * prv[w & 1023] +
-            T((int)(w >> 22)) * prv[(w >> 10) & 1023];
+        const T* p = prv + j * o.RS;
+        v = T(f[L + 1 + ((w >> 20) & 3)]) * p[w & 1023] +
+            T((int)(w >> 22)) * p[(w >> 10) & 1023];
       }
-      if (n > 0) cur[e] = v;
-      else cube[off[e] & 0x3fffffff] = double(v);
+      if (n > 0) cur[j * o.RS + e] = v;
+      else cube[j * o.CS + (off[e] & 0x3fffffff)] = double(v);
     }
     __syncthreads();
   }
 }
 
-// G[h][col] (+)= sum_h' K[col][h'] R~[h + h'] for ctn tiles of 16 columns of
-// one table (tab: its first tile), HB orders h.  A warp takes 8 orders and
-// up to two column tiles.
-__device__ __forceinline__ void hg_gemm1(const double* tab, int kt, int HK, int ctn, int HB,
-                                         const double* cube, const int* off, double* G, int gs,
+// G[h][col0 + c] (+)= sum over nj primitive quartets (cubes cs apart, tables
+// ksz apart) of sum_h' K[c][h'] R~[h + h'], c < cw, one item: 8 orders h (tile
+// nt) and up to two 16-column tiles from tile 2 m0 of ctn.
+__device__ __forceinline__ void hg_gemm1(const double* tab, size_t ksz, int nj, int kt, int HK,
+                                         int m0, int ctn, int nt, int HB, const double* cube,
+                                         int cs, const int* off, double* G, int gs, int cw,
                                          bool first) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const int nn = (HB + 7) / 8, mg = (ctn + 1) / 2;
-  const double2* t2 = reinterpret_cast<const double2*>(tab) + lane;
-  for (int it = warp; it < nn * mg; it += W) {
-    const int m0 = it / nn, nt = it - m0 * nn;
-    const int n = nt * 8 + (lane >> 2);
-    const double* rn = cube + (n < HB ? (off[n] & 0x3fffffff) : 0);
-    const bool two = 2 * m0 + 1 < ctn;
-    const double2* a0 = t2 + (size_t)(2 * m0) * kt * 32;
-    const double2* a1 = a0 + (size_t)kt * 32;
-    double c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
-    if (two) {
+  const int lane = threadIdx.x & 31;
+  const int n = nt * 8 + (lane >> 2);
+  const double* rn = cube + (n < HB ? (off[n] & 0x3fffffff) : 0);
+  const bool two = 2 * m0 + 1 < ctn;
+  const double2* a0 = reinterpret_cast<const double2*>(tab) + lane + (size_t)(2 * m0) * kt * 32;
+  double c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+  if (two) {
+    for (int j = 0; j < nj; j++, a0 += ksz / 2, rn += cs) {
+      const double2* a1 = a0 + (size_t)kt * 32;
 #pragma unroll 4
       for (int k = 0; k < kt; k++) {
         const int kk = 4 * k + (lane & 3);
@@ -259,35 +286,51 @@ __device__ __forceinline__ void hg_gemm1(const double* tab, int kt, int HK, int 
         hg_mma(c0, x, b);
         hg_mma(c1, y, b);
       }
-    } else {
+    }
+  } else if (kt == 1) {  // s kets: primitives in the inner loop, two chains
+    const double* rk = rn + ((lane & 3) < HK ? (off[lane & 3] & 0x3fffffff) : 0);
+    const size_t js = ksz / 2;
+    int j = 0;
 #pragma unroll 4
-      for (int k = 0; k < kt; k++) {
+    for (; j + 2 <= nj; j += 2) {
+      const double2 x = __ldg(a0 + j * js), y = __ldg(a0 + (j + 1) * js);
+      const double b0 = rk[j * cs], b1 = rk[(j + 1) * cs];
+      hg_mma(c0, x, b0);
+      hg_mma(c1, y, b1);
+    }
+    if (j < nj) hg_mma(c0, __ldg(a0 + j * js), rk[j * cs]);
+#pragma unroll
+    for (int t = 0; t < 4; t++) c0[t] += c1[t];
+  } else {
+    for (int j = 0; j < nj; j++, a0 += ksz / 2, rn += cs) {
+      int k = 0;
+#pragma unroll 2
+      for (; k + 2 <= kt; k += 2) {
+        const int k0 = 4 * k + (lane & 3), k1 = k0 + 4;
+        const double b0 = rn[off[k0] & 0x3fffffff];
+        const double b1 = rn[k1 < HK ? (off[k1] & 0x3fffffff) : 0];
+        const double2 x = __ldg(a0 + k * 32), y = __ldg(a0 + (k + 1) * 32);
+        hg_mma(c0, x, b0);
+        hg_mma(c1, y, b1);
+      }
+      if (k < kt) {
         const int kk = 4 * k + (lane & 3);
-        const double b = rn[kk < HK ? (off[kk] & 0x3fffffff) : 0];
-        hg_mma(c0, __ldg(a0 + k * 32), b);
+        hg_mma(c0, __ldg(a0 + k * 32), rn[kk < HK ? (off[kk] & 0x3fffffff) : 0]);
       }
     }
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int h = nt * 8 + 2 * (lane & 3) + j;
-      const double sg = (h < HB && ((off[h] >> 30) & 1)) ? -1.0 : 1.0;
-      double* g = G + (size_t)h * gs + 32 * m0 + (lane >> 2);
-      if (first) {
-        g[0] = sg * c0[j];
-        g[8] = sg * c0[2 + j];
-        if (two) {
-          g[16] = sg * c1[j];
-          g[24] = sg * c1[2 + j];
-        }
-      } else {
-        g[0] += sg * c0[j];
-        g[8] += sg * c0[2 + j];
-        if (two) {
-          g[16] += sg * c1[j];
-          g[24] += sg * c1[2 + j];
-        }
-      }
-    }
+    for (int t = 0; t < 4; t++) c0[t] += c1[t];
+  }
+  const int c = 32 * m0 + (lane >> 2);
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int h = nt * 8 + 2 * (lane & 3) + j;
+    const double sg = (h < HB && ((off[h] >> 30) & 1)) ? -1.0 : 1.0;
+    double* g = G + (size_t)h * gs + c;
+    const double v[4] = {sg * c0[j], sg * c0[2 + j], sg * c1[j], sg * c1[2 + j]};
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      if (c + 8 * t < cw && (t < 2 || two)) g[8 * t] = first ? v[t] : g[8 * t] + v[t];
   }
 }
 
@@ -310,9 +353,9 @@ __device__ __forceinline__ void hg_gemm2(const double* tab, int kt, int rtn, int
       hg_mma(c0, x, b0);
       hg_mma(c1, x, b1);
     }
-    double* m = M + (size_t)(16 * rt + (lane >> 2)) * ms + 16 * ct + 2 * (lane & 3);
+    double* m = M + hg_row(16 * rt + (lane >> 2), ms) + 16 * ct + 2 * (lane & 3);
     double2* m0 = reinterpret_cast<double2*>(m);
-    double2* m1 = reinterpret_cast<double2*>(m + 8 * (size_t)ms);
+    double2* m1 = reinterpret_cast<double2*>(m + hg_row(8, ms));
     double2 v0 = make_double2(c0[0], c0[1]), v1 = make_double2(c1[0], c1[1]);
     double2 w0 = make_double2(c0[2], c0[3]), w1 = make_double2(c1[2], c1[3]);
     if (!first) {
@@ -326,120 +369,196 @@ __device__ __forceinline__ void hg_gemm2(const double* tab, int kt, int rtn, int
   }
 }
 
+// Items of contracted classes: every listed word cut into at most `most`
+// parts of about `work` primitive quartets -- the bra's primitives in cb
+// ranges, the kets' (concatenated) in ck ones.  Without it the words of the
+// longest contractions (32 x 64 x 64 primitive quartets against a mean of a
+// few hundred) were the whole launch's tail: SMs were active for 22% of the
+// (ss|ss) gradient launch.  item = {word | FP32 << 31, b | cb << 8 | k << 16 |
+// ck << 24}.
+__global__ static void __launch_bounds__(128)
+    hg_expand_kernel(const PairDev* __restrict__ pairs, int braBeg, int ketBeg, int nTiles,
+                     const uint2* __restrict__ masks, const int* __restrict__ list64,
+                     const int* __restrict__ list32, const unsigned* __restrict__ lcount,
+                     int work, int most, uint2* __restrict__ items, unsigned* nItems) {
+  const int n64 = (int)lcount[0], n = n64 + (int)lcount[1];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const bool lo = i >= n64;
+    const int word = lo ? list32[i - n64] : list64[i];
+    const uint2 mk = masks[word];
+    const int ib = word / nTiles, jk0 = (word - ib * nTiles) * WTILE;
+    const int np = pairs[braBeg + ib].npp;
+    int nk = 0;
+    for (unsigned b = lo ? mk.y : mk.x; b; b &= b - 1u)
+      nk += pairs[ketBeg + jk0 + __ffs(b) - 1].npp;
+    const int want = max(1, min(most, (int)(((long long)np * nk + work - 1) / work)));
+    // the bra's primitives first: a batch holds ket primitives of one of them
+    const int cb = max(1, min(min(np, want), 255)), ck = max(1, min(nk, want / cb));
+    const unsigned at = atomicAdd(nItems, (unsigned)(cb * ck));
+    for (int b = 0; b < cb; b++)
+      for (int k = 0; k < ck; k++)
+        items[at + b * ck + k] =
+            make_uint2((unsigned)word | (lo ? 0x80000000u : 0u),
+                       (unsigned)b | (cb << 8) | (k << 16) | ((unsigned)ck << 24));
+  }
+}
+
 template <class D>
 __global__ void __launch_bounds__(256, 2)
     hg_kernel(const HgLaunch a, const typename D::Args args) {
   extern __shared__ double sm[];
   const int la = a.la, lb = a.lb, lc = a.lc, ld = a.ld;
   const int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld);
-  const HgLayout o = hg_layout<D>(la, lb, lc, ld, a.nru, a.ncu);
-  const int L = o.L, tid = threadIdx.x, nt = blockDim.x;
+  const HgLayout o = hg_layout<D>(la, lb, lc, ld, a.nru, a.ncu, a.nk, a.nr);
+  const int L = o.L, tid = threadIdx.x, nt = blockDim.x, cs = o.CS;
+  const int ln = 31 - __clz(a.nr);
+  const int warp = tid >> 5, W = nt >> 5;
   double* Fs = sm + o.oF;
   double* cube = sm + o.oCube;
   unsigned* rec = reinterpret_cast<unsigned*>(sm + o.oRec);
   int* off = reinterpret_cast<int*>(sm + o.oOff);
-  int* sitem = reinterpret_cast<int*>(sm + o.oItem);
-  for (int e = tid; e < nherm(L); e += nt) hg_index(e, o.S, rec[e], off[e]);
+  PairDev* Qs = reinterpret_cast<PairDev*>(sm + o.oKet);
+  int* pre = reinterpret_cast<int*>(sm + o.oPre);  // pre[q]: first primitive entry of ket q
+  int* sitem = pre + 34;
+  int* first = pre + 36;  // first[q]: ket q's first primitive of this item
+  for (int e = tid; e < o.NH; e += nt) hg_index(e, o.S, rec[e], off[e]);
   const int n64 = (int)a.lcount[0], n32 = (int)a.lcount[1];
-  const int nItems = (n64 + n32) * a.nsub * a.parts;
+  const int nItems = a.items ? (int)*a.nItems : (n64 + n32) * a.nsub;
   const int abU = a.nru * D::ABU, cdU = a.ncu * D::CDU;  // components per chunk
   for (;;) {
     if (tid == 0) *sitem = (int)atomicAdd(a.counter, 1u);
     __syncthreads();
     const int item = *sitem;
-    __syncthreads();
     if (item >= nItems) break;
-    const int part = item % a.parts, ws = item / a.parts;
-    const int sub = ws % a.nsub, w = ws / a.nsub;
-    const bool lo = w >= n64;
-    const int word = lo ? __ldg(a.list32 + (w - n64)) : __ldg(a.list64 + w);
+    uint2 it = make_uint2(0, 0);
+    if (a.items) {
+      it = __ldg(a.items + item);
+    } else {
+      const int w = item / a.nsub;
+      it.x = w < n64 ? __ldg(a.list64 + w) : (__ldg(a.list32 + (w - n64)) | 0x80000000);
+      it.y = (1u << 8) | (1u << 24);
+    }
+    const bool lo = it.x >> 31;
+    const int word = (int)(it.x & 0x7fffffff);
     const uint2 mk = __ldg(a.masks + word);
-    const int span = 32 / a.nsub;
-    unsigned bits = (lo ? mk.y : mk.x) >> (sub * span);
-    if (span < 32) bits &= (1u << span) - 1u;
-    const int ib = word / a.nTiles, jk0 = (word - ib * a.nTiles) * WTILE + sub * span;
+    unsigned bits = lo ? mk.y : mk.x;
+    if (!a.items && a.nsub > 1) {  // a share of the word's kets
+      const int span = 32 / a.nsub;
+      bits &= ((1u << span) - 1u) << (item % a.nsub * span);
+    }
+    const int nBits = __popc(bits);
+    const int ib = word / a.nTiles, jk0 = (word - ib * a.nTiles) * WTILE;
     const PairDev P = a.pairs[a.braBeg + ib];
-    for (; bits; bits &= bits - 1u) {
-      const PairDev Q = a.pairs[a.ketBeg + jk0 + __ffs(bits) - 1];
-      const int nq = Q.npp, n = P.npp * nq;
-      const int k0 = (int)((long long)n * part / a.parts);
-      const int k1 = (int)((long long)n * (part + 1) / a.parts);
-      if (k0 == k1) continue;
-      const bool one = k1 - k0 == 1;
+    const int cb = (it.y >> 8) & 255, ip0 = P.npp * (int)(it.y & 255) / cb,
+              ip1 = P.npp * (int)((it.y & 255) + 1) / cb;
+    __syncthreads();  // every thread has read the item
+    // the word's kets, and the item's share of their concatenated primitives:
+    // ket q computes entries pre[q] .. pre[q + 1] - 1, from primitive first[q]
+    if (tid < 32) {
+      int n = 0;
+      if (tid < nBits) {
+        unsigned b = bits;
+        for (int q = 0; q < tid; q++) b &= b - 1u;
+        const PairDev Q = a.pairs[a.ketBeg + jk0 + __ffs(b) - 1];
+        Qs[tid] = Q;
+        n = Q.npp;
+      }
+      int s = n;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, s, d);
+        if (tid >= d) s += t;
+      }
+      const int all = __shfl_sync(0xffffffffu, s, 31);
+      const int ck = it.y >> 24, k = (it.y >> 16) & 255;
+      const int r0 = all * k / ck, r1 = all * (k + 1) / ck;
+      if (tid == 0) pre[0] = 0;
+      pre[tid + 1] = min(max(s, r0), r1) - r0;
+      first[tid] = max(r0 - (s - n), 0);
+    }
+    __syncthreads();
+    for (int q0 = 0; q0 < nBits; q0 += a.nk) {
+      const int q1 = min(q0 + a.nk, nBits), eb0 = pre[q0], eb1 = pre[q1];
+      const int total = eb1 - eb0;
+      if (total == 0) continue;
+      const bool one = total == 1 && ip1 - ip0 == 1;
       bool haveR = false;
       for (int cd0 = 0; cd0 < ncd; cd0 += cdU)
         for (int ab0 = 0; ab0 < nab; ab0 += abU) {
-          bool firstM = true;
-          for (int kb = k0; kb < k1; kb += 32) {
-            const int nb = min(32, k1 - kb);
-            if (!(one && haveR)) {
-              if (tid < 32) {
-                if (one) {
-                  const PrimPairDev& A = a.pp[P.pp_off + kb / nq];
-                  const PrimPairDev& B = a.pp[Q.pp_off + kb % nq];
-                  if (lo) hg_boys_lanes<float>(A, B, L, Fs, a.boys32, tid);
-                  else hg_boys_lanes<double>(A, B, L, Fs, a.boys, tid);
+          for (int ip = ip0; ip < ip1; ip++) {
+            for (int eb = eb0; eb < eb1; eb += a.nr) {
+              const int nb = min(a.nr, eb1 - eb);
+              if (!(one && haveR)) {
+                const PrimPairDev& A = a.pp[P.pp_off + ip];
+                if (nb == 1) {
+                  if (tid < 32) {
+                    int q = q0;
+                    while (pre[q + 1] <= eb) q++;
+                    const PrimPairDev& B = a.pp[Qs[q].pp_off + first[q] + eb - pre[q]];
+                    if (lo) hg_boys_lanes<float>(A, B, L, Fs, a.boys32, tid);
+                    else hg_boys_lanes<double>(A, B, L, Fs, a.boys, tid);
+                  }
                 } else if (tid < nb) {
-                  const PrimPairDev& A = a.pp[P.pp_off + (kb + tid) / nq];
-                  const PrimPairDev& B = a.pp[Q.pp_off + (kb + tid) % nq];
+                  int q = q0;
+                  while (pre[q + 1] <= eb + tid) q++;
+                  const PrimPairDev& B = a.pp[Qs[q].pp_off + first[q] + eb + tid - pre[q]];
                   if (lo) hg_boys<float>(A, B, L, Fs + tid * o.FS, a.boys32);
                   else hg_boys<double>(A, B, L, Fs + tid * o.FS, a.boys);
                 }
-              }
-              __syncthreads();
-            }
-            for (int j = 0; j < nb; j++) {
-              const int ip = (kb + j) / nq, iq = (kb + j) - ip * nq;
-              if (!(one && haveR)) {
-                const double* f = Fs + j * o.FS;
+                __syncthreads();
                 if (lo)
-                  hg_R<float>(L, f, reinterpret_cast<float*>(sm + o.oR0),
+                  hg_R<float>(o, ln, nb, Fs, reinterpret_cast<float*>(sm + o.oR0),
                               reinterpret_cast<float*>(sm + o.oR1), cube, rec, off);
                 else
-                  hg_R<double>(L, f, sm + o.oR0, sm + o.oR1, cube, rec, off);
+                  hg_R<double>(o, ln, nb, Fs, sm + o.oR0, sm + o.oR1, cube, rec, off);
                 haveR = true;
               }
-              const bool firstG = iq == 0 || kb + j == k0;
-              const bool lastG = iq == nq - 1 || kb + j == k1 - 1;
+              if (one && ab0 > 0) continue;  // G is there
+              int qa = q0;
+              while (pre[qa + 1] <= eb) qa++;
+              int qb = qa;
+              while (pre[qb + 1] < eb + nb) qb++;
 #pragma unroll
               for (int q = 0; q < D::NP; q++) {
                 const int TB = D::tb(q), TK = D::tk(q);
                 const int HB = nherm(la + lb + hg_rise(TB)), HK = nherm(lc + ld + hg_rise(TK));
-                const int ktk = (HK + 3) / 4;
+                const int ktk = (HK + 3) / 4, ksz = hg_size(TK, lc, ld);
                 const int ct0 = cd0 / D::CDU * D::ctu(q);
                 const int ctn = min(a.ncu * D::ctu(q), hg_tiles(TK, lc, ld) - ct0);
-                double* G = sm + o.oG[q];
-                if (!(one && ab0 > 0)) {
+                const int nn = (HB + 7) / 8, per = nn * ((ctn + 1) / 2);
+                for (int it = warp; it < (qb - qa + 1) * per; it += W) {
+                  const int k = qa + it / per, r = it % per;
+                  const int j0 = max(pre[k], eb), j1 = min(pre[k + 1], eb + nb);
+                  if (j0 >= j1) continue;
+                  const int iq = first[k] + j0 - pre[k];
                   const double* tk = a.ket[q].tab +
-                                     (size_t)(Q.pp_off + iq - a.ket[q].ppBeg) *
-                                         hg_size(TK, lc, ld) + (size_t)ct0 * ktk * 64;
-                  hg_gemm1(tk, ktk, HK, ctn, HB, cube, off, G, o.gs[q], firstG);
+                                     (size_t)(Qs[k].pp_off + iq - a.ket[q].ppBeg) * ksz +
+                                     (size_t)ct0 * ktk * 64;
+                  hg_gemm1(tk, ksz, j1 - j0, ktk, HK, r / nn, ctn, r % nn, HB,
+                           cube + (j0 - eb) * cs, cs, off, sm + o.oG[q] + (k - q0) * o.cw[q], o.gs[q],
+                           o.cw[q], j0 == pre[k]);
                 }
               }
               __syncthreads();
-              if (lastG) {
-#pragma unroll
-                for (int q = 0; q < D::NP; q++) {
-                  const int TB = D::tb(q);
-                  const int ktb = (nherm(la + lb + hg_rise(TB)) + 3) / 4;
-                  const int ct0 = cd0 / D::CDU * D::ctu(q);
-                  const int ctn = min(a.ncu * D::ctu(q), hg_tiles(D::tk(q), lc, ld) - ct0);
-                  const int rt0 = ab0 / D::ABU * D::rtu(q);
-                  const int rtn = min(a.nru * D::rtu(q), hg_tiles(TB, la, lb) - rt0);
-                  const double* tb = a.bra[q].tab +
-                                     (size_t)(P.pp_off + ip - a.bra[q].ppBeg) *
-                                         hg_size(TB, la, lb) + (size_t)rt0 * ktb * 64;
-                  hg_gemm2(tb, ktb, rtn, ctn, sm + o.oG[q], o.gs[q], sm + o.oM[q], o.ms[q],
-                           firstM);
-                }
-                firstM = false;
-                __syncthreads();
-              }
             }
+#pragma unroll
+            for (int q = 0; q < D::NP; q++) {
+              const int TB = D::tb(q);
+              const int ktb = (nherm(la + lb + hg_rise(TB)) + 3) / 4;
+              const int rt0 = ab0 / D::ABU * D::rtu(q);
+              const int rtn = min(a.nru * D::rtu(q), hg_tiles(TB, la, lb) - rt0);
+              const double* tb = a.bra[q].tab +
+                                 (size_t)(P.pp_off + ip - a.bra[q].ppBeg) * hg_size(TB, la, lb) +
+                                 (size_t)rt0 * ktb * 64;
+              hg_gemm2(tb, ktb, rtn, ((q1 - q0) * o.cw[q] + 15) / 16, sm + o.oG[q], o.gs[q],
+                       sm + o.oM[q], o.ms[q], ip == ip0);
+            }
+            __syncthreads();
           }
           HgQuartet z;
           z.P = &P;
-          z.Q = &Q;
+          z.Q = Qs + q0;
+          z.pre = pre + q0;
+          z.nk = q1 - q0;
           z.la = la; z.lb = lb; z.lc = lc; z.ld = ld;
           z.ab0 = ab0;
           z.ab1 = min(nab, ab0 + abU);
@@ -449,12 +568,30 @@ __global__ void __launch_bounds__(256, 2)
           for (int q = 0; q < D::NP; q++) {
             z.M[q] = sm + o.oM[q];
             z.ms[q] = o.ms[q];
+            z.cw[q] = o.cw[q];
           }
+          z.st = sm + o.oSt;
           D::digest(args, z);
           __syncthreads();
         }
     }
+    __syncthreads();  // before the next item is written
   }
+}
+
+// Sum over the 2^l lanes of a group (lanes of one group call together).
+__device__ __forceinline__ double hg_group_sum(double v, int l) {
+  const int lane = threadIdx.x & 31;
+  const unsigned mask = (l == 5 ? 0xffffffffu : ((1u << (1 << l)) - 1u)) << (lane & ~((1 << l) - 1));
+  for (int o = (1 << l) >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+// log2 of the lanes that share an exchange unit: enough units for the block,
+// at most 8 and not many more than the ni contracted bra components.
+__device__ __forceinline__ int hg_share(int units, int ni) {
+  int l = 0;
+  while (l < 3 && (units << l) < (int)blockDim.x && (1 << l) < ni) l++;
+  return l;
 }
 
 // Planning pass over the words (bra pair, 32 kets) of nBra x nKet quartets:
@@ -526,87 +663,129 @@ struct HgRegion {
   long long maskWords;
   unsigned* work;
 };
-// Chunk of rows and columns: as few chunks as fit in the shared memory of
-// two blocks per SM, else of one (the R cube and the recursion buffers of
-// the f classes take up to 60 KB by themselves); 0 rows when nothing fits.
+// Chunk of rows and columns, kets and primitive quartets per batch.  A class
+// whose components fit whole batches kets (up to 32) and primitives within
+// HG_SMEM_BATCH; else one ket at a time and as few chunks as fit in the
+// shared memory of two blocks per SM, or of one (the cube and the recursion
+// buffers of the f classes take up to 60 KB by themselves).  Returns the
+// bytes, 0 when nothing fits.
+constexpr size_t HG_SMEM_BATCH = 54 * 1024;
+constexpr int HG_BATCH_WARPS = 4;
 constexpr size_t HG_SMEM_TWO = 112 * 1024;
 constexpr size_t HG_SMEM_MAX = 224 * 1024;
 template <class D>
-inline size_t hg_chunk(int la, int lb, int lc, int ld, int& nru, int& ncu) {
+inline size_t hg_chunk(HgLaunch& a, int nkMax, int nrMax) {
+  const int la = a.la, lb = a.lb, lc = a.lc, ld = a.ld;
   const int nab = ncart(la) * ncart(lb), ncd = ncart(lc) * ncart(ld);
   const int ru = (nab + D::ABU - 1) / D::ABU, cu = (ncd + D::CDU - 1) / D::CDU;
-  nru = ncu = 0;
+  auto bytes = [&](int r, int c, int k, int n) {
+    return (size_t)hg_layout<D>(la, lb, lc, ld, r, c, k, n).total * sizeof(double);
+  };
+  a.nk = a.nr = 1;
+  if (bytes(ru, cu, 1, 1) <= HG_SMEM_BATCH) {
+    a.nru = ru;
+    a.ncu = cu;
+    // kets and primitives grow together (a batch has at least one primitive
+    // quartet per ket), then the primitives alone, up to a thread each
+    for (int n = 2; n <= 32; n *= 2) {
+      const int k = std::min(n, nkMax), r = n < 2 * nrMax ? n : a.nr;
+      if (bytes(ru, cu, k, r) > HG_SMEM_BATCH) break;
+      a.nk = k;
+      a.nr = r;
+    }
+    while (a.nr >= a.nk && 2 * a.nr <= 32 * HG_BATCH_WARPS && 2 * a.nr < 2 * nrMax &&
+           bytes(ru, cu, a.nk, 2 * a.nr) <= HG_SMEM_BATCH)
+      a.nr *= 2;
+    return bytes(ru, cu, a.nk, a.nr);
+  }
   for (size_t lim : {HG_SMEM_TWO, HG_SMEM_MAX}) {
     double best = 1e30;
-    size_t bytes = 0;
+    size_t got = 0;
     for (int c = 1; c <= cu; c++)
       for (int r = 1; r <= ru; r++) {
-        const size_t b = (size_t)hg_layout<D>(la, lb, lc, ld, r, c).total * sizeof(double);
+        const size_t b = bytes(r, c, 1, 1);
         if (b > lim) break;
         const int nc = (cu + c - 1) / c, nr = (ru + r - 1) / r;
         const double cost = nc * nr + 0.01 * (r + c);  // the smallest with this chunk count
         if (cost < best) {
           best = cost;
-          nru = r;
-          ncu = c;
-          bytes = b;
+          a.nru = r;
+          a.ncu = c;
+          got = b;
         }
       }
-    // a chunk of a single row tile leaves most warps idle: take one block
-    if (bytes && (best < 24.0 || lim == HG_SMEM_MAX)) return bytes;
+    // many chunks of few tiles leave most warps idle: take one block
+    if (got && (best < 24.0 || lim == HG_SMEM_MAX)) return got;
   }
   return 0;
 }
 
-// Warps per block from the products' size (matrix instructions per
-// primitive quartet): a warp for the s and p classes, eight from d shells on.
+// Warps per block from the products' size (matrix instructions per primitive
+// quartet) and the batch.
 template <class D>
-inline int hg_warps(int la, int lb, int lc, int ld) {
+inline int hg_warps(const HgLaunch& a) {
   long long m = 0;
   for (int q = 0; q < D::NP; q++) {
-    const int hb = nherm(la + lb + hg_rise(D::tb(q)));
-    const long long ct = hg_tiles(D::tk(q), lc, ld), rt = hg_tiles(D::tb(q), la, lb);
-    m += ct * ((hb + 7) / 8) * hg_ktiles(D::tk(q), lc, ld) + 2 * ct * rt * ((hb + 3) / 4);
+    const int hb = nherm(a.la + a.lb + hg_rise(D::tb(q)));
+    const long long ct = hg_tiles(D::tk(q), a.lc, a.ld), rt = hg_tiles(D::tb(q), a.la, a.lb);
+    m += ct * ((hb + 7) / 8) * hg_ktiles(D::tk(q), a.lc, a.ld) + 2 * ct * rt * ((hb + 3) / 4);
   }
-  return m <= 48 ? 1 : (m <= 200 ? 2 : (m <= 800 ? 4 : 8));
+  if (a.nr >= 32) return HG_BATCH_WARPS;
+  m *= std::max(a.nk, a.nr);
+  return m <= 24 ? 1 : (m <= 96 ? 2 : (m <= 400 ? 4 : 8));
+}
+
+// Chunk, batch, warps and shared memory of a launch; the search takes tens of
+// microseconds for the large classes, so each thread keeps what it found for
+// a class pair and batch limits.
+struct HgShape {
+  int nkMax = 0, nrMax = 0, nru = 0, ncu = 0, nk = 0, nr = 0, W = 0;
+  size_t smem = 0;
+};
+template <class D>
+inline const HgShape& hg_shape(HgLaunch a, int nkMax, int nrMax) {
+  static thread_local HgShape memo[NCLS][NCLS];
+  HgShape& m = memo[class_id(a.la, a.lb)][class_id(a.lc, a.ld)];
+  if (m.nkMax != nkMax || m.nrMax != nrMax) {
+    m.smem = hg_chunk<D>(a, nkMax, nrMax);
+    m.nkMax = nkMax; m.nrMax = nrMax;
+    m.nru = a.nru; m.ncu = a.ncu; m.nk = a.nk; m.nr = a.nr;
+    m.W = m.smem ? hg_warps<D>(a) : 0;
+  }
+  return m;
 }
 
 // Launches the engine on one class pair (la lb | lc ld) whose planning pass
-// wrote masks and lists of nWords words; nq: quartets at most, npMax: the
-// largest product of primitive-pair counts.  *counter is zero.
+// wrote masks and lists; nItems: items at most.  *counter is zero.
 template <class D>
-inline cqf_status hg_launch(HgLaunch a, const typename D::Args& args, long long nWords,
-                            long long nq, int npMax, int nsm, cudaStream_t st) {
-  const size_t smem = hg_chunk<D>(a.la, a.lb, a.lc, a.ld, a.nru, a.ncu);
-  if (!smem) return fail(CQF_ENOTSUP, "class does not fit in shared memory");
-  const int W = hg_warps<D>(a.la, a.lb, a.lc, a.ld);
-  if (cudaFuncSetAttribute(hg_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)HG_SMEM_MAX) != cudaSuccess)
-    return fail(CQF_ECUDA, "hg_kernel: shared-memory limit");
-  // resident blocks per SM: shared memory, 2048 threads, 32 blocks, and the
-  // 128 registers per thread of the launch bound
+inline cqf_status hg_launch(HgLaunch a, const typename D::Args& args, const HgShape& m,
+                            long long nItems, int device, int nsm, cudaStream_t st) {
+  if (!m.smem) return fail(CQF_ENOTSUP, "class does not fit in shared memory");
+  a.nru = m.nru; a.ncu = m.ncu; a.nk = m.nk; a.nr = m.nr;
+  // the shared-memory limit, once per device (always the same value)
+  static std::atomic<unsigned> limited{0};
+  const unsigned bit = 1u << (device & 31);
+  if (device > 31 || !(limited.load() & bit)) {
+    if (cudaFuncSetAttribute(hg_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)HG_SMEM_MAX) != cudaSuccess)
+      return fail(CQF_ECUDA, "hg_kernel: shared-memory limit");
+    limited.fetch_or(bit);
+  }
+  // resident blocks per SM: shared memory, and the 128 registers per thread
+  // of the launch bound
   const int occ = (int)std::max<size_t>(
-      1, std::min<size_t>(std::min<size_t>(HG_SMEM_MAX / (smem + 1024), 16 / W), 32));
-  const long long slots = (long long)nsm * occ;
-  // items: enough to fill the GPU four times over, by splitting the words'
-  // quartets first and then the quartets' primitives
-  a.nsub = 1;
-  while (a.nsub < 32 && nWords * a.nsub < 4 * slots) a.nsub *= 2;
-  a.parts = 1;
-  const long long items = std::min(nq, nWords * a.nsub);
-  while (a.parts * 2 <= npMax && items * a.parts < 4 * slots) a.parts *= 2;
+      1, std::min<size_t>(HG_SMEM_MAX / (m.smem + 1024), (size_t)(16 / m.W)));
   const unsigned grid =
-      (unsigned)std::max<long long>(1, std::min(slots, nWords * a.nsub * a.parts));
-  hg_kernel<D><<<grid, 32 * W, smem, st>>>(a, args);
+      (unsigned)std::max<long long>(1, std::min((long long)nsm * occ, nItems));
+  hg_kernel<D><<<grid, 32 * m.W, m.smem, st>>>(a, args);
   return CQF_OK;
 }
-
 template <class D, class Plan>
 inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, int nBra, int ketBeg,
                               int nKet, const HgRegion& r, const typename D::Args& args,
                               cudaStream_t st, Plan plan) {
   HgLaunch h{};
-  h.pairs = B->d_pairs;
+  h.pairs = B->d_pairsHg;
   h.pp = B->d_pp;
   h.boys = B->d_boys64;
   h.boys32 = B->d_boys32;
@@ -622,7 +801,20 @@ inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, in
     h.bra[q] = {B->d_hg[tb] + B->hg_beg[tb][cb], B->cls_pp_beg[cb]};
     h.ket[q] = {B->d_hg[tk] + B->hg_beg[tk][ck], B->cls_pp_beg[ck]};
   }
-  const int slab = (int)std::max<long long>(1, r.maskWords / h.nTiles);
+  const int npb = B->cls_npp_max[cb], npk = B->cls_npp_max[ck];
+  // contracted classes: words are cut by their number of primitive quartets,
+  // into at most `most` items of 8 B beside the word's mask and list entries
+  // (16 B).  As many as leave the launch in one slab, but at least 16 (and
+  // never more than a row of words leaves room for)
+  const bool cut = npb * npk > 1;
+  const long long room = 2 * r.maskWords;
+  const int most =
+      cut ? (int)std::min(std::min(255LL, room / h.nTiles - 2),
+                          std::max(16LL, room / ((long long)nBra * h.nTiles) - 2))
+          : 0;
+  const long long words = most > 1 ? room / (2 + most) : r.maskWords;
+  const int slab = (int)std::max<long long>(1, words / h.nTiles);
+  const long long fill = 16LL * B->nsm;  // items that keep the GPU busy
   for (int ib0 = 0; ib0 < nBra; ib0 += slab) {
     const int n = std::min(slab, nBra - ib0);
     const long long nWords = (long long)n * h.nTiles;
@@ -636,8 +828,28 @@ inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, in
     const unsigned gp =
         (unsigned)std::min<long long>(((nWords + 31) / 32 + 7) / 8, (long long)B->nsm * 8);
     plan(ib0, n, r.masks, list64, list32, r.work + 2, gp);
-    const cqf_status s = hg_launch<D>(h, args, nWords, (long long)n * nKet,
-                                      B->cls_npp_max[cb] * B->cls_npp_max[ck], B->nsm, st);
+    h.nsub = 1;
+    long long nItems;
+    if (most > 1) {
+      uint2* items = r.masks + 2 * nWords;
+      h.items = items;
+      h.nItems = r.work + 1;
+      // a part's primitive quartets: the launch's (unscreened) number over
+      // the items that fill the GPU, at least a batch
+      const double all = (double)n / nBra * B->cls_npp_sum[cb] * B->cls_npp_sum[ck];
+      const int part = (int)std::min(
+          1024.0, std::max((double)hg_shape<D>(h, 32, 32 * npk).nr, all / fill));
+      hg_expand_kernel<<<(unsigned)std::min<long long>((nWords + 127) / 128, B->nsm * 8), 128, 0,
+                         st>>>(h.pairs, h.braBeg, ketBeg, h.nTiles, r.masks, list64, list32,
+                               h.lcount, part, most, items, r.work + 1);
+      nItems = nWords * most;
+    } else {
+      h.items = nullptr;
+      while (h.nsub < 32 && nWords * h.nsub < fill) h.nsub *= 2;
+      nItems = nWords * h.nsub;
+    }
+    const HgShape& m = hg_shape<D>(h, 32 / h.nsub, 32 / h.nsub * npk);
+    const cqf_status s = hg_launch<D>(h, args, m, nItems, B->device, B->nsm, st);
     if (s != CQF_OK) return s;
   }
   return CQF_OK;

@@ -100,8 +100,10 @@ struct WsLayout {
   size_t maskWords;  // mask words of each launch stream's region
 };
 // plan = false leaves the masks of a complex contraction out (its class pairs
-// with f shells then run on the generic kernel): what the fixed scratch of
-// the no-alloc entry point falls back to.
+// with f shells then run on the generic kernel) and the engine's minimum of
+// them (HG_MIN_WORDS): what the fixed scratch of the no-alloc entry point
+// falls back to.
+constexpr size_t HG_MIN_WORDS = size_t(1) << 16;
 WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan = true);
 // J and K of a class pair with an f shell (cqf_hg_eri.cu).
 cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* masks,
@@ -260,7 +262,10 @@ struct cqf_basis {
   // where each class's begin (doubles; the class's first primitive pair)
   double* d_hg[cqf::HG_NKIND] = {};
   size_t hg_beg[cqf::HG_NKIND][cqf::NCLS] = {};
+  // first primitive pair of a class, most per pair, and all of them
   int cls_pp_beg[cqf::NCLS] = {0}, cls_npp_max[cqf::NCLS] = {0};
+  long long cls_npp_sum[cqf::NCLS] = {0};
+  cqf::PairDev* d_pairsHg = nullptr;  // the pairs with their negligible primitives cut off
   void* d_relws = nullptr;
   size_t relws_bytes = 0;
   std::mutex mu;

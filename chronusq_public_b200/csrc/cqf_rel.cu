@@ -171,16 +171,15 @@ __global__ void __launch_bounds__(256)
           });
 }
 
-// left product (i f)^[a > 0] sigma_a d of a Pauli quaternion: a permutation
-// of its components with signs
-__device__ __forceinline__ Q4 left_sigma(const Q4& d, int a, double f) {
+// left product i^[a > 0] sigma_a d of a Pauli quaternion: a permutation of
+// its components with signs
+__device__ __forceinline__ Q4 left_sigma(const Q4& d, int a) {
   if (a == 0) return d;
-  // sigma_k (s + v.sigma) = v_k + s sigma_k + i (k x v).sigma; times i f
-  auto fi = [f](double2 z) { return make_double2(-f * z.y, f * z.x); };  // i f z
-  auto fr = [f](double2 z, double g) { return make_double2(f * g * z.x, f * g * z.y); };
-  if (a == 1) return Q4{fi(d.x), fi(d.s), fr(d.z, 1.0), fr(d.y, -1.0)};
-  if (a == 2) return Q4{fi(d.y), fr(d.z, -1.0), fi(d.s), fr(d.x, 1.0)};
-  return Q4{fi(d.z), fr(d.y, 1.0), fr(d.x, -1.0), fi(d.s)};
+  // sigma_k (s + v.sigma) = v_k + s sigma_k + i (k x v).sigma; times i
+  auto neg = [](double2 z) { return make_double2(-z.x, -z.y); };
+  if (a == 1) return Q4{ctimes_i(d.x), ctimes_i(d.s), d.z, neg(d.y)};
+  if (a == 2) return Q4{ctimes_i(d.y), neg(d.z), ctimes_i(d.s), d.x};
+  return Q4{ctimes_i(d.z), d.y, neg(d.x), ctimes_i(d.s)};
 }
 // sum_b (i f)^[b > 0] t_b sigma_b of four quaternions of 8 reals each
 __device__ __forceinline__ Q4 right_sigmas(const double (&t)[4][8], double f) {
@@ -204,8 +203,8 @@ __device__ __forceinline__ Q4 right_sigmas(const double (&t)[4][8], double f) {
 // TYPE 2: M[(ab, op)][(cd, op')]): the reference's updates with the sums
 // over the other two component indices taken before the one atomic of each
 // output element (J: over cd or ab; K: over the two contracted indices).
-// Work units of the exchange are (target, its bra and ket component, a share
-// of the contracted bra components); a unit sums m times the density over
+// Work units of the exchange are (target, its bra and ket component), shared
+// by a few lanes where there are few; a unit sums m times the density over
 // its elements per operator and applies the Pauli matrices once at its end.
 // The element-wise digestion this replaces sent up to 36 atomics per element
 // (11.7e9 for one Ag atom's LLSS; the L2 takes 185e9 scattered ones per
@@ -213,125 +212,162 @@ __device__ __forceinline__ Q4 right_sigmas(const double (&t)[4][8], double f) {
 template <int TYPE>
 __device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& z) {
   constexpr int NB = TYPE == 2 ? 4 : 1;
-  const PairDev &P = *z.P, &Q = *z.Q;
-  const int tid = threadIdx.x, nt = blockDim.x, ms = z.ms[0];
-  const double* M = z.M[0];
+  const PairDev& P = *z.P;
+  const int tid = threadIdx.x, nt = blockDim.x, ms = z.ms[0], msab = 4 * ms + 2;
   const size_t nc = a.ncart;
   auto ix = [nc](int r, int c) -> size_t { return (size_t)r + (size_t)c * nc; };
   const int na = ncart(z.la), nb = ncart(z.lb), ncc = ncart(z.lc), nd = ncart(z.ld);
   const int nAB = z.ab1 - z.ab0, nCD = z.cd1 - z.cd0;
-  const bool dAB = P.shA == P.shB, dCD = Q.shA == Q.shB, samePQ = P.lex == Q.lex;
-  const double s12d = dAB ? 1.0 : 2.0, s34d = dCD ? 1.0 : 2.0;
+  const bool dAB = P.shA == P.shB;
+  const double s12d = dAB ? 1.0 : 2.0;
   // the back transform adds the transpose (Hermitian completion): a
   // contribution on a pair's own diagonal block is counted twice there
-  const double w12 = dAB ? 0.5 : 1.0, w34 = dCD ? 0.5 : 1.0;
-  // Coulomb SS(1,2) from D(4,3) (:1145-1190, :2342-2380): unit (ab, op)
+  const double w12 = dAB ? 0.5 : 1.0;
+  // the densities the batch needs, in shared memory: Coulomb vectors in the
+  // order of M's rows and columns, exchange blocks (A then B) x (C then D) of
+  // each ket, 8 reals an element
+  const int nx = (na + nb) * (ncc + nd);
+  double* xk = z.st;
+  double* xab = xk + (size_t)z.nk * nx * 8;
+  double* xcd = xab + 4 * na * nb;
+  const double* const* const Xss = a.Xss;
   for (int u = tid; u < nAB * 4; u += nt) {
-    const double* m = M + (size_t)u * ms;
-    double s = 0.0;
-    for (int k = 0; k < nCD; k++) {
-      const int cd = z.cd0 + k, c = cd / nd, d = cd - c * nd;
-      const size_t e = ix(Q.cB + d, Q.cA + c);
-      if (TYPE == 1)
-        s += m[k] * __ldg(a.Xll + 2 * e);
-      else
-        s += m[4 * k] * __ldg(a.Xss[0] + 2 * e) - m[4 * k + 1] * __ldg(a.Xss[1] + 2 * e + 1) -
-             m[4 * k + 2] * __ldg(a.Xss[2] + 2 * e + 1) -
-             m[4 * k + 3] * __ldg(a.Xss[3] + 2 * e + 1);
+    const int ab = z.ab0 + (u >> 2), ai = ab / nb, bi = ab - ai * nb, op = u & 3;
+    const size_t e = 2 * ix(P.cB + bi, P.cA + ai);
+    xab[u] = op == 0 ? __ldg(Xss[0] + e) : -__ldg(Xss[op] + e + 1);
+  }
+  for (int u = tid; u < z.nk * nCD * NB; u += nt) {
+    const int q = u / (nCD * NB), v = u - q * (nCD * NB), op = v % NB;
+    const int cd = z.cd0 + v / NB, c = cd / nd, d = cd - c * nd;
+    const size_t e = 2 * ix(z.Q[q].cB + d, z.Q[q].cA + c);
+    xcd[u] = TYPE == 1 ? __ldg(a.Xll + e)
+                       : (op == 0 ? __ldg(Xss[0] + e) : -__ldg(Xss[op] + e + 1));
+  }
+  if (a.exchange)
+    for (int u = tid; u < z.nk * nx * 4; u += nt) {
+      const int comp = u & 3, v = u >> 2, q = v / nx, r = v - q * nx;
+      const int i = r / (ncc + nd), j = r - i * (ncc + nd);
+      const int gB = i < na ? P.cA + i : P.cB + i - na;
+      const int gK = j < ncc ? z.Q[q].cA + j : z.Q[q].cB + j - ncc;
+      const size_t e = TYPE == 1 ? ix(gK, gB) : ix(gB, gK);
+      reinterpret_cast<double2*>(xk)[(size_t)v * 4 + comp] = ldz(a.Xk[comp], e);
     }
+  __syncthreads();
+  // Coulomb SS(1,2) from D(4,3) (:1145-1190, :2342-2380): unit (ket, ab, op)
+  for (int uu = tid; uu < z.nk * nAB * 4; uu += nt) {
+    const int q = uu / (nAB * 4), u = uu - q * (nAB * 4);
+    if (!z.have(q)) continue;
+    const PairDev& Q = z.Q[q];
+    const double* m = z.M[0] + hg_row(u, ms) + q * z.cw[0];
+    const double* x = xcd + q * nCD * NB;
+    double s = 0.0;
+    for (int k = 0; k < nCD * NB; k++) s += m[k] * x[k];
     const int ab = z.ab0 + (u >> 2), ai = ab / nb, bi = ab - ai * nb;
-    if (s != 0.0) atomicAdd(a.Jss[u & 3] + ix(P.cA + ai, P.cB + bi), w12 * s34d * s);
+    if (s != 0.0)
+      atomicAdd(a.Jss[u & 3] + ix(P.cA + ai, P.cB + bi),
+                w12 * (Q.shA == Q.shB ? 1.0 : 2.0) * s);
   }
   // Coulomb LL(3,4) / SS(3,4) from D(2,1) (SSSS: when the pairs differ):
-  // unit (cd, op')
-  if (TYPE == 1 || !samePQ)
-    for (int u = tid; u < nCD * NB; u += nt) {
-      double s = 0.0;
-      for (int k = 0; k < nAB; k++) {
-        const int ab = z.ab0 + k, ai = ab / nb, bi = ab - ai * nb;
-        const size_t e = ix(P.cB + bi, P.cA + ai);
-        const double* m = M + (size_t)(4 * k) * ms + u;
-        s += m[0] * __ldg(a.Xss[0] + 2 * e) - m[ms] * __ldg(a.Xss[1] + 2 * e + 1) -
-             m[2 * (size_t)ms] * __ldg(a.Xss[2] + 2 * e + 1) -
-             m[3 * (size_t)ms] * __ldg(a.Xss[3] + 2 * e + 1);
-      }
-      const int cd = z.cd0 + u / NB, c = cd / nd, d = cd - c * nd;
-      if (s != 0.0)
-        atomicAdd((TYPE == 1 ? a.Jll : a.Jss[u % NB]) + ix(Q.cA + c, Q.cB + d), w34 * s12d * s);
-    }
+  // unit (ket, cd, op')
+  for (int uu = tid; uu < z.nk * nCD * NB; uu += nt) {
+    const int q = uu / (nCD * NB), u = uu - q * (nCD * NB);
+    const PairDev& Q = z.Q[q];
+    if (!z.have(q) || (TYPE == 2 && P.lex == Q.lex)) continue;
+    const double* m = z.M[0] + q * z.cw[0] + u;
+    double s = 0.0;
+    for (int k = 0; k < nAB; k++, m += msab)
+      s += m[0] * xab[4 * k] + m[ms] * xab[4 * k + 1] + m[2 * ms] * xab[4 * k + 2] +
+           m[3 * ms] * xab[4 * k + 3];
+    const int cd = z.cd0 + u / NB, c = cd / nd, d = cd - c * nd;
+    if (s != 0.0)
+      atomicAdd((TYPE == 1 ? a.Jll : a.Jss[u % NB]) + ix(Q.cA + c, Q.cB + d),
+                (Q.shA == Q.shB ? 0.5 : 1.0) * s12d * s);
+  }
   if (!a.exchange) return;
   // exchange targets (bra index of the output A or B, ket index C or D):
   // LLSS (:1200-1299) K(c,b) -= D(d,a) P, K(c,a) -= D(d,b) P^(-), ...;
   // SSSS (:2381-2445) K(a,d) -= P D(b,c) P, K(a,c), K(b,d), K(b,c)
-  const int total = 4 * (na > nb ? na : nb) * (ncc > nd ? ncc : nd);
-  for (int tgt = 0; tgt < 4; tgt++) {
-    const bool outA = TYPE == 1 ? (tgt & 1) : tgt < 2;   // output bra index: A (else B)
-    const bool outC = TYPE == 1 ? tgt < 2 : (tgt & 1);   // output ket index: C (else D)
-    if (TYPE == 1 ? ((outA && dAB) || (!outC && dCD)) : ((!outA && dAB) || (outC && dCD))) continue;
+  // Units of the four targets side by side, each shared by 2^sh lanes.
+  const int both = (na + nb) * (ncc + nd);
+  const int sh = hg_share(z.nk * both, na < nb ? na : nb);
+  for (int uu = tid; uu < ((z.nk * both) << sh); uu += nt) {
+    const int part = uu & ((1 << sh) - 1), v = uu >> sh, q = v / both, r = v - q * both;
+    const int kO2 = r / (na + nb), bO2 = r - kO2 * (na + nb);
+    const bool outA = bO2 < na, outC = kO2 < ncc;
+    const PairDev& Q = z.Q[q];
+    if (!z.have(q) || (dAB && outA == (TYPE == 1)) ||
+        (Q.shA == Q.shB && outC == (TYPE == 2)))
+      continue;
+    const int bO = outA ? bO2 : bO2 - na, kO = outC ? kO2 : kO2 - ncc;
     const double f1 = TYPE == 1 ? (outA ? -1.0 : 1.0) : (outA ? 1.0 : -1.0);
     const double f2 = TYPE == 1 ? f1 : (outC ? -1.0 : 1.0);
-    const int no = outA ? na : nb, ni = outA ? nb : na;    // bra: output, contracted
-    const int ko = outC ? ncc : nd, ki = outC ? nd : ncc;  // ket
-    const int parts = total < nt ? ni : 1;
-    for (int u = tid; u < no * ko * parts; u += nt) {
-      const int part = u / (no * ko), r = u - part * (no * ko), kO = r / no, bO = r - kO * no;
-      double t[4][8];
+    const int ni = outA ? nb : na, ki = outC ? nd : ncc;  // contracted components
+    const int abI = outA ? 1 : nb, cdI = outC ? 1 : nd;   // their steps in ab and cd
+    const int ab0 = (outA ? bO * nb : bO) - z.ab0, cd0 = (outC ? kO * nd : kO) - z.cd0;
+    const double* Mq = z.M[0] + q * z.cw[0];
+    const double* xq = xk + ((size_t)q * nx + (outA ? na : 0) * (ncc + nd) + (outC ? ncc : 0)) * 8;
+    double t[4][8];
 #pragma unroll
-      for (int b = 0; b < 4; b++)
+    for (int b = 0; b < 4; b++)
 #pragma unroll
-        for (int k = 0; k < 8; k++) t[b][k] = 0.0;
-      bool any = false;
+      for (int k = 0; k < 8; k++) t[b][k] = 0.0;
+    bool any = false;
 #pragma unroll 1
-      for (int bI = part; bI < ni; bI += parts) {
-        const int ab = (outA ? bO * nb + bI : bI * nb + bO) - z.ab0;
-        if (ab < 0 || ab >= nAB) continue;
+    for (int bI = part; bI < ni; bI += 1 << sh) {
+      const int ab = ab0 + bI * abI;
+      if (ab < 0 || ab >= nAB) continue;
+      const double* mr = Mq + ab * msab;
+      const double* xr = xq + (size_t)bI * (ncc + nd) * 8;
+      int cd = cd0;
 #pragma unroll 1
-        for (int kI = 0; kI < ki; kI++) {
-          const int cd = (outC ? kO * nd + kI : kI * nd + kO) - z.cd0;
-          if (cd < 0 || cd >= nCD) continue;
-          any = true;
-          const int gB = (outA ? P.cB : P.cA) + bI, gK = (outC ? Q.cB : Q.cA) + kI;
-          const size_t e = TYPE == 1 ? ix(gK, gB) : ix(gB, gK);
-          const Q4 d{ldz(a.Xk[0], e), ldz(a.Xk[1], e), ldz(a.Xk[2], e), ldz(a.Xk[3], e)};
-          const double* m = M + (size_t)(4 * ab) * ms + NB * cd;
-          if (TYPE == 1) {
-            // (D (m0 + i f m.sigma)): per operator m_op D
+      for (int kI = 0; kI < ki; kI++, cd += cdI, xr += 8) {
+        if (cd < 0 || cd >= nCD) continue;
+        any = true;
+        const double2* x2 = reinterpret_cast<const double2*>(xr);
+        const Q4 d{x2[0], x2[1], x2[2], x2[3]};
+        const double* m = mr + NB * cd;
+        if (TYPE == 1) {
+          // (D (m0 + i f m.sigma)): per operator m_op D
 #pragma unroll
-            for (int op = 0; op < 4; op++) {
-              const double v = m[(size_t)op * ms];
-              t[op][0] += v * d.s.x; t[op][1] += v * d.s.y;
-              t[op][2] += v * d.x.x; t[op][3] += v * d.x.y;
-              t[op][4] += v * d.y.x; t[op][5] += v * d.y.y;
-              t[op][6] += v * d.z.x; t[op][7] += v * d.z.y;
-            }
-          } else {
+          for (int op = 0; op < 4; op++) {
+            const double v = m[op * ms];
+            t[op][0] += v * d.s.x; t[op][1] += v * d.s.y;
+            t[op][2] += v * d.x.x; t[op][3] += v * d.x.y;
+            t[op][4] += v * d.y.x; t[op][5] += v * d.y.y;
+            t[op][6] += v * d.z.x; t[op][7] += v * d.z.y;
+          }
+        } else {
 #pragma unroll
-            for (int op = 0; op < 4; op++) {
-              const Q4 l = left_sigma(d, op, f1);
-              const double2 m01 = *reinterpret_cast<const double2*>(m + (size_t)op * ms);
-              const double2 m23 = *reinterpret_cast<const double2*>(m + (size_t)op * ms + 2);
-              const double v[4] = {m01.x, m01.y, m23.x, m23.y};
+          for (int op = 0; op < 4; op++) {
+            const Q4 l = left_sigma(d, op);
+            const double2 m01 = *reinterpret_cast<const double2*>(m + op * ms);
+            const double2 m23 = *reinterpret_cast<const double2*>(m + op * ms + 2);
+            const double g = op == 0 ? 1.0 : f1;
+            const double v[4] = {g * m01.x, g * m01.y, g * m23.x, g * m23.y};
 #pragma unroll
-              for (int b = 0; b < 4; b++) {
-                t[b][0] += v[b] * l.s.x; t[b][1] += v[b] * l.s.y;
-                t[b][2] += v[b] * l.x.x; t[b][3] += v[b] * l.x.y;
-                t[b][4] += v[b] * l.y.x; t[b][5] += v[b] * l.y.y;
-                t[b][6] += v[b] * l.z.x; t[b][7] += v[b] * l.z.y;
-              }
+            for (int b = 0; b < 4; b++) {
+              t[b][0] += v[b] * l.s.x; t[b][1] += v[b] * l.s.y;
+              t[b][2] += v[b] * l.x.x; t[b][3] += v[b] * l.x.y;
+              t[b][4] += v[b] * l.y.x; t[b][5] += v[b] * l.y.y;
+              t[b][6] += v[b] * l.z.x; t[b][7] += v[b] * l.z.y;
             }
           }
         }
       }
-      if (!any) continue;
-      const Q4 k4 = right_sigmas(t, f2);
-      const int gO = (outA ? P.cA : P.cB) + bO, gP = (outC ? Q.cA : Q.cB) + kO;
-      const size_t e = TYPE == 1 ? ix(gP, gO) : ix(gO, gP);
-      const double w = TYPE == 2 && samePQ ? -0.5 : -1.0;
-      addz(a.K[0], e, k4.s, w);
-      addz(a.K[1], e, k4.x, w);
-      addz(a.K[2], e, k4.y, w);
-      addz(a.K[3], e, k4.z, w);
     }
+    const Q4 k4 = right_sigmas(t, f2);
+    double o8[8] = {k4.s.x, k4.s.y, k4.x.x, k4.x.y, k4.y.x, k4.y.y, k4.z.x, k4.z.y};
+    if (sh > 0) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) o8[k] = hg_group_sum(o8[k], sh);
+      any = part == 0;
+    }
+    if (!any) continue;
+    const int gO = (outA ? P.cA : P.cB) + bO, gP = (outC ? Q.cA : Q.cB) + kO;
+    const size_t e = 2 * (TYPE == 1 ? ix(gP, gO) : ix(gO, gP));
+    const double w = TYPE == 2 && P.lex == Q.lex ? -0.5 : -1.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) atomicAdd(a.K[k >> 1] + e + (k & 1), w * o8[k]);
   }
 }
 
@@ -344,6 +380,11 @@ struct RelDig {
   __host__ __device__ static constexpr int tk(int) { return TYPE == 2 ? HG_SPIN : HG_PLAIN; }
   __host__ __device__ static constexpr int rtu(int) { return 1; }
   __host__ __device__ static constexpr int ctu(int) { return 1; }
+  __host__ __device__ static int stage(int la, int lb, int lc, int ld, int nk) {
+    return nk * ((ncart(la) + ncart(lb)) * (ncart(lc) + ncart(ld)) * 8 +
+                 ncart(lc) * ncart(ld) * (TYPE == 2 ? 4 : 1)) +
+           ncart(la) * ncart(lb) * 4;
+  }
   static __device__ __forceinline__ void digest(const RelLaunch& a, const HgQuartet& z) {
     rel_digest<TYPE>(a, z);
   }
@@ -719,13 +760,16 @@ struct GauntDig {
   __host__ __device__ static constexpr int tk(int) { return HG_D6; }
   __host__ __device__ static constexpr int rtu(int) { return 3; }
   __host__ __device__ static constexpr int ctu(int) { return 3; }
+  __host__ __device__ static constexpr int stage(int, int, int, int, int) { return 0; }
   static __device__ __forceinline__ void digest(const GauntLaunch& a, const HgQuartet& z) {
-    const PairDev &P = *z.P, &Q = *z.Q;
-    const unsigned alive = gaunt_alive(a, P, Q);
+    const PairDev& P = *z.P;
     const int nb = ncart(z.lb), nd = ncart(z.ld), nCD = z.cd1 - z.cd0;
-    for (int u = threadIdx.x; u < (z.ab1 - z.ab0) * nCD * 4; u += blockDim.x) {
+    const int per = (z.ab1 - z.ab0) * nCD * 4;
+    for (int uu = threadIdx.x; uu < z.nk * per; uu += blockDim.x) {
+      const int q = uu / per, u = uu - q * per;
+      const PairDev& Q = z.Q[q];
       const int blk = u & 3, e = u >> 2, r = e / nCD, c = e - r * nCD;
-      if (!(alive & (1u << blk))) continue;
+      if (!z.have(q) || !(gaunt_alive(a, P, Q) & (1u << blk))) continue;
       const int pb = blk >> 1, pk = blk & 1;
       const int ab = z.ab0 + r, cd = z.cd0 + c;
       const int gA = P.cA + ab / nb, gB = P.cB + ab % nb;
@@ -736,13 +780,14 @@ struct GauntDig {
       const int ydA = pk ? gD : gC, yoA = pk ? gC : gD;
       // the reference's orientation: bra X (j on X) or Y (j on Y)
       const bool xb = xd > yd || (xd == yd && xo >= yo);
-      const double* m = z.M[0] + (size_t)(r * 6 + pb * 3) * z.ms[0] + c * 6 + pk * 3;
+      const double* m = z.M[0] + q * z.cw[0] + c * 6 + pk * 3;
+      const int r0 = r * 6 + pb * 3, ms = z.ms[0];
       double v[9];
 #pragma unroll
       for (int j = 0; j < 3; j++)
 #pragma unroll
         for (int l = 0; l < 3; l++)
-          v[3 * j + l] = xb ? m[(size_t)j * z.ms[0] + l] : m[(size_t)l * z.ms[0] + j];
+          v[3 * j + l] = xb ? m[hg_row(r0 + j, ms) + l] : m[hg_row(r0 + l, ms) + j];
       if (xb) gaunt_sites(a, v, xo, xd, yd, yo, xoA, xdA, ydA, yoA);
       else gaunt_sites(a, v, yo, yd, xd, xo, yoA, ydA, xdA, xoA);
     }
@@ -1399,17 +1444,13 @@ size_t rel_core_doubles(const cqf_basis* B) {
   const size_t ga = align32(20 * 2 * nc2) + align32(16 * 2 * nc2) + align32(18 * ns2);
   return std::max(dc, ga) + 64;
 }
-// Mask words of one launch stream's region: the largest class pair (either
-// orientation) up to MASK_CAP_WORDS, at least one bra row of the widest class.
+// Mask words of one launch stream's region: the cap, and at least one bra row
+// of the widest class.
 long long rel_mask_words(const cqf_basis* B) {
-  size_t need = 1, row = 1;
-  for (int cb = 0; cb < NCLS; cb++)
-    for (int ck = 0; ck < NCLS; ck++) {
-      const size_t w = ((size_t)B->cls_cnt[ck] + WTILE - 1) / WTILE;
-      row = std::max(row, w);
-      need = std::max(need, (size_t)B->cls_cnt[cb] * w);
-    }
-  return (long long)std::max(row, std::min(need, MASK_CAP_WORDS));
+  size_t row = 1;
+  for (int c = 0; c < NCLS; c++)
+    row = std::max(row, ((size_t)B->cls_cnt[c] + WTILE - 1) / WTILE);
+  return (long long)std::max(row, MASK_CAP_WORDS);
 }
 // The contraction's arrays, then per launch stream the masks and word lists
 // (16 B a word), then four counters each.

@@ -247,11 +247,13 @@ unsigned long long cqf_fock_footprint(const cqf_shell* shells, int nshell) {
   // bases with f shells hold the Hermite-matrix engine's tables
   unsigned long long maxl = 0, tabs = 0;
   for (int s = 0; s < nshell; s++) maxl = std::max<unsigned long long>(maxl, shells[s].l);
-  if (maxl > 2)
+  if (maxl > 2) {
+    tabs = 3 * 16 * cqf::HG_MIN_WORDS;
     for (int s = 0; s < nshell; s++)
       for (int t = 0; t <= s; t++)
         tabs += 8ull * cqf::hg_size(cqf::HG_PLAIN, shells[s].l, shells[t].l) *
                 std::max(0, shells[s].nprim) * std::max(0, shells[t].nprim);
+  }
   return pairs + ws + tabs;
 }
 
