@@ -1434,8 +1434,10 @@ WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan
     }
   }
   L.maskWords = need == 0 ? 0 : std::max(row, std::min(need, MASK_CAP_WORDS));
-  // the engine cuts the words of contracted f classes into several items
-  if (plan && B->maxL > 2 && need > 0) L.maskWords = std::max(L.maskWords, HG_MIN_WORDS);
+  // the engine cuts the words of contracted f classes into several items,
+  // and the light class pairs list heavy words more than once
+  if (plan && need > 0)
+    L.maskWords = std::max(L.maskWords, B->maxL > 2 ? HG_MIN_WORDS : JK_MIN_WORDS);
   // per word: the uint2 mask and one entry in each of the two word lists
   L.oMask = take(std::max<size_t>(2 * L.maskWords * (NAUX + 1), 1));
   L.total = off;
@@ -1529,18 +1531,19 @@ void split_flags(const cqf_contraction* list, int nMat, int* fl) {
 }
 
 // Workspace (doubles) of split_core: the real contraction's | real X | real AX.
-size_t split_ws_doubles(const cqf_basis* B, int nReal, const cqf_opts& opts) {
+size_t split_ws_doubles(const cqf_basis* B, int nReal, const cqf_opts& opts, bool plan) {
   cqf_opts ro = opts;
   ro.is_complex = 0;
   ro.device_pointers = 1;
   const size_t blk = ((size_t)B->nbasis * B->nbasis + 31) / 32 * 32;
-  return ws_layout(B, nReal, ro).total + 2 * blk * nReal;
+  return ws_layout(B, nReal, ro, plan).total + 2 * blk * nReal;
 }
 
 // The split on device pointers and a caller-provided workspace; with
 // `capture` it only enqueues (stream capture), like contract_core.
 cqf_status split_core(cqf_basis* B, const cqf_contraction* list, int nMat, const cqf_opts& opts,
-                      cqf_stats* stats, double* ws, bool capture, const int* d_flags_pre) {
+                      cqf_stats* stats, double* ws, bool capture, const int* d_flags_pre,
+                      bool plan) {
   cudaStream_t st = opts.stream ? (cudaStream_t)opts.stream : B->stream;
   const size_t NN = (size_t)B->nbasis * B->nbasis;
   const size_t blk = (NN + 31) / 32 * 32;
@@ -1548,7 +1551,7 @@ cqf_status split_core(cqf_basis* B, const cqf_contraction* list, int nMat, const
   cqf_opts ro = opts;
   ro.is_complex = 0;
   ro.device_pointers = 1;
-  double* rX = ws + ws_layout(B, nReal, ro).total;
+  double* rX = ws + ws_layout(B, nReal, ro, plan).total;
   double* rA = rX + blk * nReal;
   std::vector<cqf_contraction> rl;
   std::vector<const double*> src;
@@ -1566,7 +1569,8 @@ cqf_status split_core(cqf_basis* B, const cqf_contraction* list, int nMat, const
   }
   CQF_CUDA(cudaMemsetAsync(rA, 0, blk * nReal * sizeof(double), st));
   CQF_CUDA(cudaGetLastError());
-  CQF_TRY(contract_core(B, rl.data(), nReal, ro, stats, ws, capture, d_flags_pre, src.data()));
+  CQF_TRY(contract_core(B, rl.data(), nReal, ro, stats, ws, capture, d_flags_pre, src.data(),
+                        nullptr, plan));
   for (int m = 0, r = 0; m < nMat; m++) {
     const bool k = list[m].type == CQF_EXCHANGE;
     add_complex_kernel<<<grid1(NN, 256), 256, 0, st>>>(
@@ -1593,22 +1597,23 @@ std::vector<cqf_contraction> normalized_list(const cqf_contraction* list, int nM
 // Workspace of contract_complex_split_on: [split workspace | complex X, AX
 // staging (host pointers only)].
 size_t complex_split_ws_doubles(const cqf_basis* B, const cqf_contraction* list, int nMat,
-                                const cqf_opts& opts) {
+                                const cqf_opts& opts, bool plan) {
   const size_t NN = (size_t)B->nbasis * B->nbasis;
   const size_t blk = (NN + 31) / 32 * 32;
-  const size_t inner = split_ws_doubles(B, split_real_count(list, nMat), opts);
+  const size_t inner = split_ws_doubles(B, split_real_count(list, nMat), opts, plan);
   return inner + (opts.device_pointers ? 0 : 4 * blk * nMat);
 }
 
 // The split with host pointers staged on the device.  Caller holds B->mu,
 // device current.
 cqf_status contract_complex_split_on(cqf_basis* B, const cqf_contraction* list, int nMat,
-                                     const cqf_opts& opts, cqf_stats* stats, double* ws) {
+                                     const cqf_opts& opts, cqf_stats* stats, double* ws,
+                                     bool plan) {
   cudaStream_t st = opts.stream ? (cudaStream_t)opts.stream : B->stream;
   const size_t NN = (size_t)B->nbasis * B->nbasis;
   const size_t blk = (NN + 31) / 32 * 32;
   const bool host = !opts.device_pointers;
-  const size_t inner = split_ws_doubles(B, split_real_count(list, nMat), opts);
+  const size_t inner = split_ws_doubles(B, split_real_count(list, nMat), opts, plan);
   std::vector<cqf_contraction> dl(list, list + nMat);
   if (host) {
     for (int m = 0; m < nMat; m++) {
@@ -1624,7 +1629,7 @@ cqf_status contract_complex_split_on(cqf_basis* B, const cqf_contraction* list, 
   }
   cqf_opts dopts = opts;
   dopts.device_pointers = 1;
-  CQF_TRY(split_core(B, dl.data(), nMat, dopts, stats, ws, false, nullptr));
+  CQF_TRY(split_core(B, dl.data(), nMat, dopts, stats, ws, false, nullptr, plan));
   if (host)
     for (int m = 0; m < nMat; m++)
       CQF_CUDA(cudaMemcpyAsync(list[m].AX, dl[m].AX, 2 * NN * sizeof(double),

@@ -102,7 +102,7 @@ cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* m
     c.braBeg = a.braBeg + ib0;
     c.nBra = n;
     c.braOff = ib0;
-    launch_jk_plan(c, mixed, mk, list64, list32, lcount, B->nsm, st);
+    launch_jk_plan(c, mixed, false, mk, list64, list32, lcount, B->nsm, st);
   };
   const HgRegion r{masks, maskWords, work};
   return a.cplx ? hg_contract<EriDig<true>>(B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a,

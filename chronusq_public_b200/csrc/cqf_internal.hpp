@@ -101,9 +101,10 @@ struct WsLayout {
 };
 // plan = false leaves the masks of a complex contraction out (its class pairs
 // with f shells then run on the generic kernel) and the engine's minimum of
-// them (HG_MIN_WORDS): what the fixed scratch of the no-alloc entry point
+// them (HG_MIN_WORDS, JK_MIN_WORDS): what the fixed scratch of the no-alloc entry point
 // falls back to.
 constexpr size_t HG_MIN_WORDS = size_t(1) << 16;
+constexpr size_t JK_MIN_WORDS = size_t(1) << 11;
 WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan = true);
 // J and K of a class pair with an f shell (cqf_hg_eri.cu).
 cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* masks,
@@ -143,17 +144,19 @@ bool split_eligible(const cqf_basis* B, const cqf_contraction* list, int nMat,
                     const cqf_opts& opts);
 int split_real_count(const cqf_contraction* list, int nMat);
 void split_flags(const cqf_contraction* list, int nMat, int* fl);
-size_t split_ws_doubles(const cqf_basis* B, int nReal, const cqf_opts& opts);
+size_t split_ws_doubles(const cqf_basis* B, int nReal, const cqf_opts& opts, bool plan = true);
 cqf_status split_core(cqf_basis* B, const cqf_contraction* list, int nMat, const cqf_opts& opts,
-                      cqf_stats* stats, double* ws, bool capture, const int* d_flags_pre);
+                      cqf_stats* stats, double* ws, bool capture, const int* d_flags_pre,
+                      bool plan = true);
 
 // The split for device or host pointers on a caller-provided workspace of
 // complex_split_ws_doubles() doubles (host pointers are staged in it);
 // synchronises before returning.  Caller holds B->mu, device current.
 size_t complex_split_ws_doubles(const cqf_basis* B, const cqf_contraction* list, int nMat,
-                                const cqf_opts& opts);
+                                const cqf_opts& opts, bool plan = true);
 cqf_status contract_complex_split_on(cqf_basis* B, const cqf_contraction* list, int nMat,
-                                     const cqf_opts& opts, cqf_stats* stats, double* ws);
+                                     const cqf_opts& opts, cqf_stats* stats, double* ws,
+                                     bool plan = true);
 
 // normSrc (optional, device pointers): per entry, the complex matrix whose
 // shell-block norms screen it in place of its own X (the split of a complex
@@ -261,11 +264,11 @@ struct cqf_basis {
   // coefficient tables of the Hermite-matrix engine (built on first use) and
   // where each class's begin (doubles; the class's first primitive pair)
   double* d_hg[cqf::HG_NKIND] = {};
+  cqf::PairDev* d_pairsHg = nullptr;  // the pairs with their negligible primitives cut off
   size_t hg_beg[cqf::HG_NKIND][cqf::NCLS] = {};
   // first primitive pair of a class, most per pair, and all of them
   int cls_pp_beg[cqf::NCLS] = {0}, cls_npp_max[cqf::NCLS] = {0};
   long long cls_npp_sum[cqf::NCLS] = {0};
-  cqf::PairDev* d_pairsHg = nullptr;  // the pairs with their negligible primitives cut off
   void* d_relws = nullptr;
   size_t relws_bytes = 0;
   std::mutex mu;

@@ -16,6 +16,7 @@
 #include "gen/cqf_gen_jk.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cqf {
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
 // otherwise), J_cd and the four exchange blocks with FP64 atomics.  The FP32
 // kernel forms integrals and products in FP32 from the FP32 copy of the
 // Cartesian densities; accumulation is FP64 in both.
-template <class G, bool FP32>
+template <class G, bool FP32, bool SPLIT>
 __global__ void __launch_bounds__(JK_THREADS, G::MINB)
     jk_class_kernel(const JKLaunch a, const uint2* __restrict__ masks,
                     const int* __restrict__ list, const unsigned int* __restrict__ lcount,
@@ -132,10 +133,18 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
   // largest contraction length (direct.hpp:1563-1589)
   const double peps =
       a.screen ? fmax(2.220446049250313e-16, a.thresh / (__ldg(a.maxNorm) * a.primK4)) : 0.0;
+  // SPLIT: lanes per quartet, 2^sl, named by the list entries (jk_plan_kernel)
+  int esl = 0;  // of the entry last read
   // entry e of the list: (word index, this precision's mask of it)
   auto entry = [&](int e) {
-    const int w = __ldg(list + e);
-    return make_int2(w, (int)(FP32 ? __ldg(&masks[w].y) : __ldg(&masks[w].x)));
+    const int raw = __ldg(list + e);
+    const int w = SPLIT ? raw & PLAN_WORD : raw;
+    unsigned m = FP32 ? __ldg(&masks[w].y) : __ldg(&masks[w].x);
+    if constexpr (SPLIT) {
+      esl = raw >> 24;
+      if (raw & (1 << 23)) m &= 15u << (raw >> 20 & 7) * 4;
+    }
+    return make_int2(w, (int)m);
   };
 
   for (;;) {
@@ -149,12 +158,14 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
     int2 wm = entry(e);
     unsigned m = (unsigned)wm.y;
     for (;;) {
-      // pack the next (up to) 32 named quartets of the run into the lanes
+      // pack the next (up to) 32 named quartets of the run into the lanes, or
+      // 32 / 2^sl of entries whose quartets are shared by 2^sl lanes
       int fill = 0, myW = -1, myBit = 0;
-      while (fill < 32 && e < eEnd) {
+      const int sl = SPLIT ? esl : 0, cap = 32 >> sl;
+      while (fill < cap && e < eEnd && (!SPLIT || esl == sl)) {
         const int c = __popc(m);
-        const int take = min(c, 32 - fill);
-        const int r = lane - fill;
+        const int take = min(c, cap - fill);
+        const int r = (lane >> sl) - fill;
         if (r >= 0 && r < take) {
           myW = wm.x;
           myBit = nth_set_bit(m, r);
@@ -190,9 +201,21 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
       const long long ko = __ldg(a.tileOff + a.ketTileBeg + jkc / KETT_TILE) + jkc % KETT_TILE;
       T I[G::NI];
       if constexpr (FP32)  // FP32 copies of the pair data: half the load bytes
-        G::eri(P, Q, a.pp32, KetSoAT<float>{a.ketT32 + ko}, boys, ch, I, a.ppQ, peps);
+        G::eri(P, Q, a.pp32, KetSoAT<float>{a.ketT32 + ko}, boys, ch, I, a.ppQ, peps,
+               lane & ((1 << sl) - 1), 1 << sl);
       else
-        G::eri(P, Q, a.pp, KetSoA{a.ketT + ko}, boys, ch, I, a.ppQ, peps);
+        G::eri(P, Q, a.pp, KetSoA{a.ketT + ko}, boys, ch, I, a.ppQ, peps,
+               lane & ((1 << sl) - 1), 1 << sl);
+      bool mine = work_;  // this lane digests its quartet
+      if constexpr (SPLIT) {
+        if (sl > 0) {
+#pragma unroll
+          for (int i = 0; i < G::NI; i++)
+            for (int o = (1 << sl) >> 1; o > 0; o >>= 1)
+              I[i] += __shfl_xor_sync(0xffffffffu, I[i], o);
+          mine = work_ && (lane & ((1 << sl) - 1)) == 0;
+        }
+      }
 #pragma unroll 1
       for (int mt = 0; mt < a.nMat; mt++) {
         const int fl = __ldg(a.flags + mt);
@@ -202,7 +225,7 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
         for (int i = 0; i < NA * NB; i++) jab[i] = T(0);
         double* A = a.Ac + mt * matStride;
         G::digest(I, ch, Xbase + mt * matStride, A, nc, P.cA, P.cB, Q.cA, Q.cB, sJ, sK,
-                  (fl & 4) ? -sK : sK, doJ && work_, doK && work_, jab);
+                  (fl & 4) ? -sK : sK, doJ && mine, doK && mine, jab);
         if (doJ) {
 #pragma unroll
           for (int i = 0; i < NA * NB; i++) jab[i] *= sJ;
@@ -215,7 +238,7 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
                   atomicAdd(A + (size_t)(P.cA + i / NB) + (size_t)(P.cB + i % NB) * nc,
                             double(jab[i]));
             }
-          } else if (work_) {
+          } else if (mine) {
 #pragma unroll
             for (int i = 0; i < NA * NB; i++)
               if (jab[i] != T(0))
@@ -232,7 +255,7 @@ __global__ void __launch_bounds__(JK_THREADS, G::MINB)
 // kernel sizes its items from the list's actual length).
 inline int entries_per_item(long long nWords, int nchunk, int nsm) {
   const long long per = nWords * nchunk / ((long long)nsm * 256);
-  return (int)std::min<long long>(64, std::max<long long>(4, per));
+  return (int)std::min<long long>(64, std::max<long long>(1, per));
 }
 
 // Launches the planning pass and the generated class kernels of the class
@@ -256,12 +279,16 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
       b.braTileBeg = a.ketTileBeg; b.ketTileBeg = a.braTileBeg;
     }
     b.lsum = la + lb + lc + ld;
+    constexpr bool CUTTABLE = jk_split(G64::LA + G64::LB + G64::LC + G64::LD);
     const bool mixed = b.precision == 1 && b.fp32_cut > 0.0;
     const int nTiles = (b.nKet + WTILE - 1) / WTILE;
     // slabs of bra pairs whose mask words fit the stream's region; each
     // reuses the region and the stream's counters after the last one's
     // kernels (stream order)
-    const int slab = (int)std::max<long long>(1, maskWords / nTiles);
+    // (class pairs whose lists may hold twice the words: 24 B a word)
+    const bool cut = CUTTABLE && (long long)b.nBra * nTiles <= JK_CUT_WORDS &&
+                     maskWords >= 2 * nTiles;
+    const int slab = (int)std::max<long long>(1, (cut ? maskWords * 2 / 3 : maskWords) / nTiles);
     for (int ib0 = 0; ib0 < b.nBra; ib0 += slab) {
       JKLaunch c = b;
       c.braBeg = b.braBeg + ib0;
@@ -271,20 +298,30 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
       const long long nWords = (long long)c.nBra * nTiles;
       // word lists: FP64 then FP32, nWords entries each; counts in work[2..3]
       int* list64 = reinterpret_cast<int*>(masks + nWords);
-      int* list32 = list64 + nWords;
-      launch_jk_plan(c, mixed, masks, list64, list32, work + 2, nsm, st);
+      int* list32 = list64 + (cut ? 2 : 1) * nWords;
+      launch_jk_plan(c, mixed, cut, masks, list64, list32, work + 2, nsm, st);
       constexpr int WPB = JK_THREADS / 32;
       auto grid = [&](long long items) {
         return (unsigned)std::max<long long>(
             1, std::min<long long>((items + WPB - 1) / WPB, (long long)nsm * blocksPerSm));
       };
-      const int e64 = entries_per_item(nWords, G64::NCHUNK, nsm);
-      jk_class_kernel<G64, false><<<grid((nWords + e64 - 1) / e64 * G64::NCHUNK), JK_THREADS,
-                                    0, st>>>(c, masks, list64, work + 2, e64, work);
-      if (mixed) {
-        const int e32 = entries_per_item(nWords, G32::NCHUNK, nsm);
-        jk_class_kernel<G32, true><<<grid((nWords + e32 - 1) / e32 * G32::NCHUNK), JK_THREADS,
-                                     0, st>>>(c, masks, list32, work + 3, e32, work + 1);
+      auto launch = [&](auto split) {
+        constexpr bool S = decltype(split)::value;
+        const long long n = nWords * (S ? 2 : 1);
+        const int e64 = entries_per_item(n, G64::NCHUNK, nsm);
+        jk_class_kernel<G64, false, S><<<grid((n + e64 - 1) / e64 * G64::NCHUNK), JK_THREADS, 0,
+                                         st>>>(c, masks, list64, work + 2, e64, work);
+        if (mixed) {
+          const int e32 = entries_per_item(n, G32::NCHUNK, nsm);
+          jk_class_kernel<G32, true, S><<<grid((n + e32 - 1) / e32 * G32::NCHUNK), JK_THREADS, 0,
+                                          st>>>(c, masks, list32, work + 3, e32, work + 1);
+        }
+      };
+      if constexpr (CUTTABLE) {
+        if (cut) launch(std::true_type{});
+        else launch(std::false_type{});
+      } else {
+        launch(std::false_type{});
       }
     }
     done = true;

@@ -41,8 +41,24 @@ __device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P
 // consecutive words and appends the indices of its non-empty words to one
 // list per precision (lengths in lcount[0 / 1]), so the class kernels visit
 // only words that name quartets of their precision.
+//
+// CUT (class pairs whose kernels share a quartet among lanes, jk_split): a
+// word whose quartets have long primitive loops (PLAN_HEAVY primitive
+// quartets or more) carries log2 of the lanes per quartet in its list entry,
+// and in the first eighth of the words -- pairs come in descending order of
+// their primitive counts -- it is listed as eight entries of four kets, so
+// that several warps share it; the lists then hold up to twice the words.
+// Without it one lane walked the 4096 primitive quartets of two contractions
+// of eight: 1.4 ms of a 2.3 ms build of one water molecule.
 constexpr int PLAN_RUN = 32;
-template <bool MIXED>
+constexpr int PLAN_HEAVY = 256, PLAN_EACH = 64;  // primitive quartets: heavy, a lane's share
+constexpr int PLAN_WORD = (1 << 20) - 1;         // list entry: word | sub << 20 | part << 23 | log2 << 24
+__host__ __device__ constexpr bool jk_split(int lsum) { return lsum <= 2; }
+// only launches of at most this many words: larger ones have enough quartets
+// to hide the longest loops, and the shared form costs them registers
+// ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms)
+constexpr long long JK_CUT_WORDS = 1 << 16;
+template <bool MIXED, bool CUT>
 __global__ void __launch_bounds__(256)
     jk_plan_kernel(const JKLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
                    int* __restrict__ list32, unsigned int* __restrict__ lcount) {
@@ -60,6 +76,7 @@ __global__ void __launch_bounds__(256)
     for (int word = run * PLAN_RUN; word < wEnd; word++) {
       const int ib = word / nTiles, tile = word - ib * nTiles;
       unsigned b64 = 0u, b32 = 0u;
+      int sl = 0;  // log2 of the lanes per quartet
       const int ibc = ib + a.braOff;  // the bra's position in its class
       // else: no quartet in this word (above the diagonal, or another shard's bra)
       if (!(a.same && tile * WTILE > ibc) && in_shard(a.braBeg + ib, a.shardIdx, a.shardCnt)) {
@@ -76,6 +93,10 @@ __global__ void __launch_bounds__(256)
           const double bound = sh_max_bra(a, P, Q, __ldg(a.pairNorm + a.braBeg + ib),
                                           __ldg(a.pairNorm + a.ketBeg + jk), pRef) * P.Q * Q.Q;
           screened = bound < a.thresh;
+          if (CUT && !screened) {
+            const int np = P.npp * Q.npp;
+            while (np >= PLAN_HEAVY && sl < 5 && (np >> sl) > PLAN_EACH) sl++;
+          }
           w32 = MIXED && !screened && bound < cut &&
                 fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
                               __ldg(a.pairRange + a.ketBeg + jk), a.lsum, 0, 0);
@@ -90,12 +111,30 @@ __global__ void __launch_bounds__(256)
         c64 += __popc(b64);
       }
       if (lane == 0) masks[word] = make_uint2(b64, b32);
+      int entry = word;
+      if (CUT) {
+        sl = (int)__reduce_max_sync(0xffffffffu, (unsigned)sl);
+        entry |= sl << 24;
+        if (sl > 1 && word < nWords / 8) {  // eight entries, written here
+          const unsigned s64 = b64 >> (4 * (lane & 7)) & 15u, s32 = b32 >> (4 * (lane & 7)) & 15u;
+          unsigned at = 0;
+          if (lane < 8 ? s64 != 0u : (lane < 16 && s32 != 0u))
+            at = atomicAdd(lcount + (lane < 8 ? 0 : 1), 1u);
+          const int e8 = entry | 1 << 23 | (lane & 7) << 20;
+          if (lane < 8) {
+            if (s64) list64[at] = e8;
+          } else if (lane < 16) {
+            if (s32) list32[at] = e8;
+          }
+          continue;
+        }
+      }
       if (b64) {
-        if (lane == n64) my64 = word;
+        if (lane == n64) my64 = entry;
         n64++;
       }
       if (b32) {
-        if (lane == n32) my32 = word;
+        if (lane == n32) my32 = entry;
         n32++;
       }
     }
@@ -119,15 +158,19 @@ __global__ void __launch_bounds__(256)
 
 // Launches the pass on the bra pairs [braBeg, braBeg + nBra) of `a` (a slab):
 // lcount[0 / 1], zero on entry, receive the lists' lengths.
-inline void launch_jk_plan(const JKLaunch& a, bool mixed, uint2* masks, int* list64, int* list32,
-                           unsigned int* lcount, int nsm, cudaStream_t st) {
+inline void launch_jk_plan(const JKLaunch& a, bool mixed, bool cut, uint2* masks, int* list64,
+                           int* list32, unsigned int* lcount, int nsm, cudaStream_t st) {
   const long long nWords = (long long)a.nBra * ((a.nKet + WTILE - 1) / WTILE);
   const long long nRuns = (nWords + PLAN_RUN - 1) / PLAN_RUN;
   const unsigned gp = (unsigned)std::min<long long>((nRuns + 7) / 8, (long long)nsm * 8);
-  if (mixed)
-    jk_plan_kernel<true><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
+  if (mixed && cut)
+    jk_plan_kernel<true, true><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
+  else if (mixed)
+    jk_plan_kernel<true, false><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
+  else if (cut)
+    jk_plan_kernel<false, true><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
   else
-    jk_plan_kernel<false><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
+    jk_plan_kernel<false, false><<<gp, 256, 0, st>>>(a, masks, list64, list32, lcount);
 }
 
 }  // namespace cqf

@@ -87,11 +87,15 @@ extern "C" cqf_status cqf_two_body_contract_noalloc(cqf_basis* B, const cqf_cont
   bool allHer = true;
   std::vector<cqf_contraction> list = cqf::normalized_list(listIn, nMat, &allHer);
   const bool split = allHer && cqf::split_eligible(B, list.data(), nMat, opts);
-  // without the masks of complex contractions with f shells where they do
-  // not fit (those class pairs then take the generic kernel)
-  const bool plan = split || cqf::ws_layout(B, nMat, opts).total <= kScratchDoubles;
-  const size_t need = split ? cqf::complex_split_ws_doubles(B, list.data(), nMat, opts)
-                            : cqf::ws_layout(B, nMat, opts, plan).total;
+  // where it does not fit, without the masks of complex contractions with f
+  // shells (those class pairs then take the generic kernel) and without the
+  // larger minimum of the others
+  auto doubles = [&](bool plan) {
+    return split ? cqf::complex_split_ws_doubles(B, list.data(), nMat, opts, plan)
+                 : cqf::ws_layout(B, nMat, opts, plan).total;
+  };
+  const bool plan = doubles(true) <= kScratchDoubles;
+  const size_t need = doubles(plan);
   if (need > kScratchDoubles) {
     char msg[256];
     std::snprintf(msg, sizeof msg,
@@ -107,7 +111,7 @@ extern "C" cqf_status cqf_two_body_contract_noalloc(cqf_basis* B, const cqf_cont
   double* ws = nullptr;
   s = scratch_address(B->device, &ws);
   if (s != CQF_OK) return s;
-  if (split) return cqf::contract_complex_split_on(B, list.data(), nMat, opts, stats, ws);
+  if (split) return cqf::contract_complex_split_on(B, list.data(), nMat, opts, stats, ws, plan);
   return cqf::contract_core(B, list.data(), nMat, opts, stats, ws, false, nullptr, nullptr,
                             nullptr, plan);
 }

@@ -206,7 +206,7 @@ def emit_eri_mirror(w, la, lb, lc, ld, CS, prec):
     w.line("const T PI52x2 = T(34.986836655249725693);")
     w.line("const double qbMax = eps > 0.0 ? __ldg(ppQ + P.pp_off) : 0.0;")
     w.line("#pragma unroll 1")
-    w.open("for (int iq = 0; iq < Q.npp; iq++) {")
+    w.open("for (int iq = i0; iq < Q.npp; iq += di) {")
     w.line("const double qk = eps > 0.0 ? kq.Qp(iq) : 0.0;")
     w.line("if (qk * qbMax < eps) break;")
     w.line("const T q = T(kq.p(iq)), Kcd = T(kq.Kp(iq)), o2q = T(kq.o2p(iq));")
@@ -334,9 +334,12 @@ def gen_class(la, lb, lc, ld, prec):
     # primitive quartets with Qp_ab Qp_cd < eps are skipped; a pair's
     # primitive pairs are sorted by Qp (descending), so a loop stops at the
     # first one below the bound.  eps = 0 computes every primitive quartet.
+    # The outer primitive loop takes every di-th pair from i0: di lanes can
+    # share a quartet and add their integrals.
     w.open("static __device__ __forceinline__ void eri(const PairDev& P, const PairDev& Q, "
            "const PP* __restrict__ pp, const KA& kq, const T* __restrict__ boys, "
-           "const int ch, T (&I)[%d], const double* __restrict__ ppQ, const double eps) {"
+           "const int ch, T (&I)[%d], const double* __restrict__ ppQ, const double eps, "
+           "const int i0 = 0, const int di = 1) {"
            % (NAB * CS))
     if mirror:
         emit_eri_mirror(w, la, lb, lc, ld, CS, prec)
@@ -346,7 +349,7 @@ def gen_class(la, lb, lc, ld, prec):
         w.line("const T PI52x2 = T(34.986836655249725693);")
         w.line("const double qkMax = eps > 0.0 && Q.npp > 0 ? kq.Qp(0) : 0.0;")
         w.line("#pragma unroll 1")
-        w.open("for (int ip = 0; ip < P.npp; ip++) {")
+        w.open("for (int ip = i0; ip < P.npp; ip += di) {")
         w.line("const double qb = eps > 0.0 ? __ldg(ppQ + P.pp_off + ip) : 0.0;")
         w.line("if (qb * qkMax < eps) break;")
         w.line("const auto& pa = pp[P.pp_off + ip];")

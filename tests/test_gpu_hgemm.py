@@ -60,9 +60,10 @@ def test_engine_rel(name, ctype, precision):
 
 
 @pytest.mark.parametrize("kind", ["real", "real_nonher", "complex", "complex_nonher", "mixed"])
-@pytest.mark.parametrize("name", ["f2", "mix"])
+@pytest.mark.parametrize("name", ["f2", "long", "mix"])
 def test_engine_jk(name, kind):
-    """J and K of bases with f shells: every Hermitian / complex flavour and
+    """J and K of bases with f shells, and of long contractions whose quartets
+    several lanes of the class kernels share: every Hermitian / complex flavour and
     mixed precision (three matrices a call)."""
     bs = basis(name)
     N = bs.nbasis
