@@ -488,26 +488,28 @@ __global__ void pp32_kernel(const PrimPairDev* __restrict__ pp, long long n, Pri
 }
 
 // Each pair's primitive pairs in descending order of their primitive
-// Schwarz bound (insertion sort, one thread per pair), so that the class
-// kernels' primitive loops can stop at the first pair below the screen.
-__global__ void sort_pp_kernel(const PairDev* __restrict__ pairs, int n, PrimPairDev* pp,
-                               double* ppQ) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Schwarz bound, so that the class kernels' primitive loops can stop at the
+// first pair below the screen: a warp per pair, each lane counts the
+// primitives before its own (ties keep their order).  One thread's insertion
+// sort of 64 records of 112 B took 2.1 ms.
+__global__ void sort_pp_kernel(const PairDev* __restrict__ pairs, int n,
+                               const PrimPairDev* __restrict__ pp, const double* __restrict__ ppQ,
+                               PrimPairDev* __restrict__ ppOut, double* __restrict__ qOut) {
+  const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= n) return;
   const PairDev P = pairs[i];
-  PrimPairDev* r = pp + P.pp_off;
-  double* q = ppQ + P.pp_off;
-  for (int k = 1; k < P.npp; k++) {
-    const PrimPairDev rk = r[k];
-    const double qk = q[k];
-    int j = k - 1;
-    while (j >= 0 && q[j] < qk) {
-      r[j + 1] = r[j];
-      q[j + 1] = q[j];
-      j--;
+  const double* q = ppQ + P.pp_off;
+  // NaN (which no finite input gives) sorts last: every rank stays distinct
+  auto key = [](double v) { return v == v ? v : -1.0; };
+  for (int k = lane; k < P.npp; k += 32) {
+    const double qk = key(q[k]);
+    int r = 0;
+    for (int j = 0; j < P.npp; j++) {
+      const double qj = key(q[j]);
+      r += qj > qk || (qj == qk && j < k);
     }
-    r[j + 1] = rk;
-    q[j + 1] = qk;
+    ppOut[P.pp_off + r] = pp[P.pp_off + k];
+    qOut[P.pp_off + r] = q[k];
   }
 }
 
@@ -1051,7 +1053,7 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
     if (!launch_schwarz_fast(la, lb, d_tmp, B->d_pp, B->d_boys64, B->d_sph, B->d_sphOff,
                              B->d_shells, B->cls_beg[c], B->cls_cnt[c], nshell, B->d_schwarz,
                              d_tmp, d_diag + (size_t)B->cls_beg[c] * 36, B->stream))
-      schwarz_kernel<<<grid1(B->cls_cnt[c], 64), 64, 0, B->stream>>>(
+      schwarz_kernel<<<B->cls_cnt[c], 128, 0, B->stream>>>(
           d_tmp, B->d_pp, B->d_boys64, B->d_sph, B->d_sphOff, B->d_shells, B->cls_beg[c],
           B->cls_cnt[c], nshell, B->d_schwarz, d_tmp);
   }
@@ -1106,6 +1108,14 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
       B->h_pairs[i].pp_off = (int)off2;
       off2 += B->h_pairs[i].npp;
     }
+    for (int c = 0; c < NCLS; c++) {
+      B->cls_pp_beg[c] = B->cls_cnt[c] ? B->h_pairs[B->cls_beg[c]].pp_off : 0;
+      for (int i = 0; i < B->cls_cnt[c]; i++) {
+        const int npp = B->h_pairs[B->cls_beg[c] + i].npp;
+        B->cls_npp_max[c] = std::max(B->cls_npp_max[c], npp);
+        B->cls_npp_sum[c] += npp;
+      }
+    }
     CQF_CUDA(cudaMemcpyAsync(B->d_pairs, B->h_pairs.data(), B->npair * sizeof(PairDev),
                              cudaMemcpyHostToDevice, B->stream));
     long long* d_src = nullptr;
@@ -1122,17 +1132,31 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
     // unscreened bound), then each pair's primitive pairs sorted by them
     CQF_CUDA(cudaMallocAsync(&B->d_ppQ, std::max<long long>(1, ppoff) * sizeof(double),
                              B->stream));
-    fill_kernel<<<(unsigned)std::min<long long>(grid1(std::max<long long>(1, ppoff), 256), 4096),
-                  256, 0, B->stream>>>(B->d_ppQ, std::max<long long>(1, ppoff), 1e300);
     for (int c = 0; c < NCLS; c++) {
+      if (B->cls_npp_sum[c] == 0) continue;
       int la, lb;
       class_ls(c, la, lb);
-      if (la <= 2)
-        launch_prim_schwarz(la, lb, B->d_pairs, B->d_pp, B->d_boys64, B->cls_beg[c],
-                            B->cls_cnt[c], B->d_ppQ, B->stream);
+      double* q = B->d_ppQ + B->cls_pp_beg[c];
+      if (la > 2) {
+        fill_kernel<<<(unsigned)std::min<long long>(grid1(B->cls_npp_sum[c], 256), 4096), 256, 0,
+                      B->stream>>>(q, B->cls_npp_sum[c], 1e300);
+        continue;
+      }
+      CQF_CUDA(cudaMemsetAsync(q, 0, B->cls_npp_sum[c] * sizeof(double), B->stream));
+      launch_prim_schwarz(la, lb, B->d_pairs, B->d_pp, B->d_boys64, B->cls_beg[c],
+                          B->cls_cnt[c], B->cls_npp_max[c], B->d_ppQ, B->stream);
     }
-    sort_pp_kernel<<<grid1(B->npair, 128), 128, 0, B->stream>>>(B->d_pairs, B->npair, B->d_pp,
-                                                                B->d_ppQ);
+    PrimPairDev* d_pp3 = nullptr;
+    double* d_q3 = nullptr;
+    CQF_CUDA(cudaMallocAsync(&d_pp3, std::max<long long>(1, ppoff) * sizeof(PrimPairDev),
+                             B->stream));
+    CQF_CUDA(cudaMallocAsync(&d_q3, std::max<long long>(1, ppoff) * sizeof(double), B->stream));
+    sort_pp_kernel<<<grid1(32 * (size_t)B->npair, 128), 128, 0, B->stream>>>(
+        B->d_pairs, B->npair, B->d_pp, B->d_ppQ, d_pp3, d_q3);
+    cudaFreeAsync(B->d_pp, B->stream);
+    cudaFreeAsync(B->d_ppQ, B->stream);
+    B->d_pp = d_pp3;
+    B->d_ppQ = d_q3;
     CQF_CUDA(cudaMallocAsync(&B->d_pp32, std::max<long long>(1, ppoff) * sizeof(PrimPair32),
                              B->stream));
     pp32_kernel<<<(unsigned)std::min<long long>(grid1(std::max<long long>(1, ppoff), 256), 4096),
@@ -1179,14 +1203,6 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
     pair_range_kernel<<<grid1(B->npair, 128), 128, 0, B->stream>>>(B->d_pp, B->d_pairs,
                                                                    B->npair, B->d_pairRange);
     CQF_CUDA(cudaGetLastError());
-  }
-  for (int c = 0; c < NCLS; c++) {
-    B->cls_pp_beg[c] = B->cls_cnt[c] ? B->h_pairs[B->cls_beg[c]].pp_off : 0;
-    for (int i = 0; i < B->cls_cnt[c]; i++) {
-      const int npp = B->h_pairs[B->cls_beg[c] + i].npp;
-      B->cls_npp_max[c] = std::max(B->cls_npp_max[c], npp);
-      B->cls_npp_sum[c] += npp;
-    }
   }
   B->h_schwarz.resize((size_t)nshell * nshell);
   CQF_CUDA(cudaMemcpyAsync(B->h_schwarz.data(), B->d_schwarz,

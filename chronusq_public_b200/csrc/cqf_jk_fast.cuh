@@ -336,8 +336,11 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
 
 // ----------------------------------------------------------- Schwarz (fast)
 // Diagonal (mu nu|mu nu) of the pairs of one class (LA, LB) with LA, LB <= 2
-// from the generated (ab|ab) code, one thread per (pair, chunk); the chunk's
-// share of each spherical diagonal element is added into diag[pair][mu][nu].
+// from the generated (ab|ab) code, SCHWARZ_LANES threads per (pair, chunk)
+// sharing its primitive loop (one thread each took 1.2 ms for contractions of
+// eight); each one's share of each spherical diagonal element is added into
+// diag[pair][mu][nu].
+constexpr int SCHWARZ_LANES = 16;
 template <class GC>
 __global__ void __launch_bounds__(JK_THREADS)
     schwarz_diag_kernel(const PairDev* __restrict__ pairs, const PrimPairDev* __restrict__ pp,
@@ -346,10 +349,13 @@ __global__ void __launch_bounds__(JK_THREADS)
                         int beg, int n, double* diag) {
   constexpr int NA = ncart(GC::LA), NB = ncart(GC::LB), NCH = GC::NCHUNK;
   constexpr int CS = GC::NI / (NA * NB);
-  const long long item = (long long)blockIdx.x * JK_THREADS + threadIdx.x;
+  const long long t = (long long)blockIdx.x * JK_THREADS + threadIdx.x;
+  const long long item = t / SCHWARZ_LANES;
+  const int sub = (int)(t % SCHWARZ_LANES);
   if (item >= (long long)n * NCH) return;
   const int k = (int)(item / NCH), ch = (int)(item % NCH);
   const PairDev P = pairs[beg + k];
+  if (sub >= P.npp) return;
   const ShellDev A = shells[P.shA], B = shells[P.shB];
   const int na = A.pure ? nsph(GC::LA) : NA, nb = B.pure ? nsph(GC::LB) : NB;
   const double* TA = sph + sphOff[GC::LA];
@@ -358,7 +364,8 @@ __global__ void __launch_bounds__(JK_THREADS)
   auto tb = [&](int c, int nu) { return B.pure ? TB[c * nsph(GC::LB) + nu] : (c == nu ? 1.0 : 0.0); };
   double I[GC::NI];
   GC::eri(P, P, pp, KetAoS{pp + P.pp_off, nullptr},
-                           boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr, 0.0);
+                           boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr, 0.0,
+                           sub, SCHWARZ_LANES);
   for (int mu = 0; mu < na; mu++)
     for (int nu = 0; nu < nb; nu++) {
       double s = 0.0;
@@ -423,7 +430,7 @@ inline bool launch_schwarz_fast(int la, int lb, const PairDev* pairs, const Prim
   auto go = [&](auto tag64) {
     using G = decltype(tag64);
     cudaMemsetAsync(diag, 0, (size_t)n * 36 * sizeof(double), st);
-    const long long items = (long long)n * G::NCHUNK;
+    const long long items = (long long)n * G::NCHUNK * SCHWARZ_LANES;
     schwarz_diag_kernel<G><<<(unsigned)((items + JK_THREADS - 1) / JK_THREADS), JK_THREADS, 0,
                              st>>>(pairs, pp, boys, sph, sphOff, shells, beg, n, diag);
     schwarz_finish_kernel<<<(n + 127) / 128, 128, 0, st>>>(pairs, shells, beg, n, nshell, diag,
@@ -440,8 +447,10 @@ inline bool launch_schwarz_fast(int la, int lb, const PairDev* pairs, const Prim
 // Primitive Schwarz bounds of the pairs of one class (LA, LB <= 2):
 // Qp = sqrt(max over Cartesian components |(ab|ab)|) of each primitive pair
 // alone (contraction coefficients included; the integrals the class kernels
-// form), one thread per pair.  They bound each primitive quartet's integrals
-// by Qp_ab Qp_cd (Cauchy-Schwarz), the primitive screen's estimate.
+// form), a thread per (pair, chunk of components) and primitive (blockIdx.y);
+// ppQ is zero on entry.  (A thread per pair took 235 us for d pairs.)  They
+// bound each primitive quartet's integrals by Qp_ab Qp_cd (Cauchy-Schwarz),
+// the primitive screen's estimate.
 template <class GC>
 __global__ void prim_schwarz_kernel(const PairDev* __restrict__ pairs,
                                     const PrimPairDev* __restrict__ pp,
@@ -449,38 +458,37 @@ __global__ void prim_schwarz_kernel(const PairDev* __restrict__ pairs,
                                     double* __restrict__ ppQ) {
   constexpr int NA = ncart(GC::LA), NB = ncart(GC::LB), NCH = GC::NCHUNK;
   constexpr int CS = GC::NI / (NA * NB);
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t / NCH, ch = t - k * NCH;
+  const int ip = blockIdx.y;
   if (k >= n) return;
-  const PairDev P = pairs[beg + k];
-  for (int ip = 0; ip < P.npp; ip++) {
-    PairDev P1 = P;
-    P1.npp = 1;
-    P1.pp_off = P.pp_off + ip;
-    double mx = 0.0;
-    for (int ch = 0; ch < NCH; ch++) {
-      double I[GC::NI];
-      GC::eri(P1, P1, pp, KetAoS{pp + P1.pp_off, nullptr},
-              boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr,
-              0.0);
-      for (int kk = 0; kk < CS; kk++) {
-        const int cd = ch * CS + kk;  // the diagonal element (ab | ab), ab = cd
-        if (cd < NA * NB) mx = fmax(mx, fabs(I[cd * CS + kk]));
-      }
-    }
-    ppQ[P.pp_off + ip] = sqrt(mx);
+  PairDev P1 = pairs[beg + k];
+  if (ip >= P1.npp) return;
+  P1.npp = 1;
+  P1.pp_off += ip;
+  double I[GC::NI];
+  GC::eri(P1, P1, pp, KetAoS{pp + P1.pp_off, nullptr},
+          boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr, 0.0);
+  double mx = 0.0;
+  for (int kk = 0; kk < CS; kk++) {
+    const int cd = ch * CS + kk;  // the diagonal element (ab | ab), ab = cd
+    if (cd < NA * NB) mx = fmax(mx, fabs(I[cd * CS + kk]));
   }
+  // non-negative doubles order as their bits
+  atomicMax(reinterpret_cast<unsigned long long*>(ppQ + P1.pp_off),
+            (unsigned long long)__double_as_longlong(sqrt(mx)));
 }
 
 // Primitive Schwarz bounds of one class with the generated code; false if
 // the class has none.
 inline bool launch_prim_schwarz(int la, int lb, const PairDev* pairs, const PrimPairDev* pp,
-                                const double* boys, int beg, int n, double* ppQ,
+                                const double* boys, int beg, int n, int maxNpp, double* ppQ,
                                 cudaStream_t st) {
   if (n <= 0) return true;
   bool done = false;
   auto go = [&](auto tag64) {
     using G = decltype(tag64);
-    prim_schwarz_kernel<G><<<(n + 63) / 64, 64, 0, st>>>(pairs, pp, boys, beg, n, ppQ);
+    prim_schwarz_kernel<G><<<dim3((n * G::NCHUNK + 63) / 64, maxNpp), 64, 0, st>>>(
+        pairs, pp, boys, beg, n, ppQ);
     done = true;
   };
 #define CQF_TRY_PRIM(A_, B_, C_, D_, N64, N32) \

@@ -180,12 +180,14 @@ inline void launch_jk_generic(const JKLaunch& a, int la, int lb, int lc, int ld,
 // ---------------------------------------------------------------- Schwarz
 // Q(s1,s2) = sqrt(|| D ||_inf), D(i,j) = (ij|ij) over the AOs of s1 (rows)
 // and s2 (columns): max row sum (aointegrals_utilities.cxx:78-104).
-__global__ void __launch_bounds__(64)
+// One block per pair, a thread per ket component pair (one thread per pair
+// took 48 ms for (ff|ff)).
+__global__ void __launch_bounds__(128)
     schwarz_kernel(const PairDev* __restrict__ pairs, const PrimPairDev* __restrict__ pp,
                    const double* __restrict__ boys, const double* __restrict__ sph,
                    const int* __restrict__ sphOff, const ShellDev* __restrict__ shells,
                    int beg, int n, int nshell, double* Qtab, PairDev* pairsOut) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x;
   if (k >= n) return;
   const PairDev P = pairs[beg + k];
   const ShellDev A = shells[P.shA], B = shells[P.shB];
@@ -194,33 +196,36 @@ __global__ void __launch_bounds__(64)
   const int na = A.pure ? nsph(la) : nca, nb = B.pure ? nsph(lb) : ncb;
   const double* TA = sph + sphOff[la];
   const double* TB = sph + sphOff[lb];
-  double diag[ncart(LMAX)][ncart(LMAX)];
-  for (int i = 0; i < na; i++)
-    for (int j = 0; j < nb; j++) diag[i][j] = 0.0;
+  __shared__ double diag[ncart(LMAX)][ncart(LMAX)];
+  for (int i = threadIdx.x; i < ncart(LMAX) * ncart(LMAX); i += blockDim.x)
+    diag[i / ncart(LMAX)][i % ncart(LMAX)] = 0.0;
+  __syncthreads();
   double col[RtBounds<LMAX>::NAB];
   // (mu nu|mu nu) = sum_{abcd} T_a,mu T_b,nu T_c,mu T_d,nu (ab|cd)
-  for (int c = 0; c < nca; c++)
-    for (int d = 0; d < ncb; d++) {
-      eri_column_rt<double, LMAX>(la, lb, la, lb, c, d, P, P, pp, boys, col);
-      for (int mu = 0; mu < na; mu++) {
-        const double tc = A.pure ? TA[c * nsph(la) + mu] : (c == mu ? 1.0 : 0.0);
-        if (tc == 0.0) continue;
-        for (int nu = 0; nu < nb; nu++) {
-          const double td = B.pure ? TB[d * nsph(lb) + nu] : (d == nu ? 1.0 : 0.0);
-          if (td == 0.0) continue;
-          double s = 0.0;
-          for (int ia = 0; ia < nca; ia++) {
-            const double ta = A.pure ? TA[ia * nsph(la) + mu] : (ia == mu ? 1.0 : 0.0);
-            if (ta == 0.0) continue;
-            for (int ib = 0; ib < ncb; ib++) {
-              const double tb = B.pure ? TB[ib * nsph(lb) + nu] : (ib == nu ? 1.0 : 0.0);
-              s += ta * tb * col[ia * ncb + ib];
-            }
+  for (int cd = threadIdx.x; cd < nca * ncb; cd += blockDim.x) {
+    const int c = cd / ncb, d = cd % ncb;
+    eri_column_rt<double, LMAX>(la, lb, la, lb, c, d, P, P, pp, boys, col);
+    for (int mu = 0; mu < na; mu++) {
+      const double tc = A.pure ? TA[c * nsph(la) + mu] : (c == mu ? 1.0 : 0.0);
+      if (tc == 0.0) continue;
+      for (int nu = 0; nu < nb; nu++) {
+        const double td = B.pure ? TB[d * nsph(lb) + nu] : (d == nu ? 1.0 : 0.0);
+        if (td == 0.0) continue;
+        double s = 0.0;
+        for (int ia = 0; ia < nca; ia++) {
+          const double ta = A.pure ? TA[ia * nsph(la) + mu] : (ia == mu ? 1.0 : 0.0);
+          if (ta == 0.0) continue;
+          for (int ib = 0; ib < ncb; ib++) {
+            const double tb = B.pure ? TB[ib * nsph(lb) + nu] : (ib == nu ? 1.0 : 0.0);
+            s += ta * tb * col[ia * ncb + ib];
           }
-          diag[mu][nu] += tc * td * s;
         }
+        atomicAdd(&diag[mu][nu], tc * td * s);
       }
     }
+  }
+  __syncthreads();
+  if (threadIdx.x > 0) return;
   // rows are the functions of s1 (the reference's first shell)
   const bool swp = P.shA != P.s1;
   double mx = 0.0;
