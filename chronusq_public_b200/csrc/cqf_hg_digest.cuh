@@ -122,6 +122,8 @@ __device__ __forceinline__ void hg_digest_her(const HgQuartet& z, int nc, bool e
     const PairDev& Q = z.Q[q];
     const HgRoles ro = hg_roles(P, Q);
     const double* xq = xs + q * nx + (outA ? na : 0) * (ncc + nd) + (outC ? ncc : 0);
+    int k0, k1;  // the contracted ket components in the chunk
+    hg_range(cd0, cdI, ki, nCD, k0, k1);
     double s[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) s[k] = 0.0;
@@ -130,11 +132,9 @@ __device__ __forceinline__ void hg_digest_her(const HgQuartet& z, int nc, bool e
       const int ab = ab0 + bI * abI;
       if (ab < 0 || ab >= nAB) continue;
       const double* x = xq + bI * (ncc + nd);
-      int cd = cd0;
-      for (int kI = 0; kI < ki; kI++, cd += cdI) {
-        if (cd < 0 || cd >= nCD) continue;
+      for (int kI = k0; kI < k1; kI++) {
         double v[NV];
-        val(q, ab, cd, v);
+        val(q, ab, cd0 + kI * cdI, v);
 #pragma unroll
         for (int t = 0; t < NV; t++) s[t] += v[t] * x[kI];
       }

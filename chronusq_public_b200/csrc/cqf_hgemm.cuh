@@ -404,7 +404,7 @@ __global__ static void __launch_bounds__(128)
 }
 
 template <class D>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(512, 1)
     hg_kernel(const HgLaunch a, const typename D::Args args) {
   extern __shared__ double sm[];
   const int la = a.la, lb = a.lb, lc = a.lc, ld = a.ld;
@@ -594,6 +594,12 @@ __device__ __forceinline__ int hg_share(int units, int ni) {
   return l;
 }
 
+// The steps k < n at which lo + k step (step > 0) lies in [0, end): [k0, k1).
+__device__ __forceinline__ void hg_range(int lo, int step, int n, int end, int& k0, int& k1) {
+  k0 = lo < 0 ? (-lo + step - 1) / step : 0;
+  k1 = end > lo ? min(n, (end - lo + step - 1) / step) : 0;
+}
+
 // Planning pass over the words (bra pair, 32 kets) of nBra x nKet quartets:
 // f(ib, jk, work, lo) returns whether quartet (ib, jk) exists and sets
 // whether it is computed, and with FP32 Hermite integrals.  Masks, lists of
@@ -698,32 +704,44 @@ inline size_t hg_chunk(HgLaunch& a, int nkMax, int nrMax) {
       a.nr *= 2;
     return bytes(ru, cu, a.nk, a.nr);
   }
+  // fewest chunks within each limit; one block of 16 warps per SM where that
+  // saves chunks (a chunk's digestion keeps only its share of the outputs'
+  // threads busy), else two of eight
+  int chunks2 = 1 << 30;
+  size_t got = 0;
   for (size_t lim : {HG_SMEM_TWO, HG_SMEM_MAX}) {
     double best = 1e30;
-    size_t got = 0;
+    int chunks = 1 << 30, nru = 0, ncu = 0;
+    size_t b1 = 0;
     for (int c = 1; c <= cu; c++)
       for (int r = 1; r <= ru; r++) {
         const size_t b = bytes(r, c, 1, 1);
         if (b > lim) break;
-        const int nc = (cu + c - 1) / c, nr = (ru + r - 1) / r;
-        const double cost = nc * nr + 0.01 * (r + c);  // the smallest with this chunk count
+        const int n = ((cu + c - 1) / c) * ((ru + r - 1) / r);
+        const double cost = n + 0.01 * (r + c);  // the smallest with this chunk count
         if (cost < best) {
           best = cost;
-          a.nru = r;
-          a.ncu = c;
-          got = b;
+          chunks = n;
+          nru = r;
+          ncu = c;
+          b1 = b;
         }
       }
-    // many chunks of few tiles leave most warps idle: take one block
-    if (got && (best < 24.0 || lim == HG_SMEM_MAX)) return got;
+    if (b1 && (got == 0 || chunks < chunks2)) {
+      a.nru = nru;
+      a.ncu = ncu;
+      got = b1;
+      chunks2 = chunks;
+    }
   }
-  return 0;
+  return got;
 }
 
 // Warps per block from the products' size (matrix instructions per primitive
 // quartet) and the batch.
 template <class D>
-inline int hg_warps(const HgLaunch& a) {
+inline int hg_warps(const HgLaunch& a, size_t smem) {
+  if (smem > HG_SMEM_TWO) return 16;  // one block per SM
   long long m = 0;
   for (int q = 0; q < D::NP; q++) {
     const int hb = nherm(a.la + a.lb + hg_rise(D::tb(q)));
@@ -750,7 +768,7 @@ inline const HgShape& hg_shape(HgLaunch a, int nkMax, int nrMax) {
     m.smem = hg_chunk<D>(a, nkMax, nrMax);
     m.nkMax = nkMax; m.nrMax = nrMax;
     m.nru = a.nru; m.ncu = a.ncu; m.nk = a.nk; m.nr = a.nr;
-    m.W = m.smem ? hg_warps<D>(a) : 0;
+    m.W = m.smem ? hg_warps<D>(a, m.smem) : 0;
   }
   return m;
 }

@@ -226,9 +226,10 @@ __device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& 
   // the densities the batch needs, in shared memory: Coulomb vectors in the
   // order of M's rows and columns, exchange blocks (A then B) x (C then D) of
   // each ket, 8 reals an element
-  const int nx = (na + nb) * (ncc + nd);
+  // (two more per bra component: its row starts on another bank)
+  const int xrow = (ncc + nd) * 8 + 2, nx = (na + nb) * (ncc + nd);
   double* xk = z.st;
-  double* xab = xk + (size_t)z.nk * nx * 8;
+  double* xab = xk + (size_t)z.nk * (na + nb) * xrow;
   double* xcd = xab + 4 * na * nb;
   const double* const* const Xss = a.Xss;
   for (int u = tid; u < nAB * 4; u += nt) {
@@ -250,7 +251,8 @@ __device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& 
       const int gB = i < na ? P.cA + i : P.cB + i - na;
       const int gK = j < ncc ? z.Q[q].cA + j : z.Q[q].cB + j - ncc;
       const size_t e = TYPE == 1 ? ix(gK, gB) : ix(gB, gK);
-      reinterpret_cast<double2*>(xk)[(size_t)v * 4 + comp] = ldz(a.Xk[comp], e);
+      reinterpret_cast<double2*>(xk + (q * (na + nb) + i) * xrow)[4 * j + comp] =
+          ldz(a.Xk[comp], e);
     }
   __syncthreads();
   // Coulomb SS(1,2) from D(4,3) (:1145-1190, :2342-2380): unit (ket, ab, op)
@@ -305,7 +307,9 @@ __device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& 
     const int abI = outA ? 1 : nb, cdI = outC ? 1 : nd;   // their steps in ab and cd
     const int ab0 = (outA ? bO * nb : bO) - z.ab0, cd0 = (outC ? kO * nd : kO) - z.cd0;
     const double* Mq = z.M[0] + q * z.cw[0];
-    const double* xq = xk + ((size_t)q * nx + (outA ? na : 0) * (ncc + nd) + (outC ? ncc : 0)) * 8;
+    const double* xq = xk + (q * (na + nb) + (outA ? na : 0)) * xrow + (outC ? ncc : 0) * 8;
+    int k0, k1;  // the contracted ket components in the chunk
+    hg_range(cd0, cdI, ki, nCD, k0, k1);
     double t[4][8];
 #pragma unroll
     for (int b = 0; b < 4; b++)
@@ -316,16 +320,13 @@ __device__ __forceinline__ void rel_digest(const RelLaunch& a, const HgQuartet& 
     for (int bI = part; bI < ni; bI += 1 << sh) {
       const int ab = ab0 + bI * abI;
       if (ab < 0 || ab >= nAB) continue;
-      const double* mr = Mq + ab * msab;
-      const double* xr = xq + (size_t)bI * (ncc + nd) * 8;
-      int cd = cd0;
+      const double* m = Mq + ab * msab + NB * (cd0 + k0 * cdI);
+      const double* xr = xq + bI * xrow + k0 * 8;
+      any = any || k0 < k1;
 #pragma unroll 1
-      for (int kI = 0; kI < ki; kI++, cd += cdI, xr += 8) {
-        if (cd < 0 || cd >= nCD) continue;
-        any = true;
+      for (int kI = k0; kI < k1; kI++, m += NB * cdI, xr += 8) {
         const double2* x2 = reinterpret_cast<const double2*>(xr);
         const Q4 d{x2[0], x2[1], x2[2], x2[3]};
-        const double* m = mr + NB * cd;
         if (TYPE == 1) {
           // (D (m0 + i f m.sigma)): per operator m_op D
 #pragma unroll
@@ -381,7 +382,7 @@ struct RelDig {
   __host__ __device__ static constexpr int rtu(int) { return 1; }
   __host__ __device__ static constexpr int ctu(int) { return 1; }
   __host__ __device__ static int stage(int la, int lb, int lc, int ld, int nk) {
-    return nk * ((ncart(la) + ncart(lb)) * (ncart(lc) + ncart(ld)) * 8 +
+    return nk * ((ncart(la) + ncart(lb)) * ((ncart(lc) + ncart(ld)) * 8 + 2) +
                  ncart(lc) * ncart(ld) * (TYPE == 2 ? 4 : 1)) +
            ncart(la) * ncart(lb) * 4;
   }
