@@ -358,9 +358,9 @@ class GTODirectRelERIContraction:
         GAUNT and GAUGE; None for entries the type does not use).  The AX the
         type writes are overwritten (the reference zeroes AX on entry); X and
         AX are N x N complex (numpy, or column-major CUDA complex128 tensors).
-        precision="mixed" runs the quartets whose screening bound is below
-        fp32_cutoff in FP32 arithmetic (the reference is FP64 throughout;
-        GAUNT and GAUGE always run in FP64)."""
+        precision="mixed" makes the Hermite integrals of the quartets whose
+        screening bound is below fp32_cutoff in FP32 (the reference is FP64
+        throughout; GAUNT and GAUGE always run in FP64)."""
         n = (_cabi.CQF_REL_NMAT_GAUNT if contType in (GAUNT, GAUGE)
              else _cabi.CQF_REL_NMAT)
         if len(matList) != n:

@@ -67,6 +67,9 @@ struct JKLaunch {
   int braOff;               // position of the launch's first bra pair in its class (slabs)
   int precision;            // 0 FP64, 1 mixed
   double fp32_cut;          // mixed: bound < cut -> FP32 ERIs
+  // launches whose kernels share quartets among lanes: a lane's primitive
+  // quartets, and whether every word may be listed in parts
+  int planEach, planAll;
   int shardIdx, shardCnt;   // bra pairs p with p % shardCnt == shardIdx only
   unsigned long long* counters;  // [0] visited, [1] screened, [2] fp32, [3] fp64
 };

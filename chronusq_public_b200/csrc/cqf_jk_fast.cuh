@@ -285,10 +285,18 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
     // slabs of bra pairs whose mask words fit the stream's region; each
     // reuses the region and the stream's counters after the last one's
     // kernels (stream order)
-    // (class pairs whose lists may hold twice the words: 24 B a word)
-    const bool cut = CUTTABLE && (long long)b.nBra * nTiles <= JK_CUT_WORDS &&
-                     maskWords >= 2 * nTiles;
-    const int slab = (int)std::max<long long>(1, (cut ? maskWords * 2 / 3 : maskWords) / nTiles);
+    // launches that share quartets among lanes: lists of twice the words (24 B
+    // a word), or in the smallest of eight times the words
+    const long long all = (long long)b.nBra * nTiles;
+    const bool tiny = CUTTABLE && all <= JK_TINY_WORDS && all * JK_TINY_BYTES <= maskWords * 16;
+    const bool cut = tiny || (CUTTABLE && b.lsum <= JK_CUT_LSUM && all <= JK_CUT_WORDS &&
+                              maskWords >= 2 * nTiles);
+    const int dup = tiny ? 8 : (cut ? 2 : 1);
+    b.planEach = tiny ? 8 : 64;
+    b.planAll = tiny;
+    const int slab = tiny ? b.nBra
+                          : (int)std::max<long long>(
+                                1, (cut ? maskWords * 2 / 3 : maskWords) / nTiles);
     for (int ib0 = 0; ib0 < b.nBra; ib0 += slab) {
       JKLaunch c = b;
       c.braBeg = b.braBeg + ib0;
@@ -298,7 +306,7 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
       const long long nWords = (long long)c.nBra * nTiles;
       // word lists: FP64 then FP32, nWords entries each; counts in work[2..3]
       int* list64 = reinterpret_cast<int*>(masks + nWords);
-      int* list32 = list64 + (cut ? 2 : 1) * nWords;
+      int* list32 = list64 + dup * nWords;
       launch_jk_plan(c, mixed, cut, masks, list64, list32, work + 2, nsm, st);
       constexpr int WPB = JK_THREADS / 32;
       auto grid = [&](long long items) {
@@ -307,7 +315,7 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
       };
       auto launch = [&](auto split) {
         constexpr bool S = decltype(split)::value;
-        const long long n = nWords * (S ? 2 : 1);
+        const long long n = nWords * dup;
         const int e64 = entries_per_item(n, G64::NCHUNK, nsm);
         jk_class_kernel<G64, false, S><<<grid((n + e64 - 1) / e64 * G64::NCHUNK), JK_THREADS, 0,
                                          st>>>(c, masks, list64, work + 2, e64, work);

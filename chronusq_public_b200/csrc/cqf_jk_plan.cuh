@@ -42,22 +42,27 @@ __device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P
 // list per precision (lengths in lcount[0 / 1]), so the class kernels visit
 // only words that name quartets of their precision.
 //
-// CUT (class pairs whose kernels share a quartet among lanes, jk_split): a
-// word whose quartets have long primitive loops (PLAN_HEAVY primitive
-// quartets or more) carries log2 of the lanes per quartet in its list entry,
-// and in the first eighth of the words -- pairs come in descending order of
-// their primitive counts -- it is listed as eight entries of four kets, so
-// that several warps share it; the lists then hold up to twice the words.
-// Without it one lane walked the 4096 primitive quartets of two contractions
-// of eight: 1.4 ms of a 2.3 ms build of one water molecule.
+// CUT (launches whose class kernels share a quartet among lanes): a word whose
+// quartets have long primitive loops (4 planEach primitive quartets or more)
+// carries log2 of the lanes per quartet in its list entry, and is listed as
+// eight entries of four kets, so that several warps share it: in the first
+// eighth of the words -- pairs come in descending order of their primitive
+// counts -- so that the lists hold at most twice the words, or anywhere
+// (planAll) where they have room for eight times the words.  Without it one
+// lane walked the 4096 primitive quartets of two contractions of eight: 1.4 ms
+// of a 2.3 ms build of one water molecule.
 constexpr int PLAN_RUN = 32;
-constexpr int PLAN_HEAVY = 256, PLAN_EACH = 64;  // primitive quartets: heavy, a lane's share
-constexpr int PLAN_WORD = (1 << 20) - 1;         // list entry: word | sub << 20 | part << 23 | log2 << 24
-__host__ __device__ constexpr bool jk_split(int lsum) { return lsum <= 2; }
-// only launches of at most this many words: larger ones have enough quartets
-// to hide the longest loops, and the shared form costs them registers
-// ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms)
+constexpr int PLAN_WORD = (1 << 20) - 1;  // list entry: word | sub << 20 | part << 23 | log2 << 24
+// class pairs of angular sums up to 2 in launches of up to 65536 words
+// (one water 2292 -> 917 us, eight complex 4.22 -> 3.07 ms), and of sums up to
+// 4 in launches of a few hundred, a molecule or two (917 -> 904 us, the mixed
+// four-component build of one water 3.10 -> 2.92 ms); larger ones have enough
+// quartets to hide the longest loops, and the shared form costs them
+// registers ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms)
+__host__ __device__ constexpr bool jk_split(int lsum) { return lsum <= 4; }
 constexpr long long JK_CUT_WORDS = 1 << 16;
+constexpr long long JK_TINY_WORDS = 448;
+constexpr int JK_CUT_LSUM = 2, JK_TINY_BYTES = 8 + 2 * 8 * 4;  // per word, both lists eightfold
 template <bool MIXED, bool CUT>
 __global__ void __launch_bounds__(256)
     jk_plan_kernel(const JKLaunch a, uint2* __restrict__ masks, int* __restrict__ list64,
@@ -95,7 +100,7 @@ __global__ void __launch_bounds__(256)
           screened = bound < a.thresh;
           if (CUT && !screened) {
             const int np = P.npp * Q.npp;
-            while (np >= PLAN_HEAVY && sl < 5 && (np >> sl) > PLAN_EACH) sl++;
+            while (np >= 4 * a.planEach && sl < 5 && (np >> sl) > a.planEach) sl++;
           }
           w32 = MIXED && !screened && bound < cut &&
                 fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
@@ -115,7 +120,7 @@ __global__ void __launch_bounds__(256)
       if (CUT) {
         sl = (int)__reduce_max_sync(0xffffffffu, (unsigned)sl);
         entry |= sl << 24;
-        if (sl > 1 && word < nWords / 8) {  // eight entries, written here
+        if (sl > 1 && (a.planAll || word < nWords / 8)) {  // eight entries, written here
           const unsigned s64 = b64 >> (4 * (lane & 7)) & 15u, s32 = b32 >> (4 * (lane & 7)) & 15u;
           unsigned at = 0;
           if (lane < 8 ? s64 != 0u : (lane < 16 && s32 != 0u))

@@ -254,9 +254,10 @@ typedef enum {
  * type writes are zeroed.  The densities must be
  * Hermitian, as the reference requires (:144-145).  opts->is_complex is
  * ignored (always complex); opts->device_pointers, opts->stream, opts->screen
- * apply, and opts->precision = CQF_MIXED runs the quartets whose screening
- * bound is below opts->fp32_cutoff in FP32 arithmetic (digestion and
- * accumulation stay FP64; the reference is FP64 throughout). */
+ * apply, and opts->precision = CQF_MIXED makes the Hermite integrals (Boys
+ * values and their recursion) of the quartets whose screening bound is below
+ * opts->fp32_cutoff in FP32 (the expansions, digestion and accumulation stay
+ * FP64; the reference is FP64 throughout). */
 cqf_status cqf_rel_two_body_contract(cqf_basis* basis, const void* const* X, void* const* AX,
                                      int type, int compute_exchange, const cqf_opts* opts,
                                      cqf_stats* stats);
@@ -297,7 +298,8 @@ cqf_status cqf_four_comp_gd(cqf_basis* basis, const void* const* D, void* const*
  * d(mu nu|la si)/dR_{atom,xyz}, added into AX[(3 atom + xyz) * nMat + m]
  * (3 natom nMat N x N arrays) as 1/2 (A + A^T).  shell_atom[s] is the atom
  * of shell s (ChronusQ's mapSh2Cen).  Every quartet of significant pairs is
- * computed (the reference does not screen here); FP64; at most 8 matrices;
+ * computed (the reference does not screen here) but those on a single atom,
+ * whose derivatives cancel (counted as screened); FP64; at most 8 matrices;
  * complex and non-Hermitian X are not built (the reference stops on the
  * latter).  opts: device_pointers, stream, shard_index / shard_count. */
 cqf_status cqf_grad_two_body_contract(cqf_basis* basis, const int* shell_atom, int natom,
