@@ -165,9 +165,9 @@ def fma_peaks():
 
 def build_launches(basis, Q, mixed):
     """Kernels one closed-shell J+K build launches (l <= 2 bases): block
-    norms x2, max, norms_aux, Cartesian transforms x2, the FP32 density copy
-    (mixed), per class pair and bra slab the planning pass and the FP64 (and
-    FP32) class kernel, back transforms x2.  Class sizes are the significant
+    norms of both matrices, max, norms_aux, both Cartesian transforms, the
+    FP32 density copy (mixed), per class pair and bra slab the planning pass
+    and the FP64 (and FP32) class kernel, both back transforms.  Class sizes are the significant
     pairs (nonzero Schwarz bound) per angular-momentum class; the slab size
     is the library's mask region (2^18 words per stream)."""
     sys.path.insert(0, os.path.join(ROOT, "chronusq_public_b200", "csrc"))
@@ -184,7 +184,7 @@ def build_launches(basis, Q, mixed):
     need = max([max(cnt[a] * tiles(cnt[b]), cnt[b] * tiles(cnt[a]))
                 for i, a in enumerate(cls) for b in cls[:i + 1]] + [0])
     words = max(max(tiles(n) for n in cnt.values()), min(need, 1 << 18))
-    n = 2 + 1 + 1 + 2 + (1 if mixed else 0) + 2
+    n = 1 + 1 + 1 + 1 + (1 if mixed else 0) + 1
     for i, a in enumerate(cls):
         for b in cls[:i + 1]:
             bra, ket = orientation(a, b)

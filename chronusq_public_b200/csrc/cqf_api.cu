@@ -574,8 +574,10 @@ __global__ void ket_tiles_kernel(const PrimPairDev* __restrict__ pp,
 // ------------------------------------------------------------ build kernels
 // Shell-block infinity norms (ShellBlockNorm, direct.hpp:73-90): one thread
 // per (s1, s2) block, max over rows of the absolute row sums.
-__global__ void block_norms_kernel(const double* __restrict__ X, int cplx, int N,
-                                   const ShellDev* __restrict__ sh, int ns, double* out) {
+__global__ void block_norms_kernel(const MatList l, int cplx, int N,
+                                   const ShellDev* __restrict__ sh, int ns) {
+  const double* __restrict__ X = l.src[blockIdx.y];
+  double* out = l.dst[blockIdx.y];
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ns * ns) return;
   int s1 = k % ns, s2 = k / ns;
@@ -641,10 +643,11 @@ __global__ void norms_aux_kernel(const double* __restrict__ nm, int ns,
 }
 
 // Xc = T X T^T per matrix (T: block-diagonal Cartesian -> AO transform).
-__global__ void to_cart_kernel(const double* __restrict__ X, int cplx, int N, int nc,
+__global__ void to_cart_kernel(const MatList l, int cplx, int N, int nc,
                                const ShellDev* __restrict__ sh, const int* __restrict__ c2s,
-                               const double* __restrict__ sph, const int* __restrict__ sphOff,
-                               double* Xc) {
+                               const double* __restrict__ sph, const int* __restrict__ sphOff) {
+  const double* __restrict__ X = l.src[blockIdx.y];
+  double* Xc = l.dst[blockIdx.y];
   size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (k >= (size_t)nc * nc) return;
   int ci = (int)(k % nc), cj = (int)(k / nc);
@@ -679,10 +682,12 @@ __global__ void to_cart_kernel(const double* __restrict__ X, int cplx, int N, in
 
 // AX += 1/2 (B + B^H) (Hermitian) or AX += 1/2 B, B = T^T Ac T
 // (direct.hpp:2036-2066).
-__global__ void from_cart_kernel(const double* __restrict__ Ac, int cplx, int her, int N, int nc,
+__global__ void from_cart_kernel(const MatList l, int cplx, int N, int nc,
                                  const ShellDev* __restrict__ sh, const int* __restrict__ ao2s,
-                                 const double* __restrict__ sph, const int* __restrict__ sphOff,
-                                 double* AX) {
+                                 const double* __restrict__ sph, const int* __restrict__ sphOff) {
+  const double* __restrict__ Ac = l.src[blockIdx.y];
+  double* AX = l.dst[blockIdx.y];
+  const int her = l.mode[blockIdx.y];
   size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (k >= (size_t)N * N) return;
   int i = (int)(k % N), j = (int)(k / N);
@@ -1379,11 +1384,10 @@ cqf_status cqf_four_comp_core_hamiltonian(cqf_basis* B, int natom, const double*
 
 namespace cqf {
 
-void launch_block_norms(const cqf_basis* B, const double* X, int cplx, double* out,
-                        cudaStream_t st) {
+void launch_block_norms(const cqf_basis* B, const MatList& l, int n, int cplx, cudaStream_t st) {
   const size_t ns2 = (size_t)B->nshell * B->nshell;
-  block_norms_kernel<<<grid1(ns2, 128), 128, 0, st>>>(X, cplx, B->nbasis, B->d_shells, B->nshell,
-                                                      out);
+  block_norms_kernel<<<dim3(grid1(ns2, 128), n), 128, 0, st>>>(l, cplx, B->nbasis, B->d_shells,
+                                                               B->nshell);
 }
 
 void launch_max_norms(const double* nm, int nMat, size_t ns2, double* out,
@@ -1391,18 +1395,18 @@ void launch_max_norms(const double* nm, int nMat, size_t ns2, double* out,
   max_norms_kernel<<<grid1(ns2, 256), 256, 0, st>>>(nm, nMat, ns2, out, gmax);
 }
 
-void launch_from_cart(const cqf_basis* B, const double* Ac, int cplx, int her, double* AX,
-                      cudaStream_t st) {
+void launch_from_cart(const cqf_basis* B, const MatList& l, int n, int cplx, cudaStream_t st) {
   const size_t NN = (size_t)B->nbasis * B->nbasis;
-  from_cart_kernel<<<grid1(NN, 256), 256, 0, st>>>(Ac, cplx, her, B->nbasis, B->ncart,
-                                                   B->d_shells, B->d_ao2shell, B->d_sph,
-                                                   B->d_sphOff, AX);
+  from_cart_kernel<<<dim3(grid1(NN, 256), n), 256, 0, st>>>(l, cplx, B->nbasis, B->ncart,
+                                                            B->d_shells, B->d_ao2shell, B->d_sph,
+                                                            B->d_sphOff);
 }
 
-void launch_to_cart(const cqf_basis* B, const double* X, int cplx, double* Xc, cudaStream_t st) {
+void launch_to_cart(const cqf_basis* B, const MatList& l, int n, int cplx, cudaStream_t st) {
   const size_t nc2 = (size_t)B->ncart * B->ncart;
-  to_cart_kernel<<<grid1(nc2, 256), 256, 0, st>>>(X, cplx, B->nbasis, B->ncart, B->d_shells,
-                                                  B->d_cart2shell, B->d_sph, B->d_sphOff, Xc);
+  to_cart_kernel<<<dim3(grid1(nc2, 256), n), 256, 0, st>>>(l, cplx, B->nbasis, B->ncart,
+                                                           B->d_shells, B->d_cart2shell, B->d_sph,
+                                                           B->d_sphOff);
 }
 
 cqf_status basis_workspace(cqf_basis* B, size_t bytes) { return ensure_ws(B, bytes); }
@@ -1725,24 +1729,27 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
   CQF_CUDA(cudaMemsetAsync(work, 0, NWORK * sizeof(unsigned int), st));
 
   // shell-block norms (per matrix, symmetrised when non-Hermitian), max
-  for (int m = 0; m < nMat; m++) {
-    double* nm = ws + oNmM + m * ns2;
-    block_norms_kernel<<<grid1(ns2, 128), 128, 0, st>>>(
-        normSrc ? normSrc[m] : Xd[m], normSrc ? 1 : opts.is_complex, N, B->d_shells, ns, nm);
-    if (!list[m].hermitian) sym_norms_kernel<<<grid1(ns2, 128), 128, 0, st>>>(nm, ns);
-  }
+  auto noMode = [](int) { return 0; };
+  mat_batches(
+      nMat, ns2, [&](int m) { return normSrc ? normSrc[m] : Xd[m]; },
+      [&](int m) { return ws + oNmM + m * ns2; }, noMode,
+      [&](const MatList& l, int n) {
+        launch_block_norms(B, l, n, normSrc ? 1 : opts.is_complex, st);
+      });
+  for (int m = 0; m < nMat; m++)
+    if (!list[m].hermitian)
+      sym_norms_kernel<<<grid1(ns2, 128), 128, 0, st>>>(ws + oNmM + m * ns2, ns);
   max_norms_kernel<<<grid1(ns2, 256), 256, 0, st>>>(ws + oNmM, nMat, ns2, ws + oNm,
                                                     reinterpret_cast<unsigned long long*>(ws + oG));
   norms_aux_kernel<<<grid1(std::max(ns2, (size_t)B->npair), 256), 256, 0, st>>>(
       ws + oNm, ns, B->d_pairs, B->npair, ws + Lw.oNmT, ws + Lw.oPN);
   // densities to the Cartesian AO basis, zero accumulators
-  for (int m = 0; m < nMat; m++) {
-    to_cart_kernel<<<grid1((size_t)nc * nc, 256), 256, 0, st>>>(
-        Xd[m], opts.is_complex, N, nc, B->d_shells, B->d_cart2shell, B->d_sph, B->d_sphOff,
-        ws + oXc + m * matC);
+  mat_batches(
+      nMat, matC, [&](int m) { return Xd[m]; }, [&](int m) { return ws + oXc + m * matC; }, noMode,
+      [&](const MatList& l, int n) { launch_to_cart(B, l, n, opts.is_complex, st); });
+  for (int m = 0; m < nMat; m++)
     if (!list[m].hermitian && hermitian_eff(list[m], opts.is_complex != 0))
       symmetrize_kernel<<<grid1((size_t)nc * nc, 256), 256, 0, st>>>(ws + oXc + m * matC, nc);
-  }
   CQF_CUDA(cudaMemsetAsync(ws + oAc, 0, matC * nMat * sizeof(double), st));
   float* Xc32 = reinterpret_cast<float*>(ws + Lw.oXc32);
   const bool mixedReal =
@@ -1833,12 +1840,13 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
   }
   CQF_TRY(hgRc);
   CQF_CUDA(cudaGetLastError());
-  for (int m = 0; m < nMat; m++)
-    from_cart_kernel<<<grid1((size_t)N * N, 256), 256, 0, st>>>(
-        ws + oAc + m * matC, opts.is_complex,
-        list[m].hermitian < 0 ? 2 : (hermitian_eff(list[m], opts.is_complex != 0) ? 1 : 0),
-        N, nc, B->d_shells,
-        B->d_ao2shell, B->d_sph, B->d_sphOff, AXd[m]);
+  mat_batches(
+      nMat, (size_t)N * N * (opts.is_complex ? 2 : 1),
+      [&](int m) { return ws + oAc + m * matC; }, [&](int m) { return AXd[m]; },
+      [&](int m) {
+        return list[m].hermitian < 0 ? 2 : (hermitian_eff(list[m], opts.is_complex != 0) ? 1 : 0);
+      },
+      [&](const MatList& l, int n) { launch_from_cart(B, l, n, opts.is_complex, st); });
   CQF_CUDA(cudaGetLastError());
   const bool staged = host && pinned && !capture;
   // staged downloads go in NSTAGE pieces over all matrices, an event after

@@ -185,15 +185,18 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   double* hAX = hX + (size_t)nMat * NN;
   CQF_GCUDA(cudaMemcpyAsync(dAtom, shell_atom, (size_t)B->nshell * sizeof(int),
                             cudaMemcpyHostToDevice, st));
-  for (int m = 0; m < nMat; m++) {
-    const double* X = static_cast<const double*>(list[m].X);
-    if (!o.device_pointers) {
-      CQF_GCUDA(cudaMemcpyAsync(hX + (size_t)m * NN, X, NN * sizeof(double),
+  if (!o.device_pointers)
+    for (int m = 0; m < nMat; m++)
+      CQF_GCUDA(cudaMemcpyAsync(hX + (size_t)m * NN, list[m].X, NN * sizeof(double),
                                 cudaMemcpyHostToDevice, st));
-      X = hX + (size_t)m * NN;
-    }
-    launch_to_cart(B, X, 0, Xc + (size_t)m * nc2, st);
-  }
+  auto noMode = [](int) { return 0; };
+  mat_batches(
+      nMat, nc2,
+      [&](int m) {
+        return o.device_pointers ? static_cast<const double*>(list[m].X) : hX + (size_t)m * NN;
+      },
+      [&](int m) { return Xc + (size_t)m * nc2; }, noMode,
+      [&](const MatList& l, int n) { launch_to_cart(B, l, n, 0, st); });
   CQF_GCUDA(cudaMemsetAsync(Ac, 0, (size_t)nGrad * nMat * nc2 * sizeof(double), st));
   CQF_GCUDA(cudaMemsetAsync(B->d_counters, 0, 4 * sizeof(unsigned long long), st));
   CQF_GCUDA(cudaEventRecord(B->ev0, st));
@@ -254,14 +257,17 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   }
   CQF_GCUDA(cudaGetLastError());
   // AX += 1/2 (A + A^T) per component and matrix (:2550-2560)
-  for (int k = 0; k < nGrad * nMat; k++) {
-    double* dst = static_cast<double*>(AX[k]);
-    if (!o.device_pointers) {
-      dst = hAX + (size_t)k * NN;
-      CQF_GCUDA(cudaMemcpyAsync(dst, AX[k], NN * sizeof(double), cudaMemcpyHostToDevice, st));
-    }
-    launch_from_cart(B, Ac + (size_t)k * nc2, 0, 1, dst, st);
-  }
+  if (!o.device_pointers)
+    for (int k = 0; k < nGrad * nMat; k++)
+      CQF_GCUDA(cudaMemcpyAsync(hAX + (size_t)k * NN, AX[k], NN * sizeof(double),
+                                cudaMemcpyHostToDevice, st));
+  mat_batches(
+      nGrad * nMat, NN, [&](int k) { return Ac + (size_t)k * nc2; },
+      [&](int k) {
+        return o.device_pointers ? static_cast<double*>(AX[k]) : hAX + (size_t)k * NN;
+      },
+      [](int) { return 1; },
+      [&](const MatList& l, int n) { launch_from_cart(B, l, n, 0, st); });
   CQF_GCUDA(cudaGetLastError());
   CQF_GCUDA(cudaEventRecord(B->ev1, st));
   if (!o.device_pointers)

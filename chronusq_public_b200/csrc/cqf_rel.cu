@@ -22,10 +22,10 @@
 //
 // Layout: densities and accumulators live in the Cartesian AO basis (exact
 // transforms before and after, as on the 1C path); Coulomb accumulators are
-// real, exchange accumulators complex.  One thread per unique shell quartet
-// loops over the ket's Cartesian components; for each it sums the primitive
-// quartets into the operator components of every bra component pair and
-// digests them with FP64 atomics.  Hermitian outputs are completed from the
+// real, exchange accumulators complex.  The integrals of a shell quartet come
+// from the Hermite-matrix engine (cqf_hgemm.cuh), both pairs' operator
+// components in its coefficient tables; the digestion reads them from shared
+// memory (cqf_hg_digest.cuh) and adds with FP64 atomics.  Hermitian outputs are completed from the
 // accumulated half at the back transform (the reference's "upper =
 // conj(lower)" after Hermitian digestion).
 #include <algorithm>
@@ -1321,11 +1321,14 @@ cqf_status ensure_rel_schwarz(cqf_basis* B, bool needLL, bool needSS, bool needG
 // AX (complex N x N, assigned) from a Cartesian accumulator, B = T^T Ac T:
 //   mode 0: B (complex)             mode 1: B + B^T (real Ac)
 //   mode 2: i (B - B^T) (real Ac)   mode 3: B + B^H (complex)
-__global__ void rel_from_cart_kernel(const double* __restrict__ Ac, int mode, int N, int nc,
+__global__ void rel_from_cart_kernel(const MatList l, int N, int nc,
                                      const ShellDev* __restrict__ sh,
                                      const int* __restrict__ ao2s,
                                      const double* __restrict__ sph,
-                                     const int* __restrict__ sphOff, double* AX) {
+                                     const int* __restrict__ sphOff) {
+  const double* __restrict__ Ac = l.src[blockIdx.y];
+  double* AX = l.dst[blockIdx.y];
+  const int mode = l.mode[blockIdx.y];
   size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (k >= (size_t)N * N) return;
   const int i = (int)(k % N), j = (int)(k / N);
@@ -1492,6 +1495,32 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
                               bool gauge, const cqf_opts& opts, cudaStream_t st, double* ws,
                               unsigned long long* cnt);
 
+// A list of (source, destination, mode) collected for one launch of a
+// per-matrix kernel.
+struct MatJobs {
+  std::vector<const double*> src;
+  std::vector<double*> dst;
+  std::vector<int> mode;
+  void add(const double* s, double* d, int m = 0) {
+    src.push_back(s);
+    dst.push_back(d);
+    mode.push_back(m);
+  }
+  template <class F>
+  void run(size_t span, F f) const {
+    mat_batches(
+        (int)src.size(), span, [&](int m) { return src[m]; }, [&](int m) { return dst[m]; },
+        [&](int m) { return mode[m]; }, f);
+  }
+};
+void run_back(const cqf_basis* B, const MatJobs& jobs, cudaStream_t st) {
+  const size_t NN = (size_t)B->nbasis * B->nbasis;
+  jobs.run(2 * NN, [&](const MatList& l, int n) {
+    rel_from_cart_kernel<<<dim3(rgrid(NN, 256), n), 256, 0, st>>>(
+        l, B->nbasis, B->ncart, B->d_shells, B->d_ao2shell, B->d_sph, B->d_sphOff);
+  });
+}
+
 // go(cb, ck, region, stream) for every class pair with quartets (every
 // ordered one, or ck <= cb), round-robin over the call's stream and the
 // auxiliary ones with a mask region each: the launches only add into the
@@ -1608,11 +1637,12 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
   double* Kc[4] = {accb + 5 * nc2, accb + 7 * nc2, accb + 9 * nc2, accb + 11 * nc2};
   auto XC = [&](int slot) { return xc + (size_t)slot * 2 * nc2; };
   // slots: 0 CLLMS, 1..4 CSSM*, 5..8 exchange densities
-  if (llss) launch_to_cart(B, X[CQF_CLLMS], 1, XC(0), st);
-  for (int c = 0; c < 4; c++) launch_to_cart(B, X[CQF_CSSMS + c], 1, XC(1 + c), st);
+  MatJobs cart, norms, backs;
+  if (llss) cart.add(X[CQF_CLLMS], XC(0));
+  for (int c = 0; c < 4; c++) cart.add(X[CQF_CSSMS + c], XC(1 + c));
   if (exch)
-    for (int c = 0; c < 4; c++)
-      launch_to_cart(B, X[(llss ? CQF_XLSMS : CQF_XSSMS) + c], 1, XC(5 + c), st);
+    for (int c = 0; c < 4; c++) cart.add(X[(llss ? CQF_XLSMS : CQF_XSSMS) + c], XC(5 + c));
+  cart.run(2 * nc2, [&](const MatList& l, int n) { launch_to_cart(B, l, n, 1, st); });
   // screening norms: max over CLLMS, CSSM*, XLSM* (LLSS) or CSSM* (SSSS)
   std::vector<int> smats = {CQF_CSSMS, CQF_CSSMX, CQF_CSSMY, CQF_CSSMZ};
   if (llss) {
@@ -1621,8 +1651,8 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
       if (X[CQF_XLSMS + c]) smats.push_back(CQF_XLSMS + c);
   }
   double* nmAll = nrm + ns2;
-  for (size_t i = 0; i < smats.size(); i++)
-    launch_block_norms(B, X[smats[i]], 1, nmAll + i * ns2, st);
+  for (size_t i = 0; i < smats.size(); i++) norms.add(X[smats[i]], nmAll + i * ns2);
+  norms.run(ns2, [&](const MatList& l, int n) { launch_block_norms(B, l, n, 1, st); });
   launch_max_norms(nmAll, (int)smats.size(), ns2, nrm,
                    reinterpret_cast<unsigned long long*>(nmAll + 9 * ns2), st);
   CQF_RCUDA(cudaMemsetAsync(accb, 0, 13 * nc2 * sizeof(double), st));
@@ -1670,17 +1700,14 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
         return llss ? launch_rel<1>(B, a, cb, ck, r, ls) : launch_rel<2>(B, a, cb, ck, r, ls);
       }));
   CQF_RCUDA(cudaGetLastError());
-  auto back = [&](const double* src, int mode, double* dst) {
-    rel_from_cart_kernel<<<rgrid(NN, 256), 256, 0, st>>>(src, mode, N, nc, B->d_shells,
-                                                         B->d_ao2shell, B->d_sph, B->d_sphOff,
-                                                         dst);
-  };
+  auto back = [&](const double* src, int mode, double* dst) { backs.add(src, dst, mode); };
   if (llss) back(Jll, 1, AX[CQF_CLLMS]);
   back(Jss[0], 1, AX[CQF_CSSMS]);
   for (int c = 1; c < 4; c++) back(Jss[c], 2, AX[CQF_CSSMS + c]);
   if (exch)
     for (int c = 0; c < 4; c++)
       back(Kc[c], llss ? 0 : 3, AX[(llss ? CQF_XLSMS : CQF_XSSMS) + c]);
+  run_back(B, backs, st);
   CQF_RCUDA(cudaGetLastError());
   unsigned long long h[4];
   CQF_RCUDA(cudaMemcpyAsync(h, dcnt, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
@@ -1728,9 +1755,11 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
   auto AC = [&](int slot) { return accb + (size_t)slot * 2 * nc2; };
   // density slots: 0 XLLM*, 4 XSSM*, 8 CLSM*, 12 CSLM*, 16 XSLM*
   const int src[5] = {CQF_XLLMS, CQF_XSSMS, CQF_CLSMS, CQF_CSLMS, CQF_XSLMS};
+  MatJobs cart, norms, backs;
   for (int k = 0; k < 5; k++)
     for (int c = 0; c < 4; c++)
-      if (X[src[k] + c]) launch_to_cart(B, X[src[k] + c], 1, XC(4 * k + c), st);
+      if (X[src[k] + c]) cart.add(X[src[k] + c], XC(4 * k + c));
+  cart.run(2 * nc2, [&](const MatList& l, int n) { launch_to_cart(B, l, n, 1, st); });
   // screening norms: max over XLSM*, XSLM*, XLLM*, XSSM*
   // (without exchange, the LS / SL Coulomb entries stand for the same
   // LS / SL blocks)
@@ -1743,8 +1772,8 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
       if (X[m]) smats.push_back(m);
     }
   double* nmAll = nrm + ns2;
-  for (size_t i = 0; i < smats.size(); i++)
-    launch_block_norms(B, X[smats[i]], 1, nmAll + i * ns2, st);
+  for (size_t i = 0; i < smats.size(); i++) norms.add(X[smats[i]], nmAll + i * ns2);
+  norms.run(ns2, [&](const MatList& l, int n) { launch_block_norms(B, l, n, 1, st); });
   launch_max_norms(nmAll, (int)smats.size(), ns2, nrm,
                    reinterpret_cast<unsigned long long*>(nmAll + 16 * ns2), st);
   CQF_RCUDA(cudaMemsetAsync(accb, 0, 16 * 2 * nc2 * sizeof(double), st));
@@ -1806,11 +1835,7 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
             });
       }));
   CQF_RCUDA(cudaGetLastError());
-  auto back = [&](const double* srcAcc, int mode, double* dst) {
-    rel_from_cart_kernel<<<rgrid(NN, 256), 256, 0, st>>>(srcAcc, mode, N, nc, B->d_shells,
-                                                         B->d_ao2shell, B->d_sph, B->d_sphOff,
-                                                         dst);
-  };
+  auto back = [&](const double* srcAcc, int mode, double* dst) { backs.add(srcAcc, dst, mode); };
   for (int c = 0; c < 4; c++) {
     back(AC(8 + c), 0, AX[CQF_CLSMS + c]);
     if (exch) {
@@ -1819,6 +1844,7 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
       back(AC(12 + c), 0, AX[CQF_XLSMS + c]);
     }
   }
+  run_back(B, backs, st);
   CQF_RCUDA(cudaGetLastError());
   unsigned long long h[4];
   CQF_RCUDA(cudaMemcpyAsync(h, dcnt, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));

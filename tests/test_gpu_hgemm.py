@@ -114,3 +114,35 @@ def test_engine_gradient(name):
     for g in range(6):
         for m in range(2):
             assert max_rel(cl[g][m].AX, np.asarray(ref[g][m])) < 1e-11, (g, m)
+
+
+@pytest.mark.parametrize("count", [32, 33])
+def test_many_matrices_share_outputs(count):
+    """Device matrices in batches of 32 launches; every contraction adds into
+    one J, half of the exchanges into one K, so each is the sum of its parts."""
+    torch = pytest.importorskip("torch")
+    bs = basis("one")
+    N = bs.nbasis
+    tpi = DirectTPI(bs)
+    rng = np.random.default_rng(71)
+    Ds = [d + d.T for d in rng.normal(size=(count, N, N))]
+    dev = [torch.tensor(d, device="cuda").T for d in Ds]
+    zero = lambda: torch.zeros((N, N), dtype=torch.float64, device="cuda").T
+    J, K, L = zero(), zero(), zero()
+    lst = []
+    for k, d in enumerate(dev):
+        lst.append(TwoBodyContraction(d, J, True, COULOMB))
+        lst.append(TwoBodyContraction(d, K if k % 2 else L, True, EXCHANGE))
+    GTODirectTPIContraction(tpi).twoBodyContract(lst)
+    torch.cuda.synchronize()
+    refs = [[], []]
+    for d in Ds:
+        r = [TwoBodyContraction(np.asfortranarray(d), np.zeros((N, N), order="F"), True, t)
+             for t in (COULOMB, EXCHANGE)]
+        GTODirectTPIContraction(tpi).twoBodyContract(r)
+        for t in range(2):
+            refs[t].append(r[t].AX)
+    # sums of 64 or 66 numbers of one size in another order
+    for got, ref in ((J, sum(refs[0])), (K, sum(refs[1][1::2])), (L, sum(refs[1][::2]))):
+        scale = max(np.abs(m).max() for t in refs for m in t)
+        assert np.abs(got.cpu().numpy() - ref).max() < 1e-13 * count * scale
