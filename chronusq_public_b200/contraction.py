@@ -35,26 +35,27 @@ class TwoBodyContraction:
     contType: int = COULOMB
 
 
+# cqf_shell as a record (field by field through ctypes, a basis of 96 shells
+# took 0.4 ms)
+_SHELL_DTYPE = np.dtype([("l", "i4"), ("pure", "i4"), ("nprim", "i4"), ("alpha", "u8"),
+                         ("coeff", "u8"), ("origin", "f8", 3)], align=True)
+assert _SHELL_DTYPE.itemsize == C.sizeof(_cabi.CqfShell)
+
+
 def shell_array(basis: BasisSet):
     """(cqf_shell array, owner) of a basis: the ctypes shells point into
     arrays held by `owner`, which must outlive every use of the shells."""
     f = basis.flat()
     alpha = np.ascontiguousarray(f["alpha"], dtype=np.float64)
     coef = np.ascontiguousarray(f["coef"], dtype=np.float64)
-    sh = (_cabi.CqfShell * basis.nshell)()
-    dp = C.POINTER(C.c_double)
-    off = 0
-    for s in range(basis.nshell):
-        n = int(f["nprim"][s])
-        sh[s].l = int(f["l"][s])
-        sh[s].pure = int(f["pure"][s])
-        sh[s].nprim = n
-        sh[s].alpha = C.cast(alpha.ctypes.data + 8 * off, dp)
-        sh[s].coeff = C.cast(coef.ctypes.data + 8 * off, dp)
-        for x in range(3):
-            sh[s].origin[x] = float(f["origin"][s, x])
-        off += n
-    return sh, (f, alpha, coef)
+    rec = np.zeros(basis.nshell, dtype=_SHELL_DTYPE)
+    for k in ("l", "pure", "nprim", "origin"):
+        rec[k] = f[k]
+    off = 8 * (np.cumsum(f["nprim"], dtype=np.uint64) - f["nprim"].astype(np.uint64))
+    rec["alpha"] = off + np.uint64(alpha.ctypes.data)
+    rec["coeff"] = off + np.uint64(coef.ctypes.data)
+    sh = (_cabi.CqfShell * basis.nshell).from_buffer(rec)
+    return sh, (f, alpha, coef, rec)
 
 
 class DirectTPI:
