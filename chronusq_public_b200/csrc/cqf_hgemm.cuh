@@ -42,6 +42,7 @@
 #include <atomic>
 
 #include "cqf_eri.cuh"
+#include "cqf_hg_items.hpp"
 #include "cqf_internal.hpp"
 
 namespace cqf {
@@ -374,13 +375,12 @@ __device__ __forceinline__ void hg_gemm2(const double* tab, int kt, int rtn, int
   }
 }
 
-// Items of contracted classes: every listed word cut into at most `most`
-// parts of about `work` primitive quartets -- the bra's primitives in cb
-// ranges, the kets' (concatenated) in ck ones.  Without it the words of the
-// longest contractions (32 x 64 x 64 primitive quartets against a mean of a
-// few hundred) were the whole launch's tail: SMs were active for 22% of the
-// (ss|ss) gradient launch.  item = {word | FP32 << 31, b | cb << 8 | k << 16 |
-// ck << 24}.
+// Items of contracted classes: every listed word cut into parts of about
+// `work` primitive quartets, at most `most` of them over both lists (hg_cut).
+// Without it the words of the longest contractions (32 x 64 x 64 primitive
+// quartets against a mean of a few hundred) were the whole launch's tail: SMs
+// were active for 22% of the (ss|ss) gradient launch.
+// item = {word | FP32 << 31, b | cb << 8 | k << 16 | ck << 24}.
 __global__ static void __launch_bounds__(128)
     hg_expand_kernel(const PairDev* __restrict__ pairs, int braBeg, int ketBeg, int nTiles,
                      const uint2* __restrict__ masks, const int* __restrict__ list64,
@@ -392,13 +392,15 @@ __global__ static void __launch_bounds__(128)
     const int word = lo ? list32[i - n64] : list64[i];
     const uint2 mk = masks[word];
     const int ib = word / nTiles, jk0 = (word - ib * nTiles) * WTILE;
-    const int np = pairs[braBeg + ib].npp;
-    int nk = 0;
-    for (unsigned b = lo ? mk.y : mk.x; b; b &= b - 1u)
-      nk += pairs[ketBeg + jk0 + __ffs(b) - 1].npp;
-    const int want = max(1, min(most, (int)(((long long)np * nk + work - 1) / work)));
-    // the bra's primitives first: a batch holds ket primitives of one of them
-    const int cb = max(1, min(min(np, want), 255)), ck = max(1, min(nk, want / cb));
+    // the primitives of the entry's kets and of the word's other ones
+    int nk = 0, other = 0;
+    for (unsigned b = mk.x | mk.y; b; b &= b - 1u) {
+      const int n1 = pairs[ketBeg + jk0 + __ffs(b) - 1].npp;
+      if ((lo ? mk.y : mk.x) & (b & -b)) nk += n1;
+      else other += n1;
+    }
+    const HgCut c = hg_cut(pairs[braBeg + ib].npp, nk, other, work, most);
+    const int cb = c.cb, ck = c.ck;
     const unsigned at = atomicAdd(nItems, (unsigned)(cb * ck));
     for (int b = 0; b < cb; b++)
       for (int k = 0; k < ck; k++)
@@ -825,17 +827,11 @@ inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, in
     h.ket[q] = {B->d_hg[tk] + B->hg_beg[tk][ck], B->cls_pp_beg[ck]};
   }
   const int npb = B->cls_npp_max[cb], npk = B->cls_npp_max[ck];
-  // contracted classes: words are cut by their number of primitive quartets,
-  // into at most `most` items of 8 B beside the word's mask and list entries
-  // (16 B).  As many as leave the launch in one slab, but at least 16 (and
-  // never more than a row of words leaves room for)
-  const bool cut = npb * npk > 1;
-  const long long room = 2 * r.maskWords;
-  const int most =
-      cut ? (int)std::min(std::min(255LL, room / h.nTiles - 2),
-                          std::max(16LL, room / ((long long)nBra * h.nTiles) - 2))
-          : 0;
-  const long long words = most > 1 ? room / (2 + most) : r.maskWords;
+  // contracted classes: words are cut by their number of primitive quartets
+  const HgSlab sl = npb > 1 || npk > 1 ? hg_slab(2 * r.maskWords, nBra, h.nTiles)
+                                  : HgSlab{0, r.maskWords};
+  const int most = sl.most;
+  const long long words = sl.words;
   const int slab = (int)std::max<long long>(1, words / h.nTiles);
   const long long fill = 16LL * B->nsm;  // items that keep the GPU busy
   for (int ib0 = 0; ib0 < nBra; ib0 += slab) {
@@ -853,7 +849,7 @@ inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, in
     plan(ib0, n, r.masks, list64, list32, r.work + 2, gp);
     h.nsub = 1;
     long long nItems;
-    if (most > 1) {
+    if (most) {
       uint2* items = r.masks + 2 * nWords;
       h.items = items;
       h.nItems = r.work + 1;

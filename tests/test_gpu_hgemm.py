@@ -146,3 +146,53 @@ def test_many_matrices_share_outputs(count):
     for got, ref in ((J, sum(refs[0])), (K, sum(refs[1][1::2])), (L, sum(refs[1][::2]))):
         scale = max(np.abs(m).max() for t in refs for m in t)
         assert np.abs(got.cpu().numpy() - ref).max() < 1e-13 * count * scale
+
+
+def ring_basis():
+    """24 centres with an s of 7 and an f of 3 primitives: 5400 words in
+    (ss|fs), whose items fill the launch stream's region, and (fs|fs) in two
+    slabs."""
+    t = 2 * np.pi * np.arange(24) / 24
+    mol = Molecule.from_angstrom([("H", 2 * np.cos(a), 2 * np.sin(a), 0.3 * (i % 2))
+                                  for i, a in enumerate(t)])
+    gbs = "****\nH 0\nS 7 1.00\n" + "".join("  %g %g\n" % (0.12 * 2.2 ** k, 0.2 + 0.05 * k)
+                                             for k in range(7))
+    gbs += "F 3 1.00\n  0.5 0.5\n  1.05 0.5\n  2.205 0.5\n****\n"
+    return BasisSet.build(mol, parse_gbs(gbs))
+
+
+def test_engine_items_fill_region():
+    """Words with FP64 and FP32 quartets share the items of their word: a mixed
+    build whose items fill the region equals the FP64 build, and both the
+    oracle's integrals summed over whole shell blocks without a screen (some 2e3
+    quartets a block, each within 1e-12 / 2 of its screened value)."""
+    bs = ring_basis()
+    N = bs.nbasis
+    rng = np.random.default_rng(3)
+    A = rng.standard_normal((N, N))
+    D = np.asfortranarray(0.1 * (A + A.T))
+    res = {}
+    for prec in ("fp64", "mixed"):
+        c = GTODirectTPIContraction(DirectTPI(bs))
+        lst = [TwoBodyContraction(D, np.zeros((N, N), order="F"), True, t)
+               for t in (COULOMB, EXCHANGE)]
+        c.twoBodyContract(lst, precision=prec, fp32_cutoff=1e-4)
+        res[prec] = [m.AX for m in lst]
+    assert c.last_stats["fp32"] > 3e5 and c.last_stats["fp64"] > 3e5
+    for a, b in zip(res["mixed"], res["fp64"]):
+        assert max_rel(a, b) < 1e-6
+    ob = O.OracleBasis(bs)
+    sl = [slice(o, o + s.size) for o, s in zip(bs.offsets, bs.shells)]
+    f = [s for s in range(bs.nshell) if bs.shells[s].l == 3]
+    o = [s for s in range(bs.nshell) if bs.shells[s].l == 0]
+    for a, b in ((f[0], o[0]), (o[20], o[2])):
+        J = K = 0.0
+        for c in range(bs.nshell):
+            for d in range(bs.nshell):
+                if d <= c:
+                    g = ob.eri_quartet(a, b, c, d)
+                    w = D[sl[c], sl[d]] * (1.0 if c == d else 2.0)
+                    J = J + np.einsum("abcd,cd->ab", g, w)
+                K = K + np.einsum("acbd,cd->ab", ob.eri_quartet(a, c, b, d), D[sl[c], sl[d]])
+        for got, ref in zip(res["fp64"], (J, K)):
+            assert np.abs(got[sl[a], sl[b]] - ref).max() < 1e-11 * np.abs(got).max() + 2e-9
