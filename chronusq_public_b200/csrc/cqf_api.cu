@@ -1049,15 +1049,25 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
                                                                  d_tmp, B->npair, B->d_pp);
   CQF_CUDA(cudaMallocAsync(&B->d_schwarz, (size_t)nshell * nshell * sizeof(double), B->stream));
   CQF_CUDA(cudaMemsetAsync(B->d_schwarz, 0, (size_t)nshell * nshell * sizeof(double), B->stream));
+  // partial diagonals of a class's pairs, in slabs of at most SCHWARZ_ROOM
+  // doubles (64 MiB)
+  constexpr size_t SCHWARZ_ROOM = size_t(8) << 20;
+  size_t diagRoom = 36;
+  for (int c = 0; c < NCLS; c++) {
+    int la, lb;
+    class_ls(c, la, lb);
+    diagRoom = std::max(diagRoom, (size_t)B->cls_cnt[c] * 36 * schwarz_chunks(la, lb));
+  }
+  diagRoom = std::min(diagRoom, SCHWARZ_ROOM);
   double* d_diag = nullptr;
-  CQF_CUDA(cudaMallocAsync(&d_diag, std::max(1, B->npair) * 36 * sizeof(double), B->stream));
+  CQF_CUDA(cudaMallocAsync(&d_diag, diagRoom * sizeof(double), B->stream));
   for (int c = 0; c < NCLS; c++) {
     if (B->cls_cnt[c] <= 0) continue;
     int la, lb;
     class_ls(c, la, lb);
     if (!launch_schwarz_fast(la, lb, d_tmp, B->d_pp, B->d_boys64, B->d_sph, B->d_sphOff,
                              B->d_shells, B->cls_beg[c], B->cls_cnt[c], nshell, B->d_schwarz,
-                             d_tmp, d_diag + (size_t)B->cls_beg[c] * 36, B->stream))
+                             d_tmp, d_diag, diagRoom, B->stream))
       schwarz_kernel<<<B->cls_cnt[c], 128, 0, B->stream>>>(
           d_tmp, B->d_pp, B->d_boys64, B->d_sph, B->d_sphOff, B->d_shells, B->cls_beg[c],
           B->cls_cnt[c], nshell, B->d_schwarz, d_tmp);

@@ -346,8 +346,11 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
 // Diagonal (mu nu|mu nu) of the pairs of one class (LA, LB) with LA, LB <= 2
 // from the generated (ab|ab) code, SCHWARZ_LANES threads per (pair, chunk)
 // sharing its primitive loop (one thread each took 1.2 ms for contractions of
-// eight); each one's share of each spherical diagonal element is added into
-// diag[pair][mu][nu].
+// eight).  Their shares of each spherical diagonal element are summed by a
+// shuffle tree into the chunk's diag[pair][chunk][mu][nu], and the chunks in
+// order by the finishing kernel: the bounds order the pair list, which has to
+// come out alike in every process of a sharded build, so no sum may depend on
+// the order of atomics.
 constexpr int SCHWARZ_LANES = 16;
 template <class GC>
 __global__ void __launch_bounds__(JK_THREADS)
@@ -363,7 +366,8 @@ __global__ void __launch_bounds__(JK_THREADS)
   if (item >= (long long)n * NCH) return;
   const int k = (int)(item / NCH), ch = (int)(item % NCH);
   const PairDev P = pairs[beg + k];
-  if (sub >= P.npp) return;
+  const unsigned group = ((1u << SCHWARZ_LANES) - 1u)
+                         << ((threadIdx.x & 31) / SCHWARZ_LANES * SCHWARZ_LANES);
   const ShellDev A = shells[P.shA], B = shells[P.shB];
   const int na = A.pure ? nsph(GC::LA) : NA, nb = B.pure ? nsph(GC::LB) : NB;
   const double* TA = sph + sphOff[GC::LA];
@@ -390,22 +394,34 @@ __global__ void __launch_bounds__(JK_THREADS)
         }
         s += tcd * sab;
       }
-      if (s != 0.0) atomicAdd(diag + (size_t)k * 36 + mu * 6 + nu, s);
+#pragma unroll
+      for (int o = SCHWARZ_LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(group, s, o);
+      if (sub == 0) diag[(size_t)item * 36 + mu * 6 + nu] = s;
     }
 }
 
 // Q = sqrt(max row sum |diag|) with rows the functions of s1
-// (aointegrals_utilities.cxx:78-104); writes the pair and the table.
-__global__ void schwarz_finish_kernel(const PairDev* __restrict__ pairs,
-                                      const ShellDev* __restrict__ shells, int beg, int n,
-                                      int nshell, const double* __restrict__ diag, double* Qtab,
-                                      PairDev* pairsOut) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// (aointegrals_utilities.cxx:78-104); writes the pair and the table.  A warp
+// per pair: lanes sum an element's nch chunks, in order.
+__global__ void __launch_bounds__(128)
+    schwarz_finish_kernel(const PairDev* __restrict__ pairs, const ShellDev* __restrict__ shells,
+                          int beg, int n, int nch, int nshell, const double* __restrict__ diag,
+                          double* Qtab, PairDev* pairsOut) {
+  __shared__ double sd[4][36];
+  const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (k >= n) return;
   const PairDev P = pairs[beg + k];
   const ShellDev A = shells[P.shA], B = shells[P.shB];
   const int na = A.pure ? nsph(A.l) : ncart(A.l), nb = B.pure ? nsph(B.l) : ncart(B.l);
-  const double* d = diag + (size_t)k * 36;
+  double* d = sd[threadIdx.x >> 5];
+  for (int e = lane; e < na * nb; e += 32) {
+    const int ij = e / nb * 6 + e % nb;
+    double v = 0.0;
+    for (int ch = 0; ch < nch; ch++) v += diag[((size_t)k * nch + ch) * 36 + ij];
+    d[ij] = v;
+  }
+  __syncwarp();
+  if (lane > 0) return;
   const bool swp = P.shA != P.s1;
   double mx = 0.0;
   if (!swp) {
@@ -427,22 +443,36 @@ __global__ void schwarz_finish_kernel(const PairDev* __restrict__ pairs,
   Qtab[P.s2 + (size_t)P.s1 * nshell] = q;
 }
 
+// Chunks of the class (la lb | la lb), 0 if it has no generated code.
+inline int schwarz_chunks(int la, int lb) {
+  int n = 0;
+#define CQF_SCHWARZ_CHUNKS(A_, B_, C_, D_, N64, N32) \
+  if (A_ == la && B_ == lb && C_ == la && D_ == lb) n = N64::NCHUNK;
+  CQF_GEN_JK_CLASSES(CQF_SCHWARZ_CHUNKS)
+#undef CQF_SCHWARZ_CHUNKS
+  return n;
+}
+
 // Schwarz bounds of one class with the generated code; false if the class
-// has none.  diag: n x 36 doubles (6 x 6 per pair), zeroed here.
+// has none.  diag: room for the 6 x 6 diagonals of every chunk of `room` / (36
+// chunks) pairs, at least one, at a time.
 inline bool launch_schwarz_fast(int la, int lb, const PairDev* pairs, const PrimPairDev* pp,
                                 const double* boys, const double* sph, const int* sphOff,
                                 const ShellDev* shells, int beg, int n, int nshell, double* Qtab,
-                                PairDev* pairsOut, double* diag, cudaStream_t st) {
+                                PairDev* pairsOut, double* diag, size_t room, cudaStream_t st) {
   if (n <= 0) return true;
   bool done = false;
   auto go = [&](auto tag64) {
     using G = decltype(tag64);
-    cudaMemsetAsync(diag, 0, (size_t)n * 36 * sizeof(double), st);
-    const long long items = (long long)n * G::NCHUNK * SCHWARZ_LANES;
-    schwarz_diag_kernel<G><<<(unsigned)((items + JK_THREADS - 1) / JK_THREADS), JK_THREADS, 0,
-                             st>>>(pairs, pp, boys, sph, sphOff, shells, beg, n, diag);
-    schwarz_finish_kernel<<<(n + 127) / 128, 128, 0, st>>>(pairs, shells, beg, n, nshell, diag,
-                                                          Qtab, pairsOut);
+    const int slab = (int)std::min<size_t>(n, room / (36 * G::NCHUNK));
+    for (int k = 0; k < n; k += slab) {
+      const int m = std::min(slab, n - k);
+      const long long items = (long long)m * G::NCHUNK * SCHWARZ_LANES;
+      schwarz_diag_kernel<G><<<(unsigned)((items + JK_THREADS - 1) / JK_THREADS), JK_THREADS, 0,
+                               st>>>(pairs, pp, boys, sph, sphOff, shells, beg + k, m, diag);
+      schwarz_finish_kernel<<<(m + 3) / 4, 128, 0, st>>>(pairs, shells, beg + k, m, G::NCHUNK,
+                                                         nshell, diag, Qtab, pairsOut);
+    }
     done = true;
   };
 #define CQF_TRY_SCHWARZ(A_, B_, C_, D_, N64, N32) \

@@ -181,7 +181,9 @@ inline void launch_jk_generic(const JKLaunch& a, int la, int lb, int lc, int ld,
 // Q(s1,s2) = sqrt(|| D ||_inf), D(i,j) = (ij|ij) over the AOs of s1 (rows)
 // and s2 (columns): max row sum (aointegrals_utilities.cxx:78-104).
 // One block per pair, a thread per ket component pair (one thread per pair
-// took 48 ms for (ff|ff)).
+// took 48 ms for (ff|ff)); their shares of an element are summed by shuffles
+// and the warps in order (as in schwarz_diag_kernel, no sum depends on the
+// order of atomics).
 __global__ void __launch_bounds__(128)
     schwarz_kernel(const PairDev* __restrict__ pairs, const PrimPairDev* __restrict__ pp,
                    const double* __restrict__ boys, const double* __restrict__ sph,
@@ -196,22 +198,20 @@ __global__ void __launch_bounds__(128)
   const int na = A.pure ? nsph(la) : nca, nb = B.pure ? nsph(lb) : ncb;
   const double* TA = sph + sphOff[la];
   const double* TB = sph + sphOff[lb];
-  __shared__ double diag[ncart(LMAX)][ncart(LMAX)];
-  for (int i = threadIdx.x; i < ncart(LMAX) * ncart(LMAX); i += blockDim.x)
-    diag[i / ncart(LMAX)][i % ncart(LMAX)] = 0.0;
-  __syncthreads();
+  constexpr int NT = ncart(LMAX) * ncart(LMAX);
+  static_assert(NT <= 128, "a thread per ket component pair");
+  __shared__ double part[4][NT];  // per warp
   double col[RtBounds<LMAX>::NAB];
   // (mu nu|mu nu) = sum_{abcd} T_a,mu T_b,nu T_c,mu T_d,nu (ab|cd)
-  for (int cd = threadIdx.x; cd < nca * ncb; cd += blockDim.x) {
-    const int c = cd / ncb, d = cd % ncb;
-    eri_column_rt<double, LMAX>(la, lb, la, lb, c, d, P, P, pp, boys, col);
-    for (int mu = 0; mu < na; mu++) {
-      const double tc = A.pure ? TA[c * nsph(la) + mu] : (c == mu ? 1.0 : 0.0);
-      if (tc == 0.0) continue;
-      for (int nu = 0; nu < nb; nu++) {
-        const double td = B.pure ? TB[d * nsph(lb) + nu] : (d == nu ? 1.0 : 0.0);
-        if (td == 0.0) continue;
-        double s = 0.0;
+  const int cd = threadIdx.x, c = cd / ncb, d = cd % ncb;
+  const bool has = cd < nca * ncb;
+  if (has) eri_column_rt<double, LMAX>(la, lb, la, lb, c, d, P, P, pp, boys, col);
+  for (int mu = 0; mu < na; mu++) {
+    const double tc = !has ? 0.0 : (A.pure ? TA[c * nsph(la) + mu] : (c == mu ? 1.0 : 0.0));
+    for (int nu = 0; nu < nb; nu++) {
+      const double td = !has ? 0.0 : (B.pure ? TB[d * nsph(lb) + nu] : (d == nu ? 1.0 : 0.0));
+      double s = 0.0;
+      if (tc != 0.0 && td != 0.0) {
         for (int ia = 0; ia < nca; ia++) {
           const double ta = A.pure ? TA[ia * nsph(la) + mu] : (ia == mu ? 1.0 : 0.0);
           if (ta == 0.0) continue;
@@ -220,25 +220,32 @@ __global__ void __launch_bounds__(128)
             s += ta * tb * col[ia * ncb + ib];
           }
         }
-        atomicAdd(&diag[mu][nu], tc * td * s);
+        s *= tc * td;
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][mu * nb + nu] = s;
     }
   }
   __syncthreads();
   if (threadIdx.x > 0) return;
+  auto diag = [&](int i, int j) {
+    const int e = i * nb + j;
+    return (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
+  };
   // rows are the functions of s1 (the reference's first shell)
   const bool swp = P.shA != P.s1;
   double mx = 0.0;
   if (!swp) {
     for (int i = 0; i < na; i++) {
       double r = 0.0;
-      for (int j = 0; j < nb; j++) r += fabs(diag[i][j]);
+      for (int j = 0; j < nb; j++) r += fabs(diag(i, j));
       mx = fmax(mx, r);
     }
   } else {
     for (int j = 0; j < nb; j++) {
       double r = 0.0;
-      for (int i = 0; i < na; i++) r += fabs(diag[i][j]);
+      for (int i = 0; i < na; i++) r += fabs(diag(i, j));
       mx = fmax(mx, r);
     }
   }
