@@ -3,6 +3,7 @@
 
 #include "cqf_deriv.cuh"
 #include "cqf_hgemm.cuh"
+#include "cqf_once.hpp"
 
 namespace cqf {
 namespace {
@@ -102,19 +103,28 @@ __global__ void hg_pairs_kernel(const PairDev* __restrict__ in, const double* __
 }  // namespace
 
 cqf_status hg_ensure(cqf_basis* B, int kind) {
-  if (B->d_hg[kind]) return CQF_OK;
-  if (!B->d_pairsHg) {
-    const int n = std::max(1, B->npair);
-    cudaError_t e = cudaMallocAsync((void**)&B->d_pairsHg, n * sizeof(PairDev), B->stream);
-    if (e == cudaSuccess) {
-      hg_pairs_kernel<<<(n + 127) / 128, 128, 0, B->stream>>>(B->d_pairs, B->d_ppQ, B->npair,
-                                                              B->d_pairsHg);
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess)
-      return fail(e == cudaErrorMemoryAllocation ? CQF_ENOMEM : CQF_ECUDA,
-                  std::string("hg_ensure: ") + cudaGetErrorString(e));
-  }
+  auto status = [](cudaError_t e) {
+    if (e == cudaSuccess) return CQF_OK;
+    return fail(e == cudaErrorMemoryAllocation ? CQF_ENOMEM : CQF_ECUDA,
+                std::string("hg_ensure: ") + cudaGetErrorString(e));
+  };
+  // build_once with memory of the basis' stream; fill enqueues
+  auto build = [&](auto*& slot, size_t n, auto fill) {
+    return status(build_once(
+        slot, cudaSuccess,
+        [&](auto** p) { return cudaMallocAsync((void**)p, std::max<size_t>(1, n) * sizeof(**p), B->stream); },
+        [&](auto* p) {
+          fill(p);
+          const cudaError_t e = cudaGetLastError();
+          return e != cudaSuccess ? e : cudaStreamSynchronize(B->stream);
+        },
+        [&](auto* p) { cudaFreeAsync(p, B->stream); }));
+  };
+  const cqf_status s = build(B->d_pairsHg, B->npair, [&](PairDev* p) {
+    hg_pairs_kernel<<<std::max(1, (B->npair + 127) / 128), 128, 0, B->stream>>>(
+        B->d_pairs, B->d_ppQ, B->npair, p);
+  });
+  if (s != CQF_OK || B->d_hg[kind]) return s;
   size_t total = 0;
   for (int c = 0; c < NCLS; c++) {
     B->hg_beg[kind][c] = total;
@@ -125,27 +135,18 @@ cqf_status hg_ensure(cqf_basis* B, int kind) {
     for (int i = 0; i < B->cls_cnt[c]; i++) npp += B->h_pairs[B->cls_beg[c] + i].npp;
     total += npp * hg_size(kind, la, lb);
   }
-  double* d = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d, std::max<size_t>(1, total) * sizeof(double), B->stream);
-  for (int c = 0; c < NCLS && e == cudaSuccess; c++) {
-    if (!B->cls_cnt[c]) continue;
-    int la, lb;
-    class_ls(c, la, lb);
-    const size_t smem =
-        (3 * ht_e1(la, lb) + (size_t)12 * (la + 1) * (lb + 1) * ht_fl(la, lb)) * sizeof(double);
-    hg_table_kernel<<<dim3(B->cls_cnt[c], B->cls_npp_max[c]), HT_THREADS, smem, B->stream>>>(
-        B->d_pairs, B->d_pp, B->d_shells, B->d_prim, B->cls_beg[c], B->cls_pp_beg[c], kind, la, lb,
-        d + B->hg_beg[kind][c]);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
-  if (e != cudaSuccess) {
-    if (d) cudaFreeAsync(d, B->stream);
-    return fail(e == cudaErrorMemoryAllocation ? CQF_ENOMEM : CQF_ECUDA,
-                std::string("hg_ensure: ") + cudaGetErrorString(e));
-  }
-  B->d_hg[kind] = d;
-  return CQF_OK;
+  return build(B->d_hg[kind], total, [&](double* d) {
+    for (int c = 0; c < NCLS; c++) {
+      if (!B->cls_cnt[c]) continue;
+      int la, lb;
+      class_ls(c, la, lb);
+      const size_t smem =
+          (3 * ht_e1(la, lb) + (size_t)12 * (la + 1) * (lb + 1) * ht_fl(la, lb)) * sizeof(double);
+      hg_table_kernel<<<dim3(B->cls_cnt[c], B->cls_npp_max[c]), HT_THREADS, smem, B->stream>>>(
+          B->d_pairs, B->d_pp, B->d_shells, B->d_prim, B->cls_beg[c], B->cls_pp_beg[c], kind, la,
+          lb, d + B->hg_beg[kind][c]);
+    }
+  });
 }
 
 }  // namespace cqf
