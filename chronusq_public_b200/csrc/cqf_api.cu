@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <map>
 #include <cmath>
 #include <cstring>
@@ -921,6 +922,20 @@ cqf_status boys_tables(int device, cudaStream_t st, double** d64, float** d32) {
   return CQF_OK;
 }
 
+// What a basis' coefficient tables may hold on the device (bytes): a quarter
+// of its memory, or the environment's CQF_TABLE_LIMIT_MB.
+cqf_status table_limit(int device, size_t* limit) {
+  static std::mutex mu;
+  static std::map<int, size_t> total;  // device memory does not change
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& t = total[device];
+  size_t free = 0;
+  if (!t) CQF_CUDA(cudaMemGetInfo(&free, &t));
+  const char* mb = std::getenv("CQF_TABLE_LIMIT_MB");
+  *limit = mb && *mb ? (size_t)(std::max(0.0, std::atof(mb)) * 1048576.0) : t / 4;
+  return CQF_OK;
+}
+
 cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int device,
                         cqf_basis* B) {
   int ndev = 0;
@@ -944,6 +959,7 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
   }
   B->thresh = thresh;
   B->nshell = nshell;
+  CQF_TRY(table_limit(device, &B->hg_limit));
 
   // shells, primitive data
   std::vector<double> alpha, coef;
@@ -1470,6 +1486,9 @@ WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan
     L.maskWords = std::max(L.maskWords, B->maxL > 2 ? HG_MIN_WORDS : JK_MIN_WORDS);
   // per word: the uint2 mask and one entry in each of the two word lists
   L.oMask = take(std::max<size_t>(2 * L.maskWords * (NAUX + 1), 1));
+  // windows of both sides' tables where the basis does not hold them
+  L.win = plan && need > 0 && B->maxL > 2 ? 2 * B->hg_win[HG_PLAIN] : 0;
+  L.oWin = take(L.win * (NAUX + 1));
   L.total = off;
   return L;
 }
@@ -1836,8 +1855,9 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
       if (tune) CQF_CUDA(cudaEventRecord(B->tune_ev[2 * (cb * NCLS + ck)], st));
       uint2* masks = reinterpret_cast<uint2*>(ws + Lw.oMask) + 2 * Lw.maskWords * li;
       a.braOff = 0;
-      if (lm > 2 && Lw.maskWords > 0)
-        hgRc = launch_jk_hg(B, a, cb, ck, masks, (long long)Lw.maskWords, work + 4 * li, ls);
+      if (lm > 2 && Lw.maskWords > 0 && (Lw.win || !B->hg_win[HG_PLAIN]))
+        hgRc = launch_jk_hg(B, a, cb, ck, masks, (long long)Lw.maskWords, work + 4 * li,
+                            ws + Lw.oWin + Lw.win * li, ls);
       else if (!(fastOK && lm <= 2 &&
                  launch_jk_fast(a, la, lb, lc, ld, masks, (long long)Lw.maskWords, work + 4 * li,
                                 B->nsm, ls, B->blocks_per_sm[cb][ck])))

@@ -162,19 +162,20 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   // scratch (stream-ordered): shell atoms | Cartesian X | Cartesian
   // accumulators | host staging of X and AX
   const size_t host = o.device_pointers ? 0 : (size_t)nMat * NN + (size_t)nGrad * nMat * NN;
-  // then, per launch stream, the planning pass's masks and lists and four
-  // counters
+  // then, per launch stream, the planning pass's masks and lists, four
+  // counters, and windows of the tables that the basis does not hold
   size_t row = 1;
   for (int c = 0; c < NCLS; c++)
     row = std::max(row, ((size_t)B->cls_cnt[c] + WTILE - 1) / WTILE);
   const size_t maskWords = std::max(row, MASK_CAP_WORDS);
   const size_t lists = (2 * maskWords + 2) * (NAUX + 1);
   const size_t fixed = ((size_t)nMat * nc2 + (size_t)nGrad * nMat * nc2 + host + 1) / 2 * 2;
-  const size_t doubles = fixed + lists;
   for (int k : {(int)HG_PLAIN, (int)HG_D6, (int)HG_D3}) {
     const cqf_status s = hg_ensure(B, k);
     if (s != CQF_OK) return s;
   }
+  const size_t winDoubles = hg_windows<GradDig>(B);
+  const size_t doubles = fixed + lists + winDoubles * (NAUX + 1);
   double* ws = nullptr;
   int* dAtom = nullptr;
   CQF_GCUDA(cudaMallocAsync(&ws, doubles * sizeof(double), st));
@@ -216,6 +217,7 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
   // (they only add into the accumulators), the largest first
   uint2* masks = reinterpret_cast<uint2*>(ws + fixed);
   unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
+  double* win = ws + fixed + lists;
   CQF_GCUDA(cudaEventRecord(B->evFork, st));
   cudaStream_t lanes[NAUX + 1] = {st};
   for (int i = 0; i < NAUX; i++) {
@@ -234,16 +236,13 @@ cqf_status cqf_grad_two_body_contract(cqf_basis* B, const int* shell_atom, int n
       a.same = (cb == ck);
       const int li = nlaunch++ % (NAUX + 1);
       const cudaStream_t ls = lanes[li];
-      const HgRegion r{masks + 2 * maskWords * li, (long long)maskWords, work + 4 * li};
+      const HgRegion r{masks + 2 * maskWords * li, (long long)maskWords, work + 4 * li,
+                       win + winDoubles * li};
       rc = hg_contract<GradDig>(
           B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, ls,
-          [&](int ib0, int n, uint2* mk, int* list64, int* list32, unsigned* lcount,
+          [&](const HgPart& p, uint2* mk, int* list64, int* list32, unsigned* lcount,
               unsigned gp) {
-            GradLaunch c = a;
-            c.braBeg += ib0;
-            c.braOff = ib0;
-            c.nBra = n;
-            grad_plan_kernel<<<gp, 256, 0, ls>>>(c, mk, list64, list32, lcount);
+            grad_plan_kernel<<<gp, 256, 0, ls>>>(p.of(a), mk, list64, list32, lcount);
           });
     }
   for (int i = 0; i < NAUX; i++) {

@@ -76,7 +76,7 @@ struct EriDig {
 // Planning pass and engine of one class pair (cb | ck); either side may be
 // the engine's bra: the one whose products need fewer matrix instructions.
 cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* masks,
-                        long long maskWords, unsigned* work, cudaStream_t st) {
+                        long long maskWords, unsigned* work, double* win, cudaStream_t st) {
   if (a.nBra == 0 || a.nKet == 0) return CQF_OK;
   auto cost = [](int b, int k) {
     int la, lb, lc, ld;
@@ -96,15 +96,11 @@ cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* m
   class_ls(ck, lc, ld);
   a.lsum = la + lb + lc + ld;
   const bool mixed = a.precision == 1 && a.fp32_cut > 0.0;
-  auto plan = [&](int ib0, int n, uint2* mk, int* list64, int* list32, unsigned* lcount,
+  auto plan = [&](const HgPart& p, uint2* mk, int* list64, int* list32, unsigned* lcount,
                   unsigned) {
-    JKLaunch c = a;
-    c.braBeg = a.braBeg + ib0;
-    c.nBra = n;
-    c.braOff = ib0;
-    launch_jk_plan(c, mixed, false, mk, list64, list32, lcount, B->nsm, st);
+    launch_jk_plan(p.of(a), mixed, false, mk, list64, list32, lcount, B->nsm, st);
   };
-  const HgRegion r{masks, maskWords, work};
+  const HgRegion r{masks, maskWords, work, win};
   return a.cplx ? hg_contract<EriDig<true>>(B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a,
                                             st, plan)
                 : hg_contract<EriDig<false>>(B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a,

@@ -100,6 +100,11 @@ __global__ void hg_pairs_kernel(const PairDev* __restrict__ in, const double* __
   out[i] = P;
 }
 
+// Window of a table that is not held: doubles for one side of a launch.
+// 64 MiB hold some 110 primitive pairs of two f functions with all six
+// derivatives, so that a window's building stays small beside its quartets.
+constexpr size_t HG_WINDOW = size_t(8) << 20;
+
 }  // namespace
 
 cqf_status hg_ensure(cqf_basis* B, int kind) {
@@ -125,28 +130,39 @@ cqf_status hg_ensure(cqf_basis* B, int kind) {
         B->d_pairs, B->d_ppQ, B->npair, p);
   });
   if (s != CQF_OK || B->d_hg[kind]) return s;
-  size_t total = 0;
+  if (B->hg_win[kind]) return CQF_OK;
+  size_t total = 0, pair = 0;  // doubles of the table, and of the largest pair in it
   for (int c = 0; c < NCLS; c++) {
     B->hg_beg[kind][c] = total;
     if (!B->cls_cnt[c]) continue;
     int la, lb;
     class_ls(c, la, lb);
-    size_t npp = 0;
-    for (int i = 0; i < B->cls_cnt[c]; i++) npp += B->h_pairs[B->cls_beg[c] + i].npp;
-    total += npp * hg_size(kind, la, lb);
+    total += (size_t)B->cls_npp_sum[c] * hg_size(kind, la, lb);
+    pair = std::max(pair, (size_t)B->cls_npp_max[c] * hg_size(kind, la, lb));
   }
-  return build(B->d_hg[kind], total, [&](double* d) {
-    for (int c = 0; c < NCLS; c++) {
-      if (!B->cls_cnt[c]) continue;
-      int la, lb;
-      class_ls(c, la, lb);
-      const size_t smem =
-          (3 * ht_e1(la, lb) + (size_t)12 * (la + 1) * (lb + 1) * ht_fl(la, lb)) * sizeof(double);
-      hg_table_kernel<<<dim3(B->cls_cnt[c], B->cls_npp_max[c]), HT_THREADS, smem, B->stream>>>(
-          B->d_pairs, B->d_pp, B->d_shells, B->d_prim, B->cls_beg[c], B->cls_pp_beg[c], kind, la,
-          lb, d + B->hg_beg[kind][c]);
-    }
-  });
+  if (B->hg_bytes + total * sizeof(double) <= B->hg_limit) {
+    const cqf_status t = build(B->d_hg[kind], total, [&](double* d) {
+      for (int c = 0; c < NCLS; c++)
+        if (B->cls_cnt[c])
+          hg_fill(B, kind, c, B->cls_beg[c], B->cls_cnt[c], d + B->hg_beg[kind][c], B->stream);
+    });
+    if (t == CQF_OK) B->hg_bytes += total * sizeof(double);
+    if (t != CQF_ENOMEM) return t;
+    cudaGetLastError();
+    fail(CQF_OK, "");
+  }
+  // (a table's tiles are 64 doubles; a small limit means small windows)
+  B->hg_win[kind] = std::max(pair, std::min(HG_WINDOW, B->hg_limit / 4096 * 64));
+  return CQF_OK;
+}
+
+void hg_fill(const cqf_basis* B, int kind, int c, int beg, int n, double* tab, cudaStream_t st) {
+  int la, lb;
+  class_ls(c, la, lb);
+  const size_t smem =
+      (3 * ht_e1(la, lb) + (size_t)12 * (la + 1) * (lb + 1) * ht_fl(la, lb)) * sizeof(double);
+  hg_table_kernel<<<dim3(n, B->cls_npp_max[c]), HT_THREADS, smem, st>>>(
+      B->d_pairs, B->d_pp, B->d_shells, B->d_prim, beg, B->h_pairs[beg].pp_off, kind, la, lb, tab);
 }
 
 }  // namespace cqf

@@ -668,13 +668,28 @@ __device__ __forceinline__ void hg_plan(int nBra, int nKet, uint2* __restrict__ 
 // ---------------------------------------------------------- host side
 // The engine on nBra x nKet quartets of class pair (cb | ck) in slabs of bra
 // pairs whose mask words fit the stream's region (maskWords words of 16 B;
-// work: its four counters).  plan(ib0, n, masks, list64, list32, lcount,
-// grid) launches the planning pass on bra pairs [ib0, ib0 + n) of the class;
-// digest arguments may depend on the slab: args(ib0, n).
+// work: its four counters), and of bra and ket pairs whose tables fit its
+// windows where the basis does not hold them.  plan(part, masks, list64,
+// list32, lcount, grid) launches the planning pass on a part of the class pair.
+struct HgPart {
+  int ib0, nBra, k0, nKet;  // bra pairs [ib0, ib0 + nBra) x kets [k0, k0 + nKet)
+  // launch arguments of the class pair, narrowed to the part.  braOff is the
+  // first bra's place among the kets: of one class, a ket sits at or before its bra
+  template <class A>
+  A of(A a) const {
+    a.braBeg += ib0;
+    a.nBra = nBra;
+    a.ketBeg += k0;
+    a.nKet = nKet;
+    a.braOff = ib0 - k0;
+    return a;
+  }
+};
 struct HgRegion {
   uint2* masks;
   long long maskWords;
   unsigned* work;
+  double* win;  // hg_windows<D> doubles
 };
 // Chunk of rows and columns, kets and primitive quartets per batch.  A class
 // whose components fit whole batches kets (up to 32) and primitives within
@@ -805,6 +820,27 @@ inline cqf_status hg_launch(HgLaunch a, const typename D::Args& args, const HgSh
   hg_kernel<D><<<grid, 32 * m.W, m.smem, st>>>(a, args);
   return CQF_OK;
 }
+// Doubles of a launch stream's windows of the tables that the basis does not
+// hold (hg_win), one for each pass and side.
+template <class D>
+inline size_t hg_windows(const cqf_basis* B) {
+  size_t n = 0;
+  for (int q = 0; q < D::NP; q++) n += B->hg_win[D::tb(q)] + B->hg_win[D::tk(q)];
+  return n;
+}
+// The pairs from `beg` on, at most n of them and at least one, whose tables of
+// `kind` (class c) fit its window; n where the basis holds the table.
+inline int hg_fit(const cqf_basis* B, int kind, int c, int beg, int n) {
+  if (!B->hg_win[kind]) return n;
+  int l1, l2;
+  class_ls(c, l1, l2);
+  const long long cap = (long long)(B->hg_win[kind] / hg_size(kind, l1, l2));
+  const cqf::PairDev* p = B->h_pairs.data() + beg;
+  int m = 1;
+  while (m < n && (long long)p[m].pp_off + p[m].npp - p[0].pp_off <= cap) m++;
+  return m;
+}
+
 template <class D, class Plan>
 inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, int nBra, int ketBeg,
                               int nKet, const HgRegion& r, const typename D::Args& args,
@@ -816,60 +852,78 @@ inline cqf_status hg_contract(const cqf_basis* B, int cb, int ck, int braBeg, in
   h.boys32 = B->d_boys32;
   class_ls(cb, h.la, h.lb);
   class_ls(ck, h.lc, h.ld);
-  h.ketBeg = ketBeg;
-  h.nTiles = (nKet + WTILE - 1) / WTILE;
   h.masks = r.masks;
   h.lcount = r.work + 2;
   h.counter = r.work;
+  // the tables the basis holds, or windows of them, built for each slab
+  double* win[2 * HG_MAXPASS];
+  double* next = r.win;
   for (int q = 0; q < D::NP; q++) {
     const int tb = D::tb(q), tk = D::tk(q);
     h.bra[q] = {B->d_hg[tb] + B->hg_beg[tb][cb], B->cls_pp_beg[cb]};
     h.ket[q] = {B->d_hg[tk] + B->hg_beg[tk][ck], B->cls_pp_beg[ck]};
+    win[2 * q] = next;
+    win[2 * q + 1] = next + B->hg_win[tb];
+    next += B->hg_win[tb] + B->hg_win[tk];
   }
+  auto window = [&](HgSide& s, double* w, int kind, int c, int beg, int n) {
+    if (!B->hg_win[kind]) return;
+    s = {w, B->h_pairs[beg].pp_off};
+    hg_fill(B, kind, c, beg, n, w, st);
+  };
   const int npb = B->cls_npp_max[cb], npk = B->cls_npp_max[ck];
-  // contracted classes: words are cut by their number of primitive quartets
-  const HgSlab sl = npb > 1 || npk > 1 ? hg_slab(2 * r.maskWords, nBra, h.nTiles)
-                                  : HgSlab{0, r.maskWords};
-  const int most = sl.most;
-  const long long words = sl.words;
-  const int slab = (int)std::max<long long>(1, words / h.nTiles);
   const long long fill = 16LL * B->nsm;  // items that keep the GPU busy
-  for (int ib0 = 0; ib0 < nBra; ib0 += slab) {
-    const int n = std::min(slab, nBra - ib0);
-    const long long nWords = (long long)n * h.nTiles;
-    int* list64 = reinterpret_cast<int*>(r.masks + nWords);
-    int* list32 = list64 + nWords;
-    h.list64 = list64;
-    h.list32 = list32;
-    h.braBeg = braBeg + ib0;
-    if (cudaMemsetAsync(r.work, 0, 4 * sizeof(unsigned), st) != cudaSuccess)
-      return fail(CQF_ECUDA, "hg_contract: counters");
-    const unsigned gp =
-        (unsigned)std::min<long long>(((nWords + 31) / 32 + 7) / 8, (long long)B->nsm * 8);
-    plan(ib0, n, r.masks, list64, list32, r.work + 2, gp);
-    h.nsub = 1;
-    long long nItems;
-    if (most) {
-      uint2* items = r.masks + 2 * nWords;
-      h.items = items;
-      h.nItems = r.work + 1;
-      // a part's primitive quartets: the launch's (unscreened) number over
-      // the items that fill the GPU, at least a batch
-      const double all = (double)n / nBra * B->cls_npp_sum[cb] * B->cls_npp_sum[ck];
-      const int part = (int)std::min(
-          1024.0, std::max((double)hg_shape<D>(h, 32, 32 * npk).nr, all / fill));
-      hg_expand_kernel<<<(unsigned)std::min<long long>((nWords + 127) / 128, B->nsm * 8), 128, 0,
-                         st>>>(h.pairs, h.braBeg, ketBeg, h.nTiles, r.masks, list64, list32,
-                               h.lcount, part, most, items, r.work + 1);
-      nItems = nWords * most;
-    } else {
-      h.items = nullptr;
-      while (h.nsub < 32 && nWords * h.nsub < fill) h.nsub *= 2;
-      nItems = nWords * h.nsub;
+  for (int k0 = 0, nk = 0; k0 < nKet; k0 += nk) {
+    nk = nKet - k0;
+    for (int q = 0; q < D::NP; q++) nk = std::min(nk, hg_fit(B, D::tk(q), ck, ketBeg + k0, nk));
+    for (int q = 0; q < D::NP; q++)
+      window(h.ket[q], win[2 * q + 1], D::tk(q), ck, ketBeg + k0, nk);
+    h.ketBeg = ketBeg + k0;
+    h.nTiles = (nk + WTILE - 1) / WTILE;
+    // contracted classes: words are cut by their number of primitive quartets
+    const HgSlab sl = npb > 1 || npk > 1 ? hg_slab(2 * r.maskWords, nBra, h.nTiles)
+                                         : HgSlab{0, r.maskWords};
+    const int most = sl.most;
+    const int slab = (int)std::max<long long>(1, sl.words / h.nTiles);
+    for (int ib0 = 0, n = 0; ib0 < nBra; ib0 += n) {
+      n = std::min(slab, nBra - ib0);
+      for (int q = 0; q < D::NP; q++) n = std::min(n, hg_fit(B, D::tb(q), cb, braBeg + ib0, n));
+      for (int q = 0; q < D::NP; q++) window(h.bra[q], win[2 * q], D::tb(q), cb, braBeg + ib0, n);
+      const long long nWords = (long long)n * h.nTiles;
+      int* list64 = reinterpret_cast<int*>(r.masks + nWords);
+      int* list32 = list64 + nWords;
+      h.list64 = list64;
+      h.list32 = list32;
+      h.braBeg = braBeg + ib0;
+      if (cudaMemsetAsync(r.work, 0, 4 * sizeof(unsigned), st) != cudaSuccess)
+        return fail(CQF_ECUDA, "hg_contract: counters");
+      const unsigned gp =
+          (unsigned)std::min<long long>(((nWords + 31) / 32 + 7) / 8, (long long)B->nsm * 8);
+      plan(HgPart{ib0, n, k0, nk}, r.masks, list64, list32, r.work + 2, gp);
+      h.nsub = 1;
+      long long nItems;
+      if (most) {
+        uint2* items = r.masks + 2 * nWords;
+        h.items = items;
+        h.nItems = r.work + 1;
+        // a part's primitive quartets: the launch's (unscreened) number over
+        // the items that fill the GPU, at least a batch
+        const double all = (double)n / nBra * nk / nKet * B->cls_npp_sum[cb] * B->cls_npp_sum[ck];
+        const int part = (int)std::min(
+            1024.0, std::max((double)hg_shape<D>(h, 32, 32 * npk).nr, all / fill));
+        hg_expand_kernel<<<(unsigned)std::min<long long>((nWords + 127) / 128, B->nsm * 8), 128,
+                           0, st>>>(h.pairs, h.braBeg, h.ketBeg, h.nTiles, r.masks, list64, list32,
+                                    h.lcount, part, most, items, r.work + 1);
+        nItems = nWords * most;
+      } else {
+        h.items = nullptr;
+        while (h.nsub < 32 && nWords * h.nsub < fill) h.nsub *= 2;
+        nItems = nWords * h.nsub;
+      }
+      const HgShape& m = hg_shape<D>(h, 32 / h.nsub, 32 / h.nsub * npk);
+      const cqf_status s = hg_launch<D>(h, args, m, nItems, B->device, B->nsm, st);
+      if (s != CQF_OK) return s;
     }
-    const HgShape& m = hg_shape<D>(h, 32 / h.nsub, 32 / h.nsub * npk);
-    const cqf_status s = hg_launch<D>(h, args, m, nItems, B->device, B->nsm, st);
-    if (s != CQF_OK) return s;
   }
   return CQF_OK;
 }

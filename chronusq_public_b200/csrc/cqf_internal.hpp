@@ -100,8 +100,9 @@ constexpr int NWORK = 4 * (NAUX + 1);
 // uint2 mask and two list entries); class pairs with more run in slabs
 constexpr size_t MASK_CAP_WORDS = size_t(1) << 18;
 struct WsLayout {
-  size_t oX, oAX, oXc, oAc, oNm, oNmM, oG, oNmT, oPN, oWork, oXc32, oMask, total;
+  size_t oX, oAX, oXc, oAc, oNm, oNmM, oG, oNmT, oPN, oWork, oXc32, oMask, oWin, total;
   size_t maskWords;  // mask words of each launch stream's region
+  size_t win;        // doubles of each launch stream's table windows (0: none needed)
 };
 // plan = false leaves the masks of a complex contraction out (its class pairs
 // with f shells then run on the generic kernel) and the engine's minimum of
@@ -110,9 +111,10 @@ struct WsLayout {
 constexpr size_t HG_MIN_WORDS = size_t(1) << 16;
 constexpr size_t JK_MIN_WORDS = size_t(1) << 11;
 WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan = true);
-// J and K of a class pair with an f shell (cqf_hg_eri.cu).
+// J and K of a class pair with an f shell (cqf_hg_eri.cu); win: the launch
+// stream's table windows.
 cqf_status launch_jk_hg(const cqf_basis* B, JKLaunch a, int cb, int ck, uint2* masks,
-                        long long maskWords, unsigned* work, cudaStream_t st);
+                        long long maskWords, unsigned* work, double* win, cudaStream_t st);
 cqf_status check_contract_args(const cqf_basis* B, const cqf_contraction* list, int nMat);
 // The contraction on a caller-provided device workspace of ws_layout().total
 // doubles; the caller holds B->mu and has made B's device current.
@@ -240,8 +242,12 @@ void launch_to_cart(const cqf_basis* B, const MatList& l, int n, int cplx, cudaS
 // of a real matrix with mode 2.
 void launch_from_cart(const cqf_basis* B, const MatList& l, int n, int cplx, cudaStream_t st);
 // Builds the engine's coefficient table of one kind for every primitive pair
-// of the basis (once; cqf_hgemm.cu).  Caller holds B->mu, device current.
+// of the basis (once; cqf_hgemm.cu), or, where it does not fit the basis' limit
+// or the device, settles that launches build windows of it (hg_win).  Caller
+// holds B->mu, device current.
 cqf_status hg_ensure(cqf_basis* B, int kind);
+// Enqueues the table of n pairs from `beg` of class c into tab.
+void hg_fill(const cqf_basis* B, int kind, int c, int beg, int n, double* tab, cudaStream_t st);
 // Grows the basis' contraction workspace (B->d_ws) to at least `bytes`.
 cqf_status basis_workspace(cqf_basis* B, size_t bytes);
 
@@ -310,6 +316,10 @@ struct cqf_basis {
   double* d_hg[cqf::HG_NKIND] = {};
   cqf::PairDev* d_pairsHg = nullptr;  // the pairs with their negligible primitives cut off
   size_t hg_beg[cqf::HG_NKIND][cqf::NCLS] = {};
+  // what the tables may hold together (bytes) and do; of a kind that is not
+  // held, the doubles of a window that a launch builds for one side
+  size_t hg_limit = 0, hg_bytes = 0;
+  size_t hg_win[cqf::HG_NKIND] = {};
   // first primitive pair of a class, most per pair, and all of them
   int cls_pp_beg[cqf::NCLS] = {0}, cls_npp_max[cqf::NCLS] = {0};
   long long cls_npp_sum[cqf::NCLS] = {0};

@@ -397,12 +397,8 @@ cqf_status launch_rel(cqf_basis* B, const RelLaunch& a, int cb, int ck, const Hg
                       cudaStream_t st) {
   return hg_contract<RelDig<TYPE>>(
       B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, st,
-      [&](int ib0, int n, uint2* masks, int* list64, int* list32, unsigned* lcount, unsigned gp) {
-        RelLaunch c = a;
-        c.braBeg += ib0;
-        c.braOff = ib0;
-        c.nBra = n;
-        rel_plan_kernel<TYPE><<<gp, 256, 0, st>>>(c, masks, list64, list32, lcount);
+      [&](const HgPart& p, uint2* masks, int* list64, int* list32, unsigned* lcount, unsigned gp) {
+        rel_plan_kernel<TYPE><<<gp, 256, 0, st>>>(p.of(a), masks, list64, list32, lcount);
       });
 }
 
@@ -1456,10 +1452,24 @@ long long rel_mask_words(const cqf_basis* B) {
     row = std::max(row, ((size_t)B->cls_cnt[c] + WTILE - 1) / WTILE);
   return (long long)std::max(row, MASK_CAP_WORDS);
 }
+// Table windows of one launch stream (of the kinds that are known not to be
+// held: rel_tables first).
+size_t rel_window(const cqf_basis* B) {
+  return (std::max({hg_windows<RelDig<1>>(B), hg_windows<RelDig<2>>(B),
+                    hg_windows<GauntDig>(B)}) + 31) / 32 * 32;
+}
 // The contraction's arrays, then per launch stream the masks and word lists
-// (16 B a word), then four counters each.
+// (16 B a word), four counters each, and the table windows.
 size_t rel_ws_doubles(const cqf_basis* B) {
-  return rel_core_doubles(B) + (size_t)(2 * rel_mask_words(B) + 2) * (NAUX + 1);
+  return rel_core_doubles(B) +
+         (size_t)(2 * rel_mask_words(B) + 2 + rel_window(B)) * (NAUX + 1);
+}
+// The engine's tables that a contraction type reads.
+cqf_status rel_tables(cqf_basis* B, int type) {
+  if (type == CQF_REL_LLSS || type == CQF_REL_SSSS) CQF_RTRY(hg_ensure(B, HG_SPIN));
+  if (type == CQF_REL_LLSS) CQF_RTRY(hg_ensure(B, HG_PLAIN));
+  if (type == CQF_REL_GAUNT) CQF_RTRY(hg_ensure(B, HG_D6));
+  return CQF_OK;
 }
 
 // The entries a contraction type writes (the others are neither zeroed nor
@@ -1531,6 +1541,8 @@ cqf_status for_class_pairs(cqf_basis* B, bool ordered, double* ws, cudaStream_t 
   const long long maskWords = rel_mask_words(B);
   uint2* masks = reinterpret_cast<uint2*>(ws + rel_core_doubles(B));
   unsigned* work = reinterpret_cast<unsigned*>(masks + 2 * maskWords * (NAUX + 1));
+  double* win = reinterpret_cast<double*>(work + 4 * (NAUX + 1));
+  const size_t winDoubles = rel_window(B);
   CQF_RCUDA(cudaEventRecord(B->evFork, st));
   cudaStream_t lanes[NAUX + 1] = {st};
   for (int i = 0; i < NAUX; i++) {
@@ -1543,7 +1555,10 @@ cqf_status for_class_pairs(cqf_basis* B, bool ordered, double* ws, cudaStream_t 
     for (int ck = ordered ? NCLS - 1 : cb; ck >= 0 && rc == CQF_OK; ck--) {
       if (!B->cls_cnt[cb] || !B->cls_cnt[ck]) continue;
       const int li = nlaunch++ % (NAUX + 1);
-      rc = go(cb, ck, HgRegion{masks + 2 * maskWords * li, maskWords, work + 4 * li}, lanes[li]);
+      rc = go(cb, ck,
+              HgRegion{masks + 2 * maskWords * li, maskWords, work + 4 * li,
+                       win + winDoubles * li},
+              lanes[li]);
     }
   for (int i = 0; i < NAUX; i++) {
     CQF_RCUDA(cudaEventRecord(B->evJoin[i], B->aux[i]));
@@ -1684,8 +1699,6 @@ cqf_status rel_contract_dev(cqf_basis* B, const double* const* X, double* const*
   a.shardIdx = opts.shard_index;
   a.shardCnt = std::max(1, opts.shard_count);
   a.counters = dcnt;
-  CQF_RTRY(hg_ensure(B, HG_SPIN));
-  if (llss) CQF_RTRY(hg_ensure(B, HG_PLAIN));
   CQF_RTRY(for_class_pairs(
       B, llss, ws, st, [&](int cb, int ck, const HgRegion& r, cudaStream_t ls) {
         int la, lb, lc, ld;
@@ -1808,7 +1821,6 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
   a.shardIdx = opts.shard_index;
   a.shardCnt = std::max(1, opts.shard_count);
   a.counters = dcnt;
-  if (!gauge) CQF_RTRY(hg_ensure(B, HG_D6));
   CQF_RTRY(for_class_pairs(
       B, false, ws, st, [&](int cb, int ck, const HgRegion& r, cudaStream_t ls) {
         int la, lb, lc, ld;
@@ -1825,13 +1837,9 @@ cqf_status gaunt_contract_dev(cqf_basis* B, const double* const* X, double* cons
         }
         return hg_contract<GauntDig>(
             B, cb, ck, a.braBeg, a.nBra, a.ketBeg, a.nKet, r, a, ls,
-            [&](int ib0, int n, uint2* masks, int* list64, int* list32, unsigned* lcount,
+            [&](const HgPart& p, uint2* masks, int* list64, int* list32, unsigned* lcount,
                 unsigned gp) {
-              GauntLaunch c = a;
-              c.braBeg += ib0;
-              c.braOff = ib0;
-              c.nBra = n;
-              gaunt_plan_kernel<<<gp, 256, 0, ls>>>(c, masks, list64, list32, lcount);
+              gaunt_plan_kernel<<<gp, 256, 0, ls>>>(p.of(a), masks, list64, list32, lcount);
             });
       }));
   CQF_RCUDA(cudaGetLastError());
@@ -1875,6 +1883,7 @@ cqf_status cqf_rel_two_body_contract(cqf_basis* B, const void* const* X, void* c
   const int nmat = (type >= CQF_REL_GAUNT) ? CQF_REL_NMAT_GAUNT : CQF_REL_NMAT;
   const std::vector<int> outs = rel_outputs(type, compute_exchange != 0);
   const size_t NN = (size_t)B->nbasis * B->nbasis;
+  CQF_RTRY(rel_tables(B, type));
   const size_t wsd = rel_ws_doubles(B);
   const size_t hostd = o.device_pointers ? 0 : align32(2 * NN) * 2 * nmat;
   CQF_RTRY(ensure_relws(B, (wsd + hostd) * sizeof(double)));
@@ -1950,6 +1959,9 @@ cqf_status cqf_four_comp_gd(cqf_basis* B, const void* const* D, void* const* G,
   const bool exch = std::fabs(dc.xHFX) >= 1e-12;
   // workspace: rel scratch | blocks 16 x N^2 | AX 29 x N^2 | twoeH 4 x 4N^2 |
   // K 4 x 4N^2 | D/G staging (host pointers) 8 x 4N^2, all complex
+  if (dc.dirac_coulomb) CQF_RTRY(rel_tables(B, CQF_REL_LLSS));
+  if (dc.dirac_coulomb_ssss) CQF_RTRY(rel_tables(B, CQF_REL_SSSS));
+  if (dc.gaunt) CQF_RTRY(rel_tables(B, CQF_REL_GAUNT));
   const size_t wsd = rel_ws_doubles(B);
   const size_t blkd = align32(2 * NN), bigd = align32(2 * NN2);
   const size_t total = wsd + 16 * blkd + CQF_REL_NMAT_GAUNT * blkd + 8 * bigd +

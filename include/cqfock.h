@@ -368,7 +368,10 @@ typedef struct {
  * (densities and accumulators, norms, and the class kernels' quartet masks
  * and word lists: 16 B per 32 quartets of a bra pair and a ket tile in each
  * of three launch streams' regions, at most 4 MiB each), and for bases with f
- * shells the coefficient tables of every primitive pair. */
+ * shells the coefficient tables of every primitive pair (more than a basis
+ * holds of them where they pass a quarter of the device's memory, or the
+ * CQF_TABLE_LIMIT_MB of the environment when the basis is made; launches then
+ * build the tables in windows). */
 unsigned long long cqf_fock_footprint(const cqf_shell* shells, int nshell);
 
 cqf_status cqf_server_create(const cqf_server_opts* opts, cqf_server** out);

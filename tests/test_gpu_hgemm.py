@@ -9,13 +9,16 @@ import numpy as np
 import pytest
 
 import oracle as O
+from chronusq_public_b200 import _cabi, workloads
 from chronusq_public_b200.basis import BasisSet, Molecule, parse_gbs
 from chronusq_public_b200.contraction import (COULOMB, EXCHANGE, GAUNT, LLSS, SSSS,
+                                              ContractionGraph,
                                               DirectGradContraction, DirectTPI,
                                               GTODirectRelERIContraction,
                                               GTODirectTPIContraction, TwoBodyContraction)
 from test_gpu_gaunt import OUTS_C, OUTS_X, gaunt_inputs
 from test_gpu_rel import OUTS, max_rel, rel_inputs
+from test_zz_no_alloc import _contract as noalloc_contract
 
 pytestmark = pytest.mark.gpu
 
@@ -196,3 +199,58 @@ def test_engine_items_fill_region():
                 K = K + np.einsum("acbd,cd->ab", ob.eri_quartet(a, c, b, d), D[sl[c], sl[d]])
         for got, ref in zip(res["fp64"], (J, K)):
             assert np.abs(got[sl[a], sl[b]] - ref).max() < 1e-11 * np.abs(got).max() + 2e-9
+
+
+@pytest.mark.parametrize("limit", ["0", "0.25"])
+def test_windows_of_tables(limit, monkeypatch):
+    """Tables beyond the basis' limit: launches build windows of them, of one
+    pair at the smallest (every bra pair against every ket pair by itself)."""
+    monkeypatch.setenv("CQF_TABLE_LIMIT_MB", limit)
+    for name in ("f2", "mix"):
+        for kind in ("real", "complex_nonher", "mixed"):
+            test_engine_jk(name, kind)
+        for ctype in (LLSS, SSSS):
+            test_engine_rel(name, ctype, "fp64")
+        test_engine_gaunt(name)
+        test_engine_gradient(name)
+
+
+def test_windows_under_capture(monkeypatch):
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("CQF_TABLE_LIMIT_MB", "0")
+    bs = basis("mix")
+    N = bs.nbasis
+    rng = np.random.default_rng(81)
+    A = 0.1 * rng.standard_normal((N, N))
+    X = torch.tensor(A + A.T, device="cuda").T
+    out = torch.zeros((2, N, N), dtype=torch.float64, device="cuda")
+    graph = ContractionGraph(DirectTPI(bs), [TwoBodyContraction(X, out[k].T, True, t)
+                                             for k, t in enumerate((COULOMB, EXCHANGE))])
+    for _ in range(2):
+        B = 0.1 * rng.standard_normal((N, N))
+        X.copy_(torch.tensor(B + B.T))
+        out.zero_()
+        torch.cuda.synchronize()
+        graph.launch()
+        torch.cuda.synchronize()
+        ref = O.OracleBasis(bs).contract([np.asfortranarray(B + B.T)] * 2, [1, 1], [0, 1])
+        for k in range(2):
+            assert max_rel(out[k].T.cpu().numpy(), np.asarray(ref[k])) < 1e-11
+
+
+def test_windows_beyond_fixed_scratch(monkeypatch):
+    """The windows of 43 MiB of tables with a limit of 40 (six of 5 MiB) do not
+    fit the no-alloc entry point's 32 MiB beside the matrices: it takes the generic
+    kernel."""
+    monkeypatch.setenv("CQF_TABLE_LIMIT_MB", "40")
+    bs = BasisSet.build(workloads.water_cluster(7, seed=3, box=5.0), "cc-pvtz")
+    tpi, N = DirectTPI(bs), bs.nbasis
+    A = 0.1 * np.random.default_rng(82).standard_normal((N, N))
+    D = np.asfortranarray(A + A.T)
+    res = []
+    for entry in (_cabi.lib().cqf_two_body_contract, _cabi.lib().cqf_two_body_contract_noalloc):
+        out = [np.zeros((N, N), order="F") for _ in range(2)]
+        assert noalloc_contract(entry, tpi, D, out, [COULOMB, EXCHANGE]) == _cabi.CQF_OK
+        res.append(out)
+    for a, b in zip(*res):
+        assert max_rel(a, b) < 1e-11
