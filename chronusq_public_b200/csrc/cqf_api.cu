@@ -1847,6 +1847,7 @@ cqf_status contract_core(cqf_basis* B, const cqf_contraction* list, int nMat,
       a.same = (cb == ck);
       a.braTileBeg = B->cls_tile_beg[cb];
       a.ketTileBeg = B->cls_tile_beg[ck];
+      a.maxPrimQ = (long long)B->cls_npp_max[cb] * B->cls_npp_max[ck];
       const int lm = std::max(std::max(la, lb), std::max(lc, ld));
       // autotuning times each class alone, on st, between two events
       const bool tune = B->tuning && !capture;

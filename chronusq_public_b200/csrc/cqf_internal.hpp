@@ -69,8 +69,10 @@ struct JKLaunch {
   int precision;            // 0 FP64, 1 mixed
   double fp32_cut;          // mixed: bound < cut -> FP32 ERIs
   // launches whose kernels share quartets among lanes: a lane's primitive
-  // quartets, and whether every word may be listed in parts
+  // quartets, whether every word may be listed in parts, and the most
+  // primitive quartets that a quartet of the class pair has
   int planEach, planAll;
+  long long maxPrimQ;
   int shardIdx, shardCnt;   // bra pairs p with p % shardCnt == shardIdx only
   unsigned long long* counters;  // [0] visited, [1] screened, [2] fp32, [3] fp64
 };

@@ -289,14 +289,15 @@ inline bool launch_jk_fast(JKLaunch a, int la, int lb, int lc, int ld, uint2* ma
     // a word), or in the smallest of eight times the words
     const long long all = (long long)b.nBra * nTiles;
     const bool tiny = CUTTABLE && all <= JK_TINY_WORDS && all * JK_TINY_BYTES <= maskWords * 16;
-    const bool cut = tiny || (CUTTABLE && b.lsum <= JK_CUT_LSUM && all <= JK_CUT_WORDS &&
-                              maskWords >= 2 * nTiles);
-    const int dup = tiny ? 8 : (cut ? 2 : 1);
     b.planEach = tiny ? 8 : 64;
     b.planAll = tiny;
-    const int slab = tiny ? b.nBra
-                          : (int)std::max<long long>(
-                                1, (cut ? maskWords * 2 / 3 : maskWords) / nTiles);
+    const bool cut = (tiny || (CUTTABLE && b.lsum <= JK_CUT_LSUM && all <= JK_CUT_WORDS &&
+                               maskWords >= 2 * nTiles)) &&
+                     b.maxPrimQ >= PLAN_LONG * b.planEach;
+    const int dup = !cut ? 1 : (tiny ? 8 : 2);
+    const int slab = dup == 8 ? b.nBra
+                              : (int)std::max<long long>(
+                                    1, (cut ? maskWords * 2 / 3 : maskWords) / nTiles);
     for (int ib0 = 0; ib0 < b.nBra; ib0 += slab) {
       JKLaunch c = b;
       c.braBeg = b.braBeg + ib0;

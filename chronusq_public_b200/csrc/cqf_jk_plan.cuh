@@ -43,7 +43,7 @@ __device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P
 // only words that name quartets of their precision.
 //
 // CUT (launches whose class kernels share a quartet among lanes): a word whose
-// quartets have long primitive loops (4 planEach primitive quartets or more)
+// quartets have long primitive loops (PLAN_LONG planEach primitive quartets or more)
 // carries log2 of the lanes per quartet in its list entry, and is listed as
 // eight entries of four kets, so that several warps share it: in the first
 // eighth of the words -- pairs come in descending order of their primitive
@@ -52,13 +52,17 @@ __device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P
 // lane walked the 4096 primitive quartets of two contractions of eight: 1.4 ms
 // of a 2.3 ms build of one water molecule.
 constexpr int PLAN_RUN = 32;
+constexpr int PLAN_LONG = 4;
 constexpr int PLAN_WORD = (1 << 20) - 1;  // list entry: word | sub << 20 | part << 23 | log2 << 24
 // class pairs of angular sums up to 2 in launches of up to 65536 words
 // (one water 2292 -> 917 us, eight complex 4.22 -> 3.07 ms), and of sums up to
 // 4 in launches of a few hundred, a molecule or two (917 -> 904 us, the mixed
 // four-component build of one water 3.10 -> 2.92 ms); larger ones have enough
 // quartets to hide the longest loops, and the shared form costs them
-// registers ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms)
+// registers ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms).  So the host takes it
+// only where the class pair's longest contractions reach PLAN_LONG planEach
+// (with it for every small launch 6 waters in 3-21G 262 -> 310 us, 10 in
+// def2-SVP 2.15 -> 2.29 ms)
 __host__ __device__ constexpr bool jk_split(int lsum) { return lsum <= 4; }
 constexpr long long JK_CUT_WORDS = 1 << 16;
 constexpr long long JK_TINY_WORDS = 448;
@@ -98,14 +102,14 @@ __global__ void __launch_bounds__(256)
           const double bound = sh_max_bra(a, P, Q, __ldg(a.pairNorm + a.braBeg + ib),
                                           __ldg(a.pairNorm + a.ketBeg + jk), pRef) * P.Q * Q.Q;
           screened = bound < a.thresh;
-          if (CUT && !screened) {
-            const int np = P.npp * Q.npp;
-            while (np >= 4 * a.planEach && sl < 5 && (np >> sl) > a.planEach) sl++;
-          }
           w32 = MIXED && !screened && bound < cut &&
                 fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
                               __ldg(a.pairRange + a.ketBeg + jk), a.lsum, 0, 0);
         }  // without the screen every quartet runs in FP64
+        if (CUT && visited && !screened) {  // 4 waters unscreened 2.65 -> 1.32 ms
+          const int np = P.npp * a.pairs[a.ketBeg + jk].npp;
+          while (np >= PLAN_LONG * a.planEach && sl < 5 && (np >> sl) > a.planEach) sl++;
+        }
         const unsigned bv = __ballot_sync(0xffffffffu, visited);
         const unsigned bs = __ballot_sync(0xffffffffu, visited && screened);
         b32 = __ballot_sync(0xffffffffu, visited && !screened && w32);

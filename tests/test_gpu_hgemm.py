@@ -88,6 +88,23 @@ def test_engine_jk(name, kind):
         assert max_rel(o, np.asarray(r)) < (1e-6 if kind == "mixed" else 1e-11)
 
 
+@pytest.mark.parametrize("name", ["long", "mix"])
+def test_jk_without_screen(name):
+    """Quartets are shared by lanes without the screen as well."""
+    bs = basis(name)
+    N = bs.nbasis
+    A = 0.1 * np.random.default_rng(66).standard_normal((N, N))
+    D = np.asfortranarray(A + A.T)
+    ref = O.OracleBasis(bs).contract([D, D], [1, 1], [0, 1], screen=False)
+    lst = [TwoBodyContraction(D, np.zeros((N, N), order="F"), True, t)
+           for t in (COULOMB, EXCHANGE)]
+    c = GTODirectTPIContraction(DirectTPI(bs))
+    c.twoBodyContract(lst, screen=False)
+    assert c.last_stats["screened"] == 0
+    for m, r in zip(lst, ref):
+        assert max_rel(m.AX, np.asarray(r)) < 1e-11
+
+
 @pytest.mark.parametrize("name", sorted(BASES))
 def test_engine_gaunt(name):
     bs = basis(name)
