@@ -4,7 +4,8 @@ and columns, the integrals made again for each), long contractions (a
 quartet's primitives in batches of 32 and over several blocks), one single
 shell (tiles almost empty), and FP32 Hermite integrals.  FP64 results agree
 to 1e-11 of the largest element (sums of some 1e4 terms in another order);
-mixed ones to 1e-6 at the cutoff used."""
+mixed ones, at a cutoff that divides the quartets, to 1e-6 (FP32 integrals carry
+a few 1e-7 of their bounds, which are of the outputs' size here)."""
 import numpy as np
 import pytest
 
@@ -45,6 +46,18 @@ def basis(name):
     return BasisSet.build(mol, parse_gbs("****\n%s****\n%s****\n" % (he, h)))
 
 
+def split_precision(build):
+    """build(cutoff) -> (outputs, stats) at the largest power of ten below which
+    some quartets, but not all, run in FP32."""
+    for k in range(1, -13, -1):
+        out, s = build(10.0 ** k)
+        if s["fp64"] > 0:
+            break
+    assert s["fp32"] > 0 and s["fp64"] > 0
+    assert s["fp32"] + s["fp64"] + s["screened"] == s["total"]
+    return out
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("ctype", [LLSS, SSSS])
 @pytest.mark.parametrize("name", sorted(BASES))
@@ -53,11 +66,15 @@ def test_engine_rel(name, ctype, precision):
     N = bs.nbasis
     _D, X = rel_inputs(N, 61)
     ref = O.OracleBasis(bs).rel_contract(X, ctype, True)
-    lst = [TwoBodyContraction(X[m], np.zeros((N, N), complex)) for m in range(17)]
     c = GTODirectRelERIContraction(DirectTPI(bs))
-    c.twoBodyContract(lst, ctype, precision=precision, fp32_cutoff=1e-2)
-    s = c.last_stats
-    assert s["fp32"] + s["fp64"] + s["screened"] == s["total"]
+
+    def build(cutoff):
+        lst = [TwoBodyContraction(X[m], np.zeros((N, N), complex)) for m in range(17)]
+        c.twoBodyContract(lst, ctype, precision=precision, fp32_cutoff=cutoff)
+        return lst, c.last_stats
+
+    lst = build(0.0)[0] if precision == "fp64" else split_precision(build)
+    assert precision == "mixed" or c.last_stats["fp32"] == 0
     for m in OUTS[ctype]:
         assert max_rel(lst[m].AX, ref[m]) < (1e-11 if precision == "fp64" else 1e-6), m
 
@@ -80,10 +97,15 @@ def test_engine_jk(name, kind):
         mats.append(np.asfortranarray(A + A.conj().T if her else A))
     types = [COULOMB, EXCHANGE, EXCHANGE]
     ref = O.OracleBasis(bs).contract(mats, [int(her)] * 3, types)
-    out = [np.zeros((N, N), mats[0].dtype, order="F") for _ in mats]
     c = GTODirectTPIContraction(DirectTPI(bs))
-    c.twoBodyContract([TwoBodyContraction(m, o, her, t) for m, o, t in zip(mats, out, types)],
-                      precision="mixed" if kind == "mixed" else "fp64", fp32_cutoff=1e-3)
+
+    def build(cutoff):
+        out = [np.zeros((N, N), mats[0].dtype, order="F") for _ in mats]
+        c.twoBodyContract([TwoBodyContraction(m, o, her, t) for m, o, t in zip(mats, out, types)],
+                          precision="mixed" if kind == "mixed" else "fp64", fp32_cutoff=cutoff)
+        return out, c.last_stats
+
+    out = split_precision(build) if kind == "mixed" else build(0.0)[0]
     for o, r in zip(out, ref):
         assert max_rel(o, np.asarray(r)) < (1e-6 if kind == "mixed" else 1e-11)
 
