@@ -56,7 +56,7 @@ sys.path.insert(0, ROOT)
 METRIC = ("Fock builds/s (mixed vs FP64, same B200) at <=1e-6 Eh Fock err; "
           "p50/p99 latency")
 # DRAM bytes of one mixed build from an ncu capture (profiles/), by workload
-TRAFFIC_BYTES = {"h2o16_def2svp": 1.32e8}
+TRAFFIC_BYTES = {"h2o16_def2svp": 1.309e8}
 
 
 def parse():

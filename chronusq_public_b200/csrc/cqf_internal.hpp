@@ -106,10 +106,10 @@ struct WsLayout {
   size_t maskWords;  // mask words of each launch stream's region
   size_t win;        // doubles of each launch stream's table windows (0: none needed)
 };
-// plan = false leaves the masks of a complex contraction out (its class pairs
-// with f shells then run on the generic kernel) and the engine's minimum of
-// them (HG_MIN_WORDS, JK_MIN_WORDS): what the fixed scratch of the no-alloc entry point
-// falls back to.
+// plan = false leaves the masks of a complex contraction and the table windows
+// out (the class pairs with f shells that need them then run on the generic
+// kernel) and the engine's minimum of masks (HG_MIN_WORDS, JK_MIN_WORDS): what
+// the fixed scratch of the no-alloc entry point falls back to.
 constexpr size_t HG_MIN_WORDS = size_t(1) << 16;
 constexpr size_t JK_MIN_WORDS = size_t(1) << 11;
 WsLayout ws_layout(const cqf_basis* B, int nMat, const cqf_opts& opts, bool plan = true);

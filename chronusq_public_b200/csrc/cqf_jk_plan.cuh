@@ -54,15 +54,24 @@ __device__ __forceinline__ double sh_max_bra(const JKLaunch& a, const PairDev& P
 constexpr int PLAN_RUN = 32;
 constexpr int PLAN_LONG = 4;
 constexpr int PLAN_WORD = (1 << 20) - 1;  // list entry: word | sub << 20 | part << 23 | log2 << 24
-// class pairs of angular sums up to 2 in launches of up to 65536 words
-// (one water 2292 -> 917 us, eight complex 4.22 -> 3.07 ms), and of sums up to
-// 4 in launches of a few hundred, a molecule or two (917 -> 904 us, the mixed
-// four-component build of one water 3.10 -> 2.92 ms); larger ones have enough
-// quartets to hide the longest loops, and the shared form costs them
-// registers ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms).  So the host takes it
-// only where the class pair's longest contractions reach PLAN_LONG planEach
-// (with it for every small launch 6 waters in 3-21G 262 -> 310 us, 10 in
-// def2-SVP 2.15 -> 2.29 ms)
+// Two forms (times: J and K, FP64 unless named).
+// * Angular sums up to 2 in launches of up to JK_CUT_WORDS, 14 words for each of
+//   the 4736 warps that are resident at eight blocks an SM; 64 primitive
+//   quartets a lane.  Without it 6 waters in cc-pVDZ take 3.11 ms for 1.72, up
+//   to 2^13 words 2.78; up to 2^18 12 waters would gain (5.98 -> 4.28 ms) and
+//   from 16 on nothing changes.  32 a lane: 6 waters in 6-31G(d) 1.11 -> 1.04
+//   ms, 4 in cc-pVDZ 1.33 -> 1.46; 128: 1.20 and 1.25.
+// * Angular sums up to 4 in launches of up to JK_TINY_WORDS, three words an SM
+//   and what the smallest region holds eightfold (JK_MIN_WORDS; JK_TINY_BYTES
+//   a word); 8 primitive quartets a lane.  Without it one water in def2-SVP
+//   takes 0.60 ms for 0.51 and 2 in 6-31G(d) mixed 1.09 for 0.90; up to one word
+//   an SM the latter take 0.98.  4 a lane 2-12% slower, 32 up to 9% slower
+//   (def2-SVP) or 6% faster (one water in cc-pVDZ).
+// Larger launches have enough quartets to hide the longest loops, and the
+// shared form costs registers ((H2O)16 / def2-SVP mixed 6.15 -> 6.45 ms where
+// every class pair takes it).  So the host takes it only where the class pair's
+// longest contractions reach PLAN_LONG planEach (with it for every small launch
+// 6 waters in 3-21G 262 -> 310 us, 10 in def2-SVP 2.15 -> 2.29 ms).
 __host__ __device__ constexpr bool jk_split(int lsum) { return lsum <= 4; }
 constexpr long long JK_CUT_WORDS = 1 << 16;
 constexpr long long JK_TINY_WORDS = 448;
