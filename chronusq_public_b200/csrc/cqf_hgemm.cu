@@ -14,7 +14,7 @@ constexpr int HT_THREADS = 128;
 __host__ __device__ inline int ht_fl(int la, int lb) { return la + lb + 3; }
 __host__ __device__ inline int ht_e1(int la, int lb) { return (la + 2) * (lb + 2) * (la + lb + 3); }
 
-// One block per primitive pair (pair beg + blockIdx.x, primitive blockIdx.y):
+// One block per primitive pair (pair beg + blockIdx.x, primitives from blockIdx.y on):
 // the 1D tables raised by one on both centres, the factors of every axis,
 // exponent pair and derivative type, then every entry of the table in
 // fragment order.
@@ -24,66 +24,68 @@ __global__ void __launch_bounds__(HT_THREADS)
                     int ppBeg, int kind, int la, int lb, double* __restrict__ tab) {
   extern __shared__ double sm[];
   const PairDev P = pairs[beg + blockIdx.x];
-  const int ip = blockIdx.y, tid = threadIdx.x;
-  if (ip >= P.npp) return;
-  const PrimPairDev A = pp[P.pp_off + ip];
-  double ea, eb;
-  pair_exps(shells[P.shA], shells[P.shB], prim, A, ea, eb);
-  const int E1 = ht_e1(la, lb), FL = ht_fl(la, lb);
-  double* E = sm;
-  double* fa = sm + 3 * E1;
-  if (tid < 3)
-    hermite_E_rt<double, LMAX + 1>(la + 1, lb + 1, A.o2p, A.PA[tid], A.PB[tid], E + tid * E1);
-  __syncthreads();
-  for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += HT_THREADS) {
-    const int ty = it % 4, j = (it / 4) % (lb + 1), i = (it / 4 / (lb + 1)) % (la + 1),
-              x = it / 4 / (lb + 1) / (la + 1);
-    double* f = fa + (size_t)it * FL;
-    const int n = axis_factor<double>(E + x * E1, lb + 1, la + lb + 3, i, j, ty, 2.0 * ea,
-                                      2.0 * eb, f);
-    for (int t = n; t < FL; t++) f[t] = 0.0;
-  }
-  __syncthreads();
-  const int nb = ncart(lb), nab = ncart(la) * nb, nop = hg_ops(kind);
-  const int H = nherm(la + lb + hg_rise(kind)), kt = hg_ktiles(kind, la, lb);
-  const int size = hg_size(kind, la, lb);
-  double* out = tab + (size_t)(P.pp_off + ip - ppBeg) * size;
-  for (int e = tid; e < size; e += HT_THREADS) {
-    // [row tile][order tile][lane][half]
-    const int half = e & 1, lane = (e >> 1) & 31, k = (e >> 6) % kt, rt = (e >> 6) / kt;
-    const int row = rt * 16 + half * 8 + (lane >> 2), h = k * 4 + (lane & 3);
-    double v = 0.0;
-    if (row < nab * nop && h < H) {
-      const int ab = row / nop, op = row % nop, a = ab / nb, b = ab % nb;
-      int n = 0;
-      while (nherm(n) <= h) n++;
-      const int r = h - nherm(n - 1);
-      int kk = 0;
-      while ((kk + 1) * (kk + 2) / 2 <= r) kk++;
-      const int hv = r - kk * (kk + 1) / 2, hu = kk - hv, ht = n - kk;
-      const int ax[3] = {cart_lx(la, a), cart_ly(la, a), cart_lz(la, a)};
-      const int bx[3] = {cart_lx(lb, b), cart_ly(lb, b), cart_lz(lb, b)};
-      auto f = [&](int x, int ty, int t) {
-        return t < FL ? fa[(size_t)(((x * (la + 1) + ax[x]) * (lb + 1) + bx[x]) * 4 + ty) * FL + t]
-                      : 0.0;
-      };
-      if (kind == HG_SPIN) {
-        for (int mu = 0; mu < 3; mu++)
-          for (int nu = 0; nu < 3; nu++) {
-            int o2;
-            double sg;
-            op_of(mu, nu, o2, sg);
-            if (o2 != op) continue;
-            v += sg * f(0, (mu == 0) | ((nu == 0) << 1), ht) *
-                 f(1, (mu == 1) | ((nu == 1) << 1), hu) * f(2, (mu == 2) | ((nu == 2) << 1), hv);
-          }
-      } else {
-        const int dir = kind == HG_PLAIN ? -1 : op % 3, ty = op < 3 ? 1 : 2;
-        v = f(0, dir == 0 ? ty : 0, ht) * f(1, dir == 1 ? ty : 0, hu) *
-            f(2, dir == 2 ? ty : 0, hv);
-      }
+  const int tid = threadIdx.x;
+  for (int ip = blockIdx.y; ip < P.npp; ip += gridDim.y) {
+    const PrimPairDev A = pp[P.pp_off + ip];
+    double ea, eb;
+    pair_exps(shells[P.shA], shells[P.shB], prim, A, ea, eb);
+    const int E1 = ht_e1(la, lb), FL = ht_fl(la, lb);
+    double* E = sm;
+    double* fa = sm + 3 * E1;
+    if (tid < 3)
+      hermite_E_rt<double, LMAX + 1>(la + 1, lb + 1, A.o2p, A.PA[tid], A.PB[tid], E + tid * E1);
+    __syncthreads();
+    for (int it = tid; it < 3 * (la + 1) * (lb + 1) * 4; it += HT_THREADS) {
+      const int ty = it % 4, j = (it / 4) % (lb + 1), i = (it / 4 / (lb + 1)) % (la + 1),
+                x = it / 4 / (lb + 1) / (la + 1);
+      double* f = fa + (size_t)it * FL;
+      const int n = axis_factor<double>(E + x * E1, lb + 1, la + lb + 3, i, j, ty, 2.0 * ea,
+                                        2.0 * eb, f);
+      for (int t = n; t < FL; t++) f[t] = 0.0;
     }
-    out[e] = v;
+    __syncthreads();
+    const int nb = ncart(lb), nab = ncart(la) * nb, nop = hg_ops(kind);
+    const int H = nherm(la + lb + hg_rise(kind)), kt = hg_ktiles(kind, la, lb);
+    const int size = hg_size(kind, la, lb);
+    double* out = tab + (size_t)(P.pp_off + ip - ppBeg) * size;
+    for (int e = tid; e < size; e += HT_THREADS) {
+      // [row tile][order tile][lane][half]
+      const int half = e & 1, lane = (e >> 1) & 31, k = (e >> 6) % kt, rt = (e >> 6) / kt;
+      const int row = rt * 16 + half * 8 + (lane >> 2), h = k * 4 + (lane & 3);
+      double v = 0.0;
+      if (row < nab * nop && h < H) {
+        const int ab = row / nop, op = row % nop, a = ab / nb, b = ab % nb;
+        int n = 0;
+        while (nherm(n) <= h) n++;
+        const int r = h - nherm(n - 1);
+        int kk = 0;
+        while ((kk + 1) * (kk + 2) / 2 <= r) kk++;
+        const int hv = r - kk * (kk + 1) / 2, hu = kk - hv, ht = n - kk;
+        const int ax[3] = {cart_lx(la, a), cart_ly(la, a), cart_lz(la, a)};
+        const int bx[3] = {cart_lx(lb, b), cart_ly(lb, b), cart_lz(lb, b)};
+        auto f = [&](int x, int ty, int t) {
+          return t < FL ? fa[(size_t)(((x * (la + 1) + ax[x]) * (lb + 1) + bx[x]) * 4 + ty) * FL + t]
+                        : 0.0;
+        };
+        if (kind == HG_SPIN) {
+          for (int mu = 0; mu < 3; mu++)
+            for (int nu = 0; nu < 3; nu++) {
+              int o2;
+              double sg;
+              op_of(mu, nu, o2, sg);
+              if (o2 != op) continue;
+              v += sg * f(0, (mu == 0) | ((nu == 0) << 1), ht) *
+                   f(1, (mu == 1) | ((nu == 1) << 1), hu) * f(2, (mu == 2) | ((nu == 2) << 1), hv);
+            }
+        } else {
+          const int dir = kind == HG_PLAIN ? -1 : op % 3, ty = op < 3 ? 1 : 2;
+          v = f(0, dir == 0 ? ty : 0, ht) * f(1, dir == 1 ? ty : 0, hu) *
+              f(2, dir == 2 ? ty : 0, hv);
+        }
+      }
+      out[e] = v;
+    }
+    __syncthreads();  // before the next one's factors
   }
 }
 
@@ -161,7 +163,7 @@ void hg_fill(const cqf_basis* B, int kind, int c, int beg, int n, double* tab, c
   class_ls(c, la, lb);
   const size_t smem =
       (3 * ht_e1(la, lb) + (size_t)12 * (la + 1) * (lb + 1) * ht_fl(la, lb)) * sizeof(double);
-  hg_table_kernel<<<dim3(n, B->cls_npp_max[c]), HT_THREADS, smem, st>>>(
+  hg_table_kernel<<<dim3(n, std::min(B->cls_npp_max[c], PRIM_ROWS)), HT_THREADS, smem, st>>>(
       B->d_pairs, B->d_pp, B->d_shells, B->d_prim, beg, B->h_pairs[beg].pp_off, kind, la, lb, tab);
 }
 

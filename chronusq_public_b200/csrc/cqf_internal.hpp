@@ -32,6 +32,10 @@ constexpr int KETT_NF = 13;
 constexpr int KETT_TILE = 128;
 constexpr int WTILE = 32;         // kets per mask word of the class kernels
 
+// rows of the grids that have one per primitive pair of a shell pair (a grid has
+// 65,535 at most; contractions of 256 functions have more such pairs)
+constexpr int PRIM_ROWS = 1024;
+
 // Arguments of one class-quartet J/K launch.
 struct JKLaunch {
   const PairDev* pairs;

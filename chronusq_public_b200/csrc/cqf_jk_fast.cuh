@@ -498,23 +498,24 @@ __global__ void prim_schwarz_kernel(const PairDev* __restrict__ pairs,
   constexpr int NA = ncart(GC::LA), NB = ncart(GC::LB), NCH = GC::NCHUNK;
   constexpr int CS = GC::NI / (NA * NB);
   const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t / NCH, ch = t - k * NCH;
-  const int ip = blockIdx.y;
   if (k >= n) return;
   PairDev P1 = pairs[beg + k];
-  if (ip >= P1.npp) return;
+  const int npp = P1.npp, off = P1.pp_off;
   P1.npp = 1;
-  P1.pp_off += ip;
-  double I[GC::NI];
-  GC::eri(P1, P1, pp, KetAoS{pp + P1.pp_off, nullptr},
-          boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr, 0.0);
-  double mx = 0.0;
-  for (int kk = 0; kk < CS; kk++) {
-    const int cd = ch * CS + kk;  // the diagonal element (ab | ab), ab = cd
-    if (cd < NA * NB) mx = fmax(mx, fabs(I[cd * CS + kk]));
+  for (int ip = blockIdx.y; ip < npp; ip += gridDim.y) {
+    P1.pp_off = off + ip;
+    double I[GC::NI];
+    GC::eri(P1, P1, pp, KetAoS{pp + P1.pp_off, nullptr},
+            boys + (size_t)(2 * (GC::LA + GC::LB)) * BOYS_NPTS * BOYS_ROW64, ch, I, nullptr, 0.0);
+    double mx = 0.0;
+    for (int kk = 0; kk < CS; kk++) {
+      const int cd = ch * CS + kk;  // the diagonal element (ab | ab), ab = cd
+      if (cd < NA * NB) mx = fmax(mx, fabs(I[cd * CS + kk]));
+    }
+    // non-negative doubles order as their bits
+    atomicMax(reinterpret_cast<unsigned long long*>(ppQ + P1.pp_off),
+              (unsigned long long)__double_as_longlong(sqrt(mx)));
   }
-  // non-negative doubles order as their bits
-  atomicMax(reinterpret_cast<unsigned long long*>(ppQ + P1.pp_off),
-            (unsigned long long)__double_as_longlong(sqrt(mx)));
 }
 
 // Primitive Schwarz bounds of one class with the generated code; false if
@@ -526,7 +527,7 @@ inline bool launch_prim_schwarz(int la, int lb, const PairDev* pairs, const Prim
   bool done = false;
   auto go = [&](auto tag64) {
     using G = decltype(tag64);
-    prim_schwarz_kernel<G><<<dim3((n * G::NCHUNK + 63) / 64, maxNpp), 64, 0, st>>>(
+    prim_schwarz_kernel<G><<<dim3((n * G::NCHUNK + 63) / 64, std::min(maxNpp, PRIM_ROWS)), 64, 0, st>>>(
         pairs, pp, boys, beg, n, ppQ);
     done = true;
   };

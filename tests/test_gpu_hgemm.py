@@ -158,6 +158,23 @@ def test_engine_gradient(name):
             assert max_rel(cl[g][m].AX, np.asarray(ref[g][m])) < 1e-11, (g, m)
 
 
+def test_long_contraction_in_rows():
+    """1156 primitive pairs of one shell pair: more than the grids of the set-up
+    kernels have rows (PRIM_ROWS)."""
+    gbs = "****\nH 0\nS 34 1.00\n" + "".join("  %g %g\n" % (0.1 * 1.3 ** k, 0.1 + 0.01 * k)
+                                              for k in range(34)) + "F 1 1.00\n  0.8 1.0\n****\n"
+    bs = BasisSet.build(Molecule.from_angstrom([("H", 0.1, 0.2, 0.3)]), parse_gbs(gbs))
+    N = bs.nbasis
+    A = 0.1 * np.random.default_rng(67).standard_normal((N, N))
+    D = np.asfortranarray(A + A.T)
+    ref = O.OracleBasis(bs).contract([D, D], [1, 1], [0, 1])
+    lst = [TwoBodyContraction(D, np.zeros((N, N), order="F"), True, t)
+           for t in (COULOMB, EXCHANGE)]
+    GTODirectTPIContraction(DirectTPI(bs)).twoBodyContract(lst)
+    for m, r in zip(lst, ref):
+        assert max_rel(m.AX, np.asarray(r)) < 1e-11
+
+
 @pytest.mark.parametrize("count", [32, 33])
 def test_many_matrices_share_outputs(count):
     """Device matrices in batches of 32 launches; every contraction adds into
