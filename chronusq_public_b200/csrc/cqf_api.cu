@@ -1065,16 +1065,20 @@ cqf_status basis_create(const cqf_shell* shells, int nshell, double thresh, int 
                                                                  d_tmp, B->npair, B->d_pp);
   CQF_CUDA(cudaMallocAsync(&B->d_schwarz, (size_t)nshell * nshell * sizeof(double), B->stream));
   CQF_CUDA(cudaMemsetAsync(B->d_schwarz, 0, (size_t)nshell * nshell * sizeof(double), B->stream));
-  // partial diagonals of a class's pairs, in slabs of at most SCHWARZ_ROOM
-  // doubles (64 MiB)
+  // partial diagonals of a class's pairs: room for one of every pair, and for
+  // all of a class up to SCHWARZ_ROOM doubles (64 MiB), else in slabs.  (The
+  // size moves the basis' later arrays in the memory pool, and the class kernels
+  // notice: with room for the widest class alone (H2O)16 / def2-SVP mixed ran at
+  // 158 builds/s from cold caches, with this 164; in whole 2 MiB pages at 165,
+  // but one water in 0.90 ms instead of 0.88)
   constexpr size_t SCHWARZ_ROOM = size_t(8) << 20;
-  size_t diagRoom = 36;
+  size_t diagRoom = 0;
   for (int c = 0; c < NCLS; c++) {
     int la, lb;
     class_ls(c, la, lb);
     diagRoom = std::max(diagRoom, (size_t)B->cls_cnt[c] * 36 * schwarz_chunks(la, lb));
   }
-  diagRoom = std::min(diagRoom, SCHWARZ_ROOM);
+  diagRoom = std::max((size_t)std::max(1, B->npair) * 36, std::min(diagRoom, SCHWARZ_ROOM));
   double* d_diag = nullptr;
   CQF_CUDA(cudaMallocAsync(&d_diag, diagRoom * sizeof(double), B->stream));
   for (int c = 0; c < NCLS; c++) {
