@@ -103,6 +103,10 @@ __global__ void __launch_bounds__(256)
         const bool visited = jk < a.nKet && !(a.same && jk > ibc);
         const double tileMax = __ldg(a.maxNorm) * P.Q * __ldg(a.qWin + a.ketBeg + tile * WTILE);
         bool screened = false, w32 = false;
+        auto share = [&](int ketPrim) {
+          const int np = P.npp * ketPrim;
+          while (np >= PLAN_LONG * a.planEach && sl < 5 && (np >> sl) > a.planEach) sl++;
+        };
         if (a.screen && tileMax < a.thresh) {
           screened = true;
         } else if (visited && a.screen) {
@@ -111,14 +115,13 @@ __global__ void __launch_bounds__(256)
           const double bound = sh_max_bra(a, P, Q, __ldg(a.pairNorm + a.braBeg + ib),
                                           __ldg(a.pairNorm + a.ketBeg + jk), pRef) * P.Q * Q.Q;
           screened = bound < a.thresh;
+          if (CUT && !screened) share(Q.npp);
           w32 = MIXED && !screened && bound < cut &&
                 fp32_range_ok(__ldg(a.pairRange + a.braBeg + ib),
                               __ldg(a.pairRange + a.ketBeg + jk), a.lsum, 0, 0);
+        } else if (CUT && visited) {  // 4 waters unscreened 2.65 -> 1.32 ms
+          share(a.pairs[a.ketBeg + jk].npp);
         }  // without the screen every quartet runs in FP64
-        if (CUT && visited && !screened) {  // 4 waters unscreened 2.65 -> 1.32 ms
-          const int np = P.npp * a.pairs[a.ketBeg + jk].npp;
-          while (np >= PLAN_LONG * a.planEach && sl < 5 && (np >> sl) > a.planEach) sl++;
-        }
         const unsigned bv = __ballot_sync(0xffffffffu, visited);
         const unsigned bs = __ballot_sync(0xffffffffu, visited && screened);
         b32 = __ballot_sync(0xffffffffu, visited && !screened && w32);
